@@ -3,6 +3,7 @@
 // Staged path: log+cumsum -> chunk_state -> state_passing -> fused readout, with the
 // intermediates (lcr, chunk_decay, states, states_acc) in caller-provided scratch.
 // Single-pass path: the tcgen05 kernel in scan_fused.cu when the shape is covered.
+// Otherwise, up to 128 modes: the token recurrence over segments in scan_modes.cu.
 #include "common.cuh"
 
 namespace fracssm {
@@ -33,6 +34,13 @@ int scan_fused_launch(const void *u, const void *c, const void *kappa, int ck_dt
                       const float *initial_state, void *h, void *final_state, int final_dtype,
                       void *workspace, size_t workspace_bytes, int64_t B, int64_t L, int64_t R,
                       int64_t M, int64_t T, void *stream);
+// defined in scan_modes.cu
+bool scan_few_supported(int64_t B, int64_t L, int64_t R, int64_t M, int64_t T);
+size_t scan_few_workspace_bytes(int64_t B, int64_t L, int64_t R, int64_t M);
+int scan_few_launch(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, const void *c, const void *kappa,
+                    int ck_dtype, int64_t c_sb, int64_t c_sl, int64_t k_sb, int64_t k_sl, const float *rho,
+                    int64_t r_sb, int64_t r_sl, const float *initial_state, void *h, void *final_state,
+                    int final_dtype, void *workspace, int64_t B, int64_t L, int64_t R, int64_t M, void *stream);
 
 }  // namespace fracssm
 
@@ -44,7 +52,9 @@ extern "C" size_t fracssm_frac_scan_workspace_bytes(int64_t B, int64_t L, int64_
   const size_t fused = scan_fused_workspace_bytes(B, L, R, M, T);
   if (path == 1) return staged;
   if (path == 2) return fused;
-  return staged > fused ? staged : fused;
+  // which of the two automatic routes a call takes also depends on types and strides
+  const size_t other = scan_few_supported(B, L, R, M, T) ? scan_few_workspace_bytes(B, L, R, M) : staged;
+  return other > fused ? other : fused;
 }
 
 extern "C" int fracssm_frac_scan_fwd(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl,
@@ -99,6 +109,11 @@ extern "C" int fracssm_frac_scan_fwd(const void *u, int u_dtype, int64_t u_sb, i
     return scan_fused_launch(u, c, kappa, ck_dtype, rho, initial_state, h, final_state, final_dtype,
                              workspace, workspace_bytes, B, L, R, M, T, stream);
   }
+
+  // (a caller whose workspace only holds the chunked stages keeps them)
+  if (path == 0 && scan_few_supported(B, L, R, M, T) && workspace_bytes >= scan_few_workspace_bytes(B, L, R, M))
+    return scan_few_launch(u, u_dtype, u_sb, u_sl, c, kappa, ck_dtype, c_sb, c_sl, k_sb, k_sl, rho, r_sb, r_sl,
+                           initial_state, h, final_state, final_dtype, workspace, B, L, R, M, stream);
 
   ScanScratch s = staged_layout(workspace, B, L, R, M, T);
   if (workspace_bytes < s.bytes) return fail(FRACSSM_ERR_ARG, "frac_scan: workspace too small");
