@@ -1,0 +1,637 @@
+// One decode token through all layers of the model, bfloat16, up to 64 sequences: four kernels per layer.
+//
+//   decode_linear_kernel<.., kIn>    RMSNorm of the hidden state -> in_proj -> x | gate; the rows of x also take
+//                                    the causal convolution step + SiLU (a channel needs its own history only)
+//   decode_linear_kernel<.., kProj>  rw_proj of x_conv and dyn_proj of x
+//   decode_mix_kernel                the scan parameters of a (sequence, head), its state one token further,
+//                                    readout, D skip, gate
+//   decode_linear_kernel<.., kOut>   gated RMSNorm's normalisation -> out_proj -> + hidden state
+//
+// What bounds a step: reading the weights (27 MB a layer at hidden 768, 128 modes) and, from some 16 sequences
+// on, the float32 state in and out; at one sequence the length of the kernel chain.  As separate library and
+// elementwise calls (about 30 launches a layer, most of them from Python) a step of 24 layers was bound by the
+// host.  Hence
+//   * elementwise stages sit in the prologue or epilogue of the product that reads or writes their rows;
+//   * the products stream the weights once, straight into the fragments of mma.sync (16 weight rows x 16 of the
+//     contraction x 8 sequences): with at most 64 sequences they are far below the tensor-core ridge, and a lane
+//     reads 8 consecutive weights of a row because the contraction order is free as long as both operands share
+//     it.  The 8 warps of a block split the contraction of a 16-row tile, so even 768 output rows keep 48 blocks
+//     of 8 warps busy;
+//   * every kernel is launched with programmatic stream serialisation: it requests what no kernel of this call
+//     writes (weights, the old state and convolution history) before it waits for its predecessor.
+// Whole model call, 24 layers of hidden 768, 24 heads x 128 modes, vocabulary 50280: 13.6 ms -> 0.72 ms at one
+// sequence, 13.9 ms -> 1.50 ms at 32.
+#include <mutex>
+
+#include "common.cuh"
+#include "scan_tile.cuh"
+
+namespace fracssm {
+namespace {
+
+constexpr int kThreads = 256, kWarps = 8, kTileRows = 16, kMaxSeq = 64;
+constexpr int kPre = 6;              // 32-wide steps of the contraction a warp holds weights for
+constexpr int kRedStride = 20;       // floats per sequence in the exchange buffer: 16 rows, bank-conflict free
+constexpr int kPassTiles = 2;        // groups of 8 sequences exchanged at a time
+constexpr int kMaxHidden = 2048;     // row length of the RMSNorm prologue at one or two sequences
+enum { kIn = 0, kProj = 1, kOut = 2 };
+
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+__device__ __forceinline__ uint4 ldg_weights(const void *p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                         uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ const void *param_at(const void *p, int64_t i, int dt) {
+  return reinterpret_cast<const char *>(p) + i * (dt == FRACSSM_F32 ? 4 : 2);
+}
+__device__ __forceinline__ float bf(uint32_t lo16) { return __uint_as_float(lo16 << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
+__device__ __forceinline__ float round_bf(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+__device__ __forceinline__ void unpack8(const uint4 &p, float (&f)[8]) {
+  const uint32_t w[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    f[2 * i] = bf(w[i]);
+    f[2 * i + 1] = bf_hi(w[i]);
+  }
+}
+__device__ __forceinline__ void ld_param8(const void *p, int64_t i, int dt, float (&f)[8]) {
+#pragma unroll
+  for (int e = 0; e < 8; ++e) f[e] = ld_f32(p, i + e, dt);
+}
+__device__ __forceinline__ float sum_warp(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ float sigmoid_(float x) { return 1.f / (1.f + __expf(-x)); }
+
+struct LinArgs {
+  const __nv_bfloat16 *w, *w2;   // [n][K]; kProj: w = rw_proj, w2 = dyn_proj
+  int n, n2, K, B, blocks2;      // kProj: the first blocks2 blocks take one tile of w2 each
+  const __nv_bfloat16 *act, *act2;   // kIn: hidden state; kProj: x_conv and x
+  const float *vals, *ss;        // kOut: gated values [B][K] and their partial sums of squares [B][nss]
+  int nss;
+  const void *norm_w; int norm_dt; float eps;
+  // kIn outputs and the convolution
+  __nv_bfloat16 *x, *gate, *x_conv, *new_conv;
+  const __nv_bfloat16 *old_conv, *conv_w, *conv_b;
+  int di;
+  // kProj outputs
+  float *out, *out2;
+  const __nv_bfloat16 *bias2;
+  // kOut
+  const __nv_bfloat16 *res;
+  __nv_bfloat16 *dst;
+};
+
+// NT groups of 8 sequences.
+template <int NT, int KIND>
+__global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 1) decode_linear_kernel(const LinArgs a) {
+  extern __shared__ __align__(16) uint8_t lin_smem[];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, tig = lane & 3;
+  grid_dep_launch();
+  // rows of the activation tile lie 64 mod 128 bytes apart: a quarter-warp's 16-byte reads then cover all banks
+  const uint32_t stride = a.K * 2 + ((a.K * 2) % 128 == 0 ? 64 : 128);
+  float *red = reinterpret_cast<float *>(lin_smem + 8 * NT * stride);
+  const bool second = KIND == kProj && (int)blockIdx.x < a.blocks2;
+  const __nv_bfloat16 *W = second ? a.w2 : a.w;
+  const int N = second ? a.n2 : a.n;
+  const int tile0 = KIND == kProj && !second ? blockIdx.x - a.blocks2 : blockIdx.x;
+  const int tiles = (N + kTileRows - 1) / kTileRows;
+  const int tile_step = second ? tiles : KIND == kProj ? gridDim.x - a.blocks2 : gridDim.x;
+  const int steps = a.K / 32, share = (steps + kWarps - 1) / kWarps;
+  const int k_lo = min(w * share, steps), k_hi = min(k_lo + share, steps);
+
+  uint4 wr[kPre][2];
+  auto request = [&](int tile, int k0) {
+    const int r0 = min(tile * kTileRows + g, N - 1), r1 = min(tile * kTileRows + g + 8, N - 1);
+    const __nv_bfloat16 *p0 = W + (int64_t)r0 * a.K + 8 * tig, *p1 = W + (int64_t)r1 * a.K + 8 * tig;
+#pragma unroll
+    for (int i = 0; i < kPre; ++i) {
+      if (k0 + i < k_hi) {
+        wr[i][0] = ldg_weights(p0 + (k0 + i) * 32);
+        wr[i][1] = ldg_weights(p1 + (k0 + i) * 32);
+      }
+    }
+  };
+  request(tile0, k_lo);
+  if (KIND != kProj)   // a layer's norm weight is not in L2 yet
+    for (int ch = tid; ch < a.K / 8; ch += kThreads) prefetch_l2(param_at(a.norm_w, 8 * ch, a.norm_dt));
+  // what the epilogue of this thread's first value needs and no kernel of this call writes
+  const int e_row = tid & 15, e_seq = tid >> 4;
+  uint2 cw = make_uint2(0, 0);
+  float cb = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f;
+  auto conv_inputs = [&](int n, int b) {
+    cw = *reinterpret_cast<const uint2 *>(a.conv_w + (int64_t)n * 4);
+    cb = a.conv_b ? __bfloat162float(a.conv_b[n]) : 0.f;
+    c0 = c1 = c2 = 0.f;
+    if (a.old_conv) {
+      const __nv_bfloat16 *p = a.old_conv + ((int64_t)b * a.di + n) * 3;
+      c0 = __bfloat162float(p[0]); c1 = __bfloat162float(p[1]); c2 = __bfloat162float(p[2]);
+    }
+  };
+  if (KIND == kIn && NT == 1 && e_seq < a.B && tile0 * kTileRows + e_row < a.di) conv_inputs(tile0 * kTileRows + e_row, e_seq);
+
+  grid_dep_wait();
+
+  // ---- the activation tile, bf16, rows beyond B zero
+  const int chunks = a.K / 8;
+  auto put = [&](int b, int ch, const float (&v)[8]) {
+    *reinterpret_cast<uint4 *>(lin_smem + b * stride + ch * 16) =
+        make_uint4(tile::pack2(v[0], v[1]), tile::pack2(v[2], v[3]), tile::pack2(v[4], v[5]), tile::pack2(v[6], v[7]));
+  };
+  for (int i = a.B * chunks + tid; i < 8 * NT * chunks; i += kThreads)
+    *reinterpret_cast<uint4 *>(lin_smem + (i / chunks) * stride + (i % chunks) * 16) = make_uint4(0, 0, 0, 0);
+  if (KIND == kProj) {
+    const __nv_bfloat16 *act = second ? a.act2 : a.act;
+#pragma unroll 4
+    for (int i = tid; i < a.B * chunks; i += kThreads)
+      *reinterpret_cast<uint4 *>(lin_smem + (i / chunks) * stride + (i % chunks) * 16) =
+          __ldcg(reinterpret_cast<const uint4 *>(act) + i);
+  } else if (KIND == kIn) {
+    if (NT == 1 && a.B <= 2) {   // the whole block on one row: one chunk per thread (K <= 2048)
+      for (int b = 0; b < a.B; ++b) {
+        float v[8], nw[8], ss = 0.f;
+        if (tid < chunks) {
+          unpack8(__ldcg(reinterpret_cast<const uint4 *>(a.act + (int64_t)b * a.K) + tid), v);
+          ld_param8(a.norm_w, 8 * tid, a.norm_dt, nw);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
+        }
+        ss = sum_warp(ss);
+        if (lane == 0) red[8 * b + w] = ss;
+        __syncthreads();
+        float total = 0.f;
+#pragma unroll
+        for (int i = 0; i < kWarps; ++i) total += red[8 * b + i];
+        const float rs = rsqrtf(total / (float)a.K + a.eps);
+        if (tid < chunks) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] = v[e] * rs * nw[e];
+          put(b, tid, v);
+        }
+      }
+    } else {                     // a warp per row, the raw row kept in the tile between the two passes
+      for (int b = w; b < a.B; b += kWarps) {
+        float ss = 0.f;
+        for (int ch = lane; ch < chunks; ch += 32) {
+          const uint4 raw = __ldcg(reinterpret_cast<const uint4 *>(a.act + (int64_t)b * a.K) + ch);
+          float v[8];
+          unpack8(raw, v);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
+          *reinterpret_cast<uint4 *>(lin_smem + b * stride + ch * 16) = raw;
+        }
+        const float rs = rsqrtf(sum_warp(ss) / (float)a.K + a.eps);
+        for (int ch = lane; ch < chunks; ch += 32) {
+          float v[8], nw[8];
+          unpack8(*reinterpret_cast<const uint4 *>(lin_smem + b * stride + ch * 16), v);
+          ld_param8(a.norm_w, 8 * ch, a.norm_dt, nw);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] = v[e] * rs * nw[e];
+          put(b, ch, v);
+        }
+      }
+    }
+  } else {
+    for (int b = w; b < a.B; b += kWarps) {
+      float ss = 0.f;
+      for (int i = lane; i < a.nss; i += 32) ss += __ldcg(a.ss + (int64_t)b * a.nss + i);
+      ss = sum_warp(ss);
+      if (lane == 0) red[b] = rsqrtf(ss / (float)a.K + a.eps);
+    }
+    __syncthreads();
+#pragma unroll 2
+    for (int i = tid; i < a.B * chunks; i += kThreads) {
+      const int b = i / chunks, ch = i - b * chunks;
+      const float4 lo = __ldcg(reinterpret_cast<const float4 *>(a.vals) + 2 * (int64_t)i);
+      const float4 hi = __ldcg(reinterpret_cast<const float4 *>(a.vals) + 2 * (int64_t)i + 1);
+      const float rs = red[b];
+      float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w}, nw[8];
+      ld_param8(a.norm_w, 8 * ch, a.norm_dt, nw);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = v[e] * rs * nw[e];
+      put(b, ch, v);
+    }
+  }
+  __syncthreads();
+
+  for (int tile = tile0; tile < tiles; tile += tile_step) {
+    float acc[NT][4];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
+    for (int k0 = k_lo; k0 < k_hi; k0 += kPre) {
+      if (tile != tile0 || k0 != k_lo) request(tile, k0);
+#pragma unroll
+      for (int i = 0; i < kPre; ++i) {
+        if (k0 + i < k_hi) {
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            const uint4 x = *reinterpret_cast<const uint4 *>(lin_smem + (8 * t + g) * stride + (k0 + i) * 64 + 16 * tig);
+            mma_bf16(acc[t], wr[i][0].x, wr[i][1].x, wr[i][0].y, wr[i][1].y, x.x, x.y);
+            mma_bf16(acc[t], wr[i][0].z, wr[i][1].z, wr[i][0].w, wr[i][1].w, x.z, x.w);
+          }
+        }
+      }
+    }
+    // ---- the warps' shares of the contraction are added, a value per thread
+#pragma unroll
+    for (int p = 0; p < NT; p += kPassTiles) {
+#pragma unroll
+      for (int t = p; t < p + kPassTiles && t < NT; ++t) {
+        float *d = red + (w * 8 * kPassTiles + 8 * (t - p) + 2 * tig) * kRedStride + g;
+        d[0] = acc[t][0];
+        d[kRedStride] = acc[t][1];
+        d[8] = acc[t][2];
+        d[kRedStride + 8] = acc[t][3];
+      }
+      __syncthreads();
+      const int b = 8 * p + e_seq, n = tile * kTileRows + e_row;
+      if (e_seq < 8 * (NT - p) && b < a.B && n < N) {
+        float v = 0.f;
+#pragma unroll
+        for (int i = 0; i < kWarps; ++i) v += red[(i * 8 * kPassTiles + e_seq) * kRedStride + e_row];
+        if (KIND == kIn) {
+          const __nv_bfloat16 xb = __float2bfloat16_rn(v);
+          if (n < a.di) {
+            if (NT != 1 || tile != tile0) conv_inputs(n, b);
+            const float xv = __bfloat162float(xb);
+            float y = cb;
+            y = fmaf(bf(cw.x), c0, y);
+            y = fmaf(bf_hi(cw.x), c1, y);
+            y = fmaf(bf(cw.y), c2, y);
+            y = fmaf(bf_hi(cw.y), xv, y);
+            const int64_t at = (int64_t)b * a.di + n;
+            a.x[at] = xb;
+            a.x_conv[at] = __float2bfloat16_rn(y / (1.f + __expf(-y)));
+            if (a.new_conv) {
+              __nv_bfloat16 *q = a.new_conv + at * 3;
+              q[0] = __float2bfloat16_rn(c1);
+              q[1] = __float2bfloat16_rn(c2);
+              q[2] = xb;
+            }
+          } else {
+            a.gate[(int64_t)b * a.di + n - a.di] = xb;
+          }
+        } else if (KIND == kProj) {
+          if (second) a.out2[(int64_t)b * N + n] = v + (a.bias2 ? __bfloat162float(a.bias2[n]) : 0.f);
+          else a.out[(int64_t)b * N + n] = v;
+        } else {
+          const int64_t at = (int64_t)b * N + n;
+          a.dst[at] = __float2bfloat16_rn(__bfloat162float(__ldcg(a.res + at)) + round_bf(v));
+        }
+      }
+      __syncthreads();
+    }
+  }
+}
+
+struct MixArgs {
+  const float *rw, *dyn;               // [B][2 H M], [B][3 H]
+  const __nv_bfloat16 *x_conv, *gate;  // [B][H R]
+  const float *old_state;              // [B][H][M][R] or null (zeros)
+  float *new_state;                    // or null
+  const void *dt_bias, *read_logit, *write_logit, *log_tau, *D;
+  int dt_bias_dt, read_dt, write_dt, log_tau_dt, D_dt;
+  float inv_read_temp, dt_min, dt_max, a_min, a_max, l_min, l_max, gate_bias;
+  float *vals, *ss;                    // [B][H R], [B][H splits]
+  int H, R, M, splits;
+};
+
+constexpr int kMixPre = 4;             // float4 pieces of the old state a thread requests ahead
+
+// One block per (sequence, head, share of the head's columns).
+__global__ void __launch_bounds__(kThreads) decode_mix_kernel(const MixArgs a) {
+  extern __shared__ __align__(16) float mix_smem[];
+  const int M = a.M, H = a.H, R = a.R, Mr = (M + 3) & ~3;
+  float *cc = mix_smem, *kk = cc + Mr, *rr = kk + Mr, *part = rr + Mr;   // part [groups][cols], 16-byte aligned
+  __shared__ float red[2][4][2];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int h = blockIdx.x / a.splits, sp = blockIdx.x % a.splits, b = blockIdx.y;
+  const int cols = R / a.splits, quads = cols / 4, groups = kThreads / quads;
+  const int q = tid % quads, mg = tid / quads;
+  const bool on = mg < groups;
+  grid_dep_launch();
+  const int64_t sbase = ((int64_t)b * H + h) * M * R + sp * cols + 4 * q;
+  float4 pre[kMixPre];
+#pragma unroll
+  for (int i = 0; i < kMixPre; ++i) {
+    const int m = mg + i * groups;
+    pre[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (on && m < M && a.old_state) pre[i] = *reinterpret_cast<const float4 *>(a.old_state + sbase + (int64_t)m * R);
+  }
+  const float read_gate = sigmoid_(ld_f32(a.read_logit, 0, a.read_dt)), write_gate = sigmoid_(ld_f32(a.write_logit, 0, a.write_dt));
+  const float dtb = ld_f32(a.dt_bias, h, a.dt_bias_dt);
+  for (int m = 8 * tid; m < M; m += 8 * kThreads) prefetch_l2(param_at(a.log_tau, m, a.log_tau_dt));
+  if (8 * tid < cols) prefetch_l2(param_at(a.D, (int64_t)h * R + sp * cols + 8 * tid, a.D_dt));
+  grid_dep_wait();
+
+  // ---- scan parameters (the formulas of compute_params_kernel): threads 0..127 the read side, 128..255 the write side
+  const float d0 = __ldcg(a.dyn + (int64_t)b * 3 * H + h) + dtb;
+  float dt = d0 > 20.f ? d0 : log1pf(expf(d0));
+  dt = fminf(fmaxf(dt, a.dt_min), a.dt_max);
+  const float alpha = a.a_min + sigmoid_(__ldcg(a.dyn + (int64_t)b * 3 * H + H + h)) * (a.a_max - a.a_min);
+  const float lam = a.l_min + sigmoid_(__ldcg(a.dyn + (int64_t)b * 3 * H + 2 * H + h)) * (a.l_max - a.l_min);
+  const float rate = powf(fmaxf(lam, 1e-4f), 1.f / fmaxf(alpha, 1e-4f));
+  const int side = tid >> 7, t128 = tid & 127;
+  const float *res = a.rw + (int64_t)b * 2 * H * M + (int64_t)side * H * M + (int64_t)h * M;
+  float *dst = side ? kk : cc;
+  float mx = -INFINITY;
+  for (int m = t128; m < M; m += 128) {
+    const float prior = -alpha * ld_f32(a.log_tau, m, a.log_tau_dt);
+    const float l = side ? prior + write_gate * __ldcg(res + m) : (prior + read_gate * __ldcg(res + m)) * a.inv_read_temp;
+    dst[m] = l;
+    mx = fmaxf(mx, l);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (lane == 0) red[side][w & 3][0] = mx;
+  __syncthreads();
+  mx = fmaxf(fmaxf(red[side][0][0], red[side][1][0]), fmaxf(red[side][2][0], red[side][3][0]));
+  float sum = 0.f;
+  for (int m = t128; m < M; m += 128) {
+    const float e = __expf(dst[m] - mx);
+    dst[m] = e;
+    sum += e;
+  }
+  sum = sum_warp(sum);
+  if (lane == 0) red[side][w & 3][1] = sum;
+  __syncthreads();
+  const float inv = 1.f / (red[side][0][1] + red[side][1][1] + red[side][2][1] + red[side][3][1]);
+  for (int m = t128; m < M; m += 128) {
+    if (side) {
+      float rho = expf(-dt * (rate / fmaxf(expf(ld_f32(a.log_tau, m, a.log_tau_dt)), 1e-6f)));
+      rho = fminf(fmaxf(rho, 1e-6f), 1.f - 1e-6f);
+      kk[m] = (1.f - rho) * (kk[m] * inv);
+      rr[m] = rho;
+    } else {
+      cc[m] *= inv;
+    }
+  }
+  __syncthreads();
+
+  // ---- the state one token further, and the readout
+  const int64_t col = (int64_t)b * H * R + (int64_t)h * R + sp * cols;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (on) {
+    const uint2 uw = __ldcg(reinterpret_cast<const uint2 *>(a.x_conv + col + 4 * q));
+    const float u0 = bf(uw.x), u1 = bf_hi(uw.x), u2 = bf(uw.y), u3 = bf_hi(uw.y);
+    auto step = [&](int m, float4 s) {
+      const float rho = rr[m], kap = kk[m], c = cc[m];
+      s.x = fmaf(rho, s.x, kap * u0);
+      s.y = fmaf(rho, s.y, kap * u1);
+      s.z = fmaf(rho, s.z, kap * u2);
+      s.w = fmaf(rho, s.w, kap * u3);
+      if (a.new_state) *reinterpret_cast<float4 *>(a.new_state + sbase + (int64_t)m * R) = s;
+      acc.x = fmaf(c, s.x, acc.x);
+      acc.y = fmaf(c, s.y, acc.y);
+      acc.z = fmaf(c, s.z, acc.z);
+      acc.w = fmaf(c, s.w, acc.w);
+    };
+#pragma unroll
+    for (int i = 0; i < kMixPre; ++i)
+      if (mg + i * groups < M) step(mg + i * groups, pre[i]);
+#pragma unroll 4
+    for (int m = mg + kMixPre * groups; m < M; m += groups)
+      step(m, a.old_state ? *reinterpret_cast<const float4 *>(a.old_state + sbase + (int64_t)m * R) : make_float4(0.f, 0.f, 0.f, 0.f));
+    *reinterpret_cast<float4 *>(part + mg * cols + 4 * q) = acc;
+  }
+  __syncthreads();
+  float sq = 0.f;
+  for (int c = tid; c < cols; c += kThreads) {
+    float o = 0.f;
+    for (int i = 0; i < groups; ++i) o += part[i * cols + c];
+    const float u = __bfloat162float(__ldcg(a.x_conv + col + c));
+    const float mixed = round_bf(o + u * ld_f32(a.D, (int64_t)h * R + sp * cols + c, a.D_dt));
+    const float z = round_bf(__bfloat162float(__ldcg(a.gate + col + c)) + a.gate_bias);
+    const float v = mixed * (z * sigmoid_(z));
+    a.vals[col + c] = v;
+    sq = fmaf(v, v, sq);
+  }
+  sq = sum_warp(sq);
+  __syncthreads();
+  if (lane == 0) part[w] = sq;
+  __syncthreads();
+  if (tid == 0) {
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < kWarps; ++i) t += part[i];
+    a.ss[(int64_t)b * H * a.splits + h * a.splits + sp] = t;
+  }
+}
+
+template <typename Arg>
+cudaError_t launch_dep(void (*kernel)(const Arg), dim3 grid, size_t smem, cudaStream_t st, bool dependent, const Arg &arg) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = dependent ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, arg);
+}
+
+size_t lin_smem_bytes(int nt, int64_t K) {
+  const size_t stride = K * 2 + ((K * 2) % 128 == 0 ? 64 : 128);
+  const size_t red = (size_t)kWarps * 8 * kPassTiles * kRedStride * 4;
+  return 8 * nt * stride + red;
+}
+size_t mix_smem_bytes(int64_t M) { return (size_t)(3 * ((M + 3) / 4 * 4) + kThreads * 4) * 4; }
+
+template <int NT>
+cudaError_t allow_smem() {
+  constexpr int kMost = 227 * 1024;
+  cudaError_t e = cudaFuncSetAttribute(decode_linear_kernel<NT, kIn>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_linear_kernel<NT, kProj>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_linear_kernel<NT, kOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
+  return e;
+}
+
+size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
+
+// the columns of a (sequence, head) are spread over 1, 2 or 4 blocks while the launch has fewer blocks than SMs
+int mix_splits(int64_t B, int64_t H, int64_t R) {
+  int s = 1;
+  while (s < 4 && B * H * s < 148 && R % (8 * s) == 0) s *= 2;
+  return s;
+}
+
+struct Scratch {
+  size_t x, gate, x_conv, rw, dyn, vals, ss, hid, bytes;
+};
+Scratch scratch_layout(int64_t B, int64_t d, int64_t di, int64_t H, int64_t M) {
+  Scratch s{};
+  size_t off = 0;
+  auto take = [&](size_t n) { const size_t at = off; off += align256(n); return at; };
+  s.x = take((size_t)B * di * 2);
+  s.gate = take((size_t)B * di * 2);
+  s.x_conv = take((size_t)B * di * 2);
+  s.rw = take((size_t)B * 2 * H * M * 4);
+  s.dyn = take((size_t)B * 3 * H * 4);
+  s.vals = take((size_t)B * di * 4);
+  s.ss = take((size_t)B * H * 4 * 4);
+  s.hid = take(2 * align256((size_t)B * d * 2));
+  s.bytes = off;
+  return s;
+}
+
+enum LayerPtr { kNormW, kInW, kConvW, kConvB, kDynW, kDynB, kRwW, kDtBias, kReadLogit, kWriteLogit, kLogTau, kD,
+                kOutNormW, kOutW, kOldState, kOldConv, kNewState, kNewConv, kF32Mask, kLayerPtrs };
+enum LayerNum { kEpsIn, kEpsOut, kReadTemp, kDtMin, kDtMax, kAMin, kAMax, kLMin, kLMax, kGateBias, kLayerNums };
+
+template <int NT>
+int run_layers(const uint64_t *ptrs, const float *nums, int64_t layers, const void *hidden_in, void *hidden_out,
+               char *ws, int64_t B, int64_t d, int64_t H, int64_t R, int64_t M, cudaStream_t st) {
+  static std::mutex mu;
+  static bool ready[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
+    return fail(FRACSSM_ERR_CUDA, "decode_layers: cannot identify the current device");
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (!ready[dev]) {
+      const cudaError_t e = allow_smem<NT>();
+      if (e != cudaSuccess) return fail(FRACSSM_ERR_CUDA, "decode_layers: %s", cudaGetErrorString(e));
+      ready[dev] = true;
+    }
+  }
+  const int64_t di = H * R;
+  const Scratch s = scratch_layout(B, d, di, H, M);
+  const int splits = mix_splits(B, H, R);
+  const size_t smem_d = lin_smem_bytes(NT, d), smem_di = lin_smem_bytes(NT, di), mix_smem = mix_smem_bytes(M);
+  auto at = [&](size_t off) { return ws + off; };
+  const int64_t tiles_in = ceil_div(2 * di, kTileRows), tiles_rw = ceil_div(2 * H * M, kTileRows),
+                tiles_dyn = ceil_div(3 * H, kTileRows), tiles_out = ceil_div(d, kTileRows);
+  // Up to 8 sequences a block takes one tile and all tiles are resident at once (three blocks per SM);
+  // beyond, filling the activation tile costs as much as a tile's weights: one or two blocks per SM walk over the tiles.
+  auto blocks = [&](int64_t tiles, size_t smem) -> int64_t {
+    if (NT == 1) return tiles;
+    const int64_t most = 148 * (smem <= 110 * 1024 ? 2 : 1);
+    return tiles < most ? tiles : most;
+  };
+  cudaError_t e = cudaSuccess;
+  const __nv_bfloat16 *hid = reinterpret_cast<const __nv_bfloat16 *>(hidden_in);
+  for (int64_t l = 0; l < layers && e == cudaSuccess; ++l) {
+    const uint64_t *p = ptrs + l * kLayerPtrs;
+    const float *f = nums + l * kLayerNums;
+    const uint64_t f32 = p[kF32Mask];
+    auto bfp = [&](int i) { return reinterpret_cast<const __nv_bfloat16 *>(p[i]); };
+    auto raw = [&](int i) { return reinterpret_cast<const void *>(p[i]); };
+    auto dt = [&](int i) { return (f32 >> i) & 1 ? FRACSSM_F32 : FRACSSM_BF16; };
+    __nv_bfloat16 *next = l + 1 == layers ? reinterpret_cast<__nv_bfloat16 *>(hidden_out)
+                                          : reinterpret_cast<__nv_bfloat16 *>(at(s.hid) + (l & 1) * align256((size_t)B * d * 2));
+    LinArgs in{};
+    in.w = bfp(kInW); in.n = (int)(2 * di); in.K = (int)d; in.B = (int)B;
+    in.act = hid;
+    in.norm_w = raw(kNormW); in.norm_dt = dt(kNormW); in.eps = f[kEpsIn];
+    in.x = reinterpret_cast<__nv_bfloat16 *>(at(s.x));
+    in.gate = reinterpret_cast<__nv_bfloat16 *>(at(s.gate));
+    in.x_conv = reinterpret_cast<__nv_bfloat16 *>(at(s.x_conv));
+    in.new_conv = reinterpret_cast<__nv_bfloat16 *>(p[kNewConv]);
+    in.old_conv = bfp(kOldConv);
+    in.conv_w = bfp(kConvW); in.conv_b = bfp(kConvB); in.di = (int)di;
+    e = launch_dep(decode_linear_kernel<NT, kIn>, dim3((unsigned)blocks(tiles_in, smem_d)), smem_d, st, l > 0, in);
+    if (e != cudaSuccess) break;
+
+    LinArgs pr{};
+    pr.w = bfp(kRwW); pr.n = (int)(2 * H * M); pr.w2 = bfp(kDynW); pr.n2 = (int)(3 * H); pr.K = (int)di; pr.B = (int)B;
+    pr.blocks2 = (int)tiles_dyn;
+    pr.act = in.x_conv; pr.act2 = in.x;
+    pr.out = reinterpret_cast<float *>(at(s.rw)); pr.out2 = reinterpret_cast<float *>(at(s.dyn));
+    pr.bias2 = bfp(kDynB);
+    e = launch_dep(decode_linear_kernel<NT, kProj>, dim3((unsigned)(tiles_dyn + blocks(tiles_rw, smem_di))), smem_di, st, true, pr);
+    if (e != cudaSuccess) break;
+
+    MixArgs m{};
+    m.rw = pr.out; m.dyn = pr.out2; m.x_conv = in.x_conv; m.gate = in.gate;
+    m.old_state = reinterpret_cast<const float *>(p[kOldState]);
+    m.new_state = reinterpret_cast<float *>(p[kNewState]);
+    m.dt_bias = raw(kDtBias); m.dt_bias_dt = dt(kDtBias);
+    m.read_logit = raw(kReadLogit); m.read_dt = dt(kReadLogit);
+    m.write_logit = raw(kWriteLogit); m.write_dt = dt(kWriteLogit);
+    m.log_tau = raw(kLogTau); m.log_tau_dt = dt(kLogTau);
+    m.D = raw(kD); m.D_dt = dt(kD);
+    m.inv_read_temp = 1.f / f[kReadTemp];
+    m.dt_min = f[kDtMin]; m.dt_max = f[kDtMax]; m.a_min = f[kAMin]; m.a_max = f[kAMax];
+    m.l_min = f[kLMin]; m.l_max = f[kLMax]; m.gate_bias = f[kGateBias];
+    m.vals = reinterpret_cast<float *>(at(s.vals)); m.ss = reinterpret_cast<float *>(at(s.ss));
+    m.H = (int)H; m.R = (int)R; m.M = (int)M; m.splits = splits;
+    e = launch_dep(decode_mix_kernel, dim3((unsigned)(H * splits), (unsigned)B), mix_smem, st, true, m);
+    if (e != cudaSuccess) break;
+
+    LinArgs o{};
+    o.w = bfp(kOutW); o.n = (int)d; o.K = (int)di; o.B = (int)B;
+    o.vals = m.vals; o.ss = m.ss; o.nss = (int)(H * splits);
+    o.norm_w = raw(kOutNormW); o.norm_dt = dt(kOutNormW); o.eps = f[kEpsOut];
+    o.res = hid; o.dst = next;
+    e = launch_dep(decode_linear_kernel<NT, kOut>, dim3((unsigned)blocks(tiles_out, smem_di)), smem_di, st, true, o);
+    hid = next;
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(FRACSSM_ERR_CUDA, "decode_layers: %s", cudaGetErrorString(e));
+  }
+  return check_launch("decode_layers");
+}
+
+}  // namespace
+}  // namespace fracssm
+
+extern "C" int fracssm_decode_layers_supported(int64_t B, int64_t hidden, int64_t H, int64_t R, int64_t M, int64_t K) {
+  using namespace fracssm;
+  if (B < 1 || B > kMaxSeq || hidden < 32 || hidden > kMaxHidden || H < 1 || R < 4 || M < 1 || K != 4) return 0;
+  if (H > 65536 || R > 1024 || M > 2048) return 0;
+  const int64_t di = H * R;
+  if (hidden % 32 != 0 || di % 32 != 0 || di > 65536 || R % 4 != 0 || H * M > (1 << 24)) return 0;
+  const int nt = B <= 8 ? 1 : B <= 16 ? 2 : B <= 32 ? 4 : 8;
+  return lin_smem_bytes(nt, di) <= 227 * 1024 && lin_smem_bytes(nt, hidden) <= 227 * 1024 && mix_smem_bytes(M) <= 47 * 1024;
+}
+
+extern "C" size_t fracssm_decode_layers_workspace_bytes(int64_t B, int64_t hidden, int64_t H, int64_t R, int64_t M) {
+  if (B < 1 || hidden < 1 || H < 1 || R < 1 || M < 1) return 0;
+  return fracssm::scratch_layout(B, hidden, H * R, H, M).bytes;
+}
+
+extern "C" int fracssm_decode_layers(const uint64_t *layer_ptrs, const float *layer_nums, int64_t layers,
+                                     const void *hidden_in, void *hidden_out, void *workspace, size_t workspace_bytes,
+                                     int64_t B, int64_t hidden, int64_t H, int64_t R, int64_t M, int64_t K, void *stream) {
+  using namespace fracssm;
+  if (layers < 1 || !layer_ptrs || !layer_nums || !hidden_in || !hidden_out || !workspace)
+    return fail(FRACSSM_ERR_ARG, "decode_layers: null pointer or no layer");
+  if (!fracssm_decode_layers_supported(B, hidden, H, R, M, K))
+    return fail(FRACSSM_ERR_UNSUPPORTED, "decode_layers: sizes not covered");
+  if (workspace_bytes < fracssm_decode_layers_workspace_bytes(B, hidden, H, R, M))
+    return fail(FRACSSM_ERR_ARG, "decode_layers: workspace too small");
+  uint64_t bits = (uint64_t)(uintptr_t)hidden_in | (uint64_t)(uintptr_t)hidden_out;
+  if ((uintptr_t)workspace & 255) return fail(FRACSSM_ERR_ARG, "decode_layers: workspace must be 256-byte aligned");
+  for (int64_t l = 0; l < layers; ++l) {
+    const uint64_t *p = layer_ptrs + l * kLayerPtrs;
+    for (int i = 0; i < kOldState; ++i)
+      if (!p[i] && i != kConvB && i != kDynB) return fail(FRACSSM_ERR_ARG, "decode_layers: null parameter");
+    bits |= p[kInW] | p[kDynW] | p[kRwW] | p[kOutW] | p[kOldState] | p[kNewState];
+    if (p[kConvW] & 7) return fail(FRACSSM_ERR_ARG, "decode_layers: the convolution weight must be 8-byte aligned");
+  }
+  if (bits & 15)
+    return fail(FRACSSM_ERR_ARG, "decode_layers: hidden states, projection weights and states must be 16-byte aligned");
+  const cudaStream_t st = (cudaStream_t)stream;
+  char *ws = reinterpret_cast<char *>(workspace);
+  if (B <= 8) return run_layers<1>(layer_ptrs, layer_nums, layers, hidden_in, hidden_out, ws, B, hidden, H, R, M, st);
+  if (B <= 16) return run_layers<2>(layer_ptrs, layer_nums, layers, hidden_in, hidden_out, ws, B, hidden, H, R, M, st);
+  if (B <= 32) return run_layers<4>(layer_ptrs, layer_nums, layers, hidden_in, hidden_out, ws, B, hidden, H, R, M, st);
+  return run_layers<8>(layer_ptrs, layer_nums, layers, hidden_in, hidden_out, ws, B, hidden, H, R, M, st);
+}

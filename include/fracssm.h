@@ -328,6 +328,29 @@ int fracssm_decode_step(const void *u, int u_dtype, const float *c, const float 
                         const float *D, float *state, float *out, int64_t Bt, int64_t H, int64_t R,
                         int64_t M, void *stream);
 
+/*
+ * One decode token through `layers` layers of the model (RMSNorm, mixer, residual), bfloat16 weights and
+ * activations, up to 64 sequences (fracssm_decode_layers_supported tells whether the sizes are covered).
+ * hidden_in / hidden_out [B, hidden] bf16 (may not overlap).  Host tables, read during the call only:
+ * layer_ptrs [layers][19] device pointers (as integers) of
+ *   0 norm weight [hidden]          1 in_proj weight [2 H R, hidden]   2 conv weight [H R, 4]
+ *   3 conv bias [H R] or 0          4 dyn_proj weight [3 H, H R]       5 dyn_proj bias [3 H] or 0
+ *   6 rw_proj weight [2 H M, H R]   7 dt_bias [H]                      8 read_residual_logit [1]
+ *   9 write_residual_scale [1]     10 base_log_tau [M]                11 D [H, R]
+ *  12 out_norm weight [H R]        13 out_proj weight [hidden, H R]
+ *  14 state [B, H, M, R] f32 or 0 (zeros)      15 conv state [B, H R, 3] bf16 or 0 (zeros)
+ *  16 new state or 0 (not kept)                17 new conv state or 0 (not kept)
+ *  18 bit i set: parameter i is float32 (allowed for 0 and 7..12), else bf16;
+ * layer_nums [layers][10]: eps of the norm, eps of the output norm, read_temp, dt_min, dt_max, alpha_min,
+ *   alpha_max, lambda_min, lambda_max, gate bias.
+ * Old and new states must not overlap.  Replaces the token loop of frac_ssm/models/modeling_frac.py:216-244.
+ */
+int fracssm_decode_layers_supported(int64_t B, int64_t hidden, int64_t H, int64_t R, int64_t M, int64_t K);
+size_t fracssm_decode_layers_workspace_bytes(int64_t B, int64_t hidden, int64_t H, int64_t R, int64_t M);
+int fracssm_decode_layers(const uint64_t *layer_ptrs, const float *layer_nums, int64_t layers,
+                          const void *hidden_in, void *hidden_out, void *workspace, size_t workspace_bytes,
+                          int64_t B, int64_t hidden, int64_t H, int64_t R, int64_t M, int64_t K, void *stream);
+
 #ifdef __cplusplus
 }
 #endif
