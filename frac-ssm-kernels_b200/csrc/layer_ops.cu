@@ -22,8 +22,9 @@ struct ParamArgs {
   const void *rw; int rw_dt; int64_t rw_sb, rw_sl;
   const void *x; int x_dt; int64_t x_sb, x_sl;
   const float *mask; int64_t m_sb, m_sl;
-  const float *dt_bias, *log_tau;
-  const float *read_logit, *write_logit;   // the two gate parameters, one float each, on the device
+  // the small parameters, each in its own type, on the device (the two gate parameters: one element each)
+  const void *dt_bias, *log_tau, *read_logit, *write_logit;
+  int dtb_dt, lt_dt, read_dt, write_dt;
   float inv_read_temp, dt_min, dt_max, a_min, a_max, l_min, l_max;
   void *u, *c, *kappa; int ck_dt; float *rho;
   int64_t L, H, R, M;
@@ -32,7 +33,7 @@ struct ParamArgs {
 // One warp per (bh, token): lanes stride over the M modes; two softmaxes by warp shuffles.
 __global__ void __launch_bounds__(128) compute_params_kernel(const ParamArgs a) {
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  const float read_gate = sigmoidf_(__ldg(a.read_logit)), write_gate = sigmoidf_(__ldg(a.write_logit));
+  const float read_gate = sigmoidf_(ld_f32(a.read_logit, 0, a.read_dt)), write_gate = sigmoidf_(ld_f32(a.write_logit, 0, a.write_dt));
   const int64_t l = (int64_t)blockIdx.x * 4 + warp;
   const int64_t bh = blockIdx.y;
   if (l >= a.L) return;
@@ -40,7 +41,7 @@ __global__ void __launch_bounds__(128) compute_params_kernel(const ParamArgs a) 
   const int64_t H = a.H, M = a.M, R = a.R;
 
   const int64_t dbase = b * a.dyn_sb + l * a.dyn_sl;
-  float dt = softplusf_(ld_f32(a.dyn, dbase + h, a.dyn_dt) + a.dt_bias[h]);
+  float dt = softplusf_(ld_f32(a.dyn, dbase + h, a.dyn_dt) + ld_f32(a.dt_bias, h, a.dtb_dt));
   dt = fminf(fmaxf(dt, a.dt_min), a.dt_max);
   const float alpha = a.a_min + sigmoidf_(ld_f32(a.dyn, dbase + H + h, a.dyn_dt)) * (a.a_max - a.a_min);
   const float lam = a.l_min + sigmoidf_(ld_f32(a.dyn, dbase + 2 * H + h, a.dyn_dt)) * (a.l_max - a.l_min);
@@ -51,7 +52,7 @@ __global__ void __launch_bounds__(128) compute_params_kernel(const ParamArgs a) 
   const int64_t wbase = rbase + H * M;                            // write residuals
   float rmax = -INFINITY, wmax = -INFINITY;
   for (int64_t m = lane; m < M; m += 32) {
-    const float prior = -alpha * a.log_tau[m];
+    const float prior = -alpha * ld_f32(a.log_tau, m, a.lt_dt);
     rmax = fmaxf(rmax, (prior + read_gate * ld_f32(a.rw, rbase + m, a.rw_dt)) * a.inv_read_temp);
     wmax = fmaxf(wmax, prior + write_gate * ld_f32(a.rw, wbase + m, a.rw_dt));
   }
@@ -59,14 +60,14 @@ __global__ void __launch_bounds__(128) compute_params_kernel(const ParamArgs a) 
   wmax = warp_max(wmax);
   float rsum = 0.f, wsum = 0.f;
   for (int64_t m = lane; m < M; m += 32) {
-    const float prior = -alpha * a.log_tau[m];
+    const float prior = -alpha * ld_f32(a.log_tau, m, a.lt_dt);
     rsum += __expf((prior + read_gate * ld_f32(a.rw, rbase + m, a.rw_dt)) * a.inv_read_temp - rmax);
     wsum += __expf(prior + write_gate * ld_f32(a.rw, wbase + m, a.rw_dt) - wmax);
   }
   const float rinv = 1.f / warp_sum(rsum), winv = 1.f / warp_sum(wsum);
   const int64_t obase = (bh * a.L + l) * M;
   for (int64_t m = lane; m < M; m += 32) {
-    const float lt = a.log_tau[m];
+    const float lt = ld_f32(a.log_tau, m, a.lt_dt);
     const float prior = -alpha * lt;
     const float cw = __expf((prior + read_gate * ld_f32(a.rw, rbase + m, a.rw_dt)) * a.inv_read_temp - rmax) * rinv;
     const float ww = __expf(prior + write_gate * ld_f32(a.rw, wbase + m, a.rw_dt) - wmax) * winv;
@@ -100,7 +101,7 @@ __device__ __forceinline__ void unpack4(const uint2 &p, float (&f)[4]) {
 
 __global__ void __launch_bounds__(128) compute_params_m128_kernel(const ParamArgs a) {
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  const float read_gate = sigmoidf_(__ldg(a.read_logit)), write_gate = sigmoidf_(__ldg(a.write_logit));
+  const float read_gate = sigmoidf_(ld_f32(a.read_logit, 0, a.read_dt)), write_gate = sigmoidf_(ld_f32(a.write_logit, 0, a.write_dt));
   const int64_t l0 = ((int64_t)blockIdx.x * 4 + warp) * kPrepTokens;
   const int64_t bh = blockIdx.y;
   if (l0 >= a.L) return;
@@ -110,10 +111,10 @@ __global__ void __launch_bounds__(128) compute_params_m128_kernel(const ParamArg
   float lt[4], inv_tau[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    lt[i] = a.log_tau[4 * lane + i];
+    lt[i] = ld_f32(a.log_tau, 4 * lane + i, a.lt_dt);
     inv_tau[i] = 1.f / fmaxf(expf(lt[i]), 1e-6f);
   }
-  const float dtb = a.dt_bias[h];
+  const float dtb = ld_f32(a.dt_bias, h, a.dtb_dt);
   const __nv_bfloat16 *rw = reinterpret_cast<const __nv_bfloat16 *>(a.rw);
   const int64_t l1 = min(l0 + kPrepTokens, a.L);
   // the per-token scalars (step, alpha, rate, mask) are computed once, by lane t for token l0 + t,
@@ -228,7 +229,7 @@ constexpr int kPairTokens = 32;
 __global__ void __launch_bounds__(128) compute_params_m128_pair_kernel(const ParamArgs a) {
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
   const int sub = lane >> 4, q = lane & 15;  // token of the pair; modes 8 q .. 8 q + 7
-  const float read_gate = sigmoidf_(__ldg(a.read_logit)), write_gate = sigmoidf_(__ldg(a.write_logit));
+  const float read_gate = sigmoidf_(ld_f32(a.read_logit, 0, a.read_dt)), write_gate = sigmoidf_(ld_f32(a.write_logit, 0, a.write_dt));
   const int64_t l0 = ((int64_t)blockIdx.x * 4 + warp) * kPairTokens;
   const int64_t bh = blockIdx.y;
   if (l0 >= a.L) return;
@@ -238,10 +239,10 @@ __global__ void __launch_bounds__(128) compute_params_m128_pair_kernel(const Par
   float lt[8], inv_tau[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    lt[i] = a.log_tau[8 * q + i];
+    lt[i] = ld_f32(a.log_tau, 8 * q + i, a.lt_dt);
     inv_tau[i] = 1.f / fmaxf(expf(lt[i]), 1e-6f);
   }
-  const float dtb = a.dt_bias[h];
+  const float dtb = ld_f32(a.dt_bias, h, a.dtb_dt);
   const __nv_bfloat16 *rw = reinterpret_cast<const __nv_bfloat16 *>(a.rw);
   const int64_t l1 = min(l0 + kPairTokens, a.L);
   // per-token scalars: computed once, by lane t for token l0 + t, handed over by shuffles
@@ -455,6 +456,71 @@ rmsnorm_gated_bf16_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_srow,
   }
 }
 
+// sum = x + y and norm = weight * rmsnorm(sum) in one pass: the residual addition of a block together with the
+// norm the next block starts with (sum is rounded to bf16 first, as the addition by itself would leave it).  One
+// warp per row, the row in registers; bound by memory, 4 * D * 2 bytes a row instead of 5 (an addition and a norm).
+template <int WVEC>
+__global__ void __launch_bounds__(128)
+add_rmsnorm_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ y, const void *__restrict__ w,
+                   int w_dt, float eps, __nv_bfloat16 *__restrict__ sum, __nv_bfloat16 *__restrict__ norm, int64_t rows,
+                   int64_t D) {
+  const int lane = threadIdx.x % 32;
+  const int64_t row = (int64_t)blockIdx.x * 4 + threadIdx.x / 32;
+  if (row >= rows) return;
+  const int chunks = static_cast<int>(D / 8);
+  float v[8][8];
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int ch = lane + 32 * i;
+    if (ch < chunks) {
+      float z[8];
+      unpack8(__ldcs(reinterpret_cast<const uint4 *>(x + row * D) + ch), v[i]);
+      unpack8(__ldcs(reinterpret_cast<const uint4 *>(y + row * D) + ch), z);
+      uint32_t o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[e] = pack_bf16x2(v[i][2 * e] + z[2 * e], v[i][2 * e + 1] + z[2 * e + 1]);
+      const uint4 packed = make_uint4(o[0], o[1], o[2], o[3]);
+      *(reinterpret_cast<uint4 *>(sum + row * D) + ch) = packed;
+      unpack8(packed, v[i]);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss = fmaf(v[i][e], v[i][e], ss);
+    }
+  }
+  ss = warp_sum(ss);
+  const float rs = rsqrtf(ss / (float)D + eps);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int ch = lane + 32 * i;
+    if (ch < chunks) {
+      float wv[8];
+      if (WVEC == 1) {
+        unpack8(__ldg(reinterpret_cast<const uint4 *>(w) + ch), wv);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) wv[e] = ld_f32(w, 8 * ch + e, w_dt);
+      }
+      uint32_t o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[e] = pack_bf16x2(v[i][2 * e] * rs * wv[2 * e], v[i][2 * e + 1] * rs * wv[2 * e + 1]);
+      *(reinterpret_cast<uint4 *>(norm + row * D) + ch) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
+}
+
+// state [rows][M][R] = final [rows][R][M]: a cached state lies modes first, the scan leaves it columns first
+__global__ void __launch_bounds__(256)
+state_transpose_kernel(const float *__restrict__ fin, float *__restrict__ state, int R, int M) {
+  __shared__ float tile[32][33];
+  const int64_t base = (int64_t)blockIdx.z * R * M;
+  const int m0 = blockIdx.x * 32, r0 = blockIdx.y * 32, tx = threadIdx.x % 32, ty = threadIdx.x / 32;
+  for (int i = ty; i < 32; i += 8)
+    if (r0 + i < R && m0 + tx < M) tile[i][tx] = fin[base + (int64_t)(r0 + i) * M + m0 + tx];
+  __syncthreads();
+  for (int i = ty; i < 32; i += 8)
+    if (m0 + i < M && r0 + tx < R) state[base + (int64_t)(m0 + i) * R + r0 + tx] = tile[tx][i];
+}
+
 // Modes of the epilogue kernels.  With the heads of a layer spread over several GPUs the norm spans
 // columns on other GPUs: each GPU first computes its own sum of squares per (b, l) row (partial), the
 // sums are added across GPUs, and a second pass normalises with the total (apply).
@@ -465,7 +531,7 @@ __global__ void __launch_bounds__(256)
 scan_epilogue_kernel(const void *__restrict__ h, int h_dt, int64_t h_sb, int64_t h_sl,
                      const void *__restrict__ x, int64_t x_sb, int64_t x_sl,
                      const void *__restrict__ gate, int64_t g_sb, int64_t g_sl, int dt,
-                     const float *__restrict__ Dp, const void *__restrict__ w, int w_dt,
+                     const void *__restrict__ Dp, int D_dt, const void *__restrict__ w, int w_dt,
                      float gate_bias, float eps, void *__restrict__ y, int64_t L, int64_t H,
                      int64_t R, int mode, float *__restrict__ sumsq, int64_t norm_width) {
   __shared__ float red[32];
@@ -475,7 +541,7 @@ scan_epilogue_kernel(const void *__restrict__ h, int h_dt, int64_t h_sb, int64_t
   for (int64_t j = threadIdx.x; mode != kEpilogueApply && j < HR; j += blockDim.x) {
     const int64_t hh = j / R, r = j % R;
     float v = ld_f32(h, (b * H + hh) * h_sb + l * h_sl + r, h_dt) +
-              ld_f32(x, b * x_sb + l * x_sl + j, dt) * Dp[j];
+              ld_f32(x, b * x_sb + l * x_sl + j, dt) * ld_f32(Dp, j, D_dt);
     const float z = ld_f32(gate, b * g_sb + l * g_sl + j, dt) + gate_bias;
     v *= z * sigmoidf_(z);
     ss = fmaf(v, v, ss);
@@ -493,7 +559,7 @@ scan_epilogue_kernel(const void *__restrict__ h, int h_dt, int64_t h_sb, int64_t
   for (int64_t j = threadIdx.x; j < HR; j += blockDim.x) {
     const int64_t hh = j / R, r = j % R;
     float v = ld_f32(h, (b * H + hh) * h_sb + l * h_sl + r, h_dt) +
-              ld_f32(x, b * x_sb + l * x_sl + j, dt) * Dp[j];
+              ld_f32(x, b * x_sb + l * x_sl + j, dt) * ld_f32(Dp, j, D_dt);
     const float z = ld_f32(gate, b * g_sb + l * g_sl + j, dt) + gate_bias;
     v *= z * sigmoidf_(z);
     st_f32(y, row * HR + j, dt, v * rs * ld_f32(w, j, w_dt));
@@ -510,7 +576,7 @@ __global__ void __launch_bounds__(1024)
 scan_epilogue_bf16_kernel(const __nv_bfloat16 *__restrict__ h, int64_t h_sb, int64_t h_sl,
                           const __nv_bfloat16 *__restrict__ x, int64_t x_sb, int64_t x_sl,
                           const __nv_bfloat16 *__restrict__ gate, int64_t g_sb, int64_t g_sl,
-                          const float *__restrict__ Dp, const void *__restrict__ w, int w_dt,
+                          const void *__restrict__ Dp, int D_dt, const void *__restrict__ w, int w_dt,
                           float gate_bias, float eps, __nv_bfloat16 *__restrict__ y, int64_t L, int64_t H,
                           int64_t R, int mode, float *__restrict__ sumsq, int64_t norm_width) {
   __shared__ float red[32];
@@ -527,8 +593,14 @@ scan_epilogue_bf16_kernel(const __nv_bfloat16 *__restrict__ h, int64_t h_sb, int
     unpack8(__ldcs(reinterpret_cast<const uint4 *>(h + (b * H + hh) * h_sb + l * h_sl + r)), hv);
     unpack8(__ldcs(reinterpret_cast<const uint4 *>(x + b * x_sb + l * x_sl + j)), xv);
     unpack8(__ldcs(reinterpret_cast<const uint4 *>(gate + b * g_sb + l * g_sl + j)), zv);
-    const float4 d0 = __ldg(reinterpret_cast<const float4 *>(Dp + j)), d1 = __ldg(reinterpret_cast<const float4 *>(Dp + j + 4));
-    const float dv[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+    float dv[8];
+    if (D_dt == FRACSSM_F32) {
+      const float4 d0 = __ldg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(Dp) + j));
+      const float4 d1 = __ldg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(Dp) + j + 4));
+      dv[0] = d0.x; dv[1] = d0.y; dv[2] = d0.z; dv[3] = d0.w; dv[4] = d1.x; dv[5] = d1.y; dv[6] = d1.z; dv[7] = d1.w;
+    } else {   // bf16 (checked by the launch)
+      unpack8(__ldg(reinterpret_cast<const uint4 *>(reinterpret_cast<const __nv_bfloat16 *>(Dp) + j)), dv);
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const float z = zv[i] + gate_bias;
@@ -617,17 +689,18 @@ __global__ void layer_sumsq_kernel(const float *__restrict__ ss, int64_t n_parti
 
 }  // namespace fracssm
 
-extern "C" int fracssm_compute_params(const void *dyn, int dyn_dtype, int64_t dyn_sb, int64_t dyn_sl,
-                                      const void *rw, int rw_dtype, int64_t rw_sb, int64_t rw_sl,
-                                      const void *x_conv, int x_dtype, int64_t x_sb, int64_t x_sl,
-                                      const float *mask, int64_t m_sb, int64_t m_sl,
-                                      const float *dt_bias, const float *base_log_tau,
-                                      const float *read_gate_logit, const float *write_gate_logit, float read_temp,
-                                      float dt_min, float dt_max, float alpha_min, float alpha_max,
-                                      float lambda_min, float lambda_max, void *u, void *c,
-                                      void *kappa, int ck_dtype, float *rho, int64_t Bt, int64_t L,
-                                      int64_t H, int64_t R, int64_t M, void *stream) {
-  using namespace fracssm;
+namespace fracssm {
+namespace {
+int compute_params_typed(const void *dyn, int dyn_dtype, int64_t dyn_sb, int64_t dyn_sl,
+                         const void *rw, int rw_dtype, int64_t rw_sb, int64_t rw_sl,
+                         const void *x_conv, int x_dtype, int64_t x_sb, int64_t x_sl,
+                         const float *mask, int64_t m_sb, int64_t m_sl,
+                         const void *dt_bias, int dtb_dt, const void *base_log_tau, int lt_dt,
+                         const void *read_gate_logit, int read_dt, const void *write_gate_logit, int write_dt, float read_temp,
+                         float dt_min, float dt_max, float alpha_min, float alpha_max,
+                         float lambda_min, float lambda_max, void *u, void *c,
+                         void *kappa, int ck_dtype, float *rho, int64_t Bt, int64_t L,
+                         int64_t H, int64_t R, int64_t M, void *stream) {
   if (Bt < 0 || L < 0 || H <= 0 || R <= 0 || M <= 0) return fail(FRACSSM_ERR_ARG, "compute_params: bad sizes");
   if (!known_dtype(dyn_dtype) || !known_dtype(rw_dtype) || !known_dtype(x_dtype) || !known_dtype(ck_dtype))
     return fail(FRACSSM_ERR_ARG, "compute_params: unsupported dtype");
@@ -642,6 +715,7 @@ extern "C" int fracssm_compute_params(const void *dyn, int dyn_dtype, int64_t dy
   a.x = x_conv; a.x_dt = x_dtype; a.x_sb = x_sb; a.x_sl = x_sl;
   a.mask = mask; a.m_sb = m_sb; a.m_sl = m_sl;
   a.dt_bias = dt_bias; a.log_tau = base_log_tau;
+  a.dtb_dt = dtb_dt; a.lt_dt = lt_dt; a.read_dt = read_dt; a.write_dt = write_dt;
   a.read_logit = read_gate_logit;
   a.write_logit = write_gate_logit;
   a.inv_read_temp = 1.f / read_temp;
@@ -665,6 +739,25 @@ extern "C" int fracssm_compute_params(const void *dyn, int dyn_dtype, int64_t dy
   dim3 grid((unsigned)ceil_div(L, 4), (unsigned)(Bt * H));
   compute_params_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(a);
   return check_launch("compute_params");
+}
+}  // namespace
+}  // namespace fracssm
+
+extern "C" int fracssm_compute_params(const void *dyn, int dyn_dtype, int64_t dyn_sb, int64_t dyn_sl,
+                                      const void *rw, int rw_dtype, int64_t rw_sb, int64_t rw_sl,
+                                      const void *x_conv, int x_dtype, int64_t x_sb, int64_t x_sl,
+                                      const float *mask, int64_t m_sb, int64_t m_sl,
+                                      const float *dt_bias, const float *base_log_tau,
+                                      const float *read_gate_logit, const float *write_gate_logit, float read_temp,
+                                      float dt_min, float dt_max, float alpha_min, float alpha_max,
+                                      float lambda_min, float lambda_max, void *u, void *c,
+                                      void *kappa, int ck_dtype, float *rho, int64_t Bt, int64_t L,
+                                      int64_t H, int64_t R, int64_t M, void *stream) {
+  return fracssm::compute_params_typed(dyn, dyn_dtype, dyn_sb, dyn_sl, rw, rw_dtype, rw_sb, rw_sl, x_conv, x_dtype, x_sb,
+                                       x_sl, mask, m_sb, m_sl, dt_bias, FRACSSM_F32, base_log_tau, FRACSSM_F32,
+                                       read_gate_logit, FRACSSM_F32, write_gate_logit, FRACSSM_F32, read_temp, dt_min,
+                                       dt_max, alpha_min, alpha_max, lambda_min, lambda_max, u, c, kappa, ck_dtype, rho,
+                                       Bt, L, H, R, M, stream);
 }
 
 extern "C" int fracssm_skip_mix(const void *mixed_flat, int mf_dtype, int64_t mf_sb, int64_t mf_sl,
@@ -713,7 +806,7 @@ namespace fracssm {
 namespace {
 int scan_epilogue_launch(const char *who, const void *h, int h_dtype, int64_t h_sb, int64_t h_sl,
                          const void *x_conv, int64_t x_sb, int64_t x_sl, const void *gate, int64_t g_sb,
-                         int64_t g_sl, int xg_dtype, const float *D, const void *weight, int w_dtype,
+                         int64_t g_sl, int xg_dtype, const void *D, int D_dt, const void *weight, int w_dtype,
                          float gate_bias, float eps, void *y, int64_t Bt, int64_t L, int64_t H, int64_t R,
                          int mode, float *sumsq, int64_t norm_width, void *stream) {
   if (Bt < 0 || L < 0 || H <= 0 || R <= 0) return fail(FRACSSM_ERR_ARG, "%s: bad sizes", who);
@@ -727,14 +820,14 @@ int scan_epilogue_launch(const char *who, const void *h, int h_dtype, int64_t h_
   auto al16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   const int64_t HR = H * R;
   if (h_dtype == FRACSSM_BF16 && xg_dtype == FRACSSM_BF16 && R % 8 == 0 && HR <= 8192 && al16(h) && al16(x_conv) &&
-      al16(gate) && al16(y) && al16(D) && h_sb % 8 == 0 && h_sl % 8 == 0 && x_sb % 8 == 0 && x_sl % 8 == 0 &&
+      al16(gate) && al16(y) && al16(D) && (D_dt == FRACSSM_F32 || D_dt == FRACSSM_BF16) && h_sb % 8 == 0 && h_sl % 8 == 0 && x_sb % 8 == 0 && x_sl % 8 == 0 &&
       g_sb % 8 == 0 && g_sl % 8 == 0) {
     const unsigned threads = (unsigned)(((HR / 8) + 31) / 32 * 32);
     const int wvec = (mode == kEpiloguePartial || !al16(weight)) ? 0 : w_dtype == FRACSSM_BF16 ? 1 : w_dtype == FRACSSM_F32 ? 2 : 0;
 #define FRACSSM_EPILOGUE(WV)                                                                                       \
   scan_epilogue_bf16_kernel<WV><<<(unsigned)(Bt * L), threads, 0, (cudaStream_t)stream>>>(                         \
       reinterpret_cast<const __nv_bfloat16 *>(h), h_sb, h_sl, reinterpret_cast<const __nv_bfloat16 *>(x_conv),     \
-      x_sb, x_sl, reinterpret_cast<const __nv_bfloat16 *>(gate), g_sb, g_sl, D, weight, w_dtype, gate_bias, eps,   \
+      x_sb, x_sl, reinterpret_cast<const __nv_bfloat16 *>(gate), g_sb, g_sl, D, D_dt, weight, w_dtype, gate_bias, eps, \
       reinterpret_cast<__nv_bfloat16 *>(y), L, H, R, mode, sumsq, norm_width)
     if (wvec == 1) FRACSSM_EPILOGUE(1);
     else if (wvec == 2) FRACSSM_EPILOGUE(2);
@@ -743,7 +836,7 @@ int scan_epilogue_launch(const char *who, const void *h, int h_dtype, int64_t h_
     return check_launch(who);
   }
   scan_epilogue_kernel<<<(unsigned)(Bt * L), 256, 0, (cudaStream_t)stream>>>(
-      h, h_dtype, h_sb, h_sl, x_conv, x_sb, x_sl, gate, g_sb, g_sl, xg_dtype, D, weight, w_dtype,
+      h, h_dtype, h_sb, h_sl, x_conv, x_sb, x_sl, gate, g_sb, g_sl, xg_dtype, D, D_dt, weight, w_dtype,
       gate_bias, eps, y, L, H, R, mode, sumsq, norm_width);
   return check_launch(who);
 }
@@ -758,7 +851,7 @@ extern "C" int fracssm_scan_epilogue(const void *h, int h_dtype, int64_t h_sb, i
                                      int64_t H, int64_t R, void *stream) {
   using namespace fracssm;
   return scan_epilogue_launch("scan_epilogue", h, h_dtype, h_sb, h_sl, x_conv, x_sb, x_sl, gate, g_sb, g_sl,
-                              xg_dtype, D, weight, w_dtype, gate_bias, eps, y, Bt, L, H, R, kEpilogueFull,
+                              xg_dtype, D, FRACSSM_F32, weight, w_dtype, gate_bias, eps, y, Bt, L, H, R, kEpilogueFull,
                               nullptr, H * R, stream);
 }
 
@@ -771,7 +864,7 @@ extern "C" int fracssm_scan_epilogue_sumsq(const void *h, int h_dtype, int64_t h
                                            int64_t L, int64_t H, int64_t R, void *stream) {
   using namespace fracssm;
   return scan_epilogue_launch("scan_epilogue_sumsq", h, h_dtype, h_sb, h_sl, x_conv, x_sb, x_sl, gate, g_sb,
-                              g_sl, xg_dtype, D, nullptr, FRACSSM_F32, gate_bias, 0.f, nullptr, Bt, L, H, R,
+                              g_sl, xg_dtype, D, FRACSSM_F32, nullptr, FRACSSM_F32, gate_bias, 0.f, nullptr, Bt, L, H, R,
                               kEpiloguePartial, sumsq, H * R, stream);
 }
 
@@ -786,7 +879,7 @@ extern "C" int fracssm_scan_epilogue_apply(const void *h, int h_dtype, int64_t h
                                            int64_t R, void *stream) {
   using namespace fracssm;
   return scan_epilogue_launch("scan_epilogue_apply", h, h_dtype, h_sb, h_sl, x_conv, x_sb, x_sl, gate, g_sb,
-                              g_sl, xg_dtype, D, weight, w_dtype, gate_bias, eps, y, Bt, L, H, R, kEpilogueApply,
+                              g_sl, xg_dtype, D, FRACSSM_F32, weight, w_dtype, gate_bias, eps, y, Bt, L, H, R, kEpilogueApply,
                               const_cast<float *>(sumsq), norm_width, stream);
 }
 
@@ -854,4 +947,54 @@ extern "C" int fracssm_scan_layer_norm(const void *gated, const float *ss_partia
       reinterpret_cast<const __nv_bfloat16 *>(gated), ss_partial, 4 * H, sumsq, weight, w_dtype, eps, norm_width,
       reinterpret_cast<__nv_bfloat16 *>(y), HR);
   return check_launch("scan_layer_norm");
+}
+
+extern "C" int fracssm_add_rmsnorm(const void *x, const void *y, const void *weight, int w_dtype, float eps, void *sum,
+                                   void *norm, int64_t rows, int64_t D, void *stream) {
+  using namespace fracssm;
+  if (rows < 0 || D <= 0) return fail(FRACSSM_ERR_ARG, "add_rmsnorm: bad sizes");
+  if (!known_dtype(w_dtype)) return fail(FRACSSM_ERR_ARG, "add_rmsnorm: unsupported weight dtype");
+  if (rows == 0) return FRACSSM_OK;
+  if (!x || !y || !weight || !sum || !norm) return fail(FRACSSM_ERR_ARG, "add_rmsnorm: null pointer");
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(sum) |
+                         reinterpret_cast<uintptr_t>(norm);
+  if (D % 8 != 0 || D > 2048 || (bits & 15) != 0 || ceil_div(rows, 4) >= (int64_t(1) << 31))
+    return fail(FRACSSM_ERR_UNSUPPORTED, "add_rmsnorm: rows of a multiple of 8, at most 2048 elements, 16-byte aligned");
+  const bool wvec = w_dtype == FRACSSM_BF16 && (reinterpret_cast<uintptr_t>(weight) & 15) == 0;
+  auto kernel = wvec ? add_rmsnorm_kernel<1> : add_rmsnorm_kernel<0>;
+  kernel<<<(unsigned)ceil_div(rows, 4), 128, 0, (cudaStream_t)stream>>>(
+      reinterpret_cast<const __nv_bfloat16 *>(x), reinterpret_cast<const __nv_bfloat16 *>(y), weight, w_dtype, eps,
+      reinterpret_cast<__nv_bfloat16 *>(sum), reinterpret_cast<__nv_bfloat16 *>(norm), rows, D);
+  return check_launch("add_rmsnorm");
+}
+
+// What a mixer does between its projections and out_proj, in bfloat16: parameter prep, scan, (state), epilogue.
+extern "C" int fracssm_prefill_mix(const void *dyn, const void *rw, const void *x_conv, const void *gate, int64_t gate_sl,
+                                   const float *mask, const void *const *params, int params_f32, const float *nums,
+                                   const void *u, void *c, void *kappa, int ck_dtype, float *rho, void *h,
+                                   float *final_state, float *state, void *y, void *workspace, size_t workspace_bytes,
+                                   int64_t Bt, int64_t L, int64_t H, int64_t R, int64_t M, int64_t T, void *stream) {
+  using namespace fracssm;
+  if (!params || !nums || (state && !final_state)) return fail(FRACSSM_ERR_ARG, "prefill_mix: null pointer");
+  if (Bt <= 0 || L <= 0 || H <= 0 || R <= 0 || M <= 0) return fail(FRACSSM_ERR_ARG, "prefill_mix: bad sizes");
+  if (state && (Bt * H > 65535 || ceil_div(R, 32) > 65535)) return fail(FRACSSM_ERR_UNSUPPORTED, "prefill_mix: too many rows");
+  auto dt = [&](int i) { return (params_f32 >> i) & 1 ? FRACSSM_F32 : FRACSSM_BF16; };
+  const int64_t di = H * R;
+  int rc = compute_params_typed(dyn, FRACSSM_BF16, L * 3 * H, 3 * H, rw, FRACSSM_BF16, L * 2 * H * M, 2 * H * M, x_conv,
+                                FRACSSM_BF16, L * di, di, mask, L, 1, params[0], dt(0), params[3], dt(3), params[1], dt(1),
+                                params[2], dt(2), nums[0], nums[1], nums[2], nums[3], nums[4], nums[5], nums[6], nullptr, c,
+                                kappa, ck_dtype, rho, Bt, L, H, R, M, stream);
+  if (rc) return rc;
+  rc = fracssm_frac_scan_fwd(u, FRACSSM_BF16, L * R, R, c, kappa, ck_dtype, L * M, M, L * M, M, rho, L * M, M, nullptr, h,
+                             final_state, FRACSSM_F32, workspace, workspace_bytes, Bt * H, L, R, M, T, 0, stream);
+  if (rc) return rc;
+  if (state) {
+    state_transpose_kernel<<<dim3((unsigned)ceil_div(M, 32), (unsigned)ceil_div(R, 32), (unsigned)(Bt * H)), 256, 0,
+                             (cudaStream_t)stream>>>(final_state, state, (int)R, (int)M);
+    rc = check_launch("prefill_mix");
+    if (rc) return rc;
+  }
+  return scan_epilogue_launch("prefill_mix", h, FRACSSM_BF16, L * R, R, x_conv, L * di, di, gate, L * gate_sl, gate_sl,
+                              FRACSSM_BF16, params[4], dt(4), params[5], dt(5), nums[7], nums[8], y, Bt, L, H, R,
+                              kEpilogueFull, nullptr, di, stream);
 }

@@ -189,6 +189,25 @@ causal_conv4_silu_bf16_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_sb,
   }
 }
 
+// What the convolution of the next token needs: tail[b, ch, k] = the last K - 1 inputs times their mask (rounded to
+// the input's type, like the product), zero before the first token.
+__global__ void __launch_bounds__(128)
+conv_tail_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_sb, int64_t x_sl, const float *__restrict__ mask,
+                 int64_t m_sb, int64_t m_sl, __nv_bfloat16 *__restrict__ tail, int64_t L, int64_t C, int K) {
+  const int64_t ch = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
+  if (ch >= C) return;
+  for (int k = 0; k < K - 1; ++k) {
+    const int64_t l = L - (K - 1) + k;
+    __nv_bfloat16 v = __float2bfloat16_rn(0.f);
+    if (l >= 0) {
+      v = x[b * x_sb + l * x_sl + ch];
+      if (mask)
+        v = __float2bfloat16_rn(__bfloat162float(v) * __bfloat162float(__float2bfloat16_rn(mask[b * m_sb + l * m_sl])));
+    }
+    tail[(b * C + ch) * (K - 1) + k] = v;
+  }
+}
+
 // One token of the recurrence for every (batch, head): state [M, R] float32 updated in place,
 //   state[m, r] = rho[m] * state[m, r] + kappa[m] * u[r];  out[r] = sum_m c[m] * state[m, r] + u[r] * D[r].
 // One block per (batch, head); thread r-lane strides over R, the modes are walked in the block's
@@ -284,4 +303,18 @@ extern "C" int fracssm_decode_step(const void *u, int u_dtype, const float *c, c
   decode_step_kernel<<<(unsigned)(Bt * H), dim3(tx, ty), smem, (cudaStream_t)stream>>>(u, u_dtype, c, kappa, rho, D,
                                                                                      state, out, H, R, M);
   return check_launch("decode_step");
+}
+
+extern "C" int fracssm_prefill_conv(const void *x, int64_t x_sl, const float *mask, const void *weight, const void *bias,
+                                    void *y, void *u_heads, void *tail, int64_t R, int64_t Bt, int64_t L, int64_t C,
+                                    int64_t K, void *stream) {
+  using namespace fracssm;
+  const int rc = fracssm_causal_conv_silu_heads(x, FRACSSM_BF16, L * x_sl, x_sl, mask, L, 1, weight, bias, FRACSSM_BF16, y,
+                                                FRACSSM_BF16, u_heads, R, Bt, L, C, K, stream);
+  if (rc || !tail || K < 2 || Bt == 0 || L == 0) return rc;
+  if (Bt > 65535) return fail(FRACSSM_ERR_UNSUPPORTED, "prefill_conv: batch too large for one launch");
+  conv_tail_kernel<<<dim3((unsigned)ceil_div(C, 128), (unsigned)Bt), 128, 0, (cudaStream_t)stream>>>(
+      reinterpret_cast<const __nv_bfloat16 *>(x), L * x_sl, x_sl, mask, L, 1, reinterpret_cast<__nv_bfloat16 *>(tail), L, C,
+      (int)K);
+  return check_launch("prefill_conv");
 }

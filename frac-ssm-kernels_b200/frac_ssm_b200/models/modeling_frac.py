@@ -25,6 +25,7 @@ from ..modules.rmsnorm_gated import rmsnorm_gated_fwd
 from ..ops.b200.frac_scan import frac_scan
 from .configuration_frac import FracConfig
 from .decode import decode_layers
+from .prefill import prefill_layers
 
 LayerCache = tuple  # (state [B, H, M, R] float32, conv_state [B, C, K-1])
 
@@ -226,12 +227,16 @@ class FracModel(nn.Module):
             raise ValueError("You must specify exactly one of input_ids and inputs_embeds.")
         use_cache = self.config.use_cache if use_cache is None else use_cache
         h = self.embed_tokens(input_ids) if inputs_embeds is None else inputs_embeds
-        if attention_mask is None and h.dim() == 3 and h.shape[1] == 1:
-            # one token per sequence: all layers in one native call where it covers them
-            done = decode_layers(self.layers, h, past_key_values, use_cache,
-                                 (FracBlock, RMSNorm, FracMixer, RMSNormGated))
-            if done is not None:
-                return self.norm(done[0]), done[1]
+        # all layers with few native calls where those cover the model and the call
+        classes = (FracBlock, RMSNorm, FracMixer, RMSNormGated)
+        done = None
+        if h.dim() == 3 and h.shape[1] == 1:
+            if attention_mask is None:
+                done = decode_layers(self.layers, h, past_key_values, use_cache, classes)
+        elif past_key_values is None:
+            done = prefill_layers(self.layers, h, attention_mask, use_cache, classes)
+        if done is not None:
+            return self.norm(done[0]), done[1]
         past = (None,) * len(self.layers) if past_key_values is None else past_key_values
         new_past = [] if use_cache else None
         for layer, layer_past in zip(self.layers, past):

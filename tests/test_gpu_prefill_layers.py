@@ -1,0 +1,77 @@
+"""The few-calls prefill (models/prefill.py) against the modules' own forward."""
+
+import pytest
+import torch
+
+from tests.test_gpu_decode_layers import _flat, _model
+
+pytestmark = pytest.mark.gpu
+
+
+def _hooked(model, *args, **kw):
+    """The same call with the modules' own forward: a hook keeps the native route away."""
+    handle = model.model.layers[0].register_forward_hook(lambda *a: None)
+    out = model(*args, **kw)
+    handle.remove()
+    return out
+
+
+# lengths around the convolution's history and the scan's tiles; single-pass and segment scans; odd widths
+@pytest.mark.parametrize("hidden,H,M,B,L", [(64, 2, 128, 1, 2), (128, 4, 128, 2, 3), (256, 8, 128, 2, 129), (96, 3, 7, 3, 50),
+                                            (768, 12, 8, 2, 200), (768, 24, 128, 1, 397), (72, 3, 20, 2, 33)])
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("coeff", [None, torch.bfloat16])
+def test_prefill_matches_modules(hidden, H, M, B, L, masked, coeff):
+    half = _model(hidden, H, M).to(torch.bfloat16)
+    exact_model = _model(hidden, H, M)
+    for p, q in zip(list(exact_model.parameters()) + list(exact_model.buffers()), list(half.parameters()) + list(half.buffers())):
+        p.data.copy_(q.data)
+    for layer in half.model.layers:
+        layer.mixer.coeff_dtype = coeff
+    ids = torch.randint(1, 50, (B, L), generator=torch.Generator().manual_seed(L)).cuda()
+    mask = None
+    if masked:
+        mask = torch.ones(B, L, dtype=torch.long)
+        mask[B - 1, : L // 2] = 0
+        mask = mask.cuda()
+    native = _flat(half(ids, attention_mask=mask, use_cache=True))
+    logits, none = half(ids, attention_mask=mask, use_cache=False)
+    assert none is None and torch.equal(logits, native[0])
+    modules = _flat(_hooked(half, ids, attention_mask=mask, use_cache=True))
+    exact = _flat(exact_model(ids, attention_mask=mask, use_cache=True))
+    for n, m, e in zip(native, modules, exact):
+        assert n.shape == m.shape and n.dtype == m.dtype and n.is_contiguous()
+        scale = e.float().norm().clamp_min(1e-6)
+        err, err_m = ((x.float() - e.float()).norm() / scale for x in (n, m))
+        # the same roundings at the same places: the same error up to chance
+        assert err <= 1.25 * err_m + 2e-3, (err, err_m)
+
+
+def test_mixed_parameter_types_and_other_masks():
+    half = _model(64, 2, 16).to(torch.bfloat16)
+    for layer in half.model.layers:
+        layer.mixer.base_log_tau = layer.mixer.base_log_tau.float()
+        layer.mixer.D.data = layer.mixer.D.data.float()
+        layer.norm.weight.data = layer.norm.weight.data.float()
+    ids = torch.ones(2, 40, dtype=torch.long).cuda()
+    mask = torch.ones(2, 40, device="cuda", dtype=torch.bool)
+    mask[0, 30:] = False
+    for m in (mask, mask.float() * 0.3, mask.t().contiguous().t()):
+        for a, b in zip(_flat(half(ids, attention_mask=m, use_cache=True)), _flat(_hooked(half, ids, attention_mask=m, use_cache=True))):
+            assert (a.float() - b.float()).norm() <= 2e-2 * b.float().norm() + 1e-3
+
+
+@pytest.mark.parametrize("rows,D", [(1, 8), (5, 768), (4, 2048), (3, 264)])
+@pytest.mark.parametrize("w_dtype", [torch.bfloat16, torch.float32])
+def test_add_rmsnorm(rows, D, w_dtype):
+    from frac_ssm_b200 import _cabi as C
+    g = torch.Generator().manual_seed(D)
+    x, y = (torch.randn(rows, D, generator=g).bfloat16().cuda() for _ in range(2))
+    w = (1 + 0.1 * torch.randn(D, generator=g)).to(w_dtype).cuda()
+    total, norm = torch.empty_like(x), torch.empty_like(x)
+    C.check(C.lib().fracssm_add_rmsnorm(C.ptr(x), C.ptr(y), C.ptr(w), C.dt(w), 1e-6, C.ptr(total), C.ptr(norm), rows, D,
+                                        C.stream_of(x)), "add_rmsnorm")
+    assert torch.equal(total, x + y)
+    s = total.double()
+    ref = s * torch.rsqrt(s.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    assert (norm.double() - ref).abs().max() <= 2 ** -8 * ref.abs().max()      # one rounding to bfloat16
