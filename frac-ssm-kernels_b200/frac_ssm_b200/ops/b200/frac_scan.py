@@ -11,6 +11,7 @@ from typing import Optional, Tuple
 import torch
 
 from ... import _cabi as C
+from .stages import _op
 
 # "auto": the single-pass tcgen05 kernel when it covers the shape, else the staged kernels.
 _PATHS = {"auto": C.PATH_AUTO, "staged": C.PATH_STAGED, "fused": C.PATH_FUSED}
@@ -133,7 +134,7 @@ def _launch(u, c, kappa, rho, chunk_size, initial_state, want_final, final_fp32,
 # Registered as a torch custom op (with a shape-only "fake" implementation) so that callers can put
 # the scan inside torch.compile(fullgraph=True), as the reference does for its ops
 # (frac_ssm/ops/triton/chunk_state.py:243-302).  Forward only: asking for gradients raises.
-@torch.library.custom_op("frac_ssm_b200::frac_scan_fwd", mutates_args=())
+@_op("frac_scan_fwd")
 def _frac_scan_fwd_op(u: torch.Tensor, c: torch.Tensor, kappa: torch.Tensor, rho: torch.Tensor,
                       chunk_size: int, initial_state: Optional[torch.Tensor], want_final: bool,
                       final_fp32: bool, path_code: int) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -147,13 +148,6 @@ def _(u, c, kappa, rho, chunk_size, initial_state, want_final, final_fp32, path_
     fdt = torch.float32 if final_fp32 else torch.bfloat16
     fin = torch.empty((B, R, M) if want_final else (0,), device=u.device, dtype=fdt)
     return torch.empty(B, L, R, device=u.device, dtype=u.dtype), fin
-
-
-def _no_backward(ctx, *grads):
-    raise NotImplementedError("frac_ssm_b200 implements the forward pass only")
-
-
-_frac_scan_fwd_op.register_autograd(_no_backward)
 
 
 __all__ = ["frac_scan"]

@@ -1,0 +1,33 @@
+"""When a launch function is called directly and when through its registered op (no GPU needed)."""
+
+import torch
+from torch.utils._python_dispatch import TorchDispatchMode
+
+from frac_ssm_b200.ops.b200 import stages
+
+
+class _Mode(TorchDispatchMode):
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        return func(*args, **(kwargs or {}))
+
+
+class _Sub(torch.Tensor):
+    pass
+
+
+def test_direct_only_where_nothing_observes_the_op():
+    x = torch.ones(2)
+    w = torch.ones(2, requires_grad=True)
+    assert stages._unobserved((x, 3, 1.0, None, True, torch.bfloat16))
+    assert not stages._unobserved((x, w))
+    with torch.no_grad():
+        assert stages._unobserved((x, w, torch.nn.Parameter(x)))
+    assert not stages._unobserved((x.as_subclass(_Sub),))
+    with _Mode():
+        assert not stages._unobserved((x,))
+    seen = []
+    torch.vmap(lambda t: seen.append(stages._unobserved((t,))) or t)(torch.ones(3, 2))
+    with torch.autograd.forward_ad.dual_level():
+        seen.append(stages._unobserved((x,)))
+    torch.jit.trace(lambda t: seen.append(stages._unobserved((t,))) or t + 1, x, check_trace=False)
+    assert seen and not any(seen)
