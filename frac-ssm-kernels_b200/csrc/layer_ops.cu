@@ -571,12 +571,12 @@ scan_epilogue_kernel(const void *__restrict__ h, int h_dt, int64_t h_sb, int64_t
 // instruction count as much as by memory, hence the fast-math gate (silu(z) = z / (1 + e^-z) with
 // the approximate exponential and division: about 2 ulp, the output is bf16) and the norm weight
 // read as one or two 16-byte pieces (WVEC 1: bf16, 2: f32; 0: element by element, any type).
-template <int WVEC>
+template <int WVEC, bool DF32>
 __global__ void __launch_bounds__(1024)
 scan_epilogue_bf16_kernel(const __nv_bfloat16 *__restrict__ h, int64_t h_sb, int64_t h_sl,
                           const __nv_bfloat16 *__restrict__ x, int64_t x_sb, int64_t x_sl,
                           const __nv_bfloat16 *__restrict__ gate, int64_t g_sb, int64_t g_sl,
-                          const void *__restrict__ Dp, int D_dt, const void *__restrict__ w, int w_dt,
+                          const void *__restrict__ Dp, const void *__restrict__ w, int w_dt,
                           float gate_bias, float eps, __nv_bfloat16 *__restrict__ y, int64_t L, int64_t H,
                           int64_t R, int mode, float *__restrict__ sumsq, int64_t norm_width) {
   __shared__ float red[32];
@@ -594,11 +594,11 @@ scan_epilogue_bf16_kernel(const __nv_bfloat16 *__restrict__ h, int64_t h_sb, int
     unpack8(__ldcs(reinterpret_cast<const uint4 *>(x + b * x_sb + l * x_sl + j)), xv);
     unpack8(__ldcs(reinterpret_cast<const uint4 *>(gate + b * g_sb + l * g_sl + j)), zv);
     float dv[8];
-    if (D_dt == FRACSSM_F32) {
+    if (DF32) {
       const float4 d0 = __ldg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(Dp) + j));
       const float4 d1 = __ldg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(Dp) + j + 4));
       dv[0] = d0.x; dv[1] = d0.y; dv[2] = d0.z; dv[3] = d0.w; dv[4] = d1.x; dv[5] = d1.y; dv[6] = d1.z; dv[7] = d1.w;
-    } else {   // bf16 (checked by the launch)
+    } else {   // bf16
       unpack8(__ldg(reinterpret_cast<const uint4 *>(reinterpret_cast<const __nv_bfloat16 *>(Dp) + j)), dv);
     }
 #pragma unroll
@@ -824,14 +824,20 @@ int scan_epilogue_launch(const char *who, const void *h, int h_dtype, int64_t h_
       g_sb % 8 == 0 && g_sl % 8 == 0) {
     const unsigned threads = (unsigned)(((HR / 8) + 31) / 32 * 32);
     const int wvec = (mode == kEpiloguePartial || !al16(weight)) ? 0 : w_dtype == FRACSSM_BF16 ? 1 : w_dtype == FRACSSM_F32 ? 2 : 0;
-#define FRACSSM_EPILOGUE(WV)                                                                                       \
-  scan_epilogue_bf16_kernel<WV><<<(unsigned)(Bt * L), threads, 0, (cudaStream_t)stream>>>(                         \
+#define FRACSSM_EPILOGUE(WV, DF32)                                                                                 \
+  scan_epilogue_bf16_kernel<WV, DF32><<<(unsigned)(Bt * L), threads, 0, (cudaStream_t)stream>>>(                   \
       reinterpret_cast<const __nv_bfloat16 *>(h), h_sb, h_sl, reinterpret_cast<const __nv_bfloat16 *>(x_conv),     \
-      x_sb, x_sl, reinterpret_cast<const __nv_bfloat16 *>(gate), g_sb, g_sl, D, D_dt, weight, w_dtype, gate_bias, eps, \
+      x_sb, x_sl, reinterpret_cast<const __nv_bfloat16 *>(gate), g_sb, g_sl, D, weight, w_dtype, gate_bias, eps,   \
       reinterpret_cast<__nv_bfloat16 *>(y), L, H, R, mode, sumsq, norm_width)
-    if (wvec == 1) FRACSSM_EPILOGUE(1);
-    else if (wvec == 2) FRACSSM_EPILOGUE(2);
-    else FRACSSM_EPILOGUE(0);
+    if (D_dt == FRACSSM_F32) {
+      if (wvec == 1) FRACSSM_EPILOGUE(1, true);
+      else if (wvec == 2) FRACSSM_EPILOGUE(2, true);
+      else FRACSSM_EPILOGUE(0, true);
+    } else {
+      if (wvec == 1) FRACSSM_EPILOGUE(1, false);
+      else if (wvec == 2) FRACSSM_EPILOGUE(2, false);
+      else FRACSSM_EPILOGUE(0, false);
+    }
 #undef FRACSSM_EPILOGUE
     return check_launch(who);
   }
