@@ -228,16 +228,21 @@ __global__ void __launch_bounds__(kThreads, 1)
 scan_fused_kernel(const FusedArgs a, const __grid_constant__ CUtensorMap u_map) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  // mbarriers.  Completed once per tile: cb2 / cbK / barH (tcgen05.commit), barU (TMA), fS / fW / out_bar
+  // mbarriers.  Completed once per tile: cb2 / cbK / barH (tcgen05.commit), barU (TMA), fS / fW / fL / fLb / out_bar
   // (16 worker warps), item_bar / state_bar (chain warp), read_bar (workers + MMA warp).  Completed once per HALF of the modes,
   // i.e. twice per tile, so the phase parity of half h is simply h: cb0 / cbL (tcgen05.commit) and
-  // fA / fL1 / fL / fK (16 worker warps).
+  // fA / fL1 / fK (16 worker warps).  A barrier may only be of the second kind if its second completion waits for
+  // whoever waits for the first: fA and fL1 do (the workers wait for the products in between), the rows of the levels
+  // 64 + 32 did not.  When the MMA warp was late by the time the workers need for a half (a few instruction fetches from
+  // beyond the cache), both completions were in before it looked, the parity was back where it started and the CTA waited
+  // until the limit: hence a barrier for each half (fL, fLb).
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kOffMisc);
   uint64_t *cb0 = bars + 0, *cbL = bars + 1, *cb2 = bars + 2, *cbK = bars + 3, *barH = bars + 4, *barU = bars + 5;
   uint64_t *fA = bars + 6, *fL = bars + 7, *fK = bars + 8, *fW = bars + 9, *fS = bars + 10;
   uint64_t *item_bar = bars + 11, *state_bar = bars + 12, *out_bar = bars + 13, *read_bar = bars + 14;
   uint64_t *fL1 = bars + 15;    // 16 worker warps, once per half: the rows of the levels 8 + 16 are written
-  uint32_t *tmem_s = reinterpret_cast<uint32_t *>(bars + 16);
+  uint64_t *fLb = bars + 16;    // fL for the second half of the modes
+  uint32_t *tmem_s = reinterpret_cast<uint32_t *>(bars + 17);
   volatile int *items = reinterpret_cast<volatile int *>(tmem_s + 1);  // [2], by tile parity
   volatile int *failed = reinterpret_cast<volatile int *>(tmem_s + 3);  // a wait of this CTA ran out
 
@@ -251,6 +256,7 @@ scan_fused_kernel(const FusedArgs a, const __grid_constant__ CUtensorMap u_map) 
     umma::mbar_init(out_bar, 16);
     umma::mbar_init(read_bar, 17);   // the 16 worker warps and the MMA warp, once each has read the tile's item
     umma::mbar_init(fL1, 16);
+    umma::mbar_init(fLb, 16);
     umma::fence_mbar_init();
     umma::prefetch_tmap(&u_map);
     *failed = 0;
@@ -409,7 +415,7 @@ scan_fused_kernel(const FusedArgs a, const __grid_constant__ CUtensorMap u_map) 
           umma::mma_commit(cbL);
         }
         __syncwarp();
-        FRACSSM_WAIT(fL, h);
+        FRACSSM_WAIT(h == 0 ? fL : fLb, n);
         FRACSSM_MARK(3, 3 + 4 * h)
         umma::tc_fence_after();
         if (umma::elect_one()) {
@@ -727,7 +733,7 @@ scan_fused_kernel(const FusedArgs a, const __grid_constant__ CUtensorMap u_map) 
           if (w & 8) emit_level(sb + kOffY2 + half_off + rg64 * 1024, cp, bk, true);
           else emit_level(sb + kOffZ2 + half_off + rg64 * 1024, ks, fw, true);
         }
-        warp_arrive(fL, lane);
+        warp_arrive(h == 0 ? fL : fLb, lane);
         FRACSSM_MARK(pslot, 4 + 10 * h)
         // to the tile's start (bk becomes E) and end (fw becomes F)
         if (w & 8) {
