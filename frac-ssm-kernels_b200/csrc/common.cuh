@@ -61,4 +61,12 @@ int scan_fused_launch_ex(const void *u, const void *c, const void *kappa, int ck
                          int64_t M, int64_t T, void *stream, int first_tile, unsigned long long wait_ns,
                          const ScanLayerOut *layer);
 
+// defined in frac_scan.cu: fracssm_frac_scan_fwd; where the route taken can, the final state goes to `state_modes_first`
+// ([B, M, R] float32, may be null) instead of final_state, which *modes_first reports
+int frac_scan_route(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, const void *c, const void *kappa, int ck_dtype,
+                    int64_t c_sb, int64_t c_sl, int64_t k_sb, int64_t k_sl, const float *rho, int64_t r_sb, int64_t r_sl,
+                    const float *initial_state, void *h, void *final_state, int final_dtype, void *workspace,
+                    size_t workspace_bytes, int64_t B, int64_t L, int64_t R, int64_t M, int64_t T, int path, void *stream,
+                    float *state_modes_first, bool *modes_first);
+
 }  // namespace fracssm

@@ -40,7 +40,8 @@ size_t scan_few_workspace_bytes(int64_t B, int64_t L, int64_t R, int64_t M);
 int scan_few_launch(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, const void *c, const void *kappa,
                     int ck_dtype, int64_t c_sb, int64_t c_sl, int64_t k_sb, int64_t k_sl, const float *rho,
                     int64_t r_sb, int64_t r_sl, const float *initial_state, void *h, void *final_state,
-                    int final_dtype, void *workspace, int64_t B, int64_t L, int64_t R, int64_t M, void *stream);
+                    int final_dtype, void *workspace, int64_t B, int64_t L, int64_t R, int64_t M, void *stream,
+                    bool fin_modes_first);
 
 }  // namespace fracssm
 
@@ -57,14 +58,13 @@ extern "C" size_t fracssm_frac_scan_workspace_bytes(int64_t B, int64_t L, int64_
   return other > fused ? other : fused;
 }
 
-extern "C" int fracssm_frac_scan_fwd(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl,
-                                     const void *c, const void *kappa, int ck_dtype, int64_t c_sb,
-                                     int64_t c_sl, int64_t k_sb, int64_t k_sl, const float *rho,
-                                     int64_t r_sb, int64_t r_sl, const float *initial_state,
-                                     void *h, void *final_state, int final_dtype, void *workspace,
-                                     size_t workspace_bytes, int64_t B, int64_t L, int64_t R,
-                                     int64_t M, int64_t T, int path, void *stream) {
-  using namespace fracssm;
+namespace fracssm {
+int frac_scan_route(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, const void *c, const void *kappa, int ck_dtype,
+                    int64_t c_sb, int64_t c_sl, int64_t k_sb, int64_t k_sl, const float *rho, int64_t r_sb, int64_t r_sl,
+                    const float *initial_state, void *h, void *final_state, int final_dtype, void *workspace,
+                    size_t workspace_bytes, int64_t B, int64_t L, int64_t R, int64_t M, int64_t T, int path, void *stream,
+                    float *state_modes_first, bool *modes_first) {
+  if (modes_first) *modes_first = false;
   if (B < 0 || L < 0 || R <= 0 || M <= 0 || T <= 0) return fail(FRACSSM_ERR_ARG, "frac_scan: bad sizes");
   if (!known_dtype(u_dtype) || !known_dtype(ck_dtype)) return fail(FRACSSM_ERR_ARG, "frac_scan: unsupported dtype");
   if (ck_dtype != u_dtype && ck_dtype != FRACSSM_F32)
@@ -111,9 +111,13 @@ extern "C" int fracssm_frac_scan_fwd(const void *u, int u_dtype, int64_t u_sb, i
   }
 
   // (a caller whose workspace only holds the chunked stages keeps them)
-  if (path == 0 && scan_few_supported(B, L, R, M, T) && workspace_bytes >= scan_few_workspace_bytes(B, L, R, M))
+  if (path == 0 && scan_few_supported(B, L, R, M, T) && workspace_bytes >= scan_few_workspace_bytes(B, L, R, M)) {
+    if (state_modes_first) *modes_first = true;
     return scan_few_launch(u, u_dtype, u_sb, u_sl, c, kappa, ck_dtype, c_sb, c_sl, k_sb, k_sl, rho, r_sb, r_sl,
-                           initial_state, h, final_state, final_dtype, workspace, B, L, R, M, stream);
+                           initial_state, h, state_modes_first ? state_modes_first : final_state,
+                           state_modes_first ? FRACSSM_F32 : final_dtype, workspace, B, L, R, M, stream,
+                           state_modes_first != nullptr);
+  }
 
   ScanScratch s = staged_layout(workspace, B, L, R, M, T);
   if (workspace_bytes < s.bytes) return fail(FRACSSM_ERR_ARG, "frac_scan: workspace too small");
@@ -129,4 +133,17 @@ extern "C" int fracssm_frac_scan_fwd(const void *u, int u_dtype, int64_t u_sb, i
   return fracssm_chunk_fused_readout(u, u_dtype, u_sb, u_sl, c, kappa, ck_dtype, c_sb, c_sl, k_sb,
                                      k_sl, s.states_acc, FRACSSM_F32, s.lcr, L * M, M, h, B, L, R, M,
                                      T, stream);
+}
+}  // namespace fracssm
+
+extern "C" int fracssm_frac_scan_fwd(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl,
+                                     const void *c, const void *kappa, int ck_dtype, int64_t c_sb,
+                                     int64_t c_sl, int64_t k_sb, int64_t k_sl, const float *rho,
+                                     int64_t r_sb, int64_t r_sl, const float *initial_state,
+                                     void *h, void *final_state, int final_dtype, void *workspace,
+                                     size_t workspace_bytes, int64_t B, int64_t L, int64_t R,
+                                     int64_t M, int64_t T, int path, void *stream) {
+  return fracssm::frac_scan_route(u, u_dtype, u_sb, u_sl, c, kappa, ck_dtype, c_sb, c_sl, k_sb, k_sl, rho, r_sb, r_sl,
+                                  initial_state, h, final_state, final_dtype, workspace, workspace_bytes, B, L, R, M, T,
+                                  path, stream, nullptr, nullptr);
 }

@@ -19,6 +19,7 @@ __device__ __forceinline__ float softplusf_(float x) { return x > 20.f ? x : log
 
 struct ParamArgs {
   const void *dyn; int dyn_dt; int64_t dyn_sb, dyn_sl;
+  const __nv_bfloat16 *dyn_bias;   // null, or [3 H] added to dyn (the sum rounded to bf16, as a separate addition leaves it)
   const void *rw; int rw_dt; int64_t rw_sb, rw_sl;
   const void *x; int x_dt; int64_t x_sb, x_sl;
   const float *mask; int64_t m_sb, m_sl;
@@ -29,6 +30,12 @@ struct ParamArgs {
   void *u, *c, *kappa; int ck_dt; float *rho;
   int64_t L, H, R, M;
 };
+
+// element j of a token's row of dyn (base: the row's offset)
+__device__ __forceinline__ float dyn_at(const ParamArgs &a, int64_t base, int64_t j) {
+  const float v = ld_f32(a.dyn, base + j, a.dyn_dt);
+  return a.dyn_bias ? __bfloat162float(__float2bfloat16_rn(v + __bfloat162float(a.dyn_bias[j]))) : v;
+}
 
 // One warp per (bh, token): lanes stride over the M modes; two softmaxes by warp shuffles.
 __global__ void __launch_bounds__(128) compute_params_kernel(const ParamArgs a) {
@@ -41,10 +48,10 @@ __global__ void __launch_bounds__(128) compute_params_kernel(const ParamArgs a) 
   const int64_t H = a.H, M = a.M, R = a.R;
 
   const int64_t dbase = b * a.dyn_sb + l * a.dyn_sl;
-  float dt = softplusf_(ld_f32(a.dyn, dbase + h, a.dyn_dt) + ld_f32(a.dt_bias, h, a.dtb_dt));
+  float dt = softplusf_(dyn_at(a, dbase, h) + ld_f32(a.dt_bias, h, a.dtb_dt));
   dt = fminf(fmaxf(dt, a.dt_min), a.dt_max);
-  const float alpha = a.a_min + sigmoidf_(ld_f32(a.dyn, dbase + H + h, a.dyn_dt)) * (a.a_max - a.a_min);
-  const float lam = a.l_min + sigmoidf_(ld_f32(a.dyn, dbase + 2 * H + h, a.dyn_dt)) * (a.l_max - a.l_min);
+  const float alpha = a.a_min + sigmoidf_(dyn_at(a, dbase, H + h)) * (a.a_max - a.a_min);
+  const float lam = a.l_min + sigmoidf_(dyn_at(a, dbase, 2 * H + h)) * (a.l_max - a.l_min);
   const float rate = powf(fmaxf(lam, 1e-4f), 1.f / fmaxf(alpha, 1e-4f));
   const float keep = a.mask ? a.mask[b * a.m_sb + l * a.m_sl] : 1.f;
 
@@ -122,10 +129,10 @@ __global__ void __launch_bounds__(128) compute_params_m128_kernel(const ParamArg
   float dt_l = 0.f, alpha_l = 0.f, rate_l = 0.f, keep_l = 1.f;
   if (lane < kPrepTokens && l0 + lane < l1) {
     const int64_t l = l0 + lane, dbase = b * a.dyn_sb + l * a.dyn_sl;
-    dt_l = softplusf_(ld_f32(a.dyn, dbase + h, a.dyn_dt) + dtb);
+    dt_l = softplusf_(dyn_at(a, dbase, h) + dtb);
     dt_l = fminf(fmaxf(dt_l, a.dt_min), a.dt_max);
-    alpha_l = a.a_min + sigmoidf_(ld_f32(a.dyn, dbase + H + h, a.dyn_dt)) * (a.a_max - a.a_min);
-    const float lam = a.l_min + sigmoidf_(ld_f32(a.dyn, dbase + 2 * H + h, a.dyn_dt)) * (a.l_max - a.l_min);
+    alpha_l = a.a_min + sigmoidf_(dyn_at(a, dbase, H + h)) * (a.a_max - a.a_min);
+    const float lam = a.l_min + sigmoidf_(dyn_at(a, dbase, 2 * H + h)) * (a.l_max - a.l_min);
     rate_l = powf(fmaxf(lam, 1e-4f), 1.f / fmaxf(alpha_l, 1e-4f));
     if (a.mask) keep_l = a.mask[b * a.m_sb + l * a.m_sl];
   }
@@ -191,22 +198,25 @@ __global__ void __launch_bounds__(128) compute_params_m128_kernel(const ParamArg
   }
 }
 
-// The M = 128 prep with fewer instructions per token: a half-warp owns a token (a lane eight
-// consecutive modes: one 16-byte load per residual row, 16- and 32-byte stores), so a warp works on
-// two tokens at a time, the softmax reductions take four shuffle steps instead of five, and the
-// address arithmetic, the shuffles of the per-token scalars and the loop are paid once per two tokens
-// and eight modes per lane.  The kernel above issues about 250 warp instructions per token, of which
-// about 50 are the per-mode arithmetic; this one about 95.  Measured at batch 16 x 4096 tokens x 24 heads:
-// 0.598 ms for the kernel above, 0.571 with this layout at 8 tokens per warp, 0.508 at 32 tokens per warp
-// (the per-warp setup paid less often), 0.470 with the next pair's rows requested one step ahead.
-__device__ __forceinline__ float half_warp_max(float v) {
+// The prep for 8, 16, 32, 64 or 128 modes: Q = M / 8 lanes own a token (a lane eight consecutive modes: one
+// 16-byte load per residual row, 16- and 32-byte stores), so a warp works on 32 / Q tokens at a time, the softmax
+// reductions take log2(Q) shuffle steps, and the address arithmetic, the shuffles of the per-token scalars and the
+// loop are paid once per 32 / Q tokens.  At 128 modes the kernel above issues about 250 warp instructions per token,
+// of which about 50 are the per-mode arithmetic; this one about 95.  Measured at batch 16 x 4096 tokens x 24 heads x
+// 128 modes: 0.598 ms for the kernel above, 0.571 with this layout at 8 tokens per warp, 0.508 at 32 tokens per warp
+// (the per-warp setup paid less often), 0.470 with the next tokens' rows requested one step ahead.  With few tokens
+// in all a warp takes 8 (397 tokens x 24 heads: 17.5 -> 12.8 us); 8 modes, 4 x 1000 tokens x 12 heads: 47.8 us with
+// a warp per token, 8.8 here.
+template <int Q>
+__device__ __forceinline__ float lanes_max(float v) {
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  for (int o = Q / 2; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
-__device__ __forceinline__ float half_warp_sum(float v) {
+template <int Q>
+__device__ __forceinline__ float lanes_sum(float v) {
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = Q / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 __device__ __forceinline__ void unpack8(const uint4 &p, float (&f)[8]) {
@@ -222,20 +232,22 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<const uint32_t *>(&v);
 }
 
-// tokens per warp: one lane computes the per-token scalars of one token, and the per-warp setup (the
-// time constants, the gates) is paid once per 32 tokens
+// tokens per warp, at most: one lane computes the per-token scalars of one token, and the per-warp setup (the
+// time constants, the gates) is paid once for all of them
 constexpr int kPairTokens = 32;
 
-__global__ void __launch_bounds__(128) compute_params_m128_pair_kernel(const ParamArgs a) {
+template <int Q>
+__global__ void __launch_bounds__(128) compute_params_lanes_kernel(const ParamArgs a, int per_warp) {
+  constexpr int kStep = 32 / Q;              // tokens a warp works on at a time
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  const int sub = lane >> 4, q = lane & 15;  // token of the pair; modes 8 q .. 8 q + 7
+  const int sub = lane / Q, q = lane % Q;    // token of the step; modes 8 q .. 8 q + 7
   const float read_gate = sigmoidf_(ld_f32(a.read_logit, 0, a.read_dt)), write_gate = sigmoidf_(ld_f32(a.write_logit, 0, a.write_dt));
-  const int64_t l0 = ((int64_t)blockIdx.x * 4 + warp) * kPairTokens;
+  const int64_t l0 = ((int64_t)blockIdx.x * 4 + warp) * per_warp;
   const int64_t bh = blockIdx.y;
   if (l0 >= a.L) return;
   const int64_t b = bh / a.H, h = bh % a.H;
   const int64_t H = a.H, R = a.R;
-  constexpr int64_t M = 128;
+  constexpr int64_t M = 8 * Q;
   float lt[8], inv_tau[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -244,19 +256,19 @@ __global__ void __launch_bounds__(128) compute_params_m128_pair_kernel(const Par
   }
   const float dtb = ld_f32(a.dt_bias, h, a.dtb_dt);
   const __nv_bfloat16 *rw = reinterpret_cast<const __nv_bfloat16 *>(a.rw);
-  const int64_t l1 = min(l0 + kPairTokens, a.L);
+  const int64_t l1 = min(l0 + per_warp, a.L);
   // per-token scalars: computed once, by lane t for token l0 + t, handed over by shuffles
   float dt_l = 0.f, alpha_l = 0.f, rate_l = 0.f, keep_l = 1.f;
-  if (lane < kPairTokens && l0 + lane < l1) {
+  if (lane < per_warp && l0 + lane < l1) {
     const int64_t l = l0 + lane, dbase = b * a.dyn_sb + l * a.dyn_sl;
-    dt_l = softplusf_(ld_f32(a.dyn, dbase + h, a.dyn_dt) + dtb);
+    dt_l = softplusf_(dyn_at(a, dbase, h) + dtb);
     dt_l = fminf(fmaxf(dt_l, a.dt_min), a.dt_max);
-    alpha_l = a.a_min + sigmoidf_(ld_f32(a.dyn, dbase + H + h, a.dyn_dt)) * (a.a_max - a.a_min);
-    const float lam = a.l_min + sigmoidf_(ld_f32(a.dyn, dbase + 2 * H + h, a.dyn_dt)) * (a.l_max - a.l_min);
+    alpha_l = a.a_min + sigmoidf_(dyn_at(a, dbase, H + h)) * (a.a_max - a.a_min);
+    const float lam = a.l_min + sigmoidf_(dyn_at(a, dbase, 2 * H + h)) * (a.l_max - a.l_min);
     rate_l = powf(fmaxf(lam, 1e-4f), 1.f / fmaxf(alpha_l, 1e-4f));
     if (a.mask) keep_l = a.mask[b * a.m_sb + l * a.m_sl];
   }
-  // the residual rows of the next pair of tokens are requested before this pair is worked on
+  // the residual rows of the next tokens are requested before these are worked on
   uint4 rnext = make_uint4(0, 0, 0, 0), wnext = make_uint4(0, 0, 0, 0);
   const __nv_bfloat16 *rp0 = rw + b * a.rw_sb + h * M + 8 * q;
   if (l0 + sub < l1) {
@@ -264,9 +276,9 @@ __global__ void __launch_bounds__(128) compute_params_m128_pair_kernel(const Par
     wnext = __ldcs(reinterpret_cast<const uint4 *>(rp0 + (l0 + sub) * a.rw_sl + H * M));
   }
 #pragma unroll 1
-  for (int it = 0; it < kPairTokens / 2; ++it) {
-    if (l0 + 2 * it >= l1) break;
-    const int src = 2 * it + sub;
+  for (int it = 0; it * kStep < per_warp; ++it) {
+    if (l0 + kStep * it >= l1) break;
+    const int src = kStep * it + sub;
     const int64_t l = l0 + src;
     const bool live = l < l1;
     const float dt = __shfl_sync(0xffffffffu, dt_l, src), alpha = __shfl_sync(0xffffffffu, alpha_l, src);
@@ -274,9 +286,9 @@ __global__ void __launch_bounds__(128) compute_params_m128_pair_kernel(const Par
     float rl[8], wl[8];
     {
       const uint4 rraw = rnext, wraw = wnext;
-      if (l + 2 < l1 && it + 1 < kPairTokens / 2) {
-        rnext = __ldcs(reinterpret_cast<const uint4 *>(rp0 + (l + 2) * a.rw_sl));
-        wnext = __ldcs(reinterpret_cast<const uint4 *>(rp0 + (l + 2) * a.rw_sl + H * M));
+      if (l + kStep < l1) {
+        rnext = __ldcs(reinterpret_cast<const uint4 *>(rp0 + (l + kStep) * a.rw_sl));
+        wnext = __ldcs(reinterpret_cast<const uint4 *>(rp0 + (l + kStep) * a.rw_sl + H * M));
       }
       unpack8(rraw, rl);
       unpack8(wraw, wl);
@@ -290,8 +302,8 @@ __global__ void __launch_bounds__(128) compute_params_m128_pair_kernel(const Par
       rmax = fmaxf(rmax, rl[i]);
       wmax = fmaxf(wmax, wl[i]);
     }
-    rmax = half_warp_max(rmax);
-    wmax = half_warp_max(wmax);
+    rmax = lanes_max<Q>(rmax);
+    wmax = lanes_max<Q>(wmax);
     float rsum = 0.f, wsum = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -300,7 +312,7 @@ __global__ void __launch_bounds__(128) compute_params_m128_pair_kernel(const Par
       rsum += rl[i];
       wsum += wl[i];
     }
-    const float rinv = 1.f / half_warp_sum(rsum), winv = 1.f / half_warp_sum(wsum);
+    const float rinv = 1.f / lanes_sum<Q>(rsum), winv = 1.f / lanes_sum<Q>(wsum);
     float rho[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -334,7 +346,7 @@ __global__ void __launch_bounds__(128) compute_params_m128_pair_kernel(const Par
       }
       if (a.u) {
         const int64_t xbase = b * a.x_sb + l * a.x_sl + h * R;
-        for (int64_t r = q; r < R; r += 16)
+        for (int64_t r = q; r < R; r += Q)
           st_f32(a.u, (bh * a.L + l) * R + r, a.x_dt, ld_f32(a.x, xbase + r, a.x_dt));
       }
     }
@@ -691,7 +703,7 @@ __global__ void layer_sumsq_kernel(const float *__restrict__ ss, int64_t n_parti
 
 namespace fracssm {
 namespace {
-int compute_params_typed(const void *dyn, int dyn_dtype, int64_t dyn_sb, int64_t dyn_sl,
+int compute_params_typed(const void *dyn, int dyn_dtype, int64_t dyn_sb, int64_t dyn_sl, const void *dyn_bias,
                          const void *rw, int rw_dtype, int64_t rw_sb, int64_t rw_sl,
                          const void *x_conv, int x_dtype, int64_t x_sb, int64_t x_sl,
                          const float *mask, int64_t m_sb, int64_t m_sl,
@@ -711,6 +723,7 @@ int compute_params_typed(const void *dyn, int dyn_dtype, int64_t dyn_sb, int64_t
   if (Bt * H > 65535) return fail(FRACSSM_ERR_UNSUPPORTED, "compute_params: batch*heads too large for one launch");
   ParamArgs a{};
   a.dyn = dyn; a.dyn_dt = dyn_dtype; a.dyn_sb = dyn_sb; a.dyn_sl = dyn_sl;
+  a.dyn_bias = reinterpret_cast<const __nv_bfloat16 *>(dyn_bias);
   a.rw = rw; a.rw_dt = rw_dtype; a.rw_sb = rw_sb; a.rw_sl = rw_sl;
   a.x = x_conv; a.x_dt = x_dtype; a.x_sb = x_sb; a.x_sl = x_sl;
   a.mask = mask; a.m_sb = m_sb; a.m_sl = m_sl;
@@ -724,16 +737,25 @@ int compute_params_typed(const void *dyn, int dyn_dtype, int64_t dyn_sb, int64_t
   a.u = u; a.c = c; a.kappa = kappa; a.ck_dt = ck_dtype; a.rho = rho;
   a.L = L; a.H = H; a.R = R; a.M = M;
   auto al = [](const void *p, uintptr_t n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; };
-  if (M == 128 && rw_dtype == FRACSSM_BF16 && (ck_dtype == FRACSSM_F32 || ck_dtype == FRACSSM_BF16) && al(rw, 8) &&
-      rw_sb % 4 == 0 && rw_sl % 4 == 0 && al(c, 16) && al(kappa, 16) && al(rho, 16)) {
-    // 16-byte loads of the residual rows and 16-byte stores of bf16 c / kappa need the wider alignment
-    if (al(rw, 16) && rw_sb % 8 == 0 && rw_sl % 8 == 0) {
-      dim3 grid((unsigned)ceil_div(L, 4 * kPairTokens), (unsigned)(Bt * H));
-      compute_params_m128_pair_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(a);
-    } else {
-      dim3 grid((unsigned)ceil_div(L, 4 * kPrepTokens), (unsigned)(Bt * H));
-      compute_params_m128_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(a);
-    }
+  const bool vec = rw_dtype == FRACSSM_BF16 && (ck_dtype == FRACSSM_F32 || ck_dtype == FRACSSM_BF16) && al(c, 16) &&
+                   al(kappa, 16) && al(rho, 16);
+  // 16-byte loads of the residual rows
+  if (vec && al(rw, 16) && rw_sb % 8 == 0 && rw_sl % 8 == 0 && (M == 8 || M == 16 || M == 32 || M == 64 || M == 128)) {
+    // 32 tokens per warp, or as few as 8 while that leaves the GPU less than four blocks per SM
+    int per_warp = kPairTokens;
+    while (per_warp > 8 && per_warp > 256 / M && Bt * H * ceil_div(L, 4 * per_warp) < 148 * 4) per_warp /= 2;
+    const dim3 grid((unsigned)ceil_div(L, 4 * per_warp), (unsigned)(Bt * H));
+    const cudaStream_t st = (cudaStream_t)stream;
+    if (M == 8) compute_params_lanes_kernel<1><<<grid, 128, 0, st>>>(a, per_warp);
+    else if (M == 16) compute_params_lanes_kernel<2><<<grid, 128, 0, st>>>(a, per_warp);
+    else if (M == 32) compute_params_lanes_kernel<4><<<grid, 128, 0, st>>>(a, per_warp);
+    else if (M == 64) compute_params_lanes_kernel<8><<<grid, 128, 0, st>>>(a, per_warp);
+    else compute_params_lanes_kernel<16><<<grid, 128, 0, st>>>(a, per_warp);
+    return check_launch("compute_params");
+  }
+  if (vec && M == 128 && al(rw, 8) && rw_sb % 4 == 0 && rw_sl % 4 == 0) {
+    dim3 grid((unsigned)ceil_div(L, 4 * kPrepTokens), (unsigned)(Bt * H));
+    compute_params_m128_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(a);
     return check_launch("compute_params");
   }
   dim3 grid((unsigned)ceil_div(L, 4), (unsigned)(Bt * H));
@@ -753,8 +775,8 @@ extern "C" int fracssm_compute_params(const void *dyn, int dyn_dtype, int64_t dy
                                       float lambda_min, float lambda_max, void *u, void *c,
                                       void *kappa, int ck_dtype, float *rho, int64_t Bt, int64_t L,
                                       int64_t H, int64_t R, int64_t M, void *stream) {
-  return fracssm::compute_params_typed(dyn, dyn_dtype, dyn_sb, dyn_sl, rw, rw_dtype, rw_sb, rw_sl, x_conv, x_dtype, x_sb,
-                                       x_sl, mask, m_sb, m_sl, dt_bias, FRACSSM_F32, base_log_tau, FRACSSM_F32,
+  return fracssm::compute_params_typed(dyn, dyn_dtype, dyn_sb, dyn_sl, nullptr, rw, rw_dtype, rw_sb, rw_sl, x_conv, x_dtype,
+                                       x_sb, x_sl, mask, m_sb, m_sl, dt_bias, FRACSSM_F32, base_log_tau, FRACSSM_F32,
                                        read_gate_logit, FRACSSM_F32, write_gate_logit, FRACSSM_F32, read_temp, dt_min,
                                        dt_max, alpha_min, alpha_max, lambda_min, lambda_max, u, c, kappa, ck_dtype, rho,
                                        Bt, L, H, R, M, stream);
@@ -975,7 +997,7 @@ extern "C" int fracssm_add_rmsnorm(const void *x, const void *y, const void *wei
 }
 
 // What a mixer does between its projections and out_proj, in bfloat16: parameter prep, scan, (state), epilogue.
-extern "C" int fracssm_prefill_mix(const void *dyn, const void *rw, const void *x_conv, const void *gate, int64_t gate_sl,
+extern "C" int fracssm_prefill_mix(const void *dyn, const void *dyn_bias, const void *rw, const void *x_conv, const void *gate, int64_t gate_sl,
                                    const float *mask, const void *const *params, int params_f32, const float *nums,
                                    const void *u, void *c, void *kappa, int ck_dtype, float *rho, void *h,
                                    float *final_state, float *state, void *y, void *workspace, size_t workspace_bytes,
@@ -986,15 +1008,16 @@ extern "C" int fracssm_prefill_mix(const void *dyn, const void *rw, const void *
   if (state && (Bt * H > 65535 || ceil_div(R, 32) > 65535)) return fail(FRACSSM_ERR_UNSUPPORTED, "prefill_mix: too many rows");
   auto dt = [&](int i) { return (params_f32 >> i) & 1 ? FRACSSM_F32 : FRACSSM_BF16; };
   const int64_t di = H * R;
-  int rc = compute_params_typed(dyn, FRACSSM_BF16, L * 3 * H, 3 * H, rw, FRACSSM_BF16, L * 2 * H * M, 2 * H * M, x_conv,
+  int rc = compute_params_typed(dyn, FRACSSM_BF16, L * 3 * H, 3 * H, dyn_bias, rw, FRACSSM_BF16, L * 2 * H * M, 2 * H * M, x_conv,
                                 FRACSSM_BF16, L * di, di, mask, L, 1, params[0], dt(0), params[3], dt(3), params[1], dt(1),
                                 params[2], dt(2), nums[0], nums[1], nums[2], nums[3], nums[4], nums[5], nums[6], nullptr, c,
                                 kappa, ck_dtype, rho, Bt, L, H, R, M, stream);
   if (rc) return rc;
-  rc = fracssm_frac_scan_fwd(u, FRACSSM_BF16, L * R, R, c, kappa, ck_dtype, L * M, M, L * M, M, rho, L * M, M, nullptr, h,
-                             final_state, FRACSSM_F32, workspace, workspace_bytes, Bt * H, L, R, M, T, 0, stream);
+  bool modes_first = false;
+  rc = frac_scan_route(u, FRACSSM_BF16, L * R, R, c, kappa, ck_dtype, L * M, M, L * M, M, rho, L * M, M, nullptr, h,
+                       final_state, FRACSSM_F32, workspace, workspace_bytes, Bt * H, L, R, M, T, 0, stream, state, &modes_first);
   if (rc) return rc;
-  if (state) {
+  if (state && !modes_first) {   // (the single-pass kernel writes [R, M]: a second form of that store made it 5 % slower)
     state_transpose_kernel<<<dim3((unsigned)ceil_div(M, 32), (unsigned)ceil_div(R, 32), (unsigned)(Bt * H)), 256, 0,
                              (cudaStream_t)stream>>>(final_state, state, (int)R, (int)M);
     rc = check_launch("prefill_mix");

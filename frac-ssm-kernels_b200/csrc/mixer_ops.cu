@@ -75,23 +75,54 @@ __device__ __forceinline__ void unpack4(const uint2 &p, float (&f)[4]) {
   f[3] = __uint_as_float(p.y & 0xFFFF0000u);
 }
 
-// Four channels (8 bytes) per thread, kConvTokens tokens walked with the window in registers, the next
+// What the convolution of the next token needs: tail[b, ch, k] = the last K - 1 inputs times their mask (rounded to
+// the input's type, like the product), zero before the first token.
+struct ConvTail {
+  __nv_bfloat16 *out;   // [B, C, K - 1], or null
+  int K;
+};
+__device__ __forceinline__ void conv_tail(const __nv_bfloat16 *x, int64_t x_sb, int64_t x_sl, const float *mask, int64_t m_sb,
+                                          int64_t m_sl, const ConvTail &tail, int64_t b, int64_t ch, int64_t L, int64_t C) {
+  for (int k = 0; k < tail.K - 1; ++k) {
+    const int64_t l = L - (tail.K - 1) + k;
+    __nv_bfloat16 v = __float2bfloat16_rn(0.f);
+    if (l >= 0) {
+      v = x[b * x_sb + l * x_sl + ch];
+      if (mask)
+        v = __float2bfloat16_rn(__bfloat162float(v) * __bfloat162float(__float2bfloat16_rn(mask[b * m_sb + l * m_sl])));
+    }
+    tail.out[(b * C + ch) * (tail.K - 1) + k] = v;
+  }
+}
+__global__ void __launch_bounds__(128)
+conv_tail_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_sb, int64_t x_sl, const float *__restrict__ mask,
+                 int64_t m_sb, int64_t m_sl, const ConvTail tail, int64_t L, int64_t C) {
+  const int64_t ch = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (ch < C) conv_tail(x, x_sb, x_sl, mask, m_sb, m_sl, tail, blockIdx.y, ch, L, C);
+}
+
+// Four channels (8 bytes) per thread, `tokens` (32 at full size) tokens walked with the window in registers, the next
 // four tokens requested before the current four are worked on; at most 80 registers, so 6 blocks of
 // 128 threads per SM.  At batch 16 x 4096 tokens x 1536 channels: 0.154 ms with 16 tokens per thread and
 // the loads of a group issued right before their use, 0.143 ms with 32 tokens (the three window tokens and
-// the weights are read once per 32), 0.125 ms with the loads one group ahead.
+// the weights are read once per 32), 0.125 ms with the loads one group ahead.  A short sequence is cut into runs of 16
+// or 8 tokens so that the grid covers the GPU (397 tokens: 12.2 -> 7.5 us).  With a tail, the last row of blocks writes it.
 __global__ void __launch_bounds__(128, 6)
 causal_conv4_silu_bf16_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_sb, int64_t x_sl,
                               const float *__restrict__ mask, int64_t m_sb, int64_t m_sl,
                               const void *__restrict__ w, int w_dt, const void *__restrict__ bias,
                               __nv_bfloat16 *__restrict__ y, __nv_bfloat16 *__restrict__ u_heads, int64_t R,
-                              int64_t L, int64_t C) {
+                              int64_t L, int64_t C, int tokens, const ConvTail tail) {
   const int64_t ch = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (ch >= C) return;
+  if (tail.out && blockIdx.y == gridDim.y - 1) {
+    for (int i = 0; i < 4; ++i) conv_tail(x, x_sb, x_sl, mask, m_sb, m_sl, tail, blockIdx.z, ch + i, L, C);
+    return;
+  }
   // the same four values also go to the head-major copy [Bt * H, L, R] (R a multiple of 4)
   __nv_bfloat16 *u_row = nullptr;
   if (u_heads) u_row = u_heads + ((int64_t)blockIdx.z * (C / R) + ch / R) * L * R + ch % R;
-  const int64_t b = blockIdx.z, l0 = (int64_t)blockIdx.y * kConvTokens;
+  const int64_t b = blockIdx.z, l0 = (int64_t)blockIdx.y * tokens;
   float wk[4][4], bv[4], w0[4], w1[4], w2[4];
   if (w_dt == FRACSSM_BF16) {   // 4 channels x 4 taps = 32 contiguous bytes (ch is a multiple of 4)
     const uint4 *wp = reinterpret_cast<const uint4 *>(reinterpret_cast<const __nv_bfloat16 *>(w) + ch * 4);
@@ -127,7 +158,7 @@ causal_conv4_silu_bf16_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_sb,
   in(l0 - 3, w0);
   in(l0 - 2, w1);
   in(l0 - 1, w2);
-  const int64_t l1 = min(l0 + kConvTokens, L);
+  const int64_t l1 = min(l0 + tokens, L);
   // the next four tokens are requested before the current four are worked on
   uint2 nraw[4];
   float nmk[4];
@@ -189,25 +220,6 @@ causal_conv4_silu_bf16_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_sb,
   }
 }
 
-// What the convolution of the next token needs: tail[b, ch, k] = the last K - 1 inputs times their mask (rounded to
-// the input's type, like the product), zero before the first token.
-__global__ void __launch_bounds__(128)
-conv_tail_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_sb, int64_t x_sl, const float *__restrict__ mask,
-                 int64_t m_sb, int64_t m_sl, __nv_bfloat16 *__restrict__ tail, int64_t L, int64_t C, int K) {
-  const int64_t ch = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
-  if (ch >= C) return;
-  for (int k = 0; k < K - 1; ++k) {
-    const int64_t l = L - (K - 1) + k;
-    __nv_bfloat16 v = __float2bfloat16_rn(0.f);
-    if (l >= 0) {
-      v = x[b * x_sb + l * x_sl + ch];
-      if (mask)
-        v = __float2bfloat16_rn(__bfloat162float(v) * __bfloat162float(__float2bfloat16_rn(mask[b * m_sb + l * m_sl])));
-    }
-    tail[(b * C + ch) * (K - 1) + k] = v;
-  }
-}
-
 // One token of the recurrence for every (batch, head): state [M, R] float32 updated in place,
 //   state[m, r] = rho[m] * state[m, r] + kappa[m] * u[r];  out[r] = sum_m c[m] * state[m, r] + u[r] * D[r].
 // One block per (batch, head); thread r-lane strides over R, the modes are walked in the block's
@@ -253,11 +265,11 @@ extern "C" int fracssm_causal_conv_silu(const void *x, int x_dtype, int64_t x_sb
                                         nullptr, 0, Bt, L, C, K, stream);
 }
 
-extern "C" int fracssm_causal_conv_silu_heads(const void *x, int x_dtype, int64_t x_sb, int64_t x_sl,
+static int conv_silu_heads(const void *x, int x_dtype, int64_t x_sb, int64_t x_sl,
                                               const float *mask, int64_t m_sb, int64_t m_sl,
                                               const void *weight, const void *bias, int w_dtype, void *y,
                                               int y_dtype, void *u_heads, int64_t R, int64_t Bt, int64_t L,
-                                              int64_t C, int64_t K, void *stream) {
+                                              int64_t C, int64_t K, void *stream, const fracssm::ConvTail &tail) {
   using namespace fracssm;
   if (u_heads && (R <= 0 || C % R != 0))
     return fail(FRACSSM_ERR_ARG, "causal_conv_silu: the head width must divide the channel count");
@@ -273,16 +285,36 @@ extern "C" int fracssm_causal_conv_silu_heads(const void *x, int x_dtype, int64_
   if (K == 4 && x_dtype == FRACSSM_BF16 && y_dtype == FRACSSM_BF16 && C % 8 == 0 && al16(x) && al16(y) &&
       x_sb % 8 == 0 && x_sl % 8 == 0 && (!u_heads || (R % 8 == 0 && al16(u_heads))) &&
       (w_dtype != FRACSSM_BF16 || al16(weight))) {
-    const dim3 grid((unsigned)ceil_div(C / 4, 128), (unsigned)ceil_div(L, kConvTokens), (unsigned)Bt);
+    int tokens = kConvTokens;
+    while (tokens > 8 && ceil_div(C / 4, 128) * ceil_div(L, tokens) * Bt < 148 * 4) tokens /= 2;
+    if (ceil_div(L, tokens) > 65535) tokens = kConvTokens;
+    const bool same_launch = tail.out && ceil_div(L, tokens) < 65535;
+    const dim3 grid((unsigned)ceil_div(C / 4, 128), (unsigned)(ceil_div(L, tokens) + (same_launch ? 1 : 0)), (unsigned)Bt);
     causal_conv4_silu_bf16_kernel<<<grid, block, 0, (cudaStream_t)stream>>>(
         reinterpret_cast<const __nv_bfloat16 *>(x), x_sb, x_sl, mask, m_sb, m_sl, weight, w_dtype, bias,
-        reinterpret_cast<__nv_bfloat16 *>(y), reinterpret_cast<__nv_bfloat16 *>(u_heads), R, L, C);
+        reinterpret_cast<__nv_bfloat16 *>(y), reinterpret_cast<__nv_bfloat16 *>(u_heads), R, L, C, tokens,
+        same_launch ? tail : ConvTail{nullptr, 0});
+    if (tail.out && !same_launch)
+      conv_tail_kernel<<<dim3((unsigned)ceil_div(C, 128), (unsigned)Bt), 128, 0, (cudaStream_t)stream>>>(
+          reinterpret_cast<const __nv_bfloat16 *>(x), x_sb, x_sl, mask, m_sb, m_sl, tail, L, C);
     return check_launch("causal_conv_silu");
   }
   const dim3 grid((unsigned)ceil_div(C, 128), (unsigned)ceil_div(L, kConvTokens), (unsigned)Bt);
   causal_conv_silu_kernel<<<grid, block, 0, (cudaStream_t)stream>>>(x, x_dtype, x_sb, x_sl, mask, m_sb, m_sl, weight,
                                                                  w_dtype, bias, (int)K, y, y_dtype, u_heads, R, L, C);
+  if (tail.out)
+    conv_tail_kernel<<<dim3((unsigned)ceil_div(C, 128), (unsigned)Bt), 128, 0, (cudaStream_t)stream>>>(
+        reinterpret_cast<const __nv_bfloat16 *>(x), x_sb, x_sl, mask, m_sb, m_sl, tail, L, C);
   return check_launch("causal_conv_silu");
+}
+
+extern "C" int fracssm_causal_conv_silu_heads(const void *x, int x_dtype, int64_t x_sb, int64_t x_sl,
+                                              const float *mask, int64_t m_sb, int64_t m_sl,
+                                              const void *weight, const void *bias, int w_dtype, void *y,
+                                              int y_dtype, void *u_heads, int64_t R, int64_t Bt, int64_t L,
+                                              int64_t C, int64_t K, void *stream) {
+  return conv_silu_heads(x, x_dtype, x_sb, x_sl, mask, m_sb, m_sl, weight, bias, w_dtype, y, y_dtype, u_heads, R, Bt, L, C, K,
+                         stream, fracssm::ConvTail{nullptr, 0});
 }
 
 extern "C" int fracssm_decode_step(const void *u, int u_dtype, const float *c, const float *kappa,
@@ -308,13 +340,8 @@ extern "C" int fracssm_decode_step(const void *u, int u_dtype, const float *c, c
 extern "C" int fracssm_prefill_conv(const void *x, int64_t x_sl, const float *mask, const void *weight, const void *bias,
                                     void *y, void *u_heads, void *tail, int64_t R, int64_t Bt, int64_t L, int64_t C,
                                     int64_t K, void *stream) {
-  using namespace fracssm;
-  const int rc = fracssm_causal_conv_silu_heads(x, FRACSSM_BF16, L * x_sl, x_sl, mask, L, 1, weight, bias, FRACSSM_BF16, y,
-                                                FRACSSM_BF16, u_heads, R, Bt, L, C, K, stream);
-  if (rc || !tail || K < 2 || Bt == 0 || L == 0) return rc;
-  if (Bt > 65535) return fail(FRACSSM_ERR_UNSUPPORTED, "prefill_conv: batch too large for one launch");
-  conv_tail_kernel<<<dim3((unsigned)ceil_div(C, 128), (unsigned)Bt), 128, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const __nv_bfloat16 *>(x), L * x_sl, x_sl, mask, L, 1, reinterpret_cast<__nv_bfloat16 *>(tail), L, C,
-      (int)K);
-  return check_launch("prefill_conv");
+  // bf16 in and out
+  const fracssm::ConvTail next{K >= 2 ? reinterpret_cast<__nv_bfloat16 *>(tail) : nullptr, (int)K};
+  return conv_silu_heads(x, FRACSSM_BF16, L * x_sl, x_sl, mask, L, 1, weight, bias, FRACSSM_BF16, y, FRACSSM_BF16, u_heads, R,
+                         Bt, L, C, K, stream, next);
 }

@@ -49,8 +49,8 @@ struct FewArgs {
   const float *init;           // [B, R, M] or null
   void *h;                     // [B, L, R]
   int h_vec;                   // R a multiple of 4 and h 16-byte aligned: a lane's columns go out in one store
-  void *fin;                   // [B, R, M] or null
-  int fin_dt;
+  void *fin;                   // [B, R, M] (or [B, M, R], by the strides) or null
+  int fin_dt, fin_sr, fin_sm;
   float *states;               // [B][nseg][R][Mp]
   float *decay;                // [B][nseg][Mp]
   int64_t L;
@@ -330,14 +330,14 @@ few_scan_kernel(const FewArgs a) {
 #pragma unroll
     for (int r = 0; r < kCols; ++r) {
       if (r < nr) {
-        const int64_t dst = ((int64_t)b * a.R + col0 + my + r) * a.M;
+        const int64_t dst = (int64_t)b * a.R * a.M + (int64_t)(col0 + my + r) * a.fin_sr;
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
           const int m = kModes * g + 2 * p;
           float lo, hi;
           un2(st[r][p], lo, hi);
-          if (m < a.M) st_f32(a.fin, dst + m, a.fin_dt, lo);
-          if (m + 1 < a.M) st_f32(a.fin, dst + m + 1, a.fin_dt, hi);
+          if (m < a.M) st_f32(a.fin, dst + (int64_t)m * a.fin_sm, a.fin_dt, lo);
+          if (m + 1 < a.M) st_f32(a.fin, dst + (int64_t)(m + 1) * a.fin_sm, a.fin_dt, hi);
         }
       }
     }
@@ -512,7 +512,8 @@ size_t scan_few_workspace_bytes(int64_t B, int64_t L, int64_t R, int64_t M) { re
 int scan_few_launch(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, const void *c, const void *kappa,
                     int ck_dtype, int64_t c_sb, int64_t c_sl, int64_t k_sb, int64_t k_sl, const float *rho,
                     int64_t r_sb, int64_t r_sl, const float *initial_state, void *h, void *final_state,
-                    int final_dtype, void *workspace, int64_t B, int64_t L, int64_t R, int64_t M, void *stream) {
+                    int final_dtype, void *workspace, int64_t B, int64_t L, int64_t R, int64_t M, void *stream,
+                    bool fin_modes_first) {
   const FewPlan p = few_plan(B, L, R, M);
   FewArgs a{};
   const int us = (int)dtype_size(u_dtype), ks = (int)dtype_size(ck_dtype);
@@ -528,6 +529,8 @@ int scan_few_launch(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, cons
   a.h_vec = R % 4 == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0;
   a.fin = final_state;
   a.fin_dt = final_dtype;
+  a.fin_sr = fin_modes_first ? 1 : (int)M;
+  a.fin_sm = fin_modes_first ? (int)R : 1;
   a.states = reinterpret_cast<float *>(workspace);
   a.decay = reinterpret_cast<float *>(reinterpret_cast<char *>(workspace) + align256((size_t)B * p.nseg * R * p.Mp * 4));
   a.L = L;

@@ -101,15 +101,15 @@ def prefill_layers(layers, h, attention_mask, use_cache, classes):
             C.check(lib.fracssm_prefill_conv(p_x, 2 * di, p_mask, conv_w.data_ptr(), 0 if conv_b is None else conv_b.data_ptr(),
                                              p_conv, p_u, tails[i].data_ptr() if use_cache else 0, R, B, L, di, K, stream),
                     "prefill_conv")
-            dyn = F.linear(xg.view(B, L, 2 * di)[:, :, :di], dyn_w, dyn_b)
+            dyn = F.linear(xg[:, :di], dyn_w)      # (its bias is added where it is read)
             rw = F.linear(x_conv, rw_w)
             params = (ctypes.c_void_p * 6)(dt_bias.data_ptr(), read_logit.data_ptr(), write_logit.data_ptr(),
                                            log_tau.data_ptr(), D.data_ptr(), out_norm_w.data_ptr())
             numbers = (ctypes.c_float * 9)(*nums[2:], nums[1])
-            C.check(lib.fracssm_prefill_mix(dyn.data_ptr(), rw.data_ptr(), p_conv, p_x + 2 * di, 2 * di, p_mask, params,
-                                            f32_mask >> 7 & 63, numbers, p_u, p_c, p_k, ck, p_rho, p_h, p_fin,
-                                            states[i].data_ptr() if use_cache else 0, p_y, p_ws, ws.numel(), B, L, H, R, M,
-                                            T, stream), "prefill_mix")
+            C.check(lib.fracssm_prefill_mix(dyn.data_ptr(), 0 if dyn_b is None else dyn_b.data_ptr(), rw.data_ptr(), p_conv,
+                                            p_x + 2 * di, 2 * di, p_mask, params, f32_mask >> 7 & 63, numbers, p_u, p_c,
+                                            p_k, ck, p_rho, p_h, p_fin, states[i].data_ptr() if use_cache else 0, p_y,
+                                            p_ws, ws.numel(), B, L, H, R, M, T, stream), "prefill_mix")
             out = F.linear(y, out_w)
         h = (res + out).view(B, L, d)
     return h, tuple(zip(states, tails)) if use_cache else None

@@ -360,3 +360,30 @@ def test_frac_compute_scan_params_does_not_synchronise():
         finally:
             torch.cuda.set_sync_debug_mode("default")
     assert u.shape == (2 * H, 40, R) and rho.dtype == torch.float32 and torch.isfinite(c).all()
+
+
+@pytest.mark.parametrize("M", [8, 16, 32, 64, 128])
+@pytest.mark.parametrize("B,L", [(1, 1), (2, 31), (1, 33), (3, 130), (1, 4100)])
+def test_params_with_whole_groups_of_modes_match_the_general_kernel(M, B, L):
+    """The lane-group kernel (8 modes a lane) against the warp-per-token kernel, which an odd stride of the residual
+    rows selects: edges of a warp's tokens, both counts of tokens per warp."""
+    from frac_ssm_b200.layers.compute_params import compute_params_from_projections
+    H, R = 3, 16
+    g = torch.Generator().manual_seed(M + L)
+    dyn = torch.randn(B, L, 3 * H, generator=g).bfloat16().cuda()
+    wide = torch.randn(B, L, 2 * H * M + 1, generator=g).bfloat16().cuda()
+    x = torch.randn(B, L, H * R, generator=g).bfloat16().cuda()
+    mask = (torch.rand(B, L, generator=g) < 0.8).long().cuda()
+    tail = (mask, torch.randn(H, generator=g).cuda(), -2.0, 0.3, torch.linspace(0, 11, M).cuda(), H, R, M, 1.0, 1e-4, 1.0,
+            0.2, 0.95, 0.25, 4.0)
+    odd = wide[..., 1:]
+    for coeff in (torch.float32, torch.bfloat16):
+        got = compute_params_from_projections(dyn, odd.contiguous(), x, *tail, coeff_dtype=coeff)
+        ref = compute_params_from_projections(dyn, odd, x, *tail, coeff_dtype=coeff)
+        assert torch.equal(got[0], ref[0])
+        # c: sums of M exponentials in another order, one rounding.  rho: the exponent's factor is a product here and a
+        # quotient there, two ulps (2.4e-7) of a value below 1; kappa = (1 - rho) w inherits that as an absolute error
+        # times w <= 1, however small 1 - rho is.
+        for a, b in zip(got[1:], ref[1:]):
+            tol = 2 ** -7 if a.dtype == torch.bfloat16 else 2e-6      # bfloat16: neighbours, if the halfway point lies between
+            torch.testing.assert_close(a.float(), b.float(), rtol=tol, atol=2.4e-7)
