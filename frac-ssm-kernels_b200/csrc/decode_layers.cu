@@ -1,17 +1,20 @@
 // One decode token through all layers of the model, bfloat16, up to 64 sequences: four kernels per layer.
 //
-//   decode_linear_kernel<.., kIn>    RMSNorm of the hidden state -> in_proj -> x | gate; the rows of x also take
+//   decode_linear_kernel<.., kIn>    in_proj of the normalised hidden state -> x | gate; the rows of x also take
 //                                    the causal convolution step + SiLU (a channel needs its own history only)
 //   decode_linear_kernel<.., kProj>  rw_proj of x_conv and dyn_proj of x
 //   decode_mix_kernel                the scan parameters of a (sequence, head), its state one token further,
 //                                    readout, D skip, gate
-//   decode_linear_kernel<.., kOut>   gated RMSNorm's normalisation -> out_proj -> + hidden state
+//   decode_linear_kernel<.., kOut>   out_proj of the normalised result -> + hidden state
+// and decode_first_kernel once, which does for the embedding what kOut does for the next layer's norm.
 //
 // What bounds a step: reading the weights (27 MB a layer at hidden 768, 128 modes) and, from some 16 sequences
 // on, the float32 state in and out; at one sequence the length of the kernel chain.  As separate library and
 // elementwise calls (about 30 launches a layer, most of them from Python) a step of 24 layers was bound by the
 // host.  Hence
-//   * elementwise stages sit in the prologue or epilogue of the product that reads or writes their rows;
+//   * elementwise stages sit in the epilogue of the product that writes their rows.  A norm is split: whoever writes
+//     the row also writes it times the norm's weight and the sums of squares of its part of the row, and the product
+//     that reads it scales its results by 1 / rms, so no block has to see a whole row before it can start;
 //   * the products stream the weights once, straight into the fragments of mma.sync (16 weight rows x 16 of the
 //     contraction x 8 sequences): with at most 64 sequences they are far below the tensor-core ridge, and a lane
 //     reads 8 consecutive weights of a row because the contraction order is free as long as both operands share
@@ -33,7 +36,7 @@ constexpr int kThreads = 256, kWarps = 8, kTileRows = 16, kMaxSeq = 64;
 constexpr int kPre = 6;              // 32-wide steps of the contraction a warp holds weights for
 constexpr int kRedStride = 20;       // floats per sequence in the exchange buffer: 16 rows, bank-conflict free
 constexpr int kPassTiles = 2;        // groups of 8 sequences exchanged at a time
-constexpr int kMaxHidden = 2048;     // row length of the RMSNorm prologue at one or two sequences
+constexpr int kMaxHidden = 8192;     // longest hidden state
 enum { kIn = 0, kProj = 1, kOut = 2 };
 
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -50,25 +53,9 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-__device__ __forceinline__ const void *param_at(const void *p, int64_t i, int dt) {
-  return reinterpret_cast<const char *>(p) + i * (dt == FRACSSM_F32 ? 4 : 2);
-}
 __device__ __forceinline__ float bf(uint32_t lo16) { return __uint_as_float(lo16 << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 __device__ __forceinline__ float round_bf(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-__device__ __forceinline__ void unpack8(const uint4 &p, float (&f)[8]) {
-  const uint32_t w[4] = {p.x, p.y, p.z, p.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    f[2 * i] = bf(w[i]);
-    f[2 * i + 1] = bf_hi(w[i]);
-  }
-}
-__device__ __forceinline__ void ld_param8(const void *p, int64_t i, int dt, float (&f)[8]) {
-#pragma unroll
-  for (int e = 0; e < 8; ++e) f[e] = ld_f32(p, i + e, dt);
-}
 __device__ __forceinline__ float sum_warp(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -79,10 +66,10 @@ __device__ __forceinline__ float sigmoid_(float x) { return 1.f / (1.f + __expf(
 struct LinArgs {
   const __nv_bfloat16 *w, *w2;   // [n][K]; kProj: w = rw_proj, w2 = dyn_proj
   int n, n2, K, B, blocks2;      // kProj: the first blocks2 blocks take one tile of w2 each
-  const __nv_bfloat16 *act, *act2;   // kIn: hidden state; kProj: x_conv and x
-  const float *vals, *ss;        // kOut: gated values [B][K] and their partial sums of squares [B][nss]
+  const __nv_bfloat16 *act, *act2;   // [B][K]; kProj: x_conv and x; else the row times the norm's weight
+  const float *ss;               // kIn, kOut: partial sums of squares of the rows [B][nss]
   int nss;
-  const void *norm_w; int norm_dt; float eps;
+  float eps;
   // kIn outputs and the convolution
   __nv_bfloat16 *x, *gate, *x_conv, *new_conv;
   const __nv_bfloat16 *old_conv, *conv_w, *conv_b;
@@ -90,10 +77,18 @@ struct LinArgs {
   // kProj outputs
   float *out, *out2;
   const __nv_bfloat16 *bias2;
-  // kOut
+  // kOut: dst = res + result, and for the next layer's norm (weight next_w or null) dst * next_w and a sum per tile
   const __nv_bfloat16 *res;
-  __nv_bfloat16 *dst;
+  __nv_bfloat16 *dst, *dst_w;
+  float *dst_ss;
+  const void *next_w; int next_dt;
 };
+
+// the activations of this thread's seat in the fragment: 8 consecutive values of sequence `seq`
+__device__ __forceinline__ void copy_async16(uint32_t dst, const void *src, bool on) {
+  const int n = on ? 16 : 0;   // (0: the 16 bytes are zeros, nothing is read)
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
 
 // NT groups of 8 sequences.
 template <int NT, int KIND>
@@ -103,7 +98,7 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 1) decode_linear_kerne
   grid_dep_launch();
   // rows of the activation tile lie 64 mod 128 bytes apart: a quarter-warp's 16-byte reads then cover all banks
   const uint32_t stride = a.K * 2 + ((a.K * 2) % 128 == 0 ? 64 : 128);
-  float *red = reinterpret_cast<float *>(lin_smem + 8 * NT * stride);
+  float *red = reinterpret_cast<float *>(lin_smem + (NT == 1 ? 0 : 8 * NT * stride));
   const bool second = KIND == kProj && (int)blockIdx.x < a.blocks2;
   const __nv_bfloat16 *W = second ? a.w2 : a.w;
   const int N = second ? a.n2 : a.n;
@@ -126,12 +121,10 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 1) decode_linear_kerne
     }
   };
   request(tile0, k_lo);
-  if (KIND != kProj)   // a layer's norm weight is not in L2 yet
-    for (int ch = tid; ch < a.K / 8; ch += kThreads) prefetch_l2(param_at(a.norm_w, 8 * ch, a.norm_dt));
   // what the epilogue of this thread's first value needs and no kernel of this call writes
   const int e_row = tid & 15, e_seq = tid >> 4;
   uint2 cw = make_uint2(0, 0);
-  float cb = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f;
+  float cb = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f, nw = 0.f;
   auto conv_inputs = [&](int n, int b) {
     cw = *reinterpret_cast<const uint2 *>(a.conv_w + (int64_t)n * 4);
     cb = a.conv_b ? __bfloat162float(a.conv_b[n]) : 0.f;
@@ -141,110 +134,74 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 1) decode_linear_kerne
       c0 = __bfloat162float(p[0]); c1 = __bfloat162float(p[1]); c2 = __bfloat162float(p[2]);
     }
   };
-  if (KIND == kIn && NT == 1 && e_seq < a.B && tile0 * kTileRows + e_row < a.di) conv_inputs(tile0 * kTileRows + e_row, e_seq);
+  const int e_n = tile0 * kTileRows + e_row;
+  if (KIND == kIn && NT == 1 && e_seq < a.B && e_n < a.di) conv_inputs(e_n, e_seq);
+  if (KIND == kOut && a.next_w && e_n < N) nw = ld_f32(a.next_w, e_n, a.next_dt);
 
   grid_dep_wait();
 
-  // ---- the activation tile, bf16, rows beyond B zero
-  const int chunks = a.K / 8;
-  auto put = [&](int b, int ch, const float (&v)[8]) {
-    *reinterpret_cast<uint4 *>(lin_smem + b * stride + ch * 16) =
-        make_uint4(tile::pack2(v[0], v[1]), tile::pack2(v[2], v[3]), tile::pack2(v[4], v[5]), tile::pack2(v[6], v[7]));
-  };
-  for (int i = a.B * chunks + tid; i < 8 * NT * chunks; i += kThreads)
-    *reinterpret_cast<uint4 *>(lin_smem + (i / chunks) * stride + (i % chunks) * 16) = make_uint4(0, 0, 0, 0);
-  if (KIND == kProj) {
-    const __nv_bfloat16 *act = second ? a.act2 : a.act;
-#pragma unroll 4
-    for (int i = tid; i < a.B * chunks; i += kThreads)
-      *reinterpret_cast<uint4 *>(lin_smem + (i / chunks) * stride + (i % chunks) * 16) =
-          __ldcg(reinterpret_cast<const uint4 *>(act) + i);
-  } else if (KIND == kIn) {
-    if (NT == 1 && a.B <= 2) {   // the whole block on one row: one chunk per thread (K <= 2048)
-      for (int b = 0; b < a.B; ++b) {
-        float v[8], nw[8], ss = 0.f;
-        if (tid < chunks) {
-          unpack8(__ldcg(reinterpret_cast<const uint4 *>(a.act + (int64_t)b * a.K) + tid), v);
-          ld_param8(a.norm_w, 8 * tid, a.norm_dt, nw);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
-        }
-        ss = sum_warp(ss);
-        if (lane == 0) red[8 * b + w] = ss;
-        __syncthreads();
-        float total = 0.f;
-#pragma unroll
-        for (int i = 0; i < kWarps; ++i) total += red[8 * b + i];
-        const float rs = rsqrtf(total / (float)a.K + a.eps);
-        if (tid < chunks) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) v[e] = v[e] * rs * nw[e];
-          put(b, tid, v);
-        }
+  // ---- activations (bf16, zeros beyond B): each warp its own share of the contraction.  Up to 8 sequences straight
+  // into the fragments; beyond, every tile reads them again, so they go to shared memory once.
+  const __nv_bfloat16 *act = second ? a.act2 : a.act;
+  const uint32_t act_s = (uint32_t)__cvta_generic_to_shared(lin_smem);
+  if (NT > 1) {
+    const int pieces = (k_hi - k_lo) * 4;     // 16-byte pieces of this warp's share of a row
+    for (int b = 0; b < 8 * NT; ++b)
+      for (int i = lane; i < pieces; i += 32) {
+        const int at = 4 * k_lo + i;
+        copy_async16(act_s + b * stride + at * 16, act + (int64_t)(b < a.B ? b : 0) * a.K + at * 8, b < a.B);
       }
-    } else {                     // a warp per row, the raw row kept in the tile between the two passes
-      for (int b = w; b < a.B; b += kWarps) {
-        float ss = 0.f;
-        for (int ch = lane; ch < chunks; ch += 32) {
-          const uint4 raw = __ldcg(reinterpret_cast<const uint4 *>(a.act + (int64_t)b * a.K) + ch);
-          float v[8];
-          unpack8(raw, v);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  // 1 / rms of this thread's sequences: 16 threads share one
+  constexpr int kPasses = (NT + kPassTiles - 1) / kPassTiles;
+  float rs[kPasses];
+  if (KIND != kProj) {
 #pragma unroll
-          for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
-          *reinterpret_cast<uint4 *>(lin_smem + b * stride + ch * 16) = raw;
-        }
-        const float rs = rsqrtf(sum_warp(ss) / (float)a.K + a.eps);
-        for (int ch = lane; ch < chunks; ch += 32) {
-          float v[8], nw[8];
-          unpack8(*reinterpret_cast<const uint4 *>(lin_smem + b * stride + ch * 16), v);
-          ld_param8(a.norm_w, 8 * ch, a.norm_dt, nw);
+    for (int p = 0; p < kPasses; ++p) {
+      const int b = 8 * kPassTiles * p + e_seq;
+      float t = 0.f;
+      if (b < a.B)
+        for (int i = e_row; i < a.nss; i += 16) t += __ldcg(a.ss + (int64_t)b * a.nss + i);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) v[e] = v[e] * rs * nw[e];
-          put(b, ch, v);
-        }
-      }
-    }
-  } else {
-    for (int b = w; b < a.B; b += kWarps) {
-      float ss = 0.f;
-      for (int i = lane; i < a.nss; i += 32) ss += __ldcg(a.ss + (int64_t)b * a.nss + i);
-      ss = sum_warp(ss);
-      if (lane == 0) red[b] = rsqrtf(ss / (float)a.K + a.eps);
-    }
-    __syncthreads();
-#pragma unroll 2
-    for (int i = tid; i < a.B * chunks; i += kThreads) {
-      const int b = i / chunks, ch = i - b * chunks;
-      const float4 lo = __ldcg(reinterpret_cast<const float4 *>(a.vals) + 2 * (int64_t)i);
-      const float4 hi = __ldcg(reinterpret_cast<const float4 *>(a.vals) + 2 * (int64_t)i + 1);
-      const float rs = red[b];
-      float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w}, nw[8];
-      ld_param8(a.norm_w, 8 * ch, a.norm_dt, nw);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) v[e] = v[e] * rs * nw[e];
-      put(b, ch, v);
+      for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      rs[p] = rsqrtf(t / (float)a.K + a.eps);
     }
   }
-  __syncthreads();
+  if (NT > 1) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+  }
 
   for (int tile = tile0; tile < tiles; tile += tile_step) {
     float acc[NT][4];
 #pragma unroll
     for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
     for (int k0 = k_lo; k0 < k_hi; k0 += kPre) {
-      if (tile != tile0 || k0 != k_lo) request(tile, k0);
+      if (k0 != k_lo) request(tile, k0);
+      uint4 xs[NT == 1 ? kPre : 1];
+      if (NT == 1) {
+#pragma unroll
+        for (int i = 0; i < kPre; ++i) {
+          xs[i] = make_uint4(0, 0, 0, 0);
+          if (k0 + i < k_hi && g < a.B)
+            xs[i] = __ldcg(reinterpret_cast<const uint4 *>(act + (int64_t)g * a.K + (k0 + i) * 32 + 8 * tig));
+        }
+      }
 #pragma unroll
       for (int i = 0; i < kPre; ++i) {
         if (k0 + i < k_hi) {
 #pragma unroll
           for (int t = 0; t < NT; ++t) {
-            const uint4 x = *reinterpret_cast<const uint4 *>(lin_smem + (8 * t + g) * stride + (k0 + i) * 64 + 16 * tig);
+            const uint4 x = NT == 1 ? xs[NT == 1 ? i : 0]
+                                    : *reinterpret_cast<const uint4 *>(lin_smem + (8 * t + g) * stride + (k0 + i) * 64 + 16 * tig);
             mma_bf16(acc[t], wr[i][0].x, wr[i][1].x, wr[i][0].y, wr[i][1].y, x.x, x.y);
             mma_bf16(acc[t], wr[i][0].z, wr[i][1].z, wr[i][0].w, wr[i][1].w, x.z, x.w);
           }
         }
       }
     }
+    if (tile + tile_step < tiles) request(tile + tile_step, k_lo);   // on their way during the epilogue
     // ---- the warps' shares of the contraction are added, a value per thread
 #pragma unroll
     for (int p = 0; p < NT; p += kPassTiles) {
@@ -258,10 +215,13 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 1) decode_linear_kerne
       }
       __syncthreads();
       const int b = 8 * p + e_seq, n = tile * kTileRows + e_row;
-      if (e_seq < 8 * (NT - p) && b < a.B && n < N) {
+      const bool on = e_seq < 8 * (NT - p) && b < a.B && n < N;
+      float sq = 0.f;
+      if (on) {
         float v = 0.f;
 #pragma unroll
         for (int i = 0; i < kWarps; ++i) v += red[(i * 8 * kPassTiles + e_seq) * kRedStride + e_row];
+        if (KIND != kProj) v *= rs[p / kPassTiles];
         if (KIND == kIn) {
           const __nv_bfloat16 xb = __float2bfloat16_rn(v);
           if (n < a.di) {
@@ -289,11 +249,46 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 1) decode_linear_kerne
           else a.out[(int64_t)b * N + n] = v;
         } else {
           const int64_t at = (int64_t)b * N + n;
-          a.dst[at] = __float2bfloat16_rn(__bfloat162float(__ldcg(a.res + at)) + round_bf(v));
+          const __nv_bfloat16 hb = __float2bfloat16_rn(__bfloat162float(__ldcg(a.res + at)) + round_bf(v));
+          a.dst[at] = hb;
+          if (a.next_w) {
+            if (tile != tile0) nw = ld_f32(a.next_w, n, a.next_dt);
+            const float hv = __bfloat162float(hb);
+            a.dst_w[at] = __float2bfloat16_rn(hv * nw);
+            sq = hv * hv;
+          }
         }
+      }
+      if (KIND == kOut && a.next_w) {   // the tile's 16 rows of a sequence lie in 16 neighbouring lanes
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        if (on && e_row == 0) a.dst_ss[(int64_t)b * tiles + tile] = sq;
       }
       __syncthreads();
     }
+  }
+}
+
+// The embedding times the first norm's weight, and its sums of squares (one part per row).
+__global__ void __launch_bounds__(kThreads)
+decode_first_kernel(const __nv_bfloat16 *h, const void *w, int w_dt, __nv_bfloat16 *h_w, float *ss, int d) {
+  __shared__ float red[kWarps];
+  const int64_t b = blockIdx.x;
+  grid_dep_launch();
+  float sq = 0.f;
+  for (int i = threadIdx.x; i < d; i += kThreads) {
+    const float v = __bfloat162float(h[b * d + i]);
+    h_w[b * d + i] = __float2bfloat16_rn(v * ld_f32(w, i, w_dt));
+    sq = fmaf(v, v, sq);
+  }
+  sq = sum_warp(sq);
+  if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = sq;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < kWarps; ++i) t += red[i];
+    ss[b] = t;
   }
 }
 
@@ -302,55 +297,76 @@ struct MixArgs {
   const __nv_bfloat16 *x_conv, *gate;  // [B][H R]
   const float *old_state;              // [B][H][M][R] or null (zeros)
   float *new_state;                    // or null
-  const void *dt_bias, *read_logit, *write_logit, *log_tau, *D;
-  int dt_bias_dt, read_dt, write_dt, log_tau_dt, D_dt;
+  const void *dt_bias, *read_logit, *write_logit, *log_tau, *D, *norm_w;
+  int dt_bias_dt, read_dt, write_dt, log_tau_dt, D_dt, norm_dt;
   float inv_read_temp, dt_min, dt_max, a_min, a_max, l_min, l_max, gate_bias;
-  float *vals, *ss;                    // [B][H R], [B][H splits]
+  __nv_bfloat16 *vals;                 // [B][H R]: the gated result times the output norm's weight
+  float *ss;                           // [B][H splits]: sums of squares of the gated result
   int H, R, M, splits;
 };
 
-constexpr int kMixPre = 4;             // float4 pieces of the old state a thread requests ahead
+constexpr int kMixPre = 8;             // float4 pieces of the old state a thread requests ahead
 
 // One block per (sequence, head, share of the head's columns).
 __global__ void __launch_bounds__(kThreads) decode_mix_kernel(const MixArgs a) {
   extern __shared__ __align__(16) float mix_smem[];
   const int M = a.M, H = a.H, R = a.R, Mr = (M + 3) & ~3;
-  float *cc = mix_smem, *kk = cc + Mr, *rr = kk + Mr, *part = rr + Mr;   // part [groups][cols], 16-byte aligned
-  __shared__ float red[2][4][2];
+  float *cc = mix_smem, *kk = cc + Mr, *rr = kk + Mr, *part = rr + Mr;   // part [rows][cols], 16-byte aligned
+  __shared__ float red[2][4][2], sums[kWarps];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int h = blockIdx.x / a.splits, sp = blockIdx.x % a.splits, b = blockIdx.y;
   const int cols = R / a.splits, quads = cols / 4, groups = kThreads / quads;
   const int q = tid % quads, mg = tid / quads;
   const bool on = mg < groups;
+  // a warp holds several mode groups of the same columns when quads is a power of two: they are added by shuffles
+  const bool fold = quads <= 32 && (quads & (quads - 1)) == 0;
   grid_dep_launch();
+  // ---- requested before the wait: the old state, the parameters
   const int64_t sbase = ((int64_t)b * H + h) * M * R + sp * cols + 4 * q;
   float4 pre[kMixPre];
 #pragma unroll
   for (int i = 0; i < kMixPre; ++i) {
     const int m = mg + i * groups;
     pre[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (on && m < M && a.old_state) pre[i] = *reinterpret_cast<const float4 *>(a.old_state + sbase + (int64_t)m * R);
+    if (on && m < M && a.old_state) pre[i] = __ldcs(reinterpret_cast<const float4 *>(a.old_state + sbase + (int64_t)m * R));
   }
+  const int side = tid >> 7, t128 = tid & 127;   // threads 0..127: the read side of the parameters, 128..255 the write side
   const float read_gate = sigmoid_(ld_f32(a.read_logit, 0, a.read_dt)), write_gate = sigmoid_(ld_f32(a.write_logit, 0, a.write_dt));
   const float dtb = ld_f32(a.dt_bias, h, a.dt_bias_dt);
-  for (int m = 8 * tid; m < M; m += 8 * kThreads) prefetch_l2(param_at(a.log_tau, m, a.log_tau_dt));
-  if (8 * tid < cols) prefetch_l2(param_at(a.D, (int64_t)h * R + sp * cols + 8 * tid, a.D_dt));
+  const float lt0 = t128 < M ? ld_f32(a.log_tau, t128, a.log_tau_dt) : 0.f;
+  const float tau0 = fmaxf(expf(lt0), 1e-6f);
+  float Dv = 0.f, nwv = 0.f;
+  if (tid < cols) {
+    Dv = ld_f32(a.D, (int64_t)h * R + sp * cols + tid, a.D_dt);
+    nwv = ld_f32(a.norm_w, (int64_t)h * R + sp * cols + tid, a.norm_dt);
+  }
   grid_dep_wait();
 
-  // ---- scan parameters (the formulas of compute_params_kernel): threads 0..127 the read side, 128..255 the write side
-  const float d0 = __ldcg(a.dyn + (int64_t)b * 3 * H + h) + dtb;
+  // ---- scan parameters (the formulas of compute_params_kernel)
+  const float *dyn = a.dyn + (int64_t)b * 3 * H + h;
+  const float *res = a.rw + (int64_t)b * 2 * H * M + (int64_t)side * H * M + (int64_t)h * M;
+  const float r0 = t128 < M ? __ldcg(res + t128) : 0.f;
+  const float y0 = __ldcg(dyn), y1 = __ldcg(dyn + H), y2 = __ldcg(dyn + 2 * H);
+  const int64_t col = (int64_t)b * H * R + (int64_t)h * R + sp * cols;
+  uint2 uw = make_uint2(0, 0);
+  if (on) uw = __ldcg(reinterpret_cast<const uint2 *>(a.x_conv + col + 4 * q));
+  float uc = 0.f, gc = 0.f;
+  if (tid < cols) {
+    uc = __bfloat162float(__ldcg(a.x_conv + col + tid));
+    gc = __bfloat162float(__ldcg(a.gate + col + tid));
+  }
+  const float d0 = y0 + dtb;
   float dt = d0 > 20.f ? d0 : log1pf(expf(d0));
   dt = fminf(fmaxf(dt, a.dt_min), a.dt_max);
-  const float alpha = a.a_min + sigmoid_(__ldcg(a.dyn + (int64_t)b * 3 * H + H + h)) * (a.a_max - a.a_min);
-  const float lam = a.l_min + sigmoid_(__ldcg(a.dyn + (int64_t)b * 3 * H + 2 * H + h)) * (a.l_max - a.l_min);
+  const float alpha = a.a_min + sigmoid_(y1) * (a.a_max - a.a_min);
+  const float lam = a.l_min + sigmoid_(y2) * (a.l_max - a.l_min);
   const float rate = powf(fmaxf(lam, 1e-4f), 1.f / fmaxf(alpha, 1e-4f));
-  const int side = tid >> 7, t128 = tid & 127;
-  const float *res = a.rw + (int64_t)b * 2 * H * M + (int64_t)side * H * M + (int64_t)h * M;
   float *dst = side ? kk : cc;
   float mx = -INFINITY;
   for (int m = t128; m < M; m += 128) {
-    const float prior = -alpha * ld_f32(a.log_tau, m, a.log_tau_dt);
-    const float l = side ? prior + write_gate * __ldcg(res + m) : (prior + read_gate * __ldcg(res + m)) * a.inv_read_temp;
+    const float prior = -alpha * (m == t128 ? lt0 : ld_f32(a.log_tau, m, a.log_tau_dt));
+    const float rv = m == t128 ? r0 : __ldcg(res + m);
+    const float l = side ? prior + write_gate * rv : (prior + read_gate * rv) * a.inv_read_temp;
     dst[m] = l;
     mx = fmaxf(mx, l);
   }
@@ -371,7 +387,7 @@ __global__ void __launch_bounds__(kThreads) decode_mix_kernel(const MixArgs a) {
   const float inv = 1.f / (red[side][0][1] + red[side][1][1] + red[side][2][1] + red[side][3][1]);
   for (int m = t128; m < M; m += 128) {
     if (side) {
-      float rho = expf(-dt * (rate / fmaxf(expf(ld_f32(a.log_tau, m, a.log_tau_dt)), 1e-6f)));
+      float rho = expf(-dt * (rate / (m == t128 ? tau0 : fmaxf(expf(ld_f32(a.log_tau, m, a.log_tau_dt)), 1e-6f))));
       rho = fminf(fmaxf(rho, 1e-6f), 1.f - 1e-6f);
       kk[m] = (1.f - rho) * (kk[m] * inv);
       rr[m] = rho;
@@ -382,10 +398,8 @@ __global__ void __launch_bounds__(kThreads) decode_mix_kernel(const MixArgs a) {
   __syncthreads();
 
   // ---- the state one token further, and the readout
-  const int64_t col = (int64_t)b * H * R + (int64_t)h * R + sp * cols;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   if (on) {
-    const uint2 uw = __ldcg(reinterpret_cast<const uint2 *>(a.x_conv + col + 4 * q));
     const float u0 = bf(uw.x), u1 = bf_hi(uw.x), u2 = bf(uw.y), u3 = bf_hi(uw.y);
     auto step = [&](int m, float4 s) {
       const float rho = rr[m], kap = kk[m], c = cc[m];
@@ -393,7 +407,7 @@ __global__ void __launch_bounds__(kThreads) decode_mix_kernel(const MixArgs a) {
       s.y = fmaf(rho, s.y, kap * u1);
       s.z = fmaf(rho, s.z, kap * u2);
       s.w = fmaf(rho, s.w, kap * u3);
-      if (a.new_state) *reinterpret_cast<float4 *>(a.new_state + sbase + (int64_t)m * R) = s;
+      if (a.new_state) __stcs(reinterpret_cast<float4 *>(a.new_state + sbase + (int64_t)m * R), s);
       acc.x = fmaf(c, s.x, acc.x);
       acc.y = fmaf(c, s.y, acc.y);
       acc.z = fmaf(c, s.z, acc.z);
@@ -404,29 +418,45 @@ __global__ void __launch_bounds__(kThreads) decode_mix_kernel(const MixArgs a) {
       if (mg + i * groups < M) step(mg + i * groups, pre[i]);
 #pragma unroll 4
     for (int m = mg + kMixPre * groups; m < M; m += groups)
-      step(m, a.old_state ? *reinterpret_cast<const float4 *>(a.old_state + sbase + (int64_t)m * R) : make_float4(0.f, 0.f, 0.f, 0.f));
+      step(m, a.old_state ? __ldcs(reinterpret_cast<const float4 *>(a.old_state + sbase + (int64_t)m * R)) : make_float4(0.f, 0.f, 0.f, 0.f));
+  }
+  if (fold) {
+    for (int o = quads; o < 32; o *= 2) {
+      acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+      acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+      acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
+      acc.w += __shfl_xor_sync(0xffffffffu, acc.w, o);
+    }
+    if (lane < quads) *reinterpret_cast<float4 *>(part + w * cols + 4 * q) = acc;
+  } else if (on) {
     *reinterpret_cast<float4 *>(part + mg * cols + 4 * q) = acc;
   }
   __syncthreads();
+  const int rows = fold ? kWarps : groups;
   float sq = 0.f;
   for (int c = tid; c < cols; c += kThreads) {
+    if (c != tid) {   // (heads wider than the block)
+      Dv = ld_f32(a.D, (int64_t)h * R + sp * cols + c, a.D_dt);
+      nwv = ld_f32(a.norm_w, (int64_t)h * R + sp * cols + c, a.norm_dt);
+      uc = __bfloat162float(__ldcg(a.x_conv + col + c));
+      gc = __bfloat162float(__ldcg(a.gate + col + c));
+    }
     float o = 0.f;
-    for (int i = 0; i < groups; ++i) o += part[i * cols + c];
-    const float u = __bfloat162float(__ldcg(a.x_conv + col + c));
-    const float mixed = round_bf(o + u * ld_f32(a.D, (int64_t)h * R + sp * cols + c, a.D_dt));
-    const float z = round_bf(__bfloat162float(__ldcg(a.gate + col + c)) + a.gate_bias);
+#pragma unroll 8
+    for (int i = 0; i < rows; ++i) o += part[i * cols + c];
+    const float mixed = round_bf(o + uc * Dv);
+    const float z = round_bf(gc + a.gate_bias);
     const float v = mixed * (z * sigmoid_(z));
-    a.vals[col + c] = v;
+    a.vals[col + c] = __float2bfloat16_rn(v * nwv);
     sq = fmaf(v, v, sq);
   }
   sq = sum_warp(sq);
-  __syncthreads();
-  if (lane == 0) part[w] = sq;
+  if (lane == 0) sums[w] = sq;
   __syncthreads();
   if (tid == 0) {
     float t = 0.f;
 #pragma unroll
-    for (int i = 0; i < kWarps; ++i) t += part[i];
+    for (int i = 0; i < kWarps; ++i) t += sums[i];
     a.ss[(int64_t)b * H * a.splits + h * a.splits + sp] = t;
   }
 }
@@ -449,7 +479,7 @@ cudaError_t launch_dep(void (*kernel)(const Arg), dim3 grid, size_t smem, cudaSt
 size_t lin_smem_bytes(int nt, int64_t K) {
   const size_t stride = K * 2 + ((K * 2) % 128 == 0 ? 64 : 128);
   const size_t red = (size_t)kWarps * 8 * kPassTiles * kRedStride * 4;
-  return 8 * nt * stride + red;
+  return (nt == 1 ? 0 : 8 * nt * stride) + red;
 }
 size_t mix_smem_bytes(int64_t M) { return (size_t)(3 * ((M + 3) / 4 * 4) + kThreads * 4) * 4; }
 
@@ -472,7 +502,7 @@ int mix_splits(int64_t B, int64_t H, int64_t R) {
 }
 
 struct Scratch {
-  size_t x, gate, x_conv, rw, dyn, vals, ss, hid, bytes;
+  size_t x, gate, x_conv, rw, dyn, vals, ss, hid, hid_w, hid_ss, bytes;
 };
 Scratch scratch_layout(int64_t B, int64_t d, int64_t di, int64_t H, int64_t M) {
   Scratch s{};
@@ -483,9 +513,11 @@ Scratch scratch_layout(int64_t B, int64_t d, int64_t di, int64_t H, int64_t M) {
   s.x_conv = take((size_t)B * di * 2);
   s.rw = take((size_t)B * 2 * H * M * 4);
   s.dyn = take((size_t)B * 3 * H * 4);
-  s.vals = take((size_t)B * di * 4);
+  s.vals = take((size_t)B * di * 2);
   s.ss = take((size_t)B * H * 4 * 4);
   s.hid = take(2 * align256((size_t)B * d * 2));
+  s.hid_w = take((size_t)B * d * 2);
+  s.hid_ss = take((size_t)B * ((d + kTileRows - 1) / kTileRows) * 4);
   s.bytes = off;
   return s;
 }
@@ -522,10 +554,15 @@ int run_layers(const uint64_t *ptrs, const float *nums, int64_t layers, const vo
   auto blocks = [&](int64_t tiles, size_t smem) -> int64_t {
     if (NT == 1) return tiles;
     const int64_t most = 148 * (smem <= 110 * 1024 ? 2 : 1);
-    return tiles < most ? tiles : most;
+    return ceil_div(tiles, ceil_div(tiles, most));
   };
   cudaError_t e = cudaSuccess;
   const __nv_bfloat16 *hid = reinterpret_cast<const __nv_bfloat16 *>(hidden_in);
+  __nv_bfloat16 *hid_w = reinterpret_cast<__nv_bfloat16 *>(at(s.hid_w));
+  float *hid_ss = reinterpret_cast<float *>(at(s.hid_ss));
+  decode_first_kernel<<<(unsigned)B, kThreads, 0, st>>>(hid, reinterpret_cast<const void *>(ptrs[kNormW]),
+                                                       ptrs[kF32Mask] & 1 ? FRACSSM_F32 : FRACSSM_BF16, hid_w, hid_ss, (int)d);
+  e = cudaGetLastError();
   for (int64_t l = 0; l < layers && e == cudaSuccess; ++l) {
     const uint64_t *p = ptrs + l * kLayerPtrs;
     const float *f = nums + l * kLayerNums;
@@ -537,15 +574,14 @@ int run_layers(const uint64_t *ptrs, const float *nums, int64_t layers, const vo
                                           : reinterpret_cast<__nv_bfloat16 *>(at(s.hid) + (l & 1) * align256((size_t)B * d * 2));
     LinArgs in{};
     in.w = bfp(kInW); in.n = (int)(2 * di); in.K = (int)d; in.B = (int)B;
-    in.act = hid;
-    in.norm_w = raw(kNormW); in.norm_dt = dt(kNormW); in.eps = f[kEpsIn];
+    in.act = hid_w; in.ss = hid_ss; in.nss = l == 0 ? 1 : (int)tiles_out; in.eps = f[kEpsIn];
     in.x = reinterpret_cast<__nv_bfloat16 *>(at(s.x));
     in.gate = reinterpret_cast<__nv_bfloat16 *>(at(s.gate));
     in.x_conv = reinterpret_cast<__nv_bfloat16 *>(at(s.x_conv));
     in.new_conv = reinterpret_cast<__nv_bfloat16 *>(p[kNewConv]);
     in.old_conv = bfp(kOldConv);
     in.conv_w = bfp(kConvW); in.conv_b = bfp(kConvB); in.di = (int)di;
-    e = launch_dep(decode_linear_kernel<NT, kIn>, dim3((unsigned)blocks(tiles_in, smem_d)), smem_d, st, l > 0, in);
+    e = launch_dep(decode_linear_kernel<NT, kIn>, dim3((unsigned)blocks(tiles_in, smem_d)), smem_d, st, true, in);
     if (e != cudaSuccess) break;
 
     LinArgs pr{};
@@ -569,16 +605,21 @@ int run_layers(const uint64_t *ptrs, const float *nums, int64_t layers, const vo
     m.inv_read_temp = 1.f / f[kReadTemp];
     m.dt_min = f[kDtMin]; m.dt_max = f[kDtMax]; m.a_min = f[kAMin]; m.a_max = f[kAMax];
     m.l_min = f[kLMin]; m.l_max = f[kLMax]; m.gate_bias = f[kGateBias];
-    m.vals = reinterpret_cast<float *>(at(s.vals)); m.ss = reinterpret_cast<float *>(at(s.ss));
+    m.norm_w = raw(kOutNormW); m.norm_dt = dt(kOutNormW);
+    m.vals = reinterpret_cast<__nv_bfloat16 *>(at(s.vals)); m.ss = reinterpret_cast<float *>(at(s.ss));
     m.H = (int)H; m.R = (int)R; m.M = (int)M; m.splits = splits;
     e = launch_dep(decode_mix_kernel, dim3((unsigned)(H * splits), (unsigned)B), mix_smem, st, true, m);
     if (e != cudaSuccess) break;
 
     LinArgs o{};
     o.w = bfp(kOutW); o.n = (int)d; o.K = (int)di; o.B = (int)B;
-    o.vals = m.vals; o.ss = m.ss; o.nss = (int)(H * splits);
-    o.norm_w = raw(kOutNormW); o.norm_dt = dt(kOutNormW); o.eps = f[kEpsOut];
+    o.act = m.vals; o.ss = m.ss; o.nss = (int)(H * splits); o.eps = f[kEpsOut];
     o.res = hid; o.dst = next;
+    if (l + 1 < layers) {
+      o.dst_w = hid_w; o.dst_ss = hid_ss;
+      o.next_w = reinterpret_cast<const void *>(p[kLayerPtrs + kNormW]);
+      o.next_dt = p[kLayerPtrs + kF32Mask] & 1 ? FRACSSM_F32 : FRACSSM_BF16;
+    }
     e = launch_dep(decode_linear_kernel<NT, kOut>, dim3((unsigned)blocks(tiles_out, smem_di)), smem_di, st, true, o);
     hid = next;
   }

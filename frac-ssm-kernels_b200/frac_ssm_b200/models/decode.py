@@ -9,6 +9,8 @@ sends the call back to the modules' own forward.
 from __future__ import annotations
 
 import array
+from itertools import repeat
+from operator import attrgetter, contains, itemgetter
 
 import torch
 from torch import nn
@@ -17,12 +19,10 @@ from torch.nn.modules import module as _nn_module
 from .. import _cabi as C
 
 _PTRS = 19      # columns of the pointer table of fracssm_decode_layers
+_ptr = torch.Tensor.data_ptr
 _MAY_BE_F32 = 1 << 0 | 0b111111 << 7      # the norm weights and the small parameters
-_TENSORS = (nn.Parameter, torch.Tensor)
-
-
-def _plain(m, cls):
-    return type(m) is cls and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in m.__dict__
+_PARTS = ("in_proj", "conv1d", "dyn_proj", "rw_proj", "out_norm", "out_proj")
+_TENSORS = frozenset((nn.Parameter, torch.Tensor))
 
 
 def transformed():
@@ -32,73 +32,71 @@ def transformed():
             or torch._C._len_torch_function_stack() > 0 or torch._C._functorch.peek_interpreter_stack() is not None)
 
 
-def layer_params(layer, classes, sizes, dev):
-    """One layer's 14 parameters (None for an absent bias), the bit mask of those that are float32, and its numbers,
-    in the order of the tables of fracssm_decode_layers; None when native code does not cover the layer."""
+def layer_params(layers, classes, sizes, dev):
+    """Per layer its 14 parameters (None for an absent bias), the bit mask of those that are float32, and its numbers,
+    in the order of the tables of fracssm_decode_layers; None when native code does not cover the layers.
+
+    The same question goes to all modules or parameters at once: there are hundreds of each, and asked one by one
+    the answers cost as much as the launches."""
     d, H, R, M, K, di = sizes
     block_cls, norm_cls, mixer_cls, gated_cls = classes
-    if not _plain(layer, block_cls):
+    layers = list(layers)
+    if set(map(type, layers)) != {block_cls}:
         return None
-    norm, mixer = layer._modules["norm"], layer._modules["mixer"]
-    if not _plain(norm, norm_cls) or not _plain(mixer, mixer_cls):
+    inner = [layer.__dict__["_modules"] for layer in layers]
+    norms, mixers = [m["norm"] for m in inner], [m["mixer"] for m in inner]
+    if set(map(type, mixers)) != {mixer_cls} or set(map(type, norms)) != {norm_cls}:
         return None
-    mods = mixer._modules
-    in_proj, conv1d, dyn, rw = mods["in_proj"], mods["conv1d"], mods["dyn_proj"], mods["rw_proj"]
-    out_norm, out_proj = mods["out_norm"], mods["out_proj"]
-    if not (_plain(in_proj, nn.Linear) and _plain(conv1d, nn.Conv1d) and _plain(dyn, nn.Linear)
-            and _plain(rw, nn.Linear) and _plain(out_norm, gated_cls) and _plain(out_proj, nn.Linear)):
+    parts = [list(map(m.__dict__["_modules"].__getitem__, _PARTS)) for m in mixers]
+    if any([type(p) for p in ps] != [nn.Linear, nn.Conv1d, nn.Linear, nn.Linear, gated_cls, nn.Linear] for ps in parts):
         return None
-    if in_proj._parameters["bias"] is not None or out_proj._parameters["bias"] is not None:
-        return None        # (a bias of rw_proj is not read by the modules either)
-    if mixer.num_heads != H or mixer.head_dim != R or mixer.num_modes != M or mixer.conv_kernel != K:
+    dicts = [m.__dict__ for m in layers + norms + mixers] + [p.__dict__ for ps in parts for p in ps]
+    if (any(map(itemgetter("_forward_hooks"), dicts)) or any(map(itemgetter("_forward_pre_hooks"), dicts))
+            or any(map(contains, dicts, repeat("forward")))):
         return None
-    own = mixer._parameters
-    tensors = (norm._parameters["weight"], in_proj._parameters["weight"], conv1d._parameters["weight"],
-               conv1d._parameters["bias"], dyn._parameters["weight"], dyn._parameters["bias"], rw._parameters["weight"],
-               own["dt_bias"], own["read_residual_logit"], own["write_residual_scale"], mixer._buffers["base_log_tau"],
-               own["D"], out_norm._parameters["weight"], out_proj._parameters["weight"])
-    mask = slot = 0
-    bf16, f32 = torch.bfloat16, torch.float32
-    for t, n in zip(tensors, (d, 2 * di * d, K * di, di, 3 * H * di, 3 * H, 2 * H * M * di, H, 1, 1, M, di, di, d * di)):
-        if t is None:
-            if slot != 3 and slot != 5:
-                return None
+    counts = (d, 2 * di * d, K * di, di, 3 * H * di, 3 * H, 2 * H * M * di, H, 1, 1, M, di, di, d * di)
+    found, every, expected = [], [], []
+    last_cfg = cfg_nums = None
+    for norm, mixer, ps in zip(norms, mixers, parts):
+        in_proj, conv1d, dyn, rw, out_norm, out_proj = [p.__dict__["_parameters"] for p in ps]
+        if in_proj["bias"] is not None or out_proj["bias"] is not None:
+            return None        # (a bias of rw_proj is not read by the modules either)
+        m = mixer.__dict__
+        if m["num_heads"] != H or m["head_dim"] != R or m["num_modes"] != M or m["conv_kernel"] != K:
+            return None
+        own = m["_parameters"]
+        tensors = (norm.__dict__["_parameters"]["weight"], in_proj["weight"], conv1d["weight"], conv1d["bias"], dyn["weight"],
+                   dyn["bias"], rw["weight"], own["dt_bias"], own["read_residual_logit"], own["write_residual_scale"],
+                   m["_buffers"]["base_log_tau"], own["D"], out_norm["weight"], out_proj["weight"])
+        if tensors[3] is None or tensors[5] is None:
+            every += [t for t in tensors if t is not None]
+            expected += [n for t, n in zip(tensors, counts) if t is not None]
         else:
-            if t.dtype is not bf16:
-                if t.dtype is not f32 or not _MAY_BE_F32 >> slot & 1:
+            every += tensors
+            expected += counts
+        cfg = m["config"]
+        if cfg is not last_cfg:
+            last_cfg, cfg_nums = cfg, (cfg.frac_dt_min, cfg.frac_dt_max, cfg.frac_alpha_min, cfg.frac_alpha_max,
+                                       cfg.frac_lambda_min, cfg.frac_lambda_max, cfg.frac_gate_bias_init)
+        found.append((tensors, (norm.__dict__["variance_epsilon"], ps[4].__dict__["variance_epsilon"], m["read_temp"], *cfg_nums)))
+    T = torch.Tensor
+    if not _TENSORS.issuperset(map(type, every)):      # (a missing weight is no tensor either)
+        return None
+    if set(map(T.get_device, every)) != {dev} or list(map(T.numel, every)) != expected or not all(map(T.is_contiguous, every)):
+        return None
+    bf16 = torch.bfloat16
+    if set(map(attrgetter("dtype"), every)) == {bf16}:
+        return [(tensors, 0, nums) for tensors, nums in found]
+    out = []
+    for tensors, nums in found:
+        mask = 0
+        for slot, t in enumerate(tensors):
+            if t is not None and t.dtype is not bf16:
+                if t.dtype is not torch.float32 or not _MAY_BE_F32 >> slot & 1:
                     return None
                 mask |= 1 << slot
-            if t.get_device() != dev or t.numel() != n or not t.is_contiguous() or type(t) not in _TENSORS:
-                return None
-        slot += 1
-    cfg = mixer.config
-    return tensors, mask, (norm.variance_epsilon, out_norm.variance_epsilon, mixer.read_temp, cfg.frac_dt_min,
-                           cfg.frac_dt_max, cfg.frac_alpha_min, cfg.frac_alpha_max, cfg.frac_lambda_min,
-                           cfg.frac_lambda_max, cfg.frac_gate_bias_init)
-
-
-def _layer_entry(layer, classes, sizes, B, ptrs, nums, dev, state, conv):
-    """Appends one layer's row to both tables; False when the layer is not covered."""
-    found = layer_params(layer, classes, sizes, dev)
-    if found is None:
-        return False
-    tensors, mask, numbers = found
-    d, H, R, M, K, di = sizes
-    row = [0 if t is None else t.data_ptr() for t in tensors]
-    if row[2] & 7 or (row[1] | row[4] | row[6] | row[13]) & 15:   # conv weight; projection weights
-        return False
-    ptrs += row
-    if state is None:
-        ptrs += (0, 0)
-    else:
-        if (state.dtype is not torch.float32 or state.shape != (B, H, M, R) or not state.is_contiguous()
-                or state.get_device() != dev or conv.dtype is not torch.bfloat16 or conv.shape != (B, di, 3)
-                or not conv.is_contiguous() or conv.get_device() != dev or state.data_ptr() & 15):
-            return False
-        ptrs += (state.data_ptr(), conv.data_ptr())
-    ptrs += (0, 0, mask)
-    nums += numbers
-    return True
+        out.append((tensors, mask, nums))
+    return out
 
 
 def decode_layers(layers, h, past, use_cache, classes):
@@ -123,15 +121,35 @@ def decode_layers(layers, h, past, use_cache, classes):
     dev = h.get_device()
     sizes = (d, H, R, M, K, di)
     # every layer is looked at before the first launch: a call is covered as a whole or not at all
-    ptrs, nums = [], []
-    for i, layer in enumerate(layers):
-        state = conv = None
-        if past is not None and past[i] is not None:
-            state, conv = past[i]
-            if state is None or conv is None:
-                return None
-        if not _layer_entry(layer, classes, sizes, B, ptrs, nums, dev, state, conv):
+    found = layer_params(layers, classes, sizes, dev)
+    if found is None:
+        return None
+    if past is None or all(p is None for p in past):
+        olds = [(0, 0)] * n
+    else:
+        if any(p is None or p[0] is None or p[1] is None for p in past):
             return None
+        states, convs = [p[0] for p in past], [p[1] for p in past]
+        f32, bf16 = torch.float32, torch.bfloat16
+        for ts, dtype, shape in ((states, f32, (B, H, M, R)), (convs, bf16, (B, di, 3))):
+            for t in ts:
+                if t.dtype is not dtype or t.shape != shape or not t.is_contiguous() or t.get_device() != dev:
+                    return None
+        olds = [(s.data_ptr(), c.data_ptr()) for s, c in zip(states, convs)]
+        if any(s & 15 for s, _ in olds):
+            return None
+    ptrs, nums = [], []
+    for (tensors, mask, numbers), old in zip(found, olds):
+        if tensors[3] is not None and tensors[5] is not None:
+            row = list(map(_ptr, tensors))
+        else:
+            row = [0 if t is None else t.data_ptr() for t in tensors]
+        if row[2] & 7 or (row[1] | row[4] | row[6] | row[13]) & 15:   # conv weight; projection weights
+            return None
+        ptrs += row
+        ptrs += old
+        ptrs += (0, 0, mask)
+        nums += numbers
     new_past = None
     if use_cache:
         states = torch.empty(n, B, H, M, R, device=h.device, dtype=torch.float32).unbind(0)

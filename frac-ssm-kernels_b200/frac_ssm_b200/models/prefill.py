@@ -53,15 +53,14 @@ def prefill_layers(layers, h, attention_mask, use_cache, classes):
         return None
     coeff = torch.float32 if coeff is None else coeff
     sizes = (d, H, R, M, K, di)
-    found = []
-    for layer in layers:      # a call is covered as a whole or not at all
-        entry = layer_params(layer, classes, sizes, dev)
-        if entry is None:
-            return None
+    # a call is covered as a whole or not at all
+    found = layer_params(layers, classes, sizes, dev)
+    if found is None:
+        return None
+    for layer in layers:
         m = layer.mixer
         if m.fuse_gate_into_scan or (torch.float32 if m.coeff_dtype is None else m.coeff_dtype) is not coeff or m.chunk_size != T:
             return None
-        found.append(entry)
 
     lib, bf16, f32 = C.lib(), torch.bfloat16, torch.float32
 
