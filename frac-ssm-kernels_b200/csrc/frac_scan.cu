@@ -104,8 +104,6 @@ int frac_scan_route(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, cons
   if (path == 2 && !fused_ok)
     return fail(FRACSSM_ERR_UNSUPPORTED, "frac_scan: shape, dtype, strides or alignment not covered by the single-pass kernel");
   if (fused_ok && path != 1) {
-    if (workspace_bytes < scan_fused_workspace_bytes(B, L, R, M, T))
-      return fail(FRACSSM_ERR_ARG, "frac_scan: workspace too small");
     return scan_fused_launch(u, c, kappa, ck_dtype, rho, initial_state, h, final_state, final_dtype,
                              workspace, workspace_bytes, B, L, R, M, T, stream);
   }

@@ -5,7 +5,7 @@
 //
 // Work item = (bh, tile of 128 tokens), handed out by an atomic ticket in tile-major order
 // (all bh of tile 0, then tile 1, ...).  The item (bh, j) needs the state left by (bh, j-1);
-// it waits on a per-bh counter in global memory with a time limit.  A ticket is only taken
+// it waits on a per-bh counter in global memory (few rows: on tags beside the state's values) with a time limit.  A ticket is only taken
 // by a running CTA (one item ahead of the one it is working on) and dependencies point to
 // lower tickets, so the lowest unfinished item is always being worked on and never waits.
 //
@@ -219,11 +219,27 @@ __device__ __forceinline__ void emit_pair_next_slot(uint32_t rows_s, int i, uint
   asm volatile("st.shared.b32 [%0+32768], %1;" ::"r"(addr), "r"(w0) : "memory");
 }
 
+// A piece of the state with its tile's number beside every value (LL, below): 8-byte halves are written and read whole.
+__device__ __forceinline__ uint4 ld_tagged(const uint4 *p) {
+  uint4 v;
+  asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_tagged(uint4 *p, float a, float b, uint32_t tag) {
+  asm volatile("st.volatile.global.v4.u32 [%0], {%1,%2,%3,%2};" ::"l"(p), "r"(__float_as_uint(a)), "r"(tag),
+               "r"(__float_as_uint(b)) : "memory");
+}
+
+// LL: the state is handed from tile to tile with its tile's number beside every value, and the threads that need it
+// wait for the numbers themselves.  A thread reads and writes the same 16 elements of the row's state in every tile, so
+// the hand-over is a chain of threads, without a counter, a fence or a barrier of the CTA: one L2 store and two L2
+// reads a step.  Twice the state traffic and 16 more memory instructions a tile, so it is for few rows, where a row's
+// chain of tiles is what limits the run (see scan_fused_launch_ex).
 // CKF32: c and kappa are float32 (else bf16).  LAYER: the output stage applies the skip connection and
 // the gate (its code is kept out of the plain kernel, whose loop is fetched once per tile).
 // RAGGED: L is not a multiple of the tile, so a row's last tile takes the row-by-row, predicated loads
 // (kept out of the other instances: the loop's code is fetched once per tile and its size counts).
-template <bool CKF32, bool LAYER, bool RAGGED>
+template <bool CKF32, bool LAYER, bool RAGGED, bool LL>
 __global__ void __launch_bounds__(kThreads, 1)
 scan_fused_kernel(const FusedArgs a, const __grid_constant__ CUtensorMap u_map) {
   extern __shared__ uint8_t smem_raw[];
@@ -318,6 +334,10 @@ scan_fused_kernel(const FusedArgs a, const __grid_constant__ CUtensorMap u_map) 
         umma::prefetch_l2(reinterpret_cast<const char *>(a.c) + tok * kM * kCkBytes, ntok * kM * kCkBytes);
         umma::prefetch_l2(reinterpret_cast<const char *>(a.kappa) + tok * kM * kCkBytes, ntok * kM * kCkBytes);
         umma::prefetch_l2(a.u + tok * kR, ntok * kR * 2);
+      }
+      if constexpr (LL) {   // the workers wait for the state themselves
+        item = next;
+        continue;
       }
       // the state left by the previous tile of this row
       if (lane == 0) {
@@ -594,6 +614,7 @@ scan_fused_kernel(const FusedArgs a, const __grid_constant__ CUtensorMap u_map) 
       float gt_row = 0.f;   // decay of the whole tile for the mode this thread owns in the state update
       const int m_row = 32 * Q + lane;
       float sj[16];         // incoming state: row m_row, columns 16 P .. 16 P + 15
+      uint4 *ll = reinterpret_cast<uint4 *>(a.state) + (static_cast<int64_t>(bh) * 4 + P) * 8 * kM;   // LL: [bh][P][x][m]
       auto load_state = [&]() {
         // scratch layout [bh][P][x][m][4]: the lanes of a warp touch consecutive 16-byte pieces
         const float4 *sp = reinterpret_cast<const float4 *>(a.state) +
@@ -905,8 +926,13 @@ scan_fused_kernel(const FusedArgs a, const __grid_constant__ CUtensorMap u_map) 
       FRACSSM_MARK(pslot, 24)
       };
       // ---- the chain: incoming state -> MMA operand (high | low) -> outgoing state
-      FRACSSM_WAIT(state_bar, n);
-      load_state();
+      uint32_t tag_seen = 0;
+      if constexpr (LL) {
+        if (jt > 0) tag_seen = ld_tagged(ll + 32 * Q).y;   // looked at below; on its way during the next wait
+      } else {
+        FRACSSM_WAIT(state_bar, n);
+        load_state();
+      }
       FRACSSM_WAIT(cb2, n);  // levels 64+32 product done: slots 4 / 5 are free, its accumulators complete
       FRACSSM_MARK(pslot, 20)
       // the incoming state as the MMA operand [high | low] of H = Chat S
@@ -956,16 +982,96 @@ scan_fused_kernel(const FusedArgs a, const __grid_constant__ CUtensorMap u_map) 
       // The outgoing state goes first when its own part (Sacc) is already complete: that is the case
       // when the tile had to wait for the incoming state, i.e. when the row's chain of tiles is what
       // limits the run; otherwise the operand goes first and the MMA warp gets to work earlier.
-      const bool chain_first = __shfl_sync(0xffffffffu, umma::mbar_test(cbK, n & 1u) ? 1 : 0, 0) != 0;
-      if (chain_first) {
-        state_update();
-        state_operand();
+      if constexpr (LL) {
+        // the incoming state to the outgoing one and to the operand, 8 of the thread's 16 columns at a time (the chain of
+        // either half is its own, so the second half's later reads cost the chain nothing)
+        auto state_step = [&]() {
+          uint4 v[2][4];
+          auto request = [&](int half) {
+#pragma unroll
+            for (int x = 0; x < 4; ++x) v[half][x] = jt > 0 ? ld_tagged(ll + (4 * half + x) * kM + m_row) : make_uint4(0, 0, 0, 0);
+          };
+          auto arrived = [&](int half) {
+            uint32_t miss = 0;
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+              miss |= (v[half][x].y ^ static_cast<uint32_t>(jt)) | (v[half][x].w ^ static_cast<uint32_t>(jt));
+            return __all_sync(0xffffffffu, miss == 0 || jt == 0) != 0;
+          };
+          request(0);
+          FRACSSM_WAIT(cbK, n);
+          umma::tc_fence_after();
+          const bool bad = *failed != 0;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            if (!arrived(half)) {   // read again until the tags are there (looking at one sector first made a step 0.15 us longer)
+              uint64_t t_start = 0;
+              for (uint32_t spins = 0; ok; ++spins) {
+                request(half);
+                if (arrived(half)) break;
+                if (spins == 256) t_start = umma::global_ns();
+                if (__any_sync(0xffffffffu, spins > 256 && umma::global_ns() - t_start > wait_ns)) {
+                  ok = false;
+                  *failed = 1;
+                }
+              }
+            }
+            if (half == 0) request(1);
+            float sv[8];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+              sv[2 * x] = __uint_as_float(v[half][x].x);
+              sv[2 * x + 1] = __uint_as_float(v[half][x].z);
+            }
+            if (jt == 0 && a.init) {
+#pragma unroll
+              for (int x = 0; x < 8; ++x)
+                sv[x] = a.init[(static_cast<int64_t>(bh) * kR + 16 * P + 8 * half + x) * kM + m_row];
+            }
+            float acc[8];
+            umma::tmem_ld8(lane_addr + kColS + 16 * P + 8 * half, acc);
+            umma::tmem_ld_wait();
+#pragma unroll
+            for (int x = 0; x < 8; ++x) acc[x] = bad || !ok ? kNaN : fmaf(gt_row, sv[x], acc[x]);
+            if (jt + 1 < a.ntiles) {
+#pragma unroll
+              for (int x = 0; x < 4; ++x)
+                st_tagged(ll + (4 * half + x) * kM + m_row, acc[2 * x], acc[2 * x + 1], static_cast<uint32_t>(jt + 1));
+            } else if (a.fin) {
+#pragma unroll
+              for (int x = 0; x < 8; ++x)
+                st_f32(a.fin, (static_cast<int64_t>(bh) * kR + 16 * P + 8 * half + x) * kM + m_row, a.fin_dt, acc[x]);
+            }
+            uint32_t ph[4], pl[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+              const float2 hi = bf16_round2(make_float2(sv[2 * x], sv[2 * x + 1]), ph[x]);
+              pl[x] = pack2(sv[2 * x] - hi.x, sv[2 * x + 1] - hi.y);
+            }
+            const uint32_t off = m_row * 128 + (((2 * P + half) ^ (m_row & 7)) << 4);
+            *reinterpret_cast<uint4 *>(smem + kOffS + off) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
+            *reinterpret_cast<uint4 *>(smem + kOffS + kAtom + off) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+          }
+          warp_arrive(fS, lane);
+        };
+        // a state that is not there yet: W first, which does not need it
+        const int w_at = __all_sync(0xffffffffu, tag_seen == static_cast<uint32_t>(jt)) ? 1 : 0;
+#pragma unroll 1
+        for (int part = 0; part < 2; ++part) {   // (one copy of either part: the code is fetched once per tile)
+          if (part == w_at) w_epilogue();
+          else state_step();
+        }
       } else {
-        state_operand();
-        state_update();
+        const bool chain_first = __shfl_sync(0xffffffffu, umma::mbar_test(cbK, n & 1u) ? 1 : 0, 0) != 0;
+        if (chain_first) {
+          state_update();
+          state_operand();
+        } else {
+          state_operand();
+          state_update();
+        }
+        w_epilogue();
       }
-
-      w_epilogue();
 
 
       prev_bh = bh;
@@ -985,8 +1091,19 @@ size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 }  // namespace
 
-size_t scan_fused_workspace_bytes(int64_t B, int64_t, int64_t R, int64_t M, int64_t) {
+// Rows up to which the state is handed over with tags (LL).  A step of a row's chain takes 1.0 us with tags and 2.4 us
+// through the counter (4 rows), a tile of a CTA 10.5 us against 8 (the tags' traffic and instructions), so:
+// 24 x 131072 tokens 1.73 ms with tags, 2.92 without; 48 x 65536 1.56 / 1.89; 64 x 8192 0.281 / 0.306;
+// 80 x 8192 0.343 / 0.317; 96 x 8192 0.406 / 0.351.  24 x 397 tokens, four tiles a row: 37 / 59 us.
+constexpr int64_t kTaggedRows = 64;
+static size_t plain_workspace_bytes(int64_t B, int64_t R, int64_t M) {
   return kCtrlBytes + align256((size_t)B * 4) + (size_t)B * R * M * 4;
+}
+static size_t tagged_workspace_bytes(int64_t B, int64_t R, int64_t M) {
+  return kCtrlBytes + align256((size_t)B * 4) + (size_t)B * R * M * 8;
+}
+size_t scan_fused_workspace_bytes(int64_t B, int64_t, int64_t R, int64_t M, int64_t) {
+  return B <= kTaggedRows ? tagged_workspace_bytes(B, R, M) : plain_workspace_bytes(B, R, M);
 }
 
 // first_tile / wait_ns: 0 and the default limit, except in the wait-limit self-test, which starts
@@ -998,7 +1115,7 @@ int scan_fused_launch_ex(const void *u, const void *c, const void *kappa, int ck
                          const ScanLayerOut *layer) {
   (void)T;
   const bool ckf32 = ck_dtype == FRACSSM_F32;
-  if (workspace_bytes < scan_fused_workspace_bytes(B, L, R, M, T))
+  if (workspace_bytes < plain_workspace_bytes(B, R, M))
     return fail(FRACSSM_ERR_ARG, "frac_scan: workspace too small");
   // the kernel reads c / kappa / rho and writes h with 8- and 16-byte accesses
   if (((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(kappa) |
@@ -1028,12 +1145,20 @@ int scan_fused_launch_ex(const void *u, const void *c, const void *kappa, int ck
   {
     std::lock_guard<std::mutex> lock(mu);
     if (sm_count[dev] == 0) {
-      int prc = prepare(reinterpret_cast<const void *>(&scan_fused_kernel<false, false, false>));
-      if (prc == FRACSSM_OK) prc = prepare(reinterpret_cast<const void *>(&scan_fused_kernel<true, false, false>));
-      if (prc == FRACSSM_OK) prc = prepare(reinterpret_cast<const void *>(&scan_fused_kernel<false, false, true>));
-      if (prc == FRACSSM_OK) prc = prepare(reinterpret_cast<const void *>(&scan_fused_kernel<true, false, true>));
-      if (prc == FRACSSM_OK) prc = prepare(reinterpret_cast<const void *>(&scan_fused_kernel<false, true, true>));
-      if (prc == FRACSSM_OK) prc = prepare(reinterpret_cast<const void *>(&scan_fused_kernel<true, true, true>));
+      const void *kernels[] = {
+          reinterpret_cast<const void *>(&scan_fused_kernel<false, false, false, false>),
+          reinterpret_cast<const void *>(&scan_fused_kernel<true, false, false, false>),
+          reinterpret_cast<const void *>(&scan_fused_kernel<false, false, true, false>),
+          reinterpret_cast<const void *>(&scan_fused_kernel<true, false, true, false>),
+          reinterpret_cast<const void *>(&scan_fused_kernel<false, true, true, false>),
+          reinterpret_cast<const void *>(&scan_fused_kernel<true, true, true, false>),
+          reinterpret_cast<const void *>(&scan_fused_kernel<false, false, false, true>),
+          reinterpret_cast<const void *>(&scan_fused_kernel<true, false, false, true>),
+          reinterpret_cast<const void *>(&scan_fused_kernel<false, false, true, true>),
+          reinterpret_cast<const void *>(&scan_fused_kernel<true, false, true, true>)};
+      int prc = FRACSSM_OK;
+      for (const void *k : kernels)
+        if (prc == FRACSSM_OK) prc = prepare(k);
       if (prc) return prc;
       int n = 0;
       cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
@@ -1073,23 +1198,29 @@ int scan_fused_launch_ex(const void *u, const void *c, const void *kappa, int ck
   CUtensorMap map;
   int rc = make_tmap_bf16_3d(&map, u, kR, (uint64_t)L, (uint64_t)B, kR, kTile);
   if (rc) return rc;
-  cudaError_t e = cudaMemsetAsync(ws, 0, kCtrlBytes + align256((size_t)B * 4), (cudaStream_t)stream);
+  // (one tile: nothing is handed over; a workspace of the plain size keeps the plain hand-over)
+  const bool tagged = B <= kTaggedRows && a.ntiles - first_tile > 1 && !layer &&
+                      workspace_bytes >= tagged_workspace_bytes(B, R, M);
+  // the tags start from zeros, which no tile hands over
+  cudaError_t e = cudaMemsetAsync(ws, 0, tagged ? tagged_workspace_bytes(B, R, M) : kCtrlBytes + align256((size_t)B * 4),
+                                  (cudaStream_t)stream);
   if (e != cudaSuccess) return fail(FRACSSM_ERR_CUDA, "frac_scan: %s", cudaGetErrorString(e));
   const int grid = a.total < sms ? a.total : sms;
   const cudaStream_t st = (cudaStream_t)stream;
+  const bool ragged = a.L % kTile != 0;
+#define FRACSSM_SCAN(LAYER, RAGGED, LL)                                                        \
+  if (ckf32) scan_fused_kernel<true, LAYER, RAGGED, LL><<<grid, kThreads, kSmemBytes, st>>>(a, map); \
+  else scan_fused_kernel<false, LAYER, RAGGED, LL><<<grid, kThreads, kSmemBytes, st>>>(a, map)
   if (a.gate != nullptr) {
-    if (ckf32) scan_fused_kernel<true, true, true><<<grid, kThreads, kSmemBytes, st>>>(a, map);
-    else scan_fused_kernel<false, true, true><<<grid, kThreads, kSmemBytes, st>>>(a, map);
+    FRACSSM_SCAN(true, true, false);
+  } else if (tagged) {
+    if (ragged) { FRACSSM_SCAN(false, true, true); }
+    else { FRACSSM_SCAN(false, false, true); }
   } else {
-    const bool ragged = a.L % kTile != 0;
-    if (ragged) {
-      if (ckf32) scan_fused_kernel<true, false, true><<<grid, kThreads, kSmemBytes, st>>>(a, map);
-      else scan_fused_kernel<false, false, true><<<grid, kThreads, kSmemBytes, st>>>(a, map);
-    } else {
-      if (ckf32) scan_fused_kernel<true, false, false><<<grid, kThreads, kSmemBytes, st>>>(a, map);
-      else scan_fused_kernel<false, false, false><<<grid, kThreads, kSmemBytes, st>>>(a, map);
-    }
+    if (ragged) { FRACSSM_SCAN(false, true, false); }
+    else { FRACSSM_SCAN(false, false, false); }
   }
+#undef FRACSSM_SCAN
   return check_launch("frac_scan (single-pass kernel)");
 }
 

@@ -30,7 +30,7 @@ def frac_scan(u, c, kappa, rho, chunk_size, initial_state=None, return_final_sta
         final_state_dtype: dtype of the returned state; default follows the reference
             (bfloat16 when u is bfloat16, else float32).  The state is always carried in float32.
         path: "auto", "staged" or "fused".  "auto" takes the single-pass kernel when it covers the
-            shape, and for few rows with many tokens (at most 28 rows, at least 32768 tokens) cuts
+            shape, and for very few rows with many tokens (fewer than 12 rows, at least 32768 tokens) cuts
             every row into sub-segments first, because a row is one chain of tiles and 148 SMs want
             more chains than that: one summary pass over u, kappa and rho gives every sub-segment its
             incoming state, then all sub-segments are scanned as rows (`parallel.seq_parallel_scan`).
@@ -84,12 +84,18 @@ def frac_scan(u, c, kappa, rho, chunk_size, initial_state=None, return_final_sta
     return h
 
 
+# Rows from which the single-pass kernel takes long rows as they are: its chain of tiles advances a tile per 1.05 us
+# and row, a CTA needs some 10 us a tile, and cutting the rows costs a second read of u, kappa and rho (131072 tokens:
+# 8 rows 1.17 ms whole, 1.19 cut; 12 rows 1.25 and 1.20; 16 rows 1.37 and 1.54; 24 rows of 1048576 tokens 13.7 and 16.7).
+WHOLE_ROWS = 12
+
+
 def _row_splits(u, c, chunk_size):
     """Sub-segments per row for the "auto" path: more than 1 only where the single-pass kernel covers
     both the call and the cut-up call, the tensors are dense, and the rows are few and long."""
     from ... import parallel
     B, L, R = u.shape
-    if B < 1 or not (u.is_contiguous() and c.is_contiguous()) or u.dtype != torch.bfloat16:
+    if B < 1 or B >= WHOLE_ROWS or not (u.is_contiguous() and c.is_contiguous()) or u.dtype != torch.bfloat16:
         return 1
     splits = parallel._auto_local_splits(B, L, chunk_size, 1, u.device)
     if splits > 1 and not C.lib().fracssm_scan_fused_supported(B * splits, L // splits, R, c.shape[-1],
