@@ -22,8 +22,9 @@
 //     of 8 warps busy;
 //   * every kernel is launched with programmatic stream serialisation: it requests what no kernel of this call
 //     writes (weights, the old state and convolution history) before it waits for its predecessor.
-// Whole model call, 24 layers of hidden 768, 24 heads x 128 modes, vocabulary 50280: 13.6 ms -> 0.72 ms at one
-// sequence, 13.9 ms -> 1.50 ms at 32.
+// Whole model call, 24 layers of hidden 768, 24 heads x 128 modes, vocabulary 50280, before and now: 13.6 and 0.66 ms
+// at one sequence (0.48 ms on the device, the rest is the host's 97 launches and look at 336 parameters), 13.7 and
+// 1.1 ms at 32.
 #include <mutex>
 
 #include "common.cuh"
@@ -92,7 +93,7 @@ __device__ __forceinline__ void copy_async16(uint32_t dst, const void *src, bool
 
 // NT groups of 8 sequences.
 template <int NT, int KIND>
-__global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 1) decode_linear_kernel(const LinArgs a) {
+__global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : NT <= 4 ? 2 : 1) decode_linear_kernel(const LinArgs a) {
   extern __shared__ __align__(16) uint8_t lin_smem[];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, tig = lane & 3;
   grid_dep_launch();
@@ -123,19 +124,27 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 1) decode_linear_kerne
   request(tile0, k_lo);
   // what the epilogue of this thread's first value needs and no kernel of this call writes
   const int e_row = tid & 15, e_seq = tid >> 4;
+  constexpr int kPasses = (NT + kPassTiles - 1) / kPassTiles;
   uint2 cw = make_uint2(0, 0);
-  float cb = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f, nw = 0.f;
-  auto conv_inputs = [&](int n, int b) {
+  float cb = 0.f, nw = 0.f;
+  __nv_bfloat16 ch[kPasses][3] = {};
+  auto conv_inputs = [&](int n) {   // of row n, for all of this thread's sequences
+    if (n >= a.di) return;
     cw = *reinterpret_cast<const uint2 *>(a.conv_w + (int64_t)n * 4);
     cb = a.conv_b ? __bfloat162float(a.conv_b[n]) : 0.f;
-    c0 = c1 = c2 = 0.f;
     if (a.old_conv) {
-      const __nv_bfloat16 *p = a.old_conv + ((int64_t)b * a.di + n) * 3;
-      c0 = __bfloat162float(p[0]); c1 = __bfloat162float(p[1]); c2 = __bfloat162float(p[2]);
+#pragma unroll
+      for (int p = 0; p < kPasses; ++p) {
+        const int b = 8 * kPassTiles * p + e_seq;
+        if (b < a.B) {
+          const __nv_bfloat16 *src = a.old_conv + ((int64_t)b * a.di + n) * 3;
+          ch[p][0] = src[0]; ch[p][1] = src[1]; ch[p][2] = src[2];
+        }
+      }
     }
   };
   const int e_n = tile0 * kTileRows + e_row;
-  if (KIND == kIn && NT == 1 && e_seq < a.B && e_n < a.di) conv_inputs(e_n, e_seq);
+  if (KIND == kIn) conv_inputs(e_n);
   if (KIND == kOut && a.next_w && e_n < N) nw = ld_f32(a.next_w, e_n, a.next_dt);
 
   grid_dep_wait();
@@ -146,15 +155,18 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 1) decode_linear_kerne
   const uint32_t act_s = (uint32_t)__cvta_generic_to_shared(lin_smem);
   if (NT > 1) {
     const int pieces = (k_hi - k_lo) * 4;     // 16-byte pieces of this warp's share of a row
-    for (int b = 0; b < 8 * NT; ++b)
-      for (int i = lane; i < pieces; i += 32) {
-        const int at = 4 * k_lo + i;
-        copy_async16(act_s + b * stride + at * 16, act + (int64_t)(b < a.B ? b : 0) * a.K + at * 8, b < a.B);
+    for (int i = lane; i < pieces; i += 32) {
+      const __nv_bfloat16 *src = act + (4 * k_lo + i) * 8;
+      uint32_t dst = act_s + (4 * k_lo + i) * 16;
+#pragma unroll 8
+      for (int b = 0; b < 8 * NT; ++b, dst += stride) {
+        copy_async16(dst, src, b < a.B);
+        if (b + 1 < a.B) src += a.K;
       }
+    }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   // 1 / rms of this thread's sequences: 16 threads share one
-  constexpr int kPasses = (NT + kPassTiles - 1) / kPassTiles;
   float rs[kPasses];
   if (KIND != kProj) {
 #pragma unroll
@@ -202,6 +214,7 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 1) decode_linear_kerne
       }
     }
     if (tile + tile_step < tiles) request(tile + tile_step, k_lo);   // on their way during the epilogue
+    if (KIND == kIn && tile != tile0) conv_inputs(tile * kTileRows + e_row);
     // ---- the warps' shares of the contraction are added, a value per thread
 #pragma unroll
     for (int p = 0; p < NT; p += kPassTiles) {
@@ -225,8 +238,9 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 1) decode_linear_kerne
         if (KIND == kIn) {
           const __nv_bfloat16 xb = __float2bfloat16_rn(v);
           if (n < a.di) {
-            if (NT != 1 || tile != tile0) conv_inputs(n, b);
             const float xv = __bfloat162float(xb);
+            const __nv_bfloat16 *c3 = ch[p / kPassTiles];
+            const float c0 = __bfloat162float(c3[0]), c1 = __bfloat162float(c3[1]), c2 = __bfloat162float(c3[2]);
             float y = cb;
             y = fmaf(bf(cw.x), c0, y);
             y = fmaf(bf_hi(cw.x), c1, y);
@@ -237,8 +251,8 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : 1) decode_linear_kerne
             a.x_conv[at] = __float2bfloat16_rn(y / (1.f + __expf(-y)));
             if (a.new_conv) {
               __nv_bfloat16 *q = a.new_conv + at * 3;
-              q[0] = __float2bfloat16_rn(c1);
-              q[1] = __float2bfloat16_rn(c2);
+              q[0] = c3[1];
+              q[1] = c3[2];
               q[2] = xb;
             }
           } else {
