@@ -14,7 +14,8 @@
 // host.  Hence
 //   * elementwise stages sit in the epilogue of the product that writes their rows.  A norm is split: whoever writes
 //     the row also writes it times the norm's weight and the sums of squares of its part of the row, and the product
-//     that reads it scales its results by 1 / rms, so no block has to see a whole row before it can start;
+//     that reads it scales its results by 1 / rms, so no block has to see a whole row before it can start.  What
+//     passes between the stages without going through a product (hidden state, gate, readout) stays float32;
 //   * the products stream the weights once, straight into the fragments of mma.sync (16 weight rows x 16 of the
 //     contraction x 8 sequences): with at most 64 sequences they are far below the tensor-core ridge, and a lane
 //     reads 8 consecutive weights of a row because the contraction order is free as long as both operands share
@@ -56,7 +57,6 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 }
 __device__ __forceinline__ float bf(uint32_t lo16) { return __uint_as_float(lo16 << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
-__device__ __forceinline__ float round_bf(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 __device__ __forceinline__ float sum_warp(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -72,15 +72,17 @@ struct LinArgs {
   int nss;
   float eps;
   // kIn outputs and the convolution
-  __nv_bfloat16 *x, *gate, *x_conv, *new_conv;
+  __nv_bfloat16 *x, *x_conv, *new_conv;
+  float *gate;
   const __nv_bfloat16 *old_conv, *conv_w, *conv_b;
   int di;
   // kProj outputs
   float *out, *out2;
   const __nv_bfloat16 *bias2;
   // kOut: dst = res + result, and for the next layer's norm (weight next_w or null) dst * next_w and a sum per tile
-  const __nv_bfloat16 *res;
-  __nv_bfloat16 *dst, *dst_w;
+  const float *res;              // the hidden state stays float32 from layer to layer
+  float *dst;                    // null in the last layer, which writes bfloat16 to dst_last
+  __nv_bfloat16 *dst_last, *dst_w;
   float *dst_ss;
   const void *next_w; int next_dt;
 };
@@ -256,18 +258,18 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : NT <= 4 ? 2 : 1) decod
               q[2] = xb;
             }
           } else {
-            a.gate[(int64_t)b * a.di + n - a.di] = xb;
+            a.gate[(int64_t)b * a.di + n - a.di] = v;
           }
         } else if (KIND == kProj) {
           if (second) a.out2[(int64_t)b * N + n] = v + (a.bias2 ? __bfloat162float(a.bias2[n]) : 0.f);
           else a.out[(int64_t)b * N + n] = v;
         } else {
           const int64_t at = (int64_t)b * N + n;
-          const __nv_bfloat16 hb = __float2bfloat16_rn(__bfloat162float(__ldcg(a.res + at)) + round_bf(v));
-          a.dst[at] = hb;
+          const float hv = __ldcg(a.res + at) + v;
+          if (a.dst) a.dst[at] = hv;
+          else a.dst_last[at] = __float2bfloat16_rn(hv);
           if (a.next_w) {
             if (tile != tile0) nw = ld_f32(a.next_w, n, a.next_dt);
-            const float hv = __bfloat162float(hb);
             a.dst_w[at] = __float2bfloat16_rn(hv * nw);
             sq = hv * hv;
           }
@@ -285,13 +287,14 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : NT <= 4 ? 2 : 1) decod
 
 // The embedding times the first norm's weight, and its sums of squares (one part per row).
 __global__ void __launch_bounds__(kThreads)
-decode_first_kernel(const __nv_bfloat16 *h, const void *w, int w_dt, __nv_bfloat16 *h_w, float *ss, int d) {
+decode_first_kernel(const __nv_bfloat16 *h, const void *w, int w_dt, float *h_f32, __nv_bfloat16 *h_w, float *ss, int d) {
   __shared__ float red[kWarps];
   const int64_t b = blockIdx.x;
   grid_dep_launch();
   float sq = 0.f;
   for (int i = threadIdx.x; i < d; i += kThreads) {
     const float v = __bfloat162float(h[b * d + i]);
+    h_f32[b * d + i] = v;
     h_w[b * d + i] = __float2bfloat16_rn(v * ld_f32(w, i, w_dt));
     sq = fmaf(v, v, sq);
   }
@@ -308,7 +311,8 @@ decode_first_kernel(const __nv_bfloat16 *h, const void *w, int w_dt, __nv_bfloat
 
 struct MixArgs {
   const float *rw, *dyn;               // [B][2 H M], [B][3 H]
-  const __nv_bfloat16 *x_conv, *gate;  // [B][H R]
+  const __nv_bfloat16 *x_conv;         // [B][H R]
+  const float *gate;                   // [B][H R]
   const float *old_state;              // [B][H][M][R] or null (zeros)
   float *new_state;                    // or null
   const void *dt_bias, *read_logit, *write_logit, *log_tau, *D, *norm_w;
@@ -367,7 +371,7 @@ __global__ void __launch_bounds__(kThreads) decode_mix_kernel(const MixArgs a) {
   float uc = 0.f, gc = 0.f;
   if (tid < cols) {
     uc = __bfloat162float(__ldcg(a.x_conv + col + tid));
-    gc = __bfloat162float(__ldcg(a.gate + col + tid));
+    gc = __ldcg(a.gate + col + tid);
   }
   const float d0 = y0 + dtb;
   float dt = d0 > 20.f ? d0 : log1pf(expf(d0));
@@ -453,14 +457,13 @@ __global__ void __launch_bounds__(kThreads) decode_mix_kernel(const MixArgs a) {
       Dv = ld_f32(a.D, (int64_t)h * R + sp * cols + c, a.D_dt);
       nwv = ld_f32(a.norm_w, (int64_t)h * R + sp * cols + c, a.norm_dt);
       uc = __bfloat162float(__ldcg(a.x_conv + col + c));
-      gc = __bfloat162float(__ldcg(a.gate + col + c));
+      gc = __ldcg(a.gate + col + c);
     }
     float o = 0.f;
 #pragma unroll 8
     for (int i = 0; i < rows; ++i) o += part[i * cols + c];
-    const float mixed = round_bf(o + uc * Dv);
-    const float z = round_bf(gc + a.gate_bias);
-    const float v = mixed * (z * sigmoid_(z));
+    const float z = gc + a.gate_bias;
+    const float v = (o + uc * Dv) * (z * sigmoid_(z));
     a.vals[col + c] = __float2bfloat16_rn(v * nwv);
     sq = fmaf(v, v, sq);
   }
@@ -523,13 +526,13 @@ Scratch scratch_layout(int64_t B, int64_t d, int64_t di, int64_t H, int64_t M) {
   size_t off = 0;
   auto take = [&](size_t n) { const size_t at = off; off += align256(n); return at; };
   s.x = take((size_t)B * di * 2);
-  s.gate = take((size_t)B * di * 2);
+  s.gate = take((size_t)B * di * 4);
   s.x_conv = take((size_t)B * di * 2);
   s.rw = take((size_t)B * 2 * H * M * 4);
   s.dyn = take((size_t)B * 3 * H * 4);
   s.vals = take((size_t)B * di * 2);
   s.ss = take((size_t)B * H * 4 * 4);
-  s.hid = take(2 * align256((size_t)B * d * 2));
+  s.hid = take(2 * align256((size_t)B * d * 4));
   s.hid_w = take((size_t)B * d * 2);
   s.hid_ss = take((size_t)B * ((d + kTileRows - 1) / kTileRows) * 4);
   s.bytes = off;
@@ -571,11 +574,14 @@ int run_layers(const uint64_t *ptrs, const float *nums, int64_t layers, const vo
     return ceil_div(tiles, ceil_div(tiles, most));
   };
   cudaError_t e = cudaSuccess;
-  const __nv_bfloat16 *hid = reinterpret_cast<const __nv_bfloat16 *>(hidden_in);
+  // the hidden state, float32, in two buffers in turn
+  auto hid_at = [&](int64_t l) { return reinterpret_cast<float *>(at(s.hid) + (l & 1) * align256((size_t)B * d * 4)); };
   __nv_bfloat16 *hid_w = reinterpret_cast<__nv_bfloat16 *>(at(s.hid_w));
   float *hid_ss = reinterpret_cast<float *>(at(s.hid_ss));
-  decode_first_kernel<<<(unsigned)B, kThreads, 0, st>>>(hid, reinterpret_cast<const void *>(ptrs[kNormW]),
-                                                       ptrs[kF32Mask] & 1 ? FRACSSM_F32 : FRACSSM_BF16, hid_w, hid_ss, (int)d);
+  decode_first_kernel<<<(unsigned)B, kThreads, 0, st>>>(reinterpret_cast<const __nv_bfloat16 *>(hidden_in),
+                                                       reinterpret_cast<const void *>(ptrs[kNormW]),
+                                                       ptrs[kF32Mask] & 1 ? FRACSSM_F32 : FRACSSM_BF16, hid_at(0), hid_w,
+                                                       hid_ss, (int)d);
   e = cudaGetLastError();
   for (int64_t l = 0; l < layers && e == cudaSuccess; ++l) {
     const uint64_t *p = ptrs + l * kLayerPtrs;
@@ -584,13 +590,11 @@ int run_layers(const uint64_t *ptrs, const float *nums, int64_t layers, const vo
     auto bfp = [&](int i) { return reinterpret_cast<const __nv_bfloat16 *>(p[i]); };
     auto raw = [&](int i) { return reinterpret_cast<const void *>(p[i]); };
     auto dt = [&](int i) { return (f32 >> i) & 1 ? FRACSSM_F32 : FRACSSM_BF16; };
-    __nv_bfloat16 *next = l + 1 == layers ? reinterpret_cast<__nv_bfloat16 *>(hidden_out)
-                                          : reinterpret_cast<__nv_bfloat16 *>(at(s.hid) + (l & 1) * align256((size_t)B * d * 2));
     LinArgs in{};
     in.w = bfp(kInW); in.n = (int)(2 * di); in.K = (int)d; in.B = (int)B;
     in.act = hid_w; in.ss = hid_ss; in.nss = l == 0 ? 1 : (int)tiles_out; in.eps = f[kEpsIn];
     in.x = reinterpret_cast<__nv_bfloat16 *>(at(s.x));
-    in.gate = reinterpret_cast<__nv_bfloat16 *>(at(s.gate));
+    in.gate = reinterpret_cast<float *>(at(s.gate));
     in.x_conv = reinterpret_cast<__nv_bfloat16 *>(at(s.x_conv));
     in.new_conv = reinterpret_cast<__nv_bfloat16 *>(p[kNewConv]);
     in.old_conv = bfp(kOldConv);
@@ -628,14 +632,15 @@ int run_layers(const uint64_t *ptrs, const float *nums, int64_t layers, const vo
     LinArgs o{};
     o.w = bfp(kOutW); o.n = (int)d; o.K = (int)di; o.B = (int)B;
     o.act = m.vals; o.ss = m.ss; o.nss = (int)(H * splits); o.eps = f[kEpsOut];
-    o.res = hid; o.dst = next;
+    o.res = hid_at(l);
+    if (l + 1 < layers) o.dst = hid_at(l + 1);
+    else o.dst_last = reinterpret_cast<__nv_bfloat16 *>(hidden_out);
     if (l + 1 < layers) {
       o.dst_w = hid_w; o.dst_ss = hid_ss;
       o.next_w = reinterpret_cast<const void *>(p[kLayerPtrs + kNormW]);
       o.next_dt = p[kLayerPtrs + kF32Mask] & 1 ? FRACSSM_F32 : FRACSSM_BF16;
     }
     e = launch_dep(decode_linear_kernel<NT, kOut>, dim3((unsigned)blocks(tiles_out, smem_di)), smem_di, st, true, o);
-    hid = next;
   }
   if (e != cudaSuccess) {
     cudaGetLastError();

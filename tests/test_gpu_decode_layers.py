@@ -87,7 +87,7 @@ def test_native_step_matches_modules(hidden, H, M, B, first):
         assert n.shape == m.shape and n.dtype == m.dtype and torch.equal(n, a)
         scale = e.float().norm().clamp_min(1e-6)
         err, err_m = ((x.float() - e.float()).norm() / scale for x in (n, m))
-        # both round at the same places (the native one less often): the same error up to chance
+        # the native step rounds at the same places or not at all: no larger error, up to chance
         assert err <= 1.25 * err_m + 2e-3, (err, err_m)
 
 
