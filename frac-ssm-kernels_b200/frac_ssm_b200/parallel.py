@@ -111,9 +111,8 @@ def _auto_local_splits(B, L_local, chunk_size, world, device, group=None):
     The scan kernels hand the state from tile to tile of a row, so few rows mean few independent
     chains; sub-segments are extra rows.  Splitting costs one more read of u, kappa and rho, so a
     single rank splits only where the chains are what limits the plain scan by a wide margin: at most
-    28 rows (one tile step of a chain takes about 2.8 us, a CTA needs about 7.6 us per tile, so
-    148 SMs are busy from some 54 rows on, and the extra read costs about 60 % of a scan) and at
-    least 32768 tokens (measured on 24 rows x 1,048,576 tokens: 22.7 ms plain, 16.9 ms cut in 8).
+    28 rows and at least 32768 tokens.  (The line is from when a tile step of a chain took 2.8 us; at
+    1.0 us `frac_scan` leaves 12 rows and more whole and only asks below, see its WHOLE_ROWS.)
     Each rank can only judge its own segment (segments differ by a chunk
     when the chunk count does not divide by the world size, and the last one may be ragged), so the
     ranks agree on the smallest of their candidates with one MIN all-reduce of a single integer;
