@@ -29,7 +29,8 @@ def transformed():
     """True under anything that has to see the individual operations."""
     return (torch.compiler.is_compiling() or torch.is_autocast_enabled("cuda") or bool(_nn_module._global_forward_hooks)
             or bool(_nn_module._global_forward_pre_hooks) or torch._C._len_torch_dispatch_stack() > 0
-            or torch._C._len_torch_function_stack() > 0 or torch._C._functorch.peek_interpreter_stack() is not None)
+            or torch._C._len_torch_function_stack() > 0 or torch._C._functorch.peek_interpreter_stack() is not None
+            or torch._C._get_tracing_state() is not None or torch.autograd.forward_ad._current_level >= 0)
 
 
 def layer_params(layers, classes, sizes, dev):

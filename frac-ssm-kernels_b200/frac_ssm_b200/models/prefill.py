@@ -110,6 +110,7 @@ def prefill_layers(layers, h, attention_mask, use_cache, classes):
                                             p_x + 2 * di, 2 * di, p_mask, params, f32_mask >> 7 & 63, numbers, p_u, p_c,
                                             p_k, ck, p_rho, p_h, p_fin, states[i].data_ptr() if use_cache else 0, p_y,
                                             p_ws, ws.numel(), B, L, H, R, M, T, stream), "prefill_mix")
+            del xg, dyn, rw      # (or the next layer's would be allocated beside them)
             out = F.linear(y, out_w)
         h = (res + out).view(B, L, d)
     return h, tuple(zip(states, tails)) if use_cache else None
