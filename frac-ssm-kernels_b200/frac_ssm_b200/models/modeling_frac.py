@@ -5,7 +5,8 @@ Per layer, prefill runs: in_proj (library GEMM) -> causal depthwise conv + SiLU 
 dyn_proj / rw_proj (library GEMMs) -> parameter prep (CUDA kernel) -> frac_scan (single-pass tcgen05
 kernel when the shape allows, else the staged kernels) -> skip-mix + gated RMSNorm (one CUDA kernel)
 -> out_proj (library GEMM).  Decode runs one token through the conv window, the same parameter prep
-with L = 1 and the state-update kernel.  The cache is the reference's: per layer
+with L = 1 and the state-update kernel.  bfloat16 models take the same steps through all layers with few
+native calls instead (`decode.py`, `prefill.py`).  The cache is the reference's: per layer
 (state [B, H, M, R] float32, conv_state [B, C, K-1]).
 """
 
