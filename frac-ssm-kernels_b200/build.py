@@ -51,7 +51,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OUT_DIR, exist_ok=True)
     os.makedirs(OBJ_DIR, exist_ok=True)
     nvcc = _nvcc()
-    headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
+    headers = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
     sources = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
     test_sources = sorted(glob.glob(os.path.join(CSRC, "selftest", "*.cu")))
     objs, test_objs, jobs = [], [], []

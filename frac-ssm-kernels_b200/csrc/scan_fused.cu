@@ -345,7 +345,7 @@ scan_fused_kernel(const FusedArgs a, const __grid_constant__ CUtensorMap u_map) 
           const uint64_t t_start = umma::global_ns();
           while (ld_acquire(a.flags + bh) < jt) {
             __nanosleep(100);
-            if (umma::global_ns() - t_start > wait_ns) { ok = false; *failed = 1; break; }
+            if (umma::past_limit(t_start, umma::global_ns(), wait_ns)) { ok = false; *failed = 1; break; }
           }
         }
         umma::mbar_arrive(state_bar);
@@ -1010,7 +1010,7 @@ scan_fused_kernel(const FusedArgs a, const __grid_constant__ CUtensorMap u_map) 
                 request(half);
                 if (arrived(half)) break;
                 if (spins == 256) t_start = umma::global_ns();
-                if (__any_sync(0xffffffffu, spins > 256 && umma::global_ns() - t_start > wait_ns)) {
+                if (__any_sync(0xffffffffu, spins > 256 && umma::past_limit(t_start, umma::global_ns(), wait_ns))) {
                   ok = false;
                   *failed = 1;
                 }

@@ -154,7 +154,7 @@ scan_summary_kernel(const SummaryArgs a, const __grid_constant__ CUtensorMap u_m
             const uint64_t t_start = umma::global_ns();
             while (ld_acquire(a.flags + bh) < j) {
               __nanosleep(100);
-              if (umma::global_ns() - t_start > wait_ns) { ok = false; *failed = 1; break; }
+              if (umma::past_limit(t_start, umma::global_ns(), wait_ns)) { ok = false; *failed = 1; break; }
             }
           }
           umma::mbar_arrive(state_bar);

@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "wait_limit.h"
+
 namespace fracssm {
 namespace umma {
 
@@ -58,7 +60,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint64
   const uint64_t t0 = global_ns();
   while (!mbar_test(bar, parity)) {
     __nanosleep(64);
-    if (global_ns() - t0 > limit_ns) return false;
+    if (past_limit(t0, global_ns(), limit_ns)) return false;
   }
   return true;
 }
@@ -81,7 +83,7 @@ __device__ __forceinline__ bool mbar_wait_parked(uint64_t *bar, uint32_t parity,
         : "memory");
     if (ok) return true;
     if (spins == 64) t0 = global_ns();
-    if (spins > 64 && global_ns() - t0 > limit_ns) return false;
+    if (spins > 64 && past_limit(t0, global_ns(), limit_ns)) return false;
   }
 }
 // Barrier among the first `nthreads` threads of the CTA (a multiple of 32), id 1..15.
