@@ -219,15 +219,18 @@ __device__ __forceinline__ void emit_pair_next_slot(uint32_t rows_s, int i, uint
   asm volatile("st.shared.b32 [%0+32768], %1;" ::"r"(addr), "r"(w0) : "memory");
 }
 
-// A piece of the state with its tile's number beside every value (LL, below): 8-byte halves are written and read whole.
+// A piece of the state with its tile's number beside every value (LL, below).  Value and number are one 64-bit element of
+// a strong access, which the memory model reads and writes whole (a .v4.u32 access would be four accesses in no order).
 __device__ __forceinline__ uint4 ld_tagged(const uint4 *p) {
-  uint4 v;
-  asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-  return v;
+  uint64_t lo, hi;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0,%1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+  return make_uint4(static_cast<uint32_t>(lo), static_cast<uint32_t>(lo >> 32), static_cast<uint32_t>(hi),
+                    static_cast<uint32_t>(hi >> 32));
 }
 __device__ __forceinline__ void st_tagged(uint4 *p, float a, float b, uint32_t tag) {
-  asm volatile("st.volatile.global.v4.u32 [%0], {%1,%2,%3,%2};" ::"l"(p), "r"(__float_as_uint(a)), "r"(tag),
-               "r"(__float_as_uint(b)) : "memory");
+  const uint64_t t = static_cast<uint64_t>(tag) << 32;
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1,%2};" ::"l"(p), "l"(t | __float_as_uint(a)),
+               "l"(t | __float_as_uint(b)) : "memory");
 }
 
 // LL: the state is handed from tile to tile with its tile's number beside every value, and the threads that need it
