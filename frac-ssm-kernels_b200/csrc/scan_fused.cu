@@ -994,12 +994,12 @@ scan_fused_kernel(const FusedArgs a, const __grid_constant__ CUtensorMap u_map) 
 #pragma unroll
             for (int x = 0; x < 4; ++x) v[half][x] = jt > 0 ? ld_tagged(ll + (4 * half + x) * kM + m_row) : make_uint4(0, 0, 0, 0);
           };
-          auto arrived = [&](int half) {
+          auto missing = [&](int half) {   // of this thread's own values
             uint32_t miss = 0;
 #pragma unroll
             for (int x = 0; x < 4; ++x)
               miss |= (v[half][x].y ^ static_cast<uint32_t>(jt)) | (v[half][x].w ^ static_cast<uint32_t>(jt));
-            return __all_sync(0xffffffffu, miss == 0 || jt == 0) != 0;
+            return miss != 0 && jt != 0;
           };
           request(0);
           FRACSSM_WAIT(cbK, n);
@@ -1007,13 +1007,17 @@ scan_fused_kernel(const FusedArgs a, const __grid_constant__ CUtensorMap u_map) 
           const bool bad = *failed != 0;
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
-            if (!arrived(half)) {   // read again until the tags are there (looking at one sector first made a step 0.15 us longer)
+            // read again until the tags are there (looking at one sector first made a step 0.15 us longer).  A lane waits
+            // for its own tags and votes on nothing: in the waits each lane reads the timer for itself, so `ok` may
+            // differ between lanes, and a vote inside a loop that only some of them run would have no end.  (24 x 1048576
+            // tokens 13.8 ms; 13.65 with the vote inside, 14.2 to 14.5 where the warp agrees on `ok` first.)
+            if (missing(half)) {
               uint64_t t_start = 0;
               for (uint32_t spins = 0; ok; ++spins) {
                 request(half);
-                if (arrived(half)) break;
+                if (!missing(half)) break;
                 if (spins == 256) t_start = umma::global_ns();
-                if (__any_sync(0xffffffffu, spins > 256 && umma::past_limit(t_start, umma::global_ns(), wait_ns))) {
+                if (spins > 256 && umma::past_limit(t_start, umma::global_ns(), wait_ns)) {
                   ok = false;
                   *failed = 1;
                 }

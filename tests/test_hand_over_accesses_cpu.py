@@ -19,3 +19,14 @@ def test_no_volatile_vector_access():
         if name.endswith((".cu", ".cuh")):
             text = open(os.path.join(CSRC, name)).read()
             assert not re.search(r'"(ld|st)\.volatile[.a-z]*\.v\d', text), name
+
+
+def test_no_vote_inside_a_loop_that_a_lane_leaves_for_itself():
+    """After a wait a lane's own `ok` may differ from its neighbours': a vote of the whole warp inside a loop over it
+    would wait for lanes that never come."""
+    for name in os.listdir(CSRC):
+        if name.endswith((".cu", ".cuh")):
+            text = open(os.path.join(CSRC, name)).read()
+            for head in re.finditer(r"for \([^;)]*;\s*ok\b[^;]*;[^)]*\) \{", text):
+                body = text[head.end():text.index("\n              }\n", head.end())]
+                assert not re.search(r"_sync\(|arrived\(", body), (name, head.group(0))
