@@ -17,7 +17,7 @@ from torch import nn
 from .. import _cabi as C
 from .. import parallel
 from ..modules.rmsnorm_gated import rmsnorm_gated_fwd
-from ..ops.b200.frac_scan import WHOLE_ROWS
+from ..ops.b200.frac_scan import taken_whole
 from .decode import layer_params, transformed
 
 _MAX_NORM = 2048      # longest row of fracssm_add_rmsnorm
@@ -42,7 +42,7 @@ def prefill_layers(layers, h, attention_mask, use_cache, classes):
     dev = h.get_device()
     if not 2 <= K <= 8 or not isinstance(T, int) or T < 1 or B * H > 65535:
         return None
-    if B * H < WHOLE_ROWS and parallel._auto_local_splits(B * H, L, T, 1, h.device) > 1:   # frac_scan cuts them up
+    if not taken_whole(B * H, L) and parallel._auto_local_splits(B * H, L, T, 1, h.device) > 1:   # frac_scan cuts them up
         return None
     mask = None
     if attention_mask is not None:

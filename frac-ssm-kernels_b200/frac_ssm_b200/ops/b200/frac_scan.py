@@ -31,9 +31,9 @@ def frac_scan(u, c, kappa, rho, chunk_size, initial_state=None, return_final_sta
         final_state_dtype: dtype of the returned state; default follows the reference
             (bfloat16 when u is bfloat16, else float32).  The state is always carried in float32.
         path: "auto", "staged" or "fused".  "auto" takes the single-pass kernel when it covers the
-            shape (else the segment kernels up to 128 modes, else the staged ones), and for very few rows with many tokens (fewer than 12 rows, at least 32768 tokens) cuts
-            every row into sub-segments first, because a row is one chain of tiles and 148 SMs want
-            more chains than that: one summary pass over u, kappa and rho gives every sub-segment its
+            shape (else the segment kernels up to 128 modes, else the staged ones), and for very few rows with many tokens (fewer than 12 rows from 32768 tokens on, 12
+            and 13 rows from 131072 on) cuts every row into sub-segments first, because a row is one chain of
+            tiles and 148 SMs want more chains than that: one summary pass over u, kappa and rho gives every sub-segment its
             incoming state, then all sub-segments are scanned as rows (`parallel.seq_parallel_scan`).
         check: after the launch, synchronise and raise if a bounded device-side wait of the
             single-pass kernel ran out (debugging aid; the default stays asynchronous).
@@ -85,10 +85,24 @@ def frac_scan(u, c, kappa, rho, chunk_size, initial_state=None, return_final_sta
     return h
 
 
-# Rows from which the single-pass kernel takes long rows as they are: its chain of tiles advances a tile per 1.05 us
-# and row, a CTA needs some 10 us a tile, and cutting the rows costs a second read of u, kappa and rho (131072 tokens:
-# 8 rows 1.17 ms whole, 1.19 cut; 12 rows 1.25 and 1.20; 16 rows 1.37 and 1.54; 24 rows of 1048576 tokens 13.7 and 16.7).
-WHOLE_ROWS = 12
+def taken_whole(B, L):
+    """Whether the single-pass kernel takes B rows of L tokens as they are, however long.
+
+    Whole, a row's chain of tiles advances a tile per 1.05 us and a CTA needs some 10 us a tile; cutting the rows costs
+    a second read of u, kappa and rho and a step on the host per sub-segment, some 13 us each where nothing hides it.
+    Milliseconds whole / cut, bfloat16 coefficients (float32 lies the same way):
+
+                     32768          131072         524288         1048576
+         8 rows   0.36 / 1.53    1.21 / 1.34    4.66 / 3.05    9.23 / 5.77
+        12 rows   0.42 / 0.68    1.29 / 1.21    4.91 / 4.23    9.75 / 8.23
+        13 rows   0.40 / 0.70    1.29 / 1.30    4.95 / 4.56    9.86 / 9.03
+        14 rows   0.38 / 0.70    1.33 / 1.39    5.05 / 4.90   10.01 / 10.10
+        24 rows   0.50 / 0.65    1.77 / 2.11    6.82 / 8.04   13.74 / 16.59
+
+    Below 12 rows the line stays at the 32768 tokens of `parallel._auto_local_splits`, although fewer than 131072 (and
+    up to 4 rows more) would be faster whole: both entry points cut there.
+    """
+    return B >= 14 or (B >= 12 and L < 131072)
 
 
 def _row_splits(u, c, chunk_size):
@@ -96,7 +110,7 @@ def _row_splits(u, c, chunk_size):
     both the call and the cut-up call, the tensors are dense, and the rows are few and long."""
     from ... import parallel
     B, L, R = u.shape
-    if B < 1 or B >= WHOLE_ROWS or not (u.is_contiguous() and c.is_contiguous()) or u.dtype != torch.bfloat16:
+    if B < 1 or taken_whole(B, L) or not (u.is_contiguous() and c.is_contiguous()) or u.dtype != torch.bfloat16:
         return 1
     splits = parallel._auto_local_splits(B, L, chunk_size, 1, u.device)
     if splits > 1 and not C.lib().fracssm_scan_fused_supported(B * splits, L // splits, R, c.shape[-1],

@@ -112,7 +112,7 @@ def _auto_local_splits(B, L_local, chunk_size, world, device, group=None):
     chains; sub-segments are extra rows.  Splitting costs one more read of u, kappa and rho, so a
     single rank splits only where the chains are what limits the plain scan by a wide margin: at most
     28 rows and at least 32768 tokens.  (The line is from when a tile step of a chain took 2.8 us; at
-    1.0 us `frac_scan` leaves 12 rows and more whole and only asks below, see its WHOLE_ROWS.)
+    1.0 us `frac_scan` takes more calls whole and only asks for the others, see its `taken_whole`.)
     Each rank can only judge its own segment (segments differ by a chunk
     when the chunk count does not divide by the world size, and the last one may be ragged), so the
     ranks agree on the smallest of their candidates with one MIN all-reduce of a single integer;

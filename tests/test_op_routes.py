@@ -31,3 +31,16 @@ def test_direct_only_where_nothing_observes_the_op():
         seen.append(stages._unobserved((x,)))
     torch.jit.trace(lambda t: seen.append(stages._unobserved((t,))) or t + 1, x, check_trace=False)
     assert seen and not any(seen)
+
+
+def test_few_long_rows_are_cut_where_that_was_measured_to_be_faster():
+    import importlib
+    fs = importlib.import_module("frac_ssm_b200.ops.b200.frac_scan")
+
+    def splits(B, L):
+        u = torch.empty(B, L, 64, dtype=torch.bfloat16, device="meta")
+        return fs._row_splits(u, torch.empty(B, L, 128, dtype=torch.bfloat16, device="meta"), 256)
+    assert splits(12, 1048576) == 16 and splits(13, 524288) == 16 and splits(12, 131072) == 16
+    assert splits(12, 65536) == splits(13, 32768) == 1       # 12 x 32768 tokens: 0.42 ms whole, 0.68 cut
+    assert splits(14, 1048576) == splits(24, 1048576) == 1   # 24 rows: 13.7 ms whole, 16.6 cut
+    assert splits(8, 1048576) == 32 and splits(3, 32768) == 32
