@@ -53,8 +53,17 @@ extern "C" size_t fracssm_frac_scan_workspace_bytes(int64_t B, int64_t L, int64_
   const size_t fused = scan_fused_workspace_bytes(B, L, R, M, T);
   if (path == 1) return staged;
   if (path == 2) return fused;
+  const size_t alone = fracssm_frac_scan_auto_workspace_bytes(B, L, R, M, T);
+  return staged > alone ? staged : alone;
+}
+
+extern "C" size_t fracssm_frac_scan_auto_workspace_bytes(int64_t B, int64_t L, int64_t R, int64_t M, int64_t T) {
+  using namespace fracssm;
+  if (B <= 0 || L <= 0 || R <= 0 || M <= 0 || T <= 0) return 0;
+  const size_t fused = scan_fused_workspace_bytes(B, L, R, M, T);
   // which of the two automatic routes a call takes also depends on types and strides
-  const size_t other = scan_few_supported(B, L, R, M, T) ? scan_few_workspace_bytes(B, L, R, M) : staged;
+  const size_t other = scan_few_supported(B, L, R, M, T) ? scan_few_workspace_bytes(B, L, R, M)
+                                                         : staged_layout(nullptr, B, L, R, M, T).bytes;
   return other > fused ? other : fused;
 }
 

@@ -39,6 +39,7 @@ _SIGNATURES = {
     "fracssm_chunk_fused_readout": (ci, [vp, ci, i64, i64, vp, vp, ci, i64, i64, i64, i64, vp, ci,
                                          vp, i64, i64, vp, i64, i64, i64, i64, i64, vp]),
     "fracssm_frac_scan_workspace_bytes": (sz, [i64, i64, i64, i64, i64, ci]),
+    "fracssm_frac_scan_auto_workspace_bytes": (sz, [i64, i64, i64, i64, i64]),
     "fracssm_frac_scan_fwd": (ci, [vp, ci, i64, i64, vp, vp, ci, i64, i64, i64, i64, vp, i64, i64,
                                    vp, vp, vp, ci, vp, sz, i64, i64, i64, i64, i64, ci, vp]),
     "fracssm_frac_scan_fwd_noalloc": (ci, [vp, vp, vp, vp, vp, vp, vp, ci, i64, i64, i64, i64, vp]),

@@ -71,7 +71,7 @@ def prefill_layers(layers, h, attention_mask, use_cache, classes):
     rows = B * L
     with C.trace("prefill_layers"), torch.cuda.device(dev):
         stream = C.stream_of(h)
-        nbytes = lib.fracssm_frac_scan_workspace_bytes(B * H, L, R, M, T, C.PATH_AUTO)
+        nbytes = lib.fracssm_frac_scan_auto_workspace_bytes(B * H, L, R, M, T)
         ws = empty(max(nbytes, 256), dtype=torch.uint8)
         x_conv, u, scan_out, y = empty(rows, di), empty(B * H, L, R), empty(B * H, L, R), empty(rows, di)
         c, kappa, rho = empty(B * H, L, M, dtype=coeff), empty(B * H, L, M, dtype=coeff), empty(B * H, L, M, dtype=f32)

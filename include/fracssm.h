@@ -115,13 +115,19 @@ int fracssm_chunk_fused_readout(const void *u, int u_dtype, int64_t u_sb, int64_
  * rho [B,L,M] f32; initial_state [B,R,M] f32 or NULL; h [B,L,R] in u's dtype;
  * final_state [B,R,M] (final_dtype f32 or bf16) or NULL.  workspace: device scratch of at
  * least fracssm_frac_scan_workspace_bytes(...) bytes, 256-byte aligned, caller-owned.
- * path: 0 = pick (single-pass tcgen05 kernel when the shape is covered, else staged),
+ * path: 0 = pick (single-pass tcgen05 kernel when the shape, types, strides and alignment are covered, else
+ *           up to 128 modes the segment kernels, else staged),
  *       1 = staged kernels, 2 = single-pass kernel (error if the shape is not covered).
+ * A workspace sized with path 0 serves every path.  fracssm_frac_scan_auto_workspace_bytes is what calls with
+ * path 0 need by themselves, without the intermediates of the staged kernels where no such call takes them (at
+ * 192 rows x 8192 tokens, R = 64, M = 128: 6 MB against 1.2 GB).  A path 0 call whose workspace only holds the
+ * staged kernels' intermediates takes those.
  * Replaces frac_ssm/ops/frac_scan.py:53 `frac_scan(...)` /
  * frac_ssm/ops/triton/frac_scan.py:102.
  */
 size_t fracssm_frac_scan_workspace_bytes(int64_t B, int64_t L, int64_t R, int64_t M, int64_t T,
                                          int path);
+size_t fracssm_frac_scan_auto_workspace_bytes(int64_t B, int64_t L, int64_t R, int64_t M, int64_t T);
 int fracssm_frac_scan_fwd(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, const void *c,
                           const void *kappa, int ck_dtype, int64_t c_sb, int64_t c_sl,
                           int64_t k_sb, int64_t k_sl, const float *rho, int64_t r_sb, int64_t r_sl,
@@ -367,7 +373,7 @@ int fracssm_decode_layers(const uint64_t *layer_ptrs, const float *layer_nums, i
  * read_residual_logit, write_residual_scale, base_log_tau, D, output norm weight, bit i of params_f32 set where
  * parameter i is float32, else bf16; nums (host): read_temp, dt_min, dt_max, alpha_min, alpha_max, lambda_min,
  * lambda_max, gate bias, eps.  Scratch of the caller: c, kappa [Bt*H, L, M] (ck_dtype), rho, h, final_state
- * [Bt*H, R, M] (needed with state), workspace (fracssm_frac_scan_workspace_bytes of path 0).  Results: state [Bt, H, M, R]
+ * [Bt*H, R, M] (needed with state), workspace (fracssm_frac_scan_auto_workspace_bytes).  Results: state [Bt, H, M, R]
  * (or NULL) and y [Bt, L, HR].
  */
 int fracssm_add_rmsnorm(const void *x, const void *y, const void *weight, int w_dtype, float eps, void *sum, void *norm,
