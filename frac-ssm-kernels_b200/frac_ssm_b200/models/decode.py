@@ -125,6 +125,7 @@ def decode_layers(layers, h, past, use_cache, classes):
     found = layer_params(layers, classes, sizes, dev)
     if found is None:
         return None
+    states = convs = None
     if past is None or all(p is None for p in past):
         olds = [(0, 0)] * n
     else:
@@ -153,11 +154,13 @@ def decode_layers(layers, h, past, use_cache, classes):
         nums += numbers
     new_past = None
     if use_cache:
-        states = torch.empty(n, B, H, M, R, device=h.device, dtype=torch.float32).unbind(0)
-        convs = torch.empty(n, B, di, 3, device=h.device, dtype=torch.bfloat16).unbind(0)
-        for i in range(n):
-            ptrs[i * _PTRS + 16] = states[i].data_ptr()
-            ptrs[i * _PTRS + 17] = convs[i].data_ptr()
+        # (a tensor of its own for each layer: who keeps or saves one keeps no other)
+        if states is None:
+            states = [torch.empty(B, H, M, R, device=h.device, dtype=torch.float32)] * n
+            convs = [torch.empty(B, di, 3, device=h.device, dtype=torch.bfloat16)] * n
+        states, convs = list(map(torch.empty_like, states)), list(map(torch.empty_like, convs))
+        ptrs[16::_PTRS] = map(_ptr, states)
+        ptrs[17::_PTRS] = map(_ptr, convs)
         new_past = tuple(zip(states, convs))
     table, numbers = array.array("Q", ptrs), array.array("f", nums)
     out = torch.empty(B, 1, d, device=h.device, dtype=torch.bfloat16)

@@ -79,8 +79,11 @@ def prefill_layers(layers, h, attention_mask, use_cache, classes):
         fin = states = tails = None
         if use_cache:
             fin = empty(B * H, R, M, dtype=f32)
-            states = empty(n_layers, B, H, M, R, dtype=f32).unbind(0)
-            tails = empty(n_layers, B, di, K - 1).unbind(0)
+            # (a tensor of its own for each layer: who keeps or saves one keeps no other)
+            states, tails = [empty(B, H, M, R, dtype=f32)], [empty(B, di, K - 1)]
+            for _ in range(n_layers - 1):
+                states.append(torch.empty_like(states[0]))
+                tails.append(torch.empty_like(tails[0]))
         p_ws, p_conv, p_u, p_h, p_y, p_c, p_k, p_rho, p_fin, p_norm, p_mask = (
             0 if t is None else t.data_ptr() for t in (ws, x_conv, u, scan_out, y, c, kappa, rho, fin, normed, mask))
         ck = C.dt_of(coeff)

@@ -111,6 +111,21 @@ def test_what_the_native_step_does_not_cover_still_runs():
             assert (a.float() - b.float()).norm() <= 2e-2 * b.float().norm() + 1e-3
 
 
+def test_each_layers_cache_is_a_tensor_of_its_own():
+    half = _model(64, 2, 8, layers=3).to(torch.bfloat16)
+    ids = torch.ones(2, 1, dtype=torch.long).cuda()
+    with _Count() as count:
+        first = half(ids, use_cache=True)[1]
+        then = half(ids, past_key_values=first, use_cache=True)[1]
+        assert count.n == 2
+    prompt = half(torch.ones(2, 9, dtype=torch.long).cuda(), use_cache=True)[1]
+    for past in (first, then, prompt):
+        tensors = [t for pair in past for t in pair]
+        assert len({t.untyped_storage().data_ptr() for t in tensors}) == 6
+        for t in tensors:
+            assert t.untyped_storage().nbytes() == t.numel() * t.element_size() and not t._is_view()
+
+
 def test_native_step_in_a_cuda_graph():
     half = _model(256, 4, 16).to(torch.bfloat16)
     ids = torch.ones(2, 1, dtype=torch.long).cuda()
