@@ -2,14 +2,14 @@
 
 Covers bfloat16 models on one GPU, one token per sequence, up to 64 sequences, no attention mask.  The
 parameters are looked up in the modules on every call (nothing is remembered between calls), and whatever
-this route would pass by (hooks, replaced or subclassed modules, autocast, tracing, function transforms)
+this route would pass by (hooks, replaced, patched or subclassed modules, autocast, tracing, function transforms)
 sends the call back to the modules' own forward.
 """
 
 from __future__ import annotations
 
 import array
-from itertools import repeat
+from itertools import chain, repeat
 from operator import attrgetter, contains, itemgetter
 
 import torch
@@ -21,7 +21,8 @@ from .. import _cabi as C
 _PTRS = 19      # columns of the pointer table of fracssm_decode_layers
 _ptr = torch.Tensor.data_ptr
 _MAY_BE_F32 = 1 << 0 | 0b111111 << 7      # the norm weights and the small parameters
-_PARTS = ("in_proj", "conv1d", "dyn_proj", "rw_proj", "out_norm", "out_proj")
+_parts = itemgetter("in_proj", "conv1d", "dyn_proj", "rw_proj", "out_norm", "out_proj")
+_modules, _parameters = itemgetter("_modules"), itemgetter("_parameters")
 _TENSORS = frozenset((nn.Parameter, torch.Tensor))
 
 
@@ -48,27 +49,30 @@ def layer_params(layers, classes, sizes, dev):
     norms, mixers = [m["norm"] for m in inner], [m["mixer"] for m in inner]
     if set(map(type, mixers)) != {mixer_cls} or set(map(type, norms)) != {norm_cls}:
         return None
-    parts = [list(map(m.__dict__["_modules"].__getitem__, _PARTS)) for m in mixers]
-    if any([type(p) for p in ps] != [nn.Linear, nn.Conv1d, nn.Linear, nn.Linear, gated_cls, nn.Linear] for ps in parts):
+    own = list(map(vars, mixers))
+    parts = list(chain.from_iterable(map(_parts, map(_modules, own))))      # six a layer
+    if list(map(type, parts)) != [nn.Linear, nn.Conv1d, nn.Linear, nn.Linear, gated_cls, nn.Linear] * len(layers):
         return None
-    dicts = [m.__dict__ for m in layers + norms + mixers] + [p.__dict__ for ps in parts for p in ps]
+    part_dicts = list(map(vars, parts))
+    dicts = [*map(vars, layers), *map(vars, norms), *own, *part_dicts]
     if (any(map(itemgetter("_forward_hooks"), dicts)) or any(map(itemgetter("_forward_pre_hooks"), dicts))
-            or any(map(contains, dicts, repeat("forward")))):
+            or any(map(contains, dicts, repeat("forward"))) or any(map(contains, own, repeat("_scan_params")))
+            or any(map(contains, own, repeat("_conv_state_after")))):
         return None
     counts = (d, 2 * di * d, K * di, di, 3 * H * di, 3 * H, 2 * H * M * di, H, 1, 1, M, di, di, d * di)
     found, every, expected = [], [], []
     last_cfg = cfg_nums = None
-    for norm, mixer, ps in zip(norms, mixers, parts):
-        in_proj, conv1d, dyn, rw, out_norm, out_proj = [p.__dict__["_parameters"] for p in ps]
+    held = map(_parameters, part_dicts)
+    for i, (norm, m, in_proj, conv1d, dyn, rw, out_norm, out_proj) in enumerate(zip(norms, own, held, held, held, held, held,
+                                                                                    held)):
         if in_proj["bias"] is not None or out_proj["bias"] is not None:
             return None        # (a bias of rw_proj is not read by the modules either)
-        m = mixer.__dict__
         if m["num_heads"] != H or m["head_dim"] != R or m["num_modes"] != M or m["conv_kernel"] != K:
             return None
-        own = m["_parameters"]
-        tensors = (norm.__dict__["_parameters"]["weight"], in_proj["weight"], conv1d["weight"], conv1d["bias"], dyn["weight"],
-                   dyn["bias"], rw["weight"], own["dt_bias"], own["read_residual_logit"], own["write_residual_scale"],
-                   m["_buffers"]["base_log_tau"], own["D"], out_norm["weight"], out_proj["weight"])
+        p, norm = m["_parameters"], vars(norm)
+        tensors = (norm["_parameters"]["weight"], in_proj["weight"], conv1d["weight"], conv1d["bias"], dyn["weight"],
+                   dyn["bias"], rw["weight"], p["dt_bias"], p["read_residual_logit"], p["write_residual_scale"],
+                   m["_buffers"]["base_log_tau"], p["D"], out_norm["weight"], out_proj["weight"])
         if tensors[3] is None or tensors[5] is None:
             every += [t for t in tensors if t is not None]
             expected += [n for t, n in zip(tensors, counts) if t is not None]
@@ -79,7 +83,7 @@ def layer_params(layers, classes, sizes, dev):
         if cfg is not last_cfg:
             last_cfg, cfg_nums = cfg, (cfg.frac_dt_min, cfg.frac_dt_max, cfg.frac_alpha_min, cfg.frac_alpha_max,
                                        cfg.frac_lambda_min, cfg.frac_lambda_max, cfg.frac_gate_bias_init)
-        found.append((tensors, (norm.__dict__["variance_epsilon"], ps[4].__dict__["variance_epsilon"], m["read_temp"], *cfg_nums)))
+        found.append((tensors, (norm["variance_epsilon"], part_dicts[6 * i + 4]["variance_epsilon"], m["read_temp"], *cfg_nums)))
     T = torch.Tensor
     if not _TENSORS.issuperset(map(type, every)):      # (a missing weight is no tensor either)
         return None
