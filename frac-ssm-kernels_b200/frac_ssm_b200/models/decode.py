@@ -36,9 +36,15 @@ def transformed():
 
 def layer_params(layers, classes, sizes, dev):
     """Per layer its 14 parameters (None for an absent bias), the bit mask of those that are float32, and its numbers,
-    in the order of the tables of fracssm_decode_layers; None when native code does not cover the layers.
+    in the order of the tables of fracssm_decode_layers; None when native code does not cover the layers."""
+    try:
+        return _layer_params(layers, classes, sizes, dev)
+    except (KeyError, AttributeError):      # something is not where the modules' own __init__ puts it
+        return None
 
-    The same question goes to all modules or parameters at once: there are hundreds of each, and asked one by one
+
+def _layer_params(layers, classes, sizes, dev):
+    """The same question goes to all modules or parameters at once: there are hundreds of each, and asked one by one
     the answers cost as much as the launches."""
     d, H, R, M, K, di = sizes
     block_cls, norm_cls, mixer_cls, gated_cls = classes

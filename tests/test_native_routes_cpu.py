@@ -55,3 +55,22 @@ def test_a_patched_class_or_function_keeps_the_modules(monkeypatch, owner, name)
     original = getattr(owner, name)
     monkeypatch.setattr(owner, name, lambda *a, **k: original(*a, **k))
     assert not mf.as_defined()
+
+
+@pytest.mark.parametrize("path,name", [("layers.1.norm", "weight"), ("layers.0.mixer.in_proj", "weight"), ("layers.2.mixer", "D"),
+                                       ("layers.1.mixer.dyn_proj", "bias"), ("layers.1.mixer", "base_log_tau"),
+                                       ("layers.0.mixer.conv1d", "weight"), ("layers.0.mixer.in_proj", "bias")])
+def test_a_tensor_kept_as_a_plain_attribute_keeps_the_modules(path, name):
+    """(deleted as a parameter or buffer and set again: the modules' own forward finds it all the same)"""
+    model = _model()
+    module = model.get_submodule(path)
+    value = getattr(module, name)
+    delattr(module, name)
+    object.__setattr__(module, name, None if value is None else value.detach())
+    assert _looked_at(model) is None
+
+
+def test_a_property_in_the_place_of_a_number_keeps_the_modules():
+    model = _model()
+    del model.layers[1].mixer.__dict__["read_temp"]
+    assert _looked_at(model) is None
