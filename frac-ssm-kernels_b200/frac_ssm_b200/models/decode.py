@@ -66,7 +66,7 @@ def _layer_params(layers, classes, sizes, dev):
             or any(map(contains, own, repeat("_conv_state_after")))):
         return None
     counts = (d, 2 * di * d, K * di, di, 3 * H * di, 3 * H, 2 * H * M * di, H, 1, 1, M, di, di, d * di)
-    found, every, expected = [], [], []
+    found, every, expected, products = [], [], [], []
     last_cfg = cfg_nums = None
     held = map(_parameters, part_dicts)
     for i, (norm, m, in_proj, conv1d, dyn, rw, out_norm, out_proj) in enumerate(zip(norms, own, held, held, held, held, held,
@@ -79,6 +79,7 @@ def _layer_params(layers, classes, sizes, dev):
         tensors = (norm["_parameters"]["weight"], in_proj["weight"], conv1d["weight"], conv1d["bias"], dyn["weight"],
                    dyn["bias"], rw["weight"], p["dt_bias"], p["read_residual_logit"], p["write_residual_scale"],
                    m["_buffers"]["base_log_tau"], p["D"], out_norm["weight"], out_proj["weight"])
+        products += (tensors[1], tensors[4], tensors[6], tensors[13])
         if tensors[3] is None or tensors[5] is None:
             every += [t for t in tensors if t is not None]
             expected += [n for t, n in zip(tensors, counts) if t is not None]
@@ -94,6 +95,8 @@ def _layer_params(layers, classes, sizes, dev):
     if not _TENSORS.issuperset(map(type, every)):      # (a missing weight is no tensor either)
         return None
     if set(map(T.get_device, every)) != {dev} or list(map(T.numel, every)) != expected or not all(map(T.is_contiguous, every)):
+        return None
+    if list(map(attrgetter("shape"), products)) != [(2 * di, d), (3 * H, di), (2 * H * M, di), (d, di)] * len(layers):
         return None
     bf16 = torch.bfloat16
     if set(map(attrgetter("dtype"), every)) == {bf16}:

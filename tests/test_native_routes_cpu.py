@@ -74,3 +74,12 @@ def test_a_property_in_the_place_of_a_number_keeps_the_modules():
     model = _model()
     del model.layers[1].mixer.__dict__["read_temp"]
     assert _looked_at(model) is None
+
+
+@pytest.mark.parametrize("path", ["layers.0.mixer.in_proj", "layers.2.mixer.out_proj", "layers.1.mixer.rw_proj", "layers.1.mixer.dyn_proj"])
+def test_a_weight_of_another_shape_keeps_the_modules(path):
+    """(which refuse it) although it has as many elements"""
+    model = _model()
+    module = model.get_submodule(path)
+    module.weight = torch.nn.Parameter(module.weight.detach().t().contiguous())
+    assert _looked_at(model) is None
