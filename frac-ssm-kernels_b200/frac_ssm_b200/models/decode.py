@@ -146,6 +146,8 @@ def decode_layers(layers, h, past, use_cache, classes):
             return None
         states, convs = [p[0] for p in past], [p[1] for p in past]
         f32, bf16 = torch.float32, torch.bfloat16
+        if not _TENSORS.issuperset(map(type, states)) or not _TENSORS.issuperset(map(type, convs)):
+            return None        # (a subclass may have to see the operations)
         for ts, dtype, shape in ((states, f32, (B, H, M, R)), (convs, bf16, (B, di, 3))):
             for t in ts:
                 if t.dtype is not dtype or t.shape != shape or not t.is_contiguous() or t.get_device() != dev:

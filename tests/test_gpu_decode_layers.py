@@ -111,6 +111,28 @@ def test_what_the_native_step_does_not_cover_still_runs():
             assert (a.float() - b.float()).norm() <= 2e-2 * b.float().norm() + 1e-3
 
 
+class _Seen(torch.Tensor):
+    """A tensor subclass that sees the operations on it."""
+
+    @classmethod
+    def __torch_function__(cls, func, types, args=(), kwargs=None):
+        _Seen.n += 1
+        return super().__torch_function__(func, types, args, kwargs or {})
+
+
+@pytest.mark.parametrize("which", [0, 1])
+def test_cached_tensors_that_observe_operations_keep_the_modules(which):
+    half = _model(64, 2, 8).to(torch.bfloat16)
+    ids = torch.ones(2, 1, dtype=torch.long).cuda()
+    past = _past(half, 2, torch.bfloat16)
+    seen = tuple(tuple(t.as_subclass(_Seen) if i == which else t for i, t in enumerate(pair)) for pair in past)
+    _Seen.n = 0
+    with _Count() as count:
+        half(ids, past_key_values=seen, use_cache=False)
+        assert count.n == 0
+    assert _Seen.n > 0
+
+
 def test_each_layers_cache_is_a_tensor_of_its_own():
     half = _model(64, 2, 8, layers=3).to(torch.bfloat16)
     ids = torch.ones(2, 1, dtype=torch.long).cuda()
