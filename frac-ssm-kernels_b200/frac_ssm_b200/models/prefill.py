@@ -46,9 +46,10 @@ def prefill_layers(layers, h, attention_mask, use_cache, classes):
         return None
     mask = None
     if attention_mask is not None:
-        if type(attention_mask) is not torch.Tensor or attention_mask.shape != (B, L):
+        # (the modules copy a mask over from another device, but refuse one where the cache needs it)
+        if type(attention_mask) is not torch.Tensor or attention_mask.shape != (B, L) or attention_mask.get_device() != dev:
             return None
-        mask = attention_mask.to(device=h.device, dtype=torch.float32).contiguous()
+        mask = attention_mask.to(torch.float32).contiguous()
     coeff = mixer.coeff_dtype
     if coeff not in (None, torch.float32, torch.bfloat16):
         return None

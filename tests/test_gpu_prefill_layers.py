@@ -61,6 +61,15 @@ def test_mixed_parameter_types_and_other_masks():
             assert (a.float() - b.float()).norm() <= 2e-2 * b.float().norm() + 1e-3
 
 
+def test_a_mask_on_another_device_is_refused_with_a_cache_as_by_the_modules():
+    half = _model(64, 2, 16).to(torch.bfloat16)
+    ids, mask = torch.ones(2, 40, dtype=torch.long).cuda(), torch.ones(2, 40, dtype=torch.long)
+    for run in (half, lambda *a, **k: _hooked(half, *a, **k)):
+        run(ids, attention_mask=mask, use_cache=False)
+        with pytest.raises(RuntimeError, match="same device"):
+            run(ids, attention_mask=mask, use_cache=True)
+
+
 @pytest.mark.parametrize("rows,D", [(1, 8), (5, 768), (4, 2048), (3, 264)])
 @pytest.mark.parametrize("w_dtype", [torch.bfloat16, torch.float32])
 def test_add_rmsnorm(rows, D, w_dtype):
