@@ -26,11 +26,11 @@ _PLAIN = frozenset((torch.Tensor, torch.nn.Parameter, int, float, bool, type(Non
 
 
 def _unobserved(args):
-    """True when nothing has to see the registered op: no tracing, no dispatch or function mode, no function
-    transform or forward-mode level, only plain tensors, and none that gradients are asked of."""
+    """True when nothing has to see the registered op: no tracing, no profiler, no dispatch or function mode, no
+    function transform or forward-mode level, only plain tensors, and none that gradients are asked of."""
     if (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
             or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._get_tracing_state() is not None
-            or torch.autograd.forward_ad._current_level >= 0):
+            or torch.autograd.forward_ad._current_level >= 0 or torch.autograd._profiler_enabled()):
         return False
     grad = torch.is_grad_enabled()
     for a in args:

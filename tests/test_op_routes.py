@@ -1,5 +1,6 @@
 """When a launch function is called directly and when through its registered op (no GPU needed)."""
 
+import pytest
 import torch
 from torch.utils._python_dispatch import TorchDispatchMode
 
@@ -44,3 +45,29 @@ def test_few_long_rows_are_cut_where_that_was_measured_to_be_faster():
     assert splits(12, 65536) == splits(13, 32768) == 1       # 12 x 32768 tokens: 0.42 ms whole, 0.68 cut
     assert splits(14, 1048576) == splits(24, 1048576) == 1   # 24 rows: 13.7 ms whole, 16.6 cut
     assert splits(8, 1048576) == 32 and splits(3, 32768) == 32
+
+
+@pytest.fixture(scope="module")
+def double():
+    """An op like the package's own, and how often its function ran."""
+    runs = []
+
+    @stages._op("test_double")
+    def _double_op(x: torch.Tensor, times: int) -> torch.Tensor:
+        runs.append(times)
+        return x * times
+
+    @_double_op.register_fake
+    def _(x, times):
+        return torch.empty_like(x)
+    return _double_op, runs
+
+
+def test_a_profiled_call_shows_the_registered_op(double):
+    op, runs = double
+    x = torch.ones(2)
+    op(x, 2)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        assert torch.equal(op(x, 3), x * 3)
+    assert any(e.key == "frac_ssm_b200::test_double" for e in prof.key_averages())
+    assert runs[-2:] == [2, 3]
