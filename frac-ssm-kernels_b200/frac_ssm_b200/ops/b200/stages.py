@@ -39,17 +39,34 @@ def _unobserved(args):
     return True
 
 
+class _Op:
+    """A registered op that calls its launch function itself where nothing observes the op: the dispatcher's share of
+    a call was 20 us of `frac_scan`'s 70.  Everything else about it is the op's own."""
+
+    def __init__(self, fn, op):
+        self._fn, self._op, self._direct = fn, op, True
+
+    def __call__(self, *args, **kwargs):
+        if self._direct and not kwargs and _unobserved(args):
+            return self._fn(*args)
+        return self._op(*args, **kwargs)
+
+    def __getattr__(self, name):
+        if name.startswith("__") or "_op" not in self.__dict__:
+            raise AttributeError(name)
+        value = getattr(self._op, name)
+        # whoever registers something to run instead of the function, or around it, has it run
+        if name == "set_kernel_enabled" or (name.startswith("register_") and name != "register_fake"):
+            self._direct = False
+        return value
+
+
 def _op(name):
-    """Registers a launch function as a torch custom op, and calls the function itself where nothing observes the
-    op: the dispatcher's share of a call was 20 us of `frac_scan`'s 70."""
+    """Registers a launch function as a torch custom op; see _Op."""
     def wrap(fn):
         op = torch.library.custom_op(f"frac_ssm_b200::{name}", mutates_args=())(fn)
         op.register_autograd(_no_backward)
-
-        def call(*args):
-            return fn(*args) if _unobserved(args) else op(*args)
-        call.register_fake = op.register_fake
-        return call
+        return _Op(fn, op)
     return wrap
 
 

@@ -71,3 +71,24 @@ def test_a_profiled_call_shows_the_registered_op(double):
         assert torch.equal(op(x, 3), x * 3)
     assert any(e.key == "frac_ssm_b200::test_double" for e in prof.key_averages())
     assert runs[-2:] == [2, 3]
+
+
+def test_the_returned_function_has_the_ops_own_methods(double):
+    op, runs = double
+    assert op._qualname == "frac_ssm_b200::test_double" and op._opoverload is torch.ops.frac_ssm_b200.test_double.default
+    assert op(x=torch.ones(2), times=2).sum() == 4
+    compiled = torch.compile(lambda t: op(t, 4) + 1, fullgraph=True, backend="eager")
+    assert compiled(torch.ones(2)).sum() == 10
+    for name in ("register_kernel", "register_fake", "register_autograd", "register_vmap", "register_torch_dispatch",
+                 "register_autocast", "set_kernel_enabled"):
+        assert callable(getattr(op, name)), name
+    x = torch.ones(2)
+
+    @op.register_kernel("cpu")
+    def _(x, times):
+        return x * times + 1
+    n = len(runs)
+    assert torch.equal(op(x, 2), x * 2 + 1) and len(runs) == n      # what was registered runs, not the function
+    with op.set_kernel_enabled("cpu", False):
+        assert torch.equal(op(x, 2), x * 2) and len(runs) == n + 1
+    assert torch.equal(op(x, 2), x * 2 + 1) and len(runs) == n + 1
