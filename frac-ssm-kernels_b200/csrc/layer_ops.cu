@@ -471,32 +471,40 @@ rmsnorm_gated_bf16_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_srow,
 // sum = x + y and norm = weight * rmsnorm(sum) in one pass: the residual addition of a block together with the
 // norm the next block starts with (sum is rounded to bf16 first, as the addition by itself would leave it).  One
 // warp per row, the row in registers; bound by memory, 4 * D * 2 bytes a row instead of 5 (an addition and a norm).
+// sum may be x and norm may be y: a lane writes the elements that it has read.
 template <int WVEC>
 __global__ void __launch_bounds__(128)
-add_rmsnorm_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ y, const void *__restrict__ w,
-                   int w_dt, float eps, __nv_bfloat16 *__restrict__ sum, __nv_bfloat16 *__restrict__ norm, int64_t rows,
-                   int64_t D) {
+add_rmsnorm_kernel(const __nv_bfloat16 *x, const __nv_bfloat16 *y, const void *__restrict__ w, int w_dt, float eps,
+                   __nv_bfloat16 *sum, __nv_bfloat16 *norm, int64_t rows, int64_t D) {
   const int lane = threadIdx.x % 32;
   const int64_t row = (int64_t)blockIdx.x * 4 + threadIdx.x / 32;
   if (row >= rows) return;
   const int chunks = static_cast<int>(D / 8);
-  float v[8][8];
+  uint4 xr[8], yr[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int ch = lane + 32 * i;
+    if (ch < chunks) {
+      xr[i] = __ldcs(reinterpret_cast<const uint4 *>(x + row * D) + ch);
+      yr[i] = __ldcs(reinterpret_cast<const uint4 *>(y + row * D) + ch);
+    }
+  }
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int ch = lane + 32 * i;
     if (ch < chunks) {
-      float z[8];
-      unpack8(__ldcs(reinterpret_cast<const uint4 *>(x + row * D) + ch), v[i]);
-      unpack8(__ldcs(reinterpret_cast<const uint4 *>(y + row * D) + ch), z);
+      float v[8], z[8];
+      unpack8(xr[i], v);
+      unpack8(yr[i], z);
       uint32_t o[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) o[e] = pack_bf16x2(v[i][2 * e] + z[2 * e], v[i][2 * e + 1] + z[2 * e + 1]);
-      const uint4 packed = make_uint4(o[0], o[1], o[2], o[3]);
-      *(reinterpret_cast<uint4 *>(sum + row * D) + ch) = packed;
-      unpack8(packed, v[i]);
+      for (int e = 0; e < 4; ++e) o[e] = pack_bf16x2(v[2 * e] + z[2 * e], v[2 * e + 1] + z[2 * e + 1]);
+      xr[i] = make_uint4(o[0], o[1], o[2], o[3]);
+      *(reinterpret_cast<uint4 *>(sum + row * D) + ch) = xr[i];
+      unpack8(xr[i], v);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) ss = fmaf(v[i][e], v[i][e], ss);
+      for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
     }
   }
   ss = warp_sum(ss);
@@ -505,7 +513,8 @@ add_rmsnorm_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__r
   for (int i = 0; i < 8; ++i) {
     const int ch = lane + 32 * i;
     if (ch < chunks) {
-      float wv[8];
+      float v[8], wv[8];
+      unpack8(xr[i], v);
       if (WVEC == 1) {
         unpack8(__ldg(reinterpret_cast<const uint4 *>(w) + ch), wv);
       } else {
@@ -514,7 +523,7 @@ add_rmsnorm_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__r
       }
       uint32_t o[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) o[e] = pack_bf16x2(v[i][2 * e] * rs * wv[2 * e], v[i][2 * e + 1] * rs * wv[2 * e + 1]);
+      for (int e = 0; e < 4; ++e) o[e] = pack_bf16x2(v[2 * e] * rs * wv[2 * e], v[2 * e + 1] * rs * wv[2 * e + 1]);
       *(reinterpret_cast<uint4 *>(norm + row * D) + ch) = make_uint4(o[0], o[1], o[2], o[3]);
     }
   }

@@ -74,9 +74,10 @@ def prefill_layers(layers, h, attention_mask, use_cache, classes):
         stream = C.stream_of(h)
         nbytes = lib.fracssm_frac_scan_auto_workspace_bytes(B * H, L, R, M, T)
         ws = empty(max(nbytes, 256), dtype=torch.uint8)
-        x_conv, u, scan_out, y = empty(rows, di), empty(B * H, L, R), empty(B * H, L, R), empty(rows, di)
+        x_conv, u, scan_out = empty(rows, di), empty(B * H, L, R), empty(B * H, L, R)
+        y = u.view(rows, di)      # (the epilogue writes it when the scan has read u)
         c, kappa, rho = empty(B * H, L, M, dtype=coeff), empty(B * H, L, M, dtype=coeff), empty(B * H, L, M, dtype=f32)
-        normed, sums = empty(rows, d), (empty(rows, d), empty(rows, d))
+        total = empty(rows, d) if n_layers > 1 else None      # the residual from the second layer on
         fin = states = tails = None
         if use_cache:
             fin = empty(B * H, R, M, dtype=f32)
@@ -85,8 +86,8 @@ def prefill_layers(layers, h, attention_mask, use_cache, classes):
             for _ in range(n_layers - 1):
                 states.append(torch.empty_like(states[0]))
                 tails.append(torch.empty_like(tails[0]))
-        p_ws, p_conv, p_u, p_h, p_y, p_c, p_k, p_rho, p_fin, p_norm, p_mask = (
-            0 if t is None else t.data_ptr() for t in (ws, x_conv, u, scan_out, y, c, kappa, rho, fin, normed, mask))
+        p_ws, p_conv, p_u, p_h, p_y, p_c, p_k, p_rho, p_fin, p_total, p_mask = (
+            0 if t is None else t.data_ptr() for t in (ws, x_conv, u, scan_out, y, c, kappa, rho, fin, total, mask))
         ck = C.dt_of(coeff)
         res, out, n = h.view(rows, d), None, None
         for i, (t, f32_mask, nums) in enumerate(found):
@@ -95,12 +96,13 @@ def prefill_layers(layers, h, attention_mask, use_cache, classes):
             if i == 0:
                 n = rmsnorm_gated_fwd(res, norm_w, None, nums[0])[0]
             else:
-                total = sums[i & 1]
-                C.check(lib.fracssm_add_rmsnorm(res.data_ptr(), out.data_ptr(), norm_w.data_ptr(),
-                                                C.F32 if f32_mask & 1 else C.BF16, nums[0], total.data_ptr(), p_norm, rows, d,
+                p_out = out.data_ptr()      # (the norm takes its place)
+                C.check(lib.fracssm_add_rmsnorm(res.data_ptr(), p_out, norm_w.data_ptr(),
+                                                C.F32 if f32_mask & 1 else C.BF16, nums[0], p_total, p_out, rows, d,
                                                 stream), "add_rmsnorm")
-                res, n = total, normed
+                res, n, out = total, out, None
             xg = F.linear(n, in_w)
+            n = None      # (like xg below: what is no longer read makes room)
             p_x = xg.data_ptr()
             C.check(lib.fracssm_prefill_conv(p_x, 2 * di, p_mask, conv_w.data_ptr(), 0 if conv_b is None else conv_b.data_ptr(),
                                              p_conv, p_u, tails[i].data_ptr() if use_cache else 0, R, B, L, di, K, stream),

@@ -361,7 +361,8 @@ int fracssm_decode_layers(const uint64_t *layer_ptrs, const float *layer_nums, i
  * The steps of a bfloat16 mixer's prefill around its library GEMMs, few calls per layer.
  *
  * add_rmsnorm: sum = x + y, norm = weight * sum * rsqrt(mean(sum^2) + eps); rows of D bf16 elements (D a multiple
- * of 8, at most 2048, 16-byte aligned), weight of w_dtype.  Replaces the residual addition and the norm of
+ * of 8, at most 2048, 16-byte aligned), weight of w_dtype; sum may be x and norm may be y.  Replaces the residual
+ * addition and the norm of
  * frac_ssm/models/modeling_frac.py (FracBlock).
  *
  * prefill_conv: fracssm_causal_conv_silu_heads for bf16 x [Bt, L, C] (rows x_sl elements apart, batches L * x_sl),
@@ -373,7 +374,7 @@ int fracssm_decode_layers(const uint64_t *layer_ptrs, const float *layer_nums, i
  * read_residual_logit, write_residual_scale, base_log_tau, D, output norm weight, bit i of params_f32 set where
  * parameter i is float32, else bf16; nums (host): read_temp, dt_min, dt_max, alpha_min, alpha_max, lambda_min,
  * lambda_max, gate bias, eps.  Scratch of the caller: c, kappa [Bt*H, L, M] (ck_dtype), rho, h, final_state
- * [Bt*H, R, M] (needed with state), workspace (fracssm_frac_scan_auto_workspace_bytes).  Results: state [Bt, H, M, R]
+ * [Bt*H, R, M] (needed with state), workspace (fracssm_frac_scan_auto_workspace_bytes).  y may lie in u's buffer.  Results: state [Bt, H, M, R]
  * (or NULL) and y [Bt, L, HR].
  */
 int fracssm_add_rmsnorm(const void *x, const void *y, const void *weight, int w_dtype, float eps, void *sum, void *norm,

@@ -61,6 +61,35 @@ def test_mixed_parameter_types_and_other_masks():
             assert (a.float() - b.float()).norm() <= 2e-2 * b.float().norm() + 1e-3
 
 
+@pytest.mark.parametrize("H,M,B,L", [(24, 128, 2, 3000), (24, 128, 1, 397), (12, 8, 8, 3000)])
+@pytest.mark.parametrize("use_cache", [False, True])
+def test_prefill_needs_no_more_memory_than_the_modules(H, M, B, L, use_cache):
+    """The modules with the scratch of the chunked stages, which the scan allocated before it had the segment kernels:
+    what fitted the GPU then still does."""
+    from frac_ssm_b200 import _cabi as C
+    half = _model(768, H, M, layers=4).to(torch.bfloat16)
+    ids = torch.ones(B, L, dtype=torch.long).cuda()
+    lib = C.lib()
+    alone = lib.fracssm_frac_scan_auto_workspace_bytes
+
+    def peak(run):
+        run(half, ids, use_cache=use_cache)      # (the library GEMMs' own workspace)
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        run(half, ids, use_cache=use_cache)
+        torch.cuda.synchronize()
+        return torch.cuda.max_memory_allocated() - before
+    native = peak(lambda m, *a, **k: m(*a, **k))
+    lib.fracssm_frac_scan_auto_workspace_bytes = lambda *a: lib.fracssm_frac_scan_workspace_bytes(*a, C.PATH_AUTO)
+    try:
+        modules = peak(_hooked)
+    finally:
+        lib.fracssm_frac_scan_auto_workspace_bytes = alone
+    assert native <= modules, (native / B / L, modules / B / L)
+
+
 def test_a_mask_on_another_device_is_refused_with_a_cache_as_by_the_modules():
     half = _model(64, 2, 16).to(torch.bfloat16)
     ids, mask = torch.ones(2, 40, dtype=torch.long).cuda(), torch.ones(2, 40, dtype=torch.long)
@@ -80,6 +109,10 @@ def test_add_rmsnorm(rows, D, w_dtype):
     total, norm = torch.empty_like(x), torch.empty_like(x)
     C.check(C.lib().fracssm_add_rmsnorm(C.ptr(x), C.ptr(y), C.ptr(w), C.dt(w), 1e-6, C.ptr(total), C.ptr(norm), rows, D,
                                         C.stream_of(x)), "add_rmsnorm")
+    x2, y2 = x.clone(), y.clone()          # in place: the sum over x, the norm over y
+    C.check(C.lib().fracssm_add_rmsnorm(C.ptr(x2), C.ptr(y2), C.ptr(w), C.dt(w), 1e-6, C.ptr(x2), C.ptr(y2), rows, D,
+                                        C.stream_of(x)), "add_rmsnorm")
+    assert torch.equal(x2, total) and torch.equal(y2, norm)
     assert torch.equal(total, x + y)
     s = total.double()
     ref = s * torch.rsqrt(s.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
