@@ -27,14 +27,15 @@ _PLAIN = frozenset((torch.Tensor, torch.nn.Parameter, int, float, bool, type(Non
 
 def _unobserved(args):
     """True when nothing has to see the registered op: no tracing, no profiler, no dispatch or function mode, no
-    function transform or forward-mode level, only plain tensors, and none that gradients are asked of."""
+    function transform or forward-mode level, only plain tensors, none that gradients are asked of, and none whose
+    memory holds the negated values (the dispatcher would resolve those before a function reads the memory)."""
     if (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() or torch._C._len_torch_function_stack()
             or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._get_tracing_state() is not None
             or torch.autograd.forward_ad._current_level >= 0 or torch.autograd._profiler_enabled()):
         return False
     grad = torch.is_grad_enabled()
     for a in args:
-        if type(a) not in _PLAIN or (grad and isinstance(a, torch.Tensor) and a.requires_grad):
+        if type(a) not in _PLAIN or (isinstance(a, torch.Tensor) and ((grad and a.requires_grad) or a.is_neg())):
             return False
     return True
 

@@ -24,6 +24,8 @@ def test_direct_only_where_nothing_observes_the_op():
     with torch.no_grad():
         assert stages._unobserved((x, w, torch.nn.Parameter(x)))
     assert not stages._unobserved((x.as_subclass(_Sub),))
+    negated = torch.complex(x, x).conj().imag       # its memory holds x, its values are -x
+    assert negated.is_neg() and not stages._unobserved((x, negated))
     with _Mode():
         assert not stages._unobserved((x,))
     seen = []
