@@ -46,6 +46,16 @@ class _Op:
 
     def __init__(self, fn, op):
         self._fn, self._op, self._direct = fn, op, True
+        # whoever registers something to run instead of the function, or around it, has it run: here or by the op's name
+        for name in dir(op):
+            if name == "set_kernel_enabled" or (name.startswith("register_") and name != "register_fake"):
+                setattr(op, name, self._through_the_op(getattr(op, name)))
+
+    def _through_the_op(self, method):
+        def call(*args, **kwargs):
+            self._direct = False
+            return method(*args, **kwargs)
+        return call
 
     def __call__(self, *args, **kwargs):
         if self._direct and not kwargs and _unobserved(args):
@@ -55,11 +65,7 @@ class _Op:
     def __getattr__(self, name):
         if name.startswith("__") or "_op" not in self.__dict__:
             raise AttributeError(name)
-        value = getattr(self._op, name)
-        # whoever registers something to run instead of the function, or around it, has it run
-        if name == "set_kernel_enabled" or (name.startswith("register_") and name != "register_fake"):
-            self._direct = False
-        return value
+        return getattr(self._op, name)
 
 
 def _op(name):

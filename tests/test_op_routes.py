@@ -94,3 +94,28 @@ def test_the_returned_function_has_the_ops_own_methods(double):
     with op.set_kernel_enabled("cpu", False):
         assert torch.equal(op(x, 2), x * 2) and len(runs) == n + 1
     assert torch.equal(op(x, 2), x * 2 + 1) and len(runs) == n + 1
+
+
+@pytest.mark.parametrize("register", ["register_kernel", "register_vmap", "register_torch_dispatch", "register_autocast"])
+def test_what_is_registered_by_the_ops_name_runs(register):
+    name = f"frac_ssm_b200::test_by_name_{register}"
+
+    @stages._op(name.split("::")[1])
+    def _twice_op(x: torch.Tensor) -> torch.Tensor:
+        return x * 2
+    assert _twice_op._direct
+    if register == "register_kernel":
+        torch.library.register_kernel(name, "cpu", lambda x: x * 3)
+        assert torch.equal(_twice_op(torch.ones(2)), torch.full((2,), 3.0))
+    elif register == "register_vmap":
+        torch.library.register_vmap(name, lambda info, dims, x: (x * 5, 0))
+        assert torch.equal(torch.vmap(_twice_op)(torch.ones(2)), torch.full((2,), 5.0))
+    elif register == "register_torch_dispatch":
+        torch.library.register_torch_dispatch(name, _Mode, lambda mode, func, types, args, kwargs: args[0] * 7)
+        with _Mode():
+            assert torch.equal(_twice_op(torch.ones(2)), torch.full((2,), 7.0))
+    else:
+        torch.library.register_autocast(name, "cpu", torch.bfloat16)
+        with torch.autocast("cpu", torch.bfloat16):
+            assert _twice_op(torch.ones(2)).dtype == torch.bfloat16
+    assert not _twice_op._direct
