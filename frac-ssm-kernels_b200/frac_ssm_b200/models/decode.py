@@ -113,6 +113,16 @@ def _layer_params(layers, classes, sizes, dev):
     return out
 
 
+def _pairs(past, n):
+    """Whether `past` is None or n times None or (state, conv_state), in tuples or lists.  (The modules take it from any
+    iterable, also one that can be gone through once only, and refuse other entries.)"""
+    if past is None:
+        return True
+    kinds = (tuple, list)
+    return (isinstance(past, kinds) and len(past) == n
+            and all(p is None or (isinstance(p, kinds) and len(p) == 2) for p in past))
+
+
 def decode_layers(layers, h, past, use_cache, classes):
     """h [B, 1, hidden] through `layers` -> (h, new past or None), or None when the call is not covered.
     `past`: per layer (state, conv_state), or None for a first token."""
@@ -120,7 +130,7 @@ def decode_layers(layers, h, past, use_cache, classes):
         return None
     B, _, d = h.shape
     n = len(layers)
-    if B < 1 or n < 1 or (past is not None and len(past) != n) or transformed():
+    if B < 1 or n < 1 or transformed() or not _pairs(past, n):
         return None
     if type(layers) is not nn.ModuleList or not h.is_contiguous() or h.data_ptr() & 15:
         return None

@@ -133,6 +133,21 @@ def test_cached_tensors_that_observe_operations_keep_the_modules(which):
     assert _Seen.n > 0
 
 
+def test_a_cache_that_can_be_gone_through_once_is_taken_by_the_modules():
+    half = _model(64, 2, 8).to(torch.bfloat16)
+    ids = torch.ones(2, 1, dtype=torch.long).cuda()
+    past = _past(half, 2, torch.bfloat16)
+    with _Count() as count:
+        got = half(ids, past_key_values=(pair for pair in past), use_cache=True)
+        assert count.n == 0
+        ref = half(ids, past_key_values=past, use_cache=True)
+        with pytest.raises(ValueError):      # as the modules do
+            half(ids, past_key_values=tuple((*pair, None) for pair in past), use_cache=True)
+        assert count.n == 1
+    for a, b in zip(_flat(got), _flat(ref)):
+        assert (a.float() - b.float()).norm() <= 2e-2 * b.float().norm() + 1e-3
+
+
 def test_each_layers_cache_is_a_tensor_of_its_own():
     half = _model(64, 2, 8, layers=3).to(torch.bfloat16)
     ids = torch.ones(2, 1, dtype=torch.long).cuda()

@@ -83,3 +83,13 @@ def test_a_weight_of_another_shape_keeps_the_modules(path):
     module = model.get_submodule(path)
     module.weight = torch.nn.Parameter(module.weight.detach().t().contiguous())
     assert _looked_at(model) is None
+
+
+def test_caches_in_other_containers_go_to_the_modules():
+    pair = (torch.ones(1), torch.ones(1))
+    for past in (None, (pair, pair), [None, pair], (list(pair), None)):
+        assert decode._pairs(past, 2)
+    once = (p for p in (pair, pair))
+    assert not decode._pairs(once, 2) and len(list(once)) == 2      # not touched
+    for past in ((pair,), {0: pair, 1: pair}.values(), (pair, (*pair, None)), (pair, torch.ones(2, 3)), (pair, iter(pair))):
+        assert not decode._pairs(past, 2)
