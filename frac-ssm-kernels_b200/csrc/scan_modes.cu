@@ -172,8 +172,10 @@ few_scan_kernel(const FewArgs a) {
       }
     }
   };
-  // any stride, alignment and size: element by element, when the group is due
+  // any stride, alignment and size: element by element, when the group is due.  True where an infinity or NaN of u meets
+  // padding modes: their zero coefficients would make NaN of it.
   auto copy_group = [&](int ib) {
+    bool meets = false;
     const int n = min(kGroup, ntok - ib * kGroup);
     for (int i = lane; i < n * Mp; i += lanes) {
       const int t = i / Mp, m = i % Mp;
@@ -188,7 +190,9 @@ few_scan_kernel(const FewArgs a) {
       const int t = i / a.block_cols, r = i - t * a.block_cols;
       const float v = r < cols ? ld_f32(u_p + ((int64_t)ib * kGroup + t) * a.u.sl, r, UD) : 0.f;
       wide[t * tok_floats + kOffU + r] = v;
+      meets |= !isfinite(v);
     }
+    return meets && a.M < Mp;
   };
   if (a.wide_loads) request(0);
   grid_dep_wait();
@@ -225,13 +229,14 @@ few_scan_kernel(const FewArgs a) {
   int64_t row = ((int64_t)b * a.L + t0) * a.R + col0 + my;
   for (int ib = 0; ib * kGroup < all_tok; ++ib) {
     if (ib > 0) __syncthreads();   // the previous group has been read
+    bool keep_zero = false;        // the padding modes' state
     if (a.wide_loads) {
       store_group(ib);
       request(ib + 1);
+      __syncthreads();
     } else {
-      copy_group(ib);
+      keep_zero = __syncthreads_or(copy_group(ib));
     }
-    __syncthreads();
     const int n = max(0, min(kGroup, ntok - ib * kGroup)), n_all = min(kGroup, all_tok - ib * kGroup);
     const float *tok = wide;
 #pragma unroll 1
@@ -248,6 +253,18 @@ few_scan_kernel(const FewArgs a) {
         for (int r = 0; r < kCols; ++r) {
 #pragma unroll
           for (int p = 0; p < 4; ++p) st[r][p] = fma2(rr[p], st[r][p], mul2(ka[p], uu[r]));
+        }
+        if (keep_zero) {
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {
+            const int m = kModes * g + 2 * p;
+#pragma unroll
+            for (int r = 0; r < kCols; ++r) {
+              float lo, hi;
+              un2(st[r][p], lo, hi);
+              st[r][p] = mk2(m < a.M ? lo : 0.f, m + 1 < a.M ? hi : 0.f);
+            }
+          }
         }
         if (!READOUT) {
 #pragma unroll

@@ -80,3 +80,19 @@ def test_initial_state_passes_through_masked_tokens():
     rho.fill_(1.0)
     _, fin = frac_scan(*(t.cuda() for t in (u, c, kappa, rho)), 64, init.cuda(), True)
     assert torch.equal(fin.cpu(), init)
+
+
+@pytest.mark.parametrize("M", [5, 8, 12, 20, 100])      # 8: no padding modes
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_an_infinity_stays_one_where_modes_are_padded(M, dtype):
+    from frac_ssm_b200.ops.b200 import frac_scan
+    u, c, kappa, rho, init = O.scan_inputs(2, 300, 64, M, dtype=torch.float32, gen="model_like", seed=M)
+    u, c, kappa = u.to(dtype), c.abs().add(0.01).to(dtype), kappa.abs().add(0.01).to(dtype)
+    u[0, 37, 5], u[1, 200, 63] = float("inf"), float("-inf")
+    rho = 0.9 + 0.1 * rho          # 0.9 ** 300 = 2e-14: no product of decays becomes zero, which would make NaN of it too
+    h, fin = frac_scan(*(t.cuda() for t in (u, c, kappa, rho)), 32, init.cuda(), True, final_state_dtype=torch.float32)
+    h_ref, f_ref = _exact(u, c, kappa, rho, init)
+    assert torch.isinf(h_ref).any() and not torch.isnan(h_ref).any()
+    for got, ref in ((h, h_ref), (fin, f_ref)):
+        got, finite = got.double().cpu(), torch.isfinite(ref)
+        assert torch.equal(got[~finite], ref[~finite]) and torch.isfinite(got[finite]).all()
