@@ -56,6 +56,29 @@ def test_segments_match_recurrence_and_stages(B, L, R, M, dtype, coeff):
         assert _rel(fin, fs.double().cpu()) <= 1e-5
 
 
+# more than 384 segments a row: a share of the carry kernel's 32 warps is then more than the 12 segments it keeps in
+# registers, and it reads what it overwrites a batch at a time
+@pytest.mark.parametrize("B,L,R,M", [(2, 32768, 128, 16), (1, 20011, 64, 8), (3, 7001, 20, 5)])
+@pytest.mark.parametrize("with_start", [False, True])
+def test_many_segments(B, L, R, M, with_start):
+    from frac_ssm_b200 import _cabi as C
+    from frac_ssm_b200.ops.b200 import frac_scan
+    Mp = (M + 7) // 8 * 8
+    nseg = C.lib().fracssm_frac_scan_auto_workspace_bytes(B, L, R, M, 32) // (4 * B * Mp * (R + 1))
+    assert nseg > 384
+    u, c, kappa, rho, init = O.scan_inputs(B, L, R, M, dtype=torch.float32, gen="model_like", seed=L)
+    start = init if with_start else None
+    g = [t.cuda() for t in (u, c, kappa, rho)]
+    ig = None if start is None else start.cuda()
+    h, fin = frac_scan(*g, 32, ig, True)
+    hs, fs = frac_scan(*g, 32, ig, True, path="staged")
+    h_ref, f_ref = _exact(u, c, kappa, rho, start)
+    bound = 2.0 ** -23 * L ** 0.5         # roundings of at most L steps, of either sign
+    for got, staged, ref in ((h, hs, h_ref), (fin, fs, f_ref)):
+        assert _rel(got, ref) <= bound
+        assert _rel(got, staged.double().cpu()) <= 2 * bound
+
+
 @pytest.mark.parametrize("M,R", [(16, 64), (8, 20)])
 def test_segments_take_any_stride_and_alignment(M, R):
     from frac_ssm_b200.ops.b200 import frac_scan
