@@ -21,14 +21,18 @@ def _ws(nbytes):
     return torch.zeros(max(int(nbytes), 256), dtype=torch.uint8, device="cuda")
 
 
-def test_scan_wait_runs_out_and_is_reported():
+@pytest.mark.parametrize("hand_over", ["tagged", "counted"])
+def test_scan_wait_runs_out_and_is_reported(hand_over):
     from frac_ssm_b200 import _cabi as C
     lib = selftest_lib()
     B, L = 3, 384
     u, c, kappa, rho, _ = (t.cuda() for t in O.scan_inputs(B, L, 64, 128, gen="model_like", seed=11))
     h = torch.zeros_like(u)
     fin = torch.zeros(B, 64, 128, device="cuda")
-    ws = _ws(lib.fracssm_frac_scan_workspace_bytes(B, L, 64, 128, 128, 2))
+    nbytes = lib.fracssm_frac_scan_workspace_bytes(B, L, 64, 128, 128, 2)
+    if hand_over == "counted":        # the state without the tags' half: such a workspace keeps the counter
+        nbytes -= B * 64 * 128 * 4
+    ws = _ws(nbytes)
     stream = C.stream_of(u)
     t0 = time.time()
     rc = lib.fracssm_selftest_scan_wait_limit(C.ptr(u), C.ptr(c), C.ptr(kappa), C.ptr(rho), C.ptr(h), C.ptr(fin),
