@@ -34,21 +34,24 @@ def _past(model, B, dtype, seed=0):
 
 
 class _Count:
-    """Counts the native calls."""
+    """Counts the calls of a native function."""
+
+    def __init__(self, name="fracssm_decode_layers"):
+        self.name = name
 
     def __enter__(self):
         from frac_ssm_b200 import _cabi as C
         self.lib, self.n = C.lib(), 0
-        self.fn = self.lib.fracssm_decode_layers
+        self.fn = getattr(self.lib, self.name)
 
         def counted(*a):
             self.n += 1
             return self.fn(*a)
-        self.lib.fracssm_decode_layers = counted
+        setattr(self.lib, self.name, counted)
         return self
 
     def __exit__(self, *exc):
-        self.lib.fracssm_decode_layers = self.fn
+        setattr(self.lib, self.name, self.fn)
 
 
 def _flat(out):
@@ -57,13 +60,15 @@ def _flat(out):
 
 
 # sequences around the groups of 8; widths that fill the 8 warps' shares unevenly; heads whose projections end
-# inside a 16-row tile; modes that are no multiple of 4; one and several column shares per head
-@pytest.mark.parametrize("hidden,H,M,B", [(32, 1, 8, 1), (64, 2, 7, 2), (96, 3, 16, 3), (256, 4, 128, 8), (256, 8, 33, 9),
-                                          (768, 24, 128, 1), (768, 12, 8, 17), (128, 2, 128, 33), (768, 24, 128, 64)])
+# inside a 16-row tile; modes that are no multiple of 4; one and several column shares per head; layers enough for the
+# two buffers of the hidden state to be used again
+@pytest.mark.parametrize("hidden,H,M,B,layers", [
+    (32, 1, 8, 1, 2), (64, 2, 7, 2, 2), (96, 3, 16, 3, 2), (256, 4, 128, 8, 2), (256, 8, 33, 9, 2), (768, 24, 128, 1, 2),
+    (768, 12, 8, 17, 2), (128, 2, 128, 33, 2), (768, 24, 128, 64, 2), (96, 3, 16, 2, 1), (128, 2, 20, 3, 5), (256, 4, 128, 20, 6)])
 @pytest.mark.parametrize("first", [False, True])
-def test_native_step_matches_modules(hidden, H, M, B, first):
-    half = _model(hidden, H, M).to(torch.bfloat16)
-    model = _model(hidden, H, M)
+def test_native_step_matches_modules(hidden, H, M, B, layers, first):
+    half = _model(hidden, H, M, layers).to(torch.bfloat16)
+    model = _model(hidden, H, M, layers)
     for p, q in zip(list(model.parameters()) + list(model.buffers()), list(half.parameters()) + list(half.buffers())):
         p.data.copy_(q.data)                                    # the same (rounded) weights in float32
     exact_past = None if first else _past(model, B, torch.float32)

@@ -3,7 +3,7 @@
 import pytest
 import torch
 
-from tests.test_gpu_decode_layers import _flat, _model
+from tests.test_gpu_decode_layers import _Count, _flat, _model
 
 pytestmark = pytest.mark.gpu
 
@@ -16,14 +16,16 @@ def _hooked(model, *args, **kw):
     return out
 
 
-# lengths around the convolution's history and the scan's tiles; single-pass and segment scans; odd widths
-@pytest.mark.parametrize("hidden,H,M,B,L", [(64, 2, 128, 1, 2), (128, 4, 128, 2, 3), (256, 8, 128, 2, 129), (96, 3, 7, 3, 50),
-                                            (768, 12, 8, 2, 200), (768, 24, 128, 1, 397), (72, 3, 20, 2, 33)])
+# lengths around the convolution's history and the scan's tiles; single-pass and segment scans; odd widths; one layer,
+# and layers enough for every buffer that they share to be used again
+@pytest.mark.parametrize("hidden,H,M,B,L,layers", [
+    (64, 2, 128, 1, 2, 2), (128, 4, 128, 2, 3, 2), (256, 8, 128, 2, 129, 2), (96, 3, 7, 3, 50, 2), (768, 12, 8, 2, 200, 2),
+    (768, 24, 128, 1, 397, 2), (72, 3, 20, 2, 33, 2), (72, 3, 20, 2, 33, 1), (128, 4, 128, 2, 150, 5), (96, 3, 7, 3, 50, 4)])
 @pytest.mark.parametrize("masked", [False, True])
 @pytest.mark.parametrize("coeff", [None, torch.bfloat16])
-def test_prefill_matches_modules(hidden, H, M, B, L, masked, coeff):
-    half = _model(hidden, H, M).to(torch.bfloat16)
-    exact_model = _model(hidden, H, M)
+def test_prefill_matches_modules(hidden, H, M, B, L, layers, masked, coeff):
+    half = _model(hidden, H, M, layers).to(torch.bfloat16)
+    exact_model = _model(hidden, H, M, layers)
     for p, q in zip(list(exact_model.parameters()) + list(exact_model.buffers()), list(half.parameters()) + list(half.buffers())):
         p.data.copy_(q.data)
     for layer in half.model.layers:
@@ -34,10 +36,13 @@ def test_prefill_matches_modules(hidden, H, M, B, L, masked, coeff):
         mask = torch.ones(B, L, dtype=torch.long)
         mask[B - 1, : L // 2] = 0
         mask = mask.cuda()
-    native = _flat(half(ids, attention_mask=mask, use_cache=True))
-    logits, none = half(ids, attention_mask=mask, use_cache=False)
-    assert none is None and torch.equal(logits, native[0])
-    modules = _flat(_hooked(half, ids, attention_mask=mask, use_cache=True))
+    with _Count("fracssm_prefill_mix") as count:
+        native = _flat(half(ids, attention_mask=mask, use_cache=True))
+        logits, none = half(ids, attention_mask=mask, use_cache=False)
+        assert count.n == 2 * layers
+        assert none is None and torch.equal(logits, native[0])
+        modules = _flat(_hooked(half, ids, attention_mask=mask, use_cache=True))
+        assert count.n == 2 * layers
     exact = _flat(exact_model(ids, attention_mask=mask, use_cache=True))
     for n, m, e in zip(native, modules, exact):
         assert n.shape == m.shape and n.dtype == m.dtype and n.is_contiguous()
@@ -57,7 +62,10 @@ def test_mixed_parameter_types_and_other_masks():
     mask = torch.ones(2, 40, device="cuda", dtype=torch.bool)
     mask[0, 30:] = False
     for m in (mask, mask.float() * 0.3, mask.t().contiguous().t()):
-        for a, b in zip(_flat(half(ids, attention_mask=m, use_cache=True)), _flat(_hooked(half, ids, attention_mask=m, use_cache=True))):
+        with _Count("fracssm_prefill_mix") as count:
+            native = _flat(half(ids, attention_mask=m, use_cache=True))
+            assert count.n == 2
+        for a, b in zip(native, _flat(_hooked(half, ids, attention_mask=m, use_cache=True))):
             assert (a.float() - b.float()).norm() <= 2e-2 * b.float().norm() + 1e-3
 
 
