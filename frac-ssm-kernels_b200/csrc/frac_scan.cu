@@ -3,7 +3,7 @@
 // Staged path: log+cumsum -> chunk_state -> state_passing -> fused readout, with the
 // intermediates (lcr, chunk_decay, states, states_acc) in caller-provided scratch.
 // Single-pass path: the tcgen05 kernel in scan_fused.cu when the shape is covered.
-// Otherwise, up to 128 modes: the token recurrence over segments in scan_modes.cu.
+// Otherwise, up to 128 modes: the token recurrence over segments in scan_modes.cu, where that is the faster one.
 #include "common.cuh"
 
 namespace fracssm {
@@ -37,6 +37,11 @@ int scan_fused_launch(const void *u, const void *c, const void *kappa, int ck_dt
 // defined in scan_modes.cu
 bool scan_few_supported(int64_t B, int64_t L, int64_t R, int64_t M, int64_t T);
 size_t scan_few_workspace_bytes(int64_t B, int64_t L, int64_t R, int64_t M);
+bool scan_few_narrow_slower(int64_t B, int64_t L, int64_t R, int64_t M, int64_t T);
+bool scan_few_shape_loads_wide(int64_t R, int64_t M);
+bool scan_few_loads_wide(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, const void *c, const void *kappa,
+                         int ck_dtype, int64_t c_sb, int64_t c_sl, int64_t k_sb, int64_t k_sl, const float *rho,
+                         int64_t r_sb, int64_t r_sl, int64_t R, int64_t M);
 int scan_few_launch(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, const void *c, const void *kappa,
                     int ck_dtype, int64_t c_sb, int64_t c_sl, int64_t k_sb, int64_t k_sl, const float *rho,
                     int64_t r_sb, int64_t r_sl, const float *initial_state, void *h, void *final_state,
@@ -61,10 +66,14 @@ extern "C" size_t fracssm_frac_scan_auto_workspace_bytes(int64_t B, int64_t L, i
   using namespace fracssm;
   if (B <= 0 || L <= 0 || R <= 0 || M <= 0 || T <= 0) return 0;
   const size_t fused = scan_fused_workspace_bytes(B, L, R, M, T);
-  // which of the two automatic routes a call takes also depends on types and strides
-  const size_t other = scan_few_supported(B, L, R, M, T) ? scan_few_workspace_bytes(B, L, R, M)
-                                                         : staged_layout(nullptr, B, L, R, M, T).bytes;
-  return other > fused ? other : fused;
+  // which of the automatic routes a call takes also depends on types and strides
+  size_t most = fused;
+  auto also = [&](size_t n) { most = n > most ? n : most; };
+  const bool few = scan_few_supported(B, L, R, M, T);
+  if (few) also(scan_few_workspace_bytes(B, L, R, M));
+  if (!few || (!scan_few_shape_loads_wide(R, M) && scan_few_narrow_slower(B, L, R, M, T)))
+    also(staged_layout(nullptr, B, L, R, M, T).bytes);
+  return most;
 }
 
 namespace fracssm {
@@ -117,8 +126,12 @@ int frac_scan_route(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, cons
                              workspace, workspace_bytes, B, L, R, M, T, stream);
   }
 
-  // (a caller whose workspace only holds the chunked stages keeps them)
-  if (path == 0 && scan_few_supported(B, L, R, M, T) && workspace_bytes >= scan_few_workspace_bytes(B, L, R, M)) {
+  ScanScratch s = staged_layout(workspace, B, L, R, M, T);
+  // (a caller whose workspace holds the intermediates of one of the two only keeps those kernels)
+  bool few = path == 0 && scan_few_supported(B, L, R, M, T) && workspace_bytes >= scan_few_workspace_bytes(B, L, R, M);
+  if (few && workspace_bytes >= s.bytes && scan_few_narrow_slower(B, L, R, M, T))
+    few = scan_few_loads_wide(u, u_dtype, u_sb, u_sl, c, kappa, ck_dtype, c_sb, c_sl, k_sb, k_sl, rho, r_sb, r_sl, R, M);
+  if (few) {
     if (state_modes_first) *modes_first = true;
     return scan_few_launch(u, u_dtype, u_sb, u_sl, c, kappa, ck_dtype, c_sb, c_sl, k_sb, k_sl, rho, r_sb, r_sl,
                            initial_state, h, state_modes_first ? state_modes_first : final_state,
@@ -126,7 +139,6 @@ int frac_scan_route(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, cons
                            state_modes_first != nullptr);
   }
 
-  ScanScratch s = staged_layout(workspace, B, L, R, M, T);
   if (workspace_bytes < s.bytes) return fail(FRACSSM_ERR_ARG, "frac_scan: workspace too small");
   const int64_t N = ceil_div(L, T);
   int rc = fracssm_chunk_cumsum(rho, r_sb, r_sl, 1, s.lcr, s.chunk_decay, B, L, M, T, stream);

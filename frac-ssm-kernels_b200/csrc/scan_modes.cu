@@ -44,6 +44,10 @@ struct Rows {                  // one input: base and strides in bytes
   int64_t sb, sl;
 };
 
+Rows few_rows(const void *p, int64_t sb, int64_t sl, int size) {
+  return Rows{reinterpret_cast<const char *>(p), sb * size, sl * size};
+}
+
 struct FewArgs {
   Rows u, c, kappa, rho;
   const float *init;           // [B, R, M] or null
@@ -450,6 +454,43 @@ FewPlan few_plan(int64_t B, int64_t L, int64_t R, int64_t M) {
   return p;
 }
 
+// 16-byte loads: every row starts on a 16-byte boundary and fills whole pieces, there is no padding among the modes or
+// columns, and a segment has the threads for one piece of rho each (64 columns or more).
+bool few_wide_shape(const FewPlan &p, int64_t R, int64_t M, int u_size) {
+  const int pieces = p.block_cols * u_size / 16;
+  return p.block_cols * u_size % 16 == 0 && M == p.Mp && R % p.block_cols == 0 && (pieces & (pieces - 1)) == 0 &&
+         p.lanes >= 16 * p.G;
+}
+bool few_wide_rows(const Rows &u, const Rows &c, const Rows &kappa, const Rows &rho) {
+  uint64_t bits = 0;
+  for (const Rows *r : {&u, &c, &kappa, &rho}) bits |= (uint64_t)(uintptr_t)r->p | (uint64_t)r->sb | (uint64_t)r->sl;
+  return (bits & 15) == 0;
+}
+
+// Work (B L R Mp) up to which these kernels are the faster ones for calls that are cut into segments and load element by
+// element: such a load is waited for anew in every group of 8 tokens, and a cut row is loaded twice.  How long the chunked
+// stages take depends on the chunk: at 32, 128 and 256 tokens 1.5, 1.1 and 1.4 times as long as at 64.  Stages / segments
+// in us, bfloat16, chunk 64:
+//      2 x 32768 tokens, 128 columns x 40 modes  422 / 310       2 x 32768, 256 x 72  1143 / 1877
+//      8 x 8192,          64 x 60                236 / 172       8 x 8192,  128 x 60   412 / 428
+//     16 x 16384,         64 x 24                668 / 491      16 x 16384, 64 x 40    855 / 1091
+//     16 x 2048,         192 x 20                186 / 177       8 x 8192,  192 x 20   375 / 462
+// (192 columns are three blocks' worth of 64 but lie in two of 96, whose loads also divide by a number that is no power
+// of two.)  At 16 or fewer modes, at 32 or fewer columns and wherever rows are taken whole or loads are wide, the
+// segments were the faster in every one of some 500 such pairs but for 4 % at 192 x 12.
+double few_narrow_limit(const FewPlan &p, int64_t B, int64_t R, int64_t T) {
+  if (R <= 32 || p.Mp <= 16) return 1e30;
+  const bool odd = (p.block_cols & (p.block_cols - 1)) != 0;
+  if (T < 48 || T >= 192) {
+    if (p.Mp <= (odd ? 32 : 64)) return 1e30;
+    return (odd ? 1.2e9 : 2e9) * (B > 32 ? 3 : 1);
+  }
+  double limit;
+  if (odd) limit = p.Mp == 32 ? 256e6 : B <= 2 ? 100e6 : 64e6;
+  else limit = B <= 2 ? 800e6 : p.Mp == 32 && B <= 32 ? 600e6 : 400e6;
+  return T < 96 ? limit : 2 * limit;
+}
+
 template <typename... P, typename... Args>
 cudaError_t few_launch_dep(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, bool dependent,
                            Args... args) {
@@ -472,14 +513,8 @@ template <int G, int UD, int CK>
 int few_launch(FewArgs &a, const FewPlan &p, cudaStream_t st) {
   constexpr int Mp = kModes * G, kUs = UD == FRACSSM_F32 ? 4 : 2;
   const int threads = (int)(ceil_div(p.lanes * p.per_block, 32) * 32);
-  // 16-byte loads: every row starts on a 16-byte boundary and fills whole pieces, there is no padding among the
-  // modes or columns, and a segment has the threads for one piece of rho each (64 columns or more)
-  const uint64_t bits = (uint64_t)(uintptr_t)a.u.p | (uint64_t)(uintptr_t)a.c.p | (uint64_t)(uintptr_t)a.kappa.p |
-                        (uint64_t)(uintptr_t)a.rho.p | (uint64_t)a.u.sb | (uint64_t)a.u.sl | (uint64_t)a.c.sb |
-                        (uint64_t)a.c.sl | (uint64_t)a.kappa.sb | (uint64_t)a.kappa.sl | (uint64_t)a.rho.sb |
-                        (uint64_t)a.rho.sl | (uint64_t)(p.block_cols * kUs);
   const int pieces = p.block_cols * kUs / 16;
-  a.wide_loads = (bits & 15) == 0 && a.M == Mp && a.R % p.block_cols == 0 && (pieces & (pieces - 1)) == 0 && p.lanes >= 16 * G;
+  a.wide_loads = few_wide_shape(p, a.R, a.M, kUs) && few_wide_rows(a.u, a.c, a.kappa, a.rho);
   a.u_shift = 0;
   while ((1 << a.u_shift) < pieces) ++a.u_shift;
   const size_t sum_smem = (size_t)p.per_block * kGroup * (2 * Mp + p.block_cols) * 4;
@@ -526,6 +561,25 @@ bool scan_few_supported(int64_t B, int64_t L, int64_t R, int64_t M, int64_t T) {
 
 size_t scan_few_workspace_bytes(int64_t B, int64_t L, int64_t R, int64_t M) { return few_plan(B, L, R, M).bytes; }
 
+// Whether the chunked stages are the faster kernels for a call that loads element by element; for one that takes its
+// rows in 16-byte pieces they never are.
+bool scan_few_narrow_slower(int64_t B, int64_t L, int64_t R, int64_t M, int64_t T) {
+  const FewPlan p = few_plan(B, L, R, M);
+  return p.nseg > 1 && (double)B * L * R * p.Mp > few_narrow_limit(p, B, R, T);
+}
+bool scan_few_shape_loads_wide(int64_t R, int64_t M) {
+  const FewPlan p = few_plan(1, 1, R, M);
+  return few_wide_shape(p, R, M, 2) && few_wide_shape(p, R, M, 4);
+}
+bool scan_few_loads_wide(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, const void *c, const void *kappa,
+                         int ck_dtype, int64_t c_sb, int64_t c_sl, int64_t k_sb, int64_t k_sl, const float *rho,
+                         int64_t r_sb, int64_t r_sl, int64_t R, int64_t M) {
+  const int us = (int)dtype_size(u_dtype), ks = (int)dtype_size(ck_dtype);
+  return few_wide_shape(few_plan(1, 1, R, M), R, M, us) &&
+         few_wide_rows(few_rows(u, u_sb, u_sl, us), few_rows(c, c_sb, c_sl, ks), few_rows(kappa, k_sb, k_sl, ks),
+                       few_rows(rho, r_sb, r_sl, 4));
+}
+
 int scan_few_launch(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, const void *c, const void *kappa,
                     int ck_dtype, int64_t c_sb, int64_t c_sl, int64_t k_sb, int64_t k_sl, const float *rho,
                     int64_t r_sb, int64_t r_sl, const float *initial_state, void *h, void *final_state,
@@ -534,13 +588,10 @@ int scan_few_launch(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, cons
   const FewPlan p = few_plan(B, L, R, M);
   FewArgs a{};
   const int us = (int)dtype_size(u_dtype), ks = (int)dtype_size(ck_dtype);
-  auto rows = [](const void *ptr, int64_t sb, int64_t sl, int size) {
-    return Rows{reinterpret_cast<const char *>(ptr), sb * size, sl * size};
-  };
-  a.u = rows(u, u_sb, u_sl, us);
-  a.c = rows(c, c_sb, c_sl, ks);
-  a.kappa = rows(kappa, k_sb, k_sl, ks);
-  a.rho = rows(rho, r_sb, r_sl, 4);
+  a.u = few_rows(u, u_sb, u_sl, us);
+  a.c = few_rows(c, c_sb, c_sl, ks);
+  a.kappa = few_rows(kappa, k_sb, k_sl, ks);
+  a.rho = few_rows(rho, r_sb, r_sl, 4);
   a.init = initial_state;
   a.h = h;
   a.h_vec = R % 4 == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0;

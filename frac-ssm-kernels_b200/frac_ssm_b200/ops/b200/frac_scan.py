@@ -137,8 +137,11 @@ def _launch(u, c, kappa, rho, chunk_size, initial_state, want_final, final_fp32,
     if B > 0:
         lib = C.lib()
         with C.trace("frac_scan"), torch.cuda.device(u.device):
-            nbytes = (lib.fracssm_frac_scan_auto_workspace_bytes(B, L, R, M, chunk_size) if path_code == C.PATH_AUTO
-                      else lib.fracssm_frac_scan_workspace_bytes(B, L, R, M, chunk_size, path_code))
+            # (strided inputs may take the chunked stages where dense ones take the segment kernels)
+            if path_code == C.PATH_AUTO and all(t.is_contiguous() for t in (u, c, kappa, rho)):
+                nbytes = lib.fracssm_frac_scan_auto_workspace_bytes(B, L, R, M, chunk_size)
+            else:
+                nbytes = lib.fracssm_frac_scan_workspace_bytes(B, L, R, M, chunk_size, path_code)
             ws = torch.empty(max(nbytes, 256), device=u.device, dtype=torch.uint8)
             C.check(lib.fracssm_frac_scan_fwd(
                 C.ptr(u), C.dt(u), u.stride(0), u.stride(1), C.ptr(c), C.ptr(kappa), C.dt(c),

@@ -116,7 +116,8 @@ int fracssm_chunk_fused_readout(const void *u, int u_dtype, int64_t u_sb, int64_
  * final_state [B,R,M] (final_dtype f32 or bf16) or NULL.  workspace: device scratch of at
  * least fracssm_frac_scan_workspace_bytes(...) bytes, 256-byte aligned, caller-owned.
  * path: 0 = pick (single-pass tcgen05 kernel when the shape, types, strides and alignment are covered, else
- *           up to 128 modes the segment kernels, else staged),
+ *           up to 128 modes the segment kernels, else staged; large calls whose rows the segment kernels could not
+ *           load in 16-byte pieces take the staged kernels too),
  *       1 = staged kernels, 2 = single-pass kernel (error if the shape is not covered).
  * A workspace sized with path 0 serves every path.  fracssm_frac_scan_auto_workspace_bytes is what calls with
  * path 0 need by themselves, without the intermediates of the staged kernels where no such call takes them (at

@@ -79,6 +79,24 @@ def test_many_segments(B, L, R, M, with_start):
         assert _rel(got, staged.double().cpu()) <= 2 * bound
 
 
+@pytest.mark.parametrize("B,L,R,M,T,strided", [(8, 8192, 192, 40, 64, False), (16, 4096, 128, 72, 128, False), (8, 8192, 128, 128, 64, True)])
+def test_large_calls_that_load_by_element_take_the_stages(B, L, R, M, T, strided):
+    """A segment is then the slower way (8 x 8192 tokens, 192 columns x 40 modes: 819 us against 541)."""
+    from frac_ssm_b200.ops.b200 import frac_scan
+    g = torch.Generator(device="cuda").manual_seed(M)
+
+    def rows(n, lo, hi, dtype):
+        x = lo + (hi - lo) * torch.rand(B, L, n + strided, device="cuda", generator=g)
+        return x.to(dtype)[:, :, int(strided):]
+    bf = torch.bfloat16
+    args = rows(R, -1, 1, bf), rows(M, 0, 1 / M, bf), rows(M, 0, 1, bf), rows(M, 0.9, 1, torch.float32)
+    auto, staged = (frac_scan(*args, T, None, True, path=path) for path in ("auto", "staged"))
+    assert torch.equal(auto[0], staged[0]) and torch.equal(auto[1], staged[1])
+    few = frac_scan(*(t[:1, :4000] for t in args), T)      # below the line: the same values by the segments
+    want = staged[0][:1, :4000]
+    assert not torch.equal(few, want) and _rel(few, want.double().cpu()) <= 2 ** -7
+
+
 @pytest.mark.parametrize("M,R", [(16, 64), (8, 20)])
 def test_segments_take_any_stride_and_alignment(M, R):
     from frac_ssm_b200.ops.b200 import frac_scan

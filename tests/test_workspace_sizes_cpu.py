@@ -23,3 +23,13 @@ def test_scratch_of_the_automatic_path_alone():
     # the headline shape: the single-pass kernel's state, not the chunked stages' gigabyte
     assert lib.fracssm_frac_scan_auto_workspace_bytes(192, 8192, 64, 128, 256) < 8 << 20
     assert lib.fracssm_frac_scan_auto_workspace_bytes(0, 8192, 64, 128, 256) == 0
+
+
+@pytest.mark.parametrize("shape,staged", [((8, 8192, 192, 40, 64), True), ((8, 8192, 192, 40, 32), False), ((8, 8192, 128, 128, 64), False),
+                                          ((16, 16384, 64, 72, 128), True), ((2, 32768, 128, 40, 64), False),
+                                          ((400, 2048, 192, 40, 64), False), ((16, 16384, 16, 100, 64), False)])
+def test_scratch_of_the_automatic_path_holds_the_stages_where_dense_calls_take_them(shape, staged):
+    """(they do where the segment kernels would load element by element and were measured to be slower)"""
+    lib = C.lib()
+    need = lib.fracssm_frac_scan_auto_workspace_bytes(*shape)
+    assert (need >= lib.fracssm_frac_scan_workspace_bytes(*shape, C.PATH_STAGED)) == staged
