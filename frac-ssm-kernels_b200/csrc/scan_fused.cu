@@ -1098,11 +1098,23 @@ size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 }  // namespace
 
-// Rows up to which the state is handed over with tags (LL).  A step of a row's chain takes 1.0 us with tags and 2.4 us
-// through the counter (4 rows), a tile of a CTA 10.5 us against 8 (the tags' traffic and instructions), so:
-// 24 x 131072 tokens 1.73 ms with tags, 2.92 without; 48 x 65536 1.56 / 1.89; 64 x 8192 0.281 / 0.306;
-// 80 x 8192 0.343 / 0.317; 96 x 8192 0.406 / 0.351.  24 x 397 tokens, four tiles a row: 37 / 59 us.
+// Where the state is handed over with tags (LL).  A step of a row's chain takes 1.0 us with tags and 2.4 us through the
+// counter (4 rows), a tile of a CTA 10.5 us against 8 (the tags' traffic and instructions), and the tags start from zeros.
+// So with more rows the chain has to be longer before it counts.  Counter / tags in us (bfloat16 coefficients; float32
+// lies the same way):
+//   tiles a row        2             4             6            12            24            32
+//      8 rows    18.5 / 19.7   22.6 / 21.7                                               92 /  55
+//     24 rows    18.6 / 20.2   23.4 / 21.9   29.2 / 23.8   48.7 / 37.7   87.6 / 66.7   109 /  84
+//     32 rows    18.5 / 20.4   23.7 / 22.7   32.6 / 30.9   54.2 / 47.8   96.3 / 79.7   121 /  97
+//     40 rows    18.6 / 20.6   25.4 / 29.8   34.0 / 33.8   56.6 / 54.9   97.4 / 89.4   125 / 110
+//     48 rows    18.6 / 20.6   28.2 / 29.9   35.0 / 34.4   57.8 / 57.2    107 /  99    135 / 122
+//     64 rows    18.8 / 20.6   30.1 / 31.9   41.4 / 42.8   67.8 / 68.8    131 / 123    157 / 149
+//     80 rows, 64 tiles 317 / 343; 96 rows, 64 tiles 351 / 406
+// (24 x 131072 tokens 2.92 / 1.76 ms, 48 x 65536 1.89 / 1.56 ms.)
 constexpr int64_t kTaggedRows = 64;
+static bool tags_pay(int64_t rows, int64_t tiles) {
+  return rows <= kTaggedRows && tiles >= (rows <= 32 ? 4 : rows <= 48 ? 12 : 24);
+}
 static size_t plain_workspace_bytes(int64_t B, int64_t R, int64_t M) {
   return kCtrlBytes + align256((size_t)B * 4) + (size_t)B * R * M * 4;
 }
@@ -1205,8 +1217,8 @@ int scan_fused_launch_ex(const void *u, const void *c, const void *kappa, int ck
   CUtensorMap map;
   int rc = make_tmap_bf16_3d(&map, u, kR, (uint64_t)L, (uint64_t)B, kR, kTile);
   if (rc) return rc;
-  // (one tile: nothing is handed over; a workspace of the plain size keeps the plain hand-over)
-  const bool tagged = B <= kTaggedRows && a.ntiles - first_tile > 1 && !layer &&
+  // (a workspace of the plain size keeps the plain hand-over)
+  const bool tagged = tags_pay(B, a.ntiles - first_tile) && !layer &&
                       workspace_bytes >= tagged_workspace_bytes(B, R, M);
   // the tags start from zeros, which no tile hands over
   cudaError_t e = cudaMemsetAsync(ws, 0, tagged ? tagged_workspace_bytes(B, R, M) : kCtrlBytes + align256((size_t)B * 4),

@@ -1,5 +1,5 @@
-"""The single-pass scan's two ways of handing the state from tile to tile: up to 64 rows with tags beside the values,
-beyond through a counter.  The arithmetic is the same, so the results are the same bits."""
+"""The single-pass scan's two ways of handing the state from tile to tile: with tags beside the values for few and long
+rows (from 4 tiles on, with more than 32 rows from 12 and with more than 48 from 24, up to 64 rows), else through a counter.  The arithmetic is the same, so the results are the same bits."""
 
 import pytest
 import torch
@@ -9,7 +9,8 @@ from oracle import frac_oracle as O
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("L", [1, 128, 129, 256, 1000, 2560])       # one tile, edges of tiles, several chains deep
+# one tile, edges of tiles, several chains deep; either side of 4, 12 and 24 tiles
+@pytest.mark.parametrize("L", [1, 128, 129, 256, 384, 385, 1000, 1408, 1409, 2560, 2944, 2945])
 @pytest.mark.parametrize("coeff", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("start,final", [(False, False), (True, True)])
 def test_tagged_and_counted_hand_over_give_the_same_bits(L, coeff, start, final):
@@ -23,6 +24,6 @@ def test_tagged_and_counted_hand_over_give_the_same_bits(L, coeff, start, final)
                         final_state_dtype=torch.float32, path="fused", check=True)
         return out if final else (out,)
     ref = run(slice(0, B))
-    for rows in (slice(0, 1), slice(3, 5), slice(1, 65)):
+    for rows in (slice(0, 1), slice(3, 5), slice(0, 33), slice(16, 64), slice(1, 65)):
         for got, want in zip(run(rows), ref):
             assert torch.equal(got, want[rows])

@@ -25,7 +25,7 @@ def _ws(nbytes):
 def test_scan_wait_runs_out_and_is_reported(hand_over):
     from frac_ssm_b200 import _cabi as C
     lib = selftest_lib()
-    B, L = 3, 384
+    B, L = 3, 640        # (four tiles in the launch: the fewest that take the tags)
     u, c, kappa, rho, _ = (t.cuda() for t in O.scan_inputs(B, L, 64, 128, gen="model_like", seed=11))
     h = torch.zeros_like(u)
     fin = torch.zeros(B, 64, 128, device="cuda")
