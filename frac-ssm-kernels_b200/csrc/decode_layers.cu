@@ -46,7 +46,8 @@ __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol
 
 __device__ __forceinline__ uint4 ldg_weights(const void *p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
   return v;
 }
 __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
@@ -87,9 +88,9 @@ struct LinArgs {
   const void *next_w; int next_dt;
 };
 
-// the activations of this thread's seat in the fragment: 8 consecutive values of sequence `seq`
+// 16 bytes to shared memory, zeros where `on` is false
 __device__ __forceinline__ void copy_async16(uint32_t dst, const void *src, bool on) {
-  const int n = on ? 16 : 0;   // (0: the 16 bytes are zeros, nothing is read)
+  const int n = on ? 16 : 0;   // (0: nothing is read)
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 
@@ -208,7 +209,8 @@ __global__ void __launch_bounds__(kThreads, NT == 1 ? 3 : NT <= 4 ? 2 : 1) decod
 #pragma unroll
           for (int t = 0; t < NT; ++t) {
             const uint4 x = NT == 1 ? xs[NT == 1 ? i : 0]
-                                    : *reinterpret_cast<const uint4 *>(lin_smem + (8 * t + g) * stride + (k0 + i) * 64 + 16 * tig);
+                                    : *reinterpret_cast<const uint4 *>(lin_smem + (8 * t + g) * stride +
+                                                                       (k0 + i) * 64 + 16 * tig);
             mma_bf16(acc[t], wr[i][0].x, wr[i][1].x, wr[i][0].y, wr[i][1].y, x.x, x.y);
             mma_bf16(acc[t], wr[i][0].z, wr[i][1].z, wr[i][0].w, wr[i][1].w, x.z, x.w);
           }
@@ -346,10 +348,13 @@ __global__ void __launch_bounds__(kThreads) decode_mix_kernel(const MixArgs a) {
   for (int i = 0; i < kMixPre; ++i) {
     const int m = mg + i * groups;
     pre[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (on && m < M && a.old_state) pre[i] = __ldcs(reinterpret_cast<const float4 *>(a.old_state + sbase + (int64_t)m * R));
+    if (on && m < M && a.old_state)
+      pre[i] = __ldcs(reinterpret_cast<const float4 *>(a.old_state + sbase + (int64_t)m * R));
   }
-  const int side = tid >> 7, t128 = tid & 127;   // threads 0..127: the read side of the parameters, 128..255 the write side
-  const float read_gate = sigmoid_(ld_f32(a.read_logit, 0, a.read_dt)), write_gate = sigmoid_(ld_f32(a.write_logit, 0, a.write_dt));
+  // threads 0..127: the read side of the parameters, 128..255 the write side
+  const int side = tid >> 7, t128 = tid & 127;
+  const float read_gate = sigmoid_(ld_f32(a.read_logit, 0, a.read_dt));
+  const float write_gate = sigmoid_(ld_f32(a.write_logit, 0, a.write_dt));
   const float dtb = ld_f32(a.dt_bias, h, a.dt_bias_dt);
   const float lt0 = t128 < M ? ld_f32(a.log_tau, t128, a.log_tau_dt) : 0.f;
   const float tau0 = fmaxf(expf(lt0), 1e-6f);
@@ -436,7 +441,8 @@ __global__ void __launch_bounds__(kThreads) decode_mix_kernel(const MixArgs a) {
       if (mg + i * groups < M) step(mg + i * groups, pre[i]);
 #pragma unroll 4
     for (int m = mg + kMixPre * groups; m < M; m += groups)
-      step(m, a.old_state ? __ldcs(reinterpret_cast<const float4 *>(a.old_state + sbase + (int64_t)m * R)) : make_float4(0.f, 0.f, 0.f, 0.f));
+      step(m, a.old_state ? __ldcs(reinterpret_cast<const float4 *>(a.old_state + sbase + (int64_t)m * R))
+                          : make_float4(0.f, 0.f, 0.f, 0.f));
   }
   if (fold) {
     for (int o = quads; o < 32; o *= 2) {
@@ -503,9 +509,10 @@ size_t mix_smem_bytes(int64_t M) { return (size_t)(3 * ((M + 3) / 4 * 4) + kThre
 template <int NT>
 cudaError_t allow_smem() {
   constexpr int kMost = 227 * 1024;
-  cudaError_t e = cudaFuncSetAttribute(decode_linear_kernel<NT, kIn>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_linear_kernel<NT, kProj>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_linear_kernel<NT, kOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
+  constexpr cudaFuncAttribute kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  cudaError_t e = cudaFuncSetAttribute(decode_linear_kernel<NT, kIn>, kAttr, kMost);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_linear_kernel<NT, kProj>, kAttr, kMost);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_linear_kernel<NT, kOut>, kAttr, kMost);
   return e;
 }
 
@@ -566,8 +573,9 @@ int run_layers(const uint64_t *ptrs, const float *nums, int64_t layers, const vo
   auto at = [&](size_t off) { return ws + off; };
   const int64_t tiles_in = ceil_div(2 * di, kTileRows), tiles_rw = ceil_div(2 * H * M, kTileRows),
                 tiles_dyn = ceil_div(3 * H, kTileRows), tiles_out = ceil_div(d, kTileRows);
-  // Up to 8 sequences a block takes one tile and all tiles are resident at once (three blocks per SM);
-  // beyond, filling the activation tile costs as much as a tile's weights: one or two blocks per SM walk over the tiles.
+  // Up to 8 sequences a block takes one tile (three blocks per SM: up to 444 tiles, 7104 output rows, are resident at
+  // once, which the products of a model of hidden 768 are).  Beyond, filling the activation tile costs as much as a
+  // tile's weights: one or two blocks per SM walk over the tiles.
   auto blocks = [&](int64_t tiles, size_t smem) -> int64_t {
     if (NT == 1) return tiles;
     const int64_t most = 148 * (smem <= 110 * 1024 ? 2 : 1);
@@ -608,7 +616,8 @@ int run_layers(const uint64_t *ptrs, const float *nums, int64_t layers, const vo
     pr.act = in.x_conv; pr.act2 = in.x;
     pr.out = reinterpret_cast<float *>(at(s.rw)); pr.out2 = reinterpret_cast<float *>(at(s.dyn));
     pr.bias2 = bfp(kDynB);
-    e = launch_dep(decode_linear_kernel<NT, kProj>, dim3((unsigned)(tiles_dyn + blocks(tiles_rw, smem_di))), smem_di, st, true, pr);
+    const dim3 pr_grid((unsigned)(tiles_dyn + blocks(tiles_rw, smem_di)));
+    e = launch_dep(decode_linear_kernel<NT, kProj>, pr_grid, smem_di, st, true, pr);
     if (e != cudaSuccess) break;
 
     MixArgs m{};
@@ -659,7 +668,8 @@ extern "C" int fracssm_decode_layers_supported(int64_t B, int64_t hidden, int64_
   const int64_t di = H * R;
   if (hidden % 32 != 0 || di % 32 != 0 || di > 65536 || R % 4 != 0 || H * M > (1 << 24)) return 0;
   const int nt = B <= 8 ? 1 : B <= 16 ? 2 : B <= 32 ? 4 : 8;
-  return lin_smem_bytes(nt, di) <= 227 * 1024 && lin_smem_bytes(nt, hidden) <= 227 * 1024 && mix_smem_bytes(M) <= 47 * 1024;
+  return lin_smem_bytes(nt, di) <= 227 * 1024 && lin_smem_bytes(nt, hidden) <= 227 * 1024 &&
+         mix_smem_bytes(M) <= 47 * 1024;
 }
 
 extern "C" size_t fracssm_decode_layers_workspace_bytes(int64_t B, int64_t hidden, int64_t H, int64_t R, int64_t M) {

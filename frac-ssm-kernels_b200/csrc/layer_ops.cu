@@ -19,7 +19,8 @@ __device__ __forceinline__ float softplusf_(float x) { return x > 20.f ? x : log
 
 struct ParamArgs {
   const void *dyn; int dyn_dt; int64_t dyn_sb, dyn_sl;
-  const __nv_bfloat16 *dyn_bias;   // null, or [3 H] added to dyn (the sum rounded to bf16, as a separate addition leaves it)
+  // null, or [3 H] added to dyn (the sum rounded to bf16, as a separate addition leaves it)
+  const __nv_bfloat16 *dyn_bias;
   const void *rw; int rw_dt; int64_t rw_sb, rw_sl;
   const void *x; int x_dt; int64_t x_sb, x_sl;
   const float *mask; int64_t m_sb, m_sl;
@@ -40,7 +41,8 @@ __device__ __forceinline__ float dyn_at(const ParamArgs &a, int64_t base, int64_
 // One warp per (bh, token): lanes stride over the M modes; two softmaxes by warp shuffles.
 __global__ void __launch_bounds__(128) compute_params_kernel(const ParamArgs a) {
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  const float read_gate = sigmoidf_(ld_f32(a.read_logit, 0, a.read_dt)), write_gate = sigmoidf_(ld_f32(a.write_logit, 0, a.write_dt));
+  const float read_gate = sigmoidf_(ld_f32(a.read_logit, 0, a.read_dt));
+  const float write_gate = sigmoidf_(ld_f32(a.write_logit, 0, a.write_dt));
   const int64_t l = (int64_t)blockIdx.x * 4 + warp;
   const int64_t bh = blockIdx.y;
   if (l >= a.L) return;
@@ -108,7 +110,8 @@ __device__ __forceinline__ void unpack4(const uint2 &p, float (&f)[4]) {
 
 __global__ void __launch_bounds__(128) compute_params_m128_kernel(const ParamArgs a) {
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  const float read_gate = sigmoidf_(ld_f32(a.read_logit, 0, a.read_dt)), write_gate = sigmoidf_(ld_f32(a.write_logit, 0, a.write_dt));
+  const float read_gate = sigmoidf_(ld_f32(a.read_logit, 0, a.read_dt));
+  const float write_gate = sigmoidf_(ld_f32(a.write_logit, 0, a.write_dt));
   const int64_t l0 = ((int64_t)blockIdx.x * 4 + warp) * kPrepTokens;
   const int64_t bh = blockIdx.y;
   if (l0 >= a.L) return;
@@ -241,7 +244,8 @@ __global__ void __launch_bounds__(128) compute_params_lanes_kernel(const ParamAr
   constexpr int kStep = 32 / Q;              // tokens a warp works on at a time
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
   const int sub = lane / Q, q = lane % Q;    // token of the step; modes 8 q .. 8 q + 7
-  const float read_gate = sigmoidf_(ld_f32(a.read_logit, 0, a.read_dt)), write_gate = sigmoidf_(ld_f32(a.write_logit, 0, a.write_dt));
+  const float read_gate = sigmoidf_(ld_f32(a.read_logit, 0, a.read_dt));
+  const float write_gate = sigmoidf_(ld_f32(a.write_logit, 0, a.write_dt));
   const int64_t l0 = ((int64_t)blockIdx.x * 4 + warp) * per_warp;
   const int64_t bh = blockIdx.y;
   if (l0 >= a.L) return;
@@ -851,7 +855,8 @@ int scan_epilogue_launch(const char *who, const void *h, int h_dtype, int64_t h_
   auto al16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   const int64_t HR = H * R;
   if (h_dtype == FRACSSM_BF16 && xg_dtype == FRACSSM_BF16 && R % 8 == 0 && HR <= 8192 && al16(h) && al16(x_conv) &&
-      al16(gate) && al16(y) && al16(D) && (D_dt == FRACSSM_F32 || D_dt == FRACSSM_BF16) && h_sb % 8 == 0 && h_sl % 8 == 0 && x_sb % 8 == 0 && x_sl % 8 == 0 &&
+      al16(gate) && al16(y) && al16(D) && (D_dt == FRACSSM_F32 || D_dt == FRACSSM_BF16) && h_sb % 8 == 0 &&
+      h_sl % 8 == 0 && x_sb % 8 == 0 && x_sl % 8 == 0 &&
       g_sb % 8 == 0 && g_sl % 8 == 0) {
     const unsigned threads = (unsigned)(((HR / 8) + 31) / 32 * 32);
     const int wvec = (mode == kEpiloguePartial || !al16(weight)) ? 0 : w_dtype == FRACSSM_BF16 ? 1 : w_dtype == FRACSSM_F32 ? 2 : 0;
@@ -1006,7 +1011,8 @@ extern "C" int fracssm_add_rmsnorm(const void *x, const void *y, const void *wei
 }
 
 // What a mixer does between its projections and out_proj, in bfloat16: parameter prep, scan, (state), epilogue.
-extern "C" int fracssm_prefill_mix(const void *dyn, const void *dyn_bias, const void *rw, const void *x_conv, const void *gate, int64_t gate_sl,
+extern "C" int fracssm_prefill_mix(const void *dyn, const void *dyn_bias, const void *rw, const void *x_conv,
+                                   const void *gate, int64_t gate_sl,
                                    const float *mask, const void *const *params, int params_f32, const float *nums,
                                    const void *u, void *c, void *kappa, int ck_dtype, float *rho, void *h,
                                    float *final_state, float *state, void *y, void *workspace, size_t workspace_bytes,
@@ -1014,17 +1020,19 @@ extern "C" int fracssm_prefill_mix(const void *dyn, const void *dyn_bias, const 
   using namespace fracssm;
   if (!params || !nums || (state && !final_state)) return fail(FRACSSM_ERR_ARG, "prefill_mix: null pointer");
   if (Bt <= 0 || L <= 0 || H <= 0 || R <= 0 || M <= 0) return fail(FRACSSM_ERR_ARG, "prefill_mix: bad sizes");
-  if (state && (Bt * H > 65535 || ceil_div(R, 32) > 65535)) return fail(FRACSSM_ERR_UNSUPPORTED, "prefill_mix: too many rows");
+  if (state && (Bt * H > 65535 || ceil_div(R, 32) > 65535))
+    return fail(FRACSSM_ERR_UNSUPPORTED, "prefill_mix: too many rows");
   auto dt = [&](int i) { return (params_f32 >> i) & 1 ? FRACSSM_F32 : FRACSSM_BF16; };
   const int64_t di = H * R;
-  int rc = compute_params_typed(dyn, FRACSSM_BF16, L * 3 * H, 3 * H, dyn_bias, rw, FRACSSM_BF16, L * 2 * H * M, 2 * H * M, x_conv,
-                                FRACSSM_BF16, L * di, di, mask, L, 1, params[0], dt(0), params[3], dt(3), params[1], dt(1),
+  int rc = compute_params_typed(dyn, FRACSSM_BF16, L * 3 * H, 3 * H, dyn_bias, rw, FRACSSM_BF16, L * 2 * H * M,
+                                2 * H * M, x_conv, FRACSSM_BF16, L * di, di, mask, L, 1, params[0], dt(0), params[3], dt(3), params[1], dt(1),
                                 params[2], dt(2), nums[0], nums[1], nums[2], nums[3], nums[4], nums[5], nums[6], nullptr, c,
                                 kappa, ck_dtype, rho, Bt, L, H, R, M, stream);
   if (rc) return rc;
   bool modes_first = false;
   rc = frac_scan_route(u, FRACSSM_BF16, L * R, R, c, kappa, ck_dtype, L * M, M, L * M, M, rho, L * M, M, nullptr, h,
-                       final_state, FRACSSM_F32, workspace, workspace_bytes, Bt * H, L, R, M, T, 0, stream, state, &modes_first);
+                       final_state, FRACSSM_F32, workspace, workspace_bytes, Bt * H, L, R, M, T, 0, stream, state,
+                       &modes_first);
   if (rc) return rc;
   if (state && !modes_first) {   // (the single-pass kernel writes [R, M]: a second form of that store made it 5 % slower)
     state_transpose_kernel<<<dim3((unsigned)ceil_div(M, 32), (unsigned)ceil_div(R, 32), (unsigned)(Bt * H)), 256, 0,

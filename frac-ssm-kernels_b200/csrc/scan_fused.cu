@@ -5,9 +5,10 @@
 //
 // Work item = (bh, tile of 128 tokens), handed out by an atomic ticket in tile-major order
 // (all bh of tile 0, then tile 1, ...).  The item (bh, j) needs the state left by (bh, j-1);
-// it waits on a per-bh counter in global memory (few rows: on tags beside the state's values) with a time limit.  A ticket is only taken
-// by a running CTA (one item ahead of the one it is working on) and dependencies point to
-// lower tickets, so the lowest unfinished item is always being worked on and never waits.
+// it waits on a per-bh counter in global memory (few long rows: on tags beside the state's values)
+// with a time limit.  A ticket is only taken by a running CTA (one item ahead of the one it is
+// working on) and dependencies point to lower tickets, so the lowest unfinished item is always
+// being worked on and never waits.
 //
 // One CTA per SM, 20 warps.  Warps 0-15 ("workers") turn the raw inputs into bf16 operand tiles in
 // shared memory and run the epilogues; warp 16 ("MMA warp") issues the TMA load of u and every
@@ -23,7 +24,10 @@
 // A tile is processed in two passes over the modes (64 + 64): a worker thread owns 8 token rows x 2
 // modes per pass, so its per-token factors (32 registers) and the raw inputs of the other pass
 // (32 registers, requested one pass ahead in two batches of four token rows; full tiles use one
-// address per thread and immediate row offsets) fit in registers without spilling; each operand tile's two
+// address per thread and immediate row offsets) fit in its 96 registers with float32 coefficients; with
+// bfloat16 ones the counted instances spill one register (4 bytes stored, 40 loaded a thread), in layer mode
+// one or two, and the tagged instances, which hold two halves of tagged values as well, 24 to 98 bytes
+// stored and 24 to 104 loaded; each operand tile's two
 // 64-column halves are filled by the two passes and the level / base products are issued per pass
 // (4 of their 8 contraction steps), accumulating in tensor memory.
 //
@@ -237,7 +241,8 @@ __device__ __forceinline__ void st_tagged(uint4 *p, float a, float b, uint32_t t
 // wait for the numbers themselves.  A thread reads and writes the same 16 elements of the row's state in every tile, so
 // the hand-over is a chain of threads, without a counter, a fence or a barrier of the CTA: one L2 store and two L2
 // reads a step.  Twice the state traffic and 16 more memory instructions a tile, so it is for few rows, where a row's
-// chain of tiles is what limits the run (see scan_fused_launch_ex).
+// chain of tiles is what limits the run (see tags_pay).  (A flag beside every value is the published method of NCCL's LL
+// protocol; this is one 64-bit access of either kind, written for this hand-over.)
 // CKF32: c and kappa are float32 (else bf16).  LAYER: the output stage applies the skip connection and
 // the gate (its code is kept out of the plain kernel, whose loop is fetched once per tile).
 // RAGGED: L is not a multiple of the tile, so a row's last tile takes the row-by-row, predicated loads
@@ -248,8 +253,8 @@ scan_fused_kernel(const FusedArgs a, const __grid_constant__ CUtensorMap u_map) 
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   // mbarriers.  Completed once per tile: cb2 / cbK / barH (tcgen05.commit), barU (TMA), fS / fW / fL / fLb / out_bar
-  // (16 worker warps), item_bar / state_bar (chain warp), read_bar (workers + MMA warp).  Completed once per HALF of the modes,
-  // i.e. twice per tile, so the phase parity of half h is simply h: cb0 / cbL (tcgen05.commit) and
+  // (16 worker warps), item_bar / state_bar (chain warp), read_bar (workers + MMA warp).  Completed once per HALF of the
+  // modes, i.e. twice per tile, so the phase parity of half h is simply h: cb0 / cbL (tcgen05.commit) and
   // fA / fL1 / fK (16 worker warps).  A barrier may only be of the second kind if its second completion waits for
   // whoever waits for the first: fA and fL1 do (the workers wait for the products in between), the rows of the levels
   // 64 + 32 did not.  When the MMA warp was late by the time the workers need for a half (a few instruction fetches from

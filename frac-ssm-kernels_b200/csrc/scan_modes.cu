@@ -14,7 +14,9 @@
 // owns 4 columns of u and 8 modes (32 elements), so that registers leave room for 16 warps per SM.  (8 columns
 // need fewer instructions in all, but 160 registers: 2.5 warps per scheduler, and the whole was slower.)
 // What is not arithmetic is kept small: a group of 8 tokens is requested a group ahead into registers, widened
-// to float32 once per block and read from shared memory by all its threads; with cp.async and the conversions in every thread a token took 188 instructions a warp.
+// to float32 once per block and read from shared memory by all its threads; with cp.async and the conversions in every
+// thread a token took 188 instructions a warp.  (Calls whose rows do not load in 16-byte pieces request a group when it
+// is due; large ones among them are left to the chunked stages, see few_narrow_limit.)
 // Whole call, 2 rows x 32768 tokens, 128 columns, 16 modes, bfloat16: 328 us with the chunked stages, 80 us
 // with the first form of these kernels, 62 us here.
 #include "common.cuh"
@@ -102,7 +104,8 @@ few_scan_kernel(const FewArgs a) {
   extern __shared__ __align__(16) float few_smem[];
   const int lanes = a.lanes, sub = threadIdx.x / lanes, lane = threadIdx.x - sub * lanes;
   const int tok_floats = kOffU + a.block_cols;
-  float *wide = few_smem + min(sub, a.per_block - 1) * kGroup * tok_floats;   // (threads beyond the last segment idle along)
+  // (threads beyond the last segment idle along)
+  float *wide = few_smem + min(sub, a.per_block - 1) * kGroup * tok_floats;
   const int segs = READOUT ? a.nseg : a.nseg - 1;
   const int64_t items = (int64_t)a.B * segs, item = (int64_t)blockIdx.x * a.per_block + sub;
   const bool owner = sub < a.per_block && item < items;
@@ -172,7 +175,8 @@ few_scan_kernel(const FewArgs a) {
         widen<UD>(q_u[i], f);
         float *d = wide + ut * tok_floats + kOffU + kN * uq;
 #pragma unroll
-        for (int e = 0; e < kN; e += 4) *reinterpret_cast<float4 *>(d + e) = make_float4(f[e], f[e + 1], f[e + 2], f[e + 3]);
+        for (int e = 0; e < kN; e += 4)
+          *reinterpret_cast<float4 *>(d + e) = make_float4(f[e], f[e + 1], f[e + 2], f[e + 3]);
       }
     }
   };
@@ -314,7 +318,8 @@ few_scan_kernel(const FewArgs a) {
           const int r0 = b0 ? 2 : 0;
           if constexpr (G == 2) {
             if (a.h_vec && nw == kCols && UD != FRACSSM_F16) {
-              if (UD == FRACSSM_F32) *reinterpret_cast<float2 *>(reinterpret_cast<float *>(a.h) + row + r0) = make_float2(x0, x1);
+              if (UD == FRACSSM_F32)
+                *reinterpret_cast<float2 *>(reinterpret_cast<float *>(a.h) + row + r0) = make_float2(x0, x1);
               else *reinterpret_cast<uint32_t *>(reinterpret_cast<__nv_bfloat16 *>(a.h) + row + r0) = tile::pack2(x0, x1);
             } else {
               if (r0 < nw) st_f32(a.h, row + r0, UD, x0);
@@ -527,8 +532,8 @@ int few_launch(FewArgs &a, const FewPlan &p, cudaStream_t st) {
     int warps = (int)ceil_div(p.nseg, 8);
     if (warps > kCarryWarps) warps = kCarryWarps;
     if (e == cudaSuccess)
-      e = few_launch_dep(few_carry_kernel, dim3((unsigned)ceil_div((int64_t)a.R * Mp, 32), (unsigned)a.B), 32 * warps, 0, st,
-                         true, a.states, a.decay, a.init, p.nseg, a.R, a.M, Mp);
+      e = few_launch_dep(few_carry_kernel, dim3((unsigned)ceil_div((int64_t)a.R * Mp, 32), (unsigned)a.B), 32 * warps,
+                         0, st, true, a.states, a.decay, a.init, p.nseg, a.R, a.M, Mp);
   }
   if (e == cudaSuccess)
     e = few_launch_dep(few_scan_kernel<G, UD, CK, true>, blocks(p.nseg), threads, out_smem, st, p.nseg > 1, a);
@@ -551,7 +556,8 @@ int few_launch_modes(FewArgs &a, const FewPlan &p, cudaStream_t st) {
 }  // namespace
 
 // Up to 128 modes the state of 4 columns fits the registers of at most 16 threads (half a warp, which adds the
-// readout by shuffles); beyond, the chunked stages stay.  The other limits are those of the chunked stages (a launch's grid).
+// readout by shuffles); beyond, the chunked stages stay.  The other limits are those of the chunked stages (a launch's
+// grid).
 bool scan_few_supported(int64_t B, int64_t L, int64_t R, int64_t M, int64_t T) {
   if (B < 1 || L < 1 || R < 1 || M < 1 || M > 128 || R > 65535 || B > 65535 || L >= (int64_t(1) << 30)) return false;
   if (ceil_div(L, T) > 65535) return false;

@@ -13,8 +13,8 @@ import torch
 from ... import _cabi as C
 from .stages import _op
 
-# "auto": the single-pass tcgen05 kernel when it covers the shape, else the segment kernels (up to 128 modes), else
-# the staged kernels.
+# "auto": the single-pass tcgen05 kernel when it covers the shape, else the segment kernels (up to 128 modes, where they
+# are the faster ones), else the staged kernels.
 _PATHS = {"auto": C.PATH_AUTO, "staged": C.PATH_STAGED, "fused": C.PATH_FUSED}
 
 def frac_scan(u, c, kappa, rho, chunk_size, initial_state=None, return_final_state=False, *,
@@ -31,10 +31,13 @@ def frac_scan(u, c, kappa, rho, chunk_size, initial_state=None, return_final_sta
         final_state_dtype: dtype of the returned state; default follows the reference
             (bfloat16 when u is bfloat16, else float32).  The state is always carried in float32.
         path: "auto", "staged" or "fused".  "auto" takes the single-pass kernel when it covers the
-            shape (else the segment kernels up to 128 modes, else the staged ones), and for very few rows with many tokens (fewer than 12 rows from 32768 tokens on, 12
-            and 13 rows from 131072 on) cuts every row into sub-segments first, because a row is one chain of
-            tiles and 148 SMs want more chains than that: one summary pass over u, kappa and rho gives every sub-segment its
-            incoming state, then all sub-segments are scanned as rows (`parallel.seq_parallel_scan`).
+            shape, else up to 128 modes the segment kernels (but for large calls whose rows these
+            could not load in 16-byte pieces), else the staged ones.  For very few rows with many
+            tokens (fewer than 12 rows from 32768 tokens on, 12 and 13 rows from 131072 on) it cuts
+            every row into sub-segments first, because a row is one chain of tiles and 148 SMs want
+            more chains than that: one summary pass over u, kappa and rho gives every sub-segment
+            its incoming state, then all sub-segments are scanned as rows
+            (`parallel.seq_parallel_scan`).
         check: after the launch, synchronise and raise if a bounded device-side wait of the
             single-pass kernel ran out (debugging aid; the default stays asynchronous).
     Returns:

@@ -370,19 +370,20 @@ int fracssm_decode_layers(const uint64_t *layer_ptrs, const float *layer_nums, i
  * mask [Bt, L] or NULL, and, if tail is not NULL, tail [Bt, C, K-1] = the last K-1 masked inputs (zeros before the
  * first token).
  *
- * prefill_mix: compute_params, frac_scan and scan_epilogue of one layer.  dyn [Bt, L, 3H] (dyn_bias [3H] or NULL is added), rw [Bt, L, 2HM], x_conv
- * [Bt, L, HR], gate rows gate_sl apart, u [Bt*H, L, R], all bf16; params (host array of device pointers): dt_bias,
+ * prefill_mix: compute_params, frac_scan and scan_epilogue of one layer.  dyn [Bt, L, 3H] (dyn_bias [3H] or NULL is
+ * added), rw [Bt, L, 2HM], x_conv [Bt, L, HR], gate rows gate_sl apart, u [Bt*H, L, R], all bf16; params (host array of device pointers): dt_bias,
  * read_residual_logit, write_residual_scale, base_log_tau, D, output norm weight, bit i of params_f32 set where
  * parameter i is float32, else bf16; nums (host): read_temp, dt_min, dt_max, alpha_min, alpha_max, lambda_min,
  * lambda_max, gate bias, eps.  Scratch of the caller: c, kappa [Bt*H, L, M] (ck_dtype), rho, h, final_state
- * [Bt*H, R, M] (needed with state), workspace (fracssm_frac_scan_auto_workspace_bytes).  y may lie in u's buffer.  Results: state [Bt, H, M, R]
- * (or NULL) and y [Bt, L, HR].
+ * [Bt*H, R, M] (needed with state), workspace (fracssm_frac_scan_auto_workspace_bytes).  y may lie in u's buffer.
+ * Results: state [Bt, H, M, R] (or NULL) and y [Bt, L, HR].
  */
 int fracssm_add_rmsnorm(const void *x, const void *y, const void *weight, int w_dtype, float eps, void *sum, void *norm,
                         int64_t rows, int64_t D, void *stream);
 int fracssm_prefill_conv(const void *x, int64_t x_sl, const float *mask, const void *weight, const void *bias, void *y,
                          void *u_heads, void *tail, int64_t R, int64_t Bt, int64_t L, int64_t C, int64_t K, void *stream);
-int fracssm_prefill_mix(const void *dyn, const void *dyn_bias, const void *rw, const void *x_conv, const void *gate, int64_t gate_sl,
+int fracssm_prefill_mix(const void *dyn, const void *dyn_bias, const void *rw, const void *x_conv, const void *gate,
+                        int64_t gate_sl,
                         const float *mask, const void *const *params, int params_f32, const float *nums, const void *u,
                         void *c, void *kappa, int ck_dtype, float *rho, void *h, float *final_state, float *state,
                         void *y, void *workspace, size_t workspace_bytes, int64_t Bt, int64_t L, int64_t H, int64_t R,
