@@ -101,28 +101,30 @@ conv_tail_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_sb, int64_t x_sl
   if (ch < C) conv_tail(x, x_sb, x_sl, mask, m_sb, m_sl, tail, blockIdx.y, ch, L, C);
 }
 
-// Four channels (8 bytes) per thread, `tokens` (32 at full size) tokens walked with the window in registers, the next
+// Four channels (8 bytes) per thread, TOKENS (32 at full size) tokens walked with the window in registers, the next
 // four tokens requested before the current four are worked on; at most 80 registers, so 6 blocks of
 // 128 threads per SM.  At batch 16 x 4096 tokens x 1536 channels: 0.154 ms with 16 tokens per thread and
 // the loads of a group issued right before their use, 0.143 ms with 32 tokens (the three window tokens and
 // the weights are read once per 32), 0.125 ms with the loads one group ahead.  A short sequence is cut into runs of 16
-// or 8 tokens so that the grid covers the GPU (397 tokens: 12.2 -> 7.5 us).  With a tail, the last row of blocks writes it.
+// or 8 tokens so that the grid covers the GPU (397 tokens: 12.2 -> 7.5 us).  With TAIL, the last row of blocks writes it;
+// at full size a launch of its own does, since that branch costs the kernel registers and 6 % of its time.
+template <int TOKENS, bool TAIL>
 __global__ void __launch_bounds__(128, 6)
 causal_conv4_silu_bf16_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_sb, int64_t x_sl,
                               const float *__restrict__ mask, int64_t m_sb, int64_t m_sl,
                               const void *__restrict__ w, int w_dt, const void *__restrict__ bias,
                               __nv_bfloat16 *__restrict__ y, __nv_bfloat16 *__restrict__ u_heads, int64_t R,
-                              int64_t L, int64_t C, int tokens, const ConvTail tail) {
+                              int64_t L, int64_t C, const ConvTail tail) {
   const int64_t ch = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (ch >= C) return;
-  if (tail.out && blockIdx.y == gridDim.y - 1) {
+  if (TAIL && blockIdx.y == gridDim.y - 1) {
     for (int i = 0; i < 4; ++i) conv_tail(x, x_sb, x_sl, mask, m_sb, m_sl, tail, blockIdx.z, ch + i, L, C);
     return;
   }
   // the same four values also go to the head-major copy [Bt * H, L, R] (R a multiple of 4)
   __nv_bfloat16 *u_row = nullptr;
   if (u_heads) u_row = u_heads + ((int64_t)blockIdx.z * (C / R) + ch / R) * L * R + ch % R;
-  const int64_t b = blockIdx.z, l0 = (int64_t)blockIdx.y * tokens;
+  const int64_t b = blockIdx.z, l0 = (int64_t)blockIdx.y * TOKENS;
   float wk[4][4], bv[4], w0[4], w1[4], w2[4];
   if (w_dt == FRACSSM_BF16) {   // 4 channels x 4 taps = 32 contiguous bytes (ch is a multiple of 4)
     const uint4 *wp = reinterpret_cast<const uint4 *>(reinterpret_cast<const __nv_bfloat16 *>(w) + ch * 4);
@@ -158,7 +160,7 @@ causal_conv4_silu_bf16_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_sb,
   in(l0 - 3, w0);
   in(l0 - 2, w1);
   in(l0 - 1, w2);
-  const int64_t l1 = min(l0 + tokens, L);
+  const int64_t l1 = min(l0 + TOKENS, L);
   // the next four tokens are requested before the current four are worked on
   uint2 nraw[4];
   float nmk[4];
@@ -288,12 +290,14 @@ static int conv_silu_heads(const void *x, int x_dtype, int64_t x_sb, int64_t x_s
     int tokens = kConvTokens;
     while (tokens > 8 && ceil_div(C / 4, 128) * ceil_div(L, tokens) * Bt < 148 * 4) tokens /= 2;
     if (ceil_div(L, tokens) > 65535) tokens = kConvTokens;
-    const bool same_launch = tail.out && ceil_div(L, tokens) < 65535;
+    const bool same_launch = tail.out && tokens < kConvTokens && ceil_div(L, tokens) < 65535;
     const dim3 grid((unsigned)ceil_div(C / 4, 128), (unsigned)(ceil_div(L, tokens) + (same_launch ? 1 : 0)), (unsigned)Bt);
-    causal_conv4_silu_bf16_kernel<<<grid, block, 0, (cudaStream_t)stream>>>(
+    auto kernel = causal_conv4_silu_bf16_kernel<kConvTokens, false>;
+    if (tokens == 16) kernel = same_launch ? causal_conv4_silu_bf16_kernel<16, true> : causal_conv4_silu_bf16_kernel<16, false>;
+    if (tokens == 8) kernel = same_launch ? causal_conv4_silu_bf16_kernel<8, true> : causal_conv4_silu_bf16_kernel<8, false>;
+    kernel<<<grid, block, 0, (cudaStream_t)stream>>>(
         reinterpret_cast<const __nv_bfloat16 *>(x), x_sb, x_sl, mask, m_sb, m_sl, weight, w_dtype, bias,
-        reinterpret_cast<__nv_bfloat16 *>(y), reinterpret_cast<__nv_bfloat16 *>(u_heads), R, L, C, tokens,
-        same_launch ? tail : ConvTail{nullptr, 0});
+        reinterpret_cast<__nv_bfloat16 *>(y), reinterpret_cast<__nv_bfloat16 *>(u_heads), R, L, C, tail);
     if (tail.out && !same_launch)
       conv_tail_kernel<<<dim3((unsigned)ceil_div(C, 128), (unsigned)Bt), 128, 0, (cudaStream_t)stream>>>(
           reinterpret_cast<const __nv_bfloat16 *>(x), x_sb, x_sl, mask, m_sb, m_sl, tail, L, C);

@@ -125,3 +125,22 @@ def test_add_rmsnorm(rows, D, w_dtype):
     s = total.double()
     ref = s * torch.rsqrt(s.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
     assert (norm.double() - ref).abs().max() <= 2 ** -8 * ref.abs().max()      # one rounding to bfloat16
+
+
+# runs of 8, 16 and 32 tokens a thread: with the shorter ones the tail is written by the same launch
+@pytest.mark.parametrize("B,L,C", [(1, 2, 64), (2, 50, 72), (4, 1000, 1536), (8, 3000, 1536), (64, 200, 520)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_prefill_conv_and_its_tail(B, L, C, masked):
+    from frac_ssm_b200 import _cabi as abi
+    from frac_ssm_b200.models.modeling_frac import causal_conv_silu
+    g = torch.Generator(device="cuda").manual_seed(L + C)
+    xg = torch.randn(B, L, 2 * C, device="cuda", generator=g).bfloat16()
+    x, w = xg[..., :C], torch.randn(C, 1, 4, device="cuda", generator=g).bfloat16()
+    bias = torch.randn(C, device="cuda", generator=g).bfloat16()
+    mask = (torch.rand(B, L, device="cuda", generator=g) > 0.3).float() if masked else None
+    y, tail = torch.empty(B, L, C, device="cuda", dtype=torch.bfloat16), torch.empty(B, C, 3, device="cuda", dtype=torch.bfloat16)
+    abi.check(abi.lib().fracssm_prefill_conv(abi.ptr(x), 2 * C, abi.ptr(mask), abi.ptr(w), abi.ptr(bias), abi.ptr(y), None,
+                                             abi.ptr(tail), 0, B, L, C, 4, abi.stream_of(x)), "prefill_conv")
+    assert torch.equal(y, causal_conv_silu(x, w, bias, mask))
+    kept = x if mask is None else x * mask[..., None].bfloat16()
+    assert torch.equal(tail, torch.nn.functional.pad(kept.transpose(1, 2), (3, 0))[..., -3:])
