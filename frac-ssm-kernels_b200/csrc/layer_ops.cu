@@ -29,8 +29,44 @@ struct ParamArgs {
   int dtb_dt, lt_dt, read_dt, write_dt;
   float inv_read_temp, dt_min, dt_max, a_min, a_max, l_min, l_max;
   void *u, *c, *kappa; int ck_dt; float *rho;
+  int u_pieces;                            // 16-byte pieces of a row of u and x, 0 where rows are no such pieces
   int64_t L, H, R, M;
 };
+
+// N consecutive values: one look at the type, so that the loads are on their way together
+template <int N>
+__device__ __forceinline__ void ld_run(const void *p, int64_t i0, int dt, float (&f)[N]) {
+  if (dt == FRACSSM_F32) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) f[i] = reinterpret_cast<const float *>(p)[i0 + i];
+  } else if (dt == FRACSSM_BF16) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) f[i] = __bfloat162float(reinterpret_cast<const __nv_bfloat16 *>(p)[i0 + i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) f[i] = __half2float(reinterpret_cast<const __half *>(p)[i0 + i]);
+  }
+}
+
+// u[bh, l0 .. l1) = x's columns of head h, by a whole warp: the rows of u lie one after the other.
+__device__ __forceinline__ void copy_u(const ParamArgs &a, int64_t b, int64_t h, int64_t bh, int64_t l0, int64_t l1,
+                                       int lane) {
+  if (a.u_pieces) {
+    const int es = a.x_dt == FRACSSM_F32 ? 4 : 2, n = (int)(l1 - l0) * a.u_pieces;
+    const char *src = reinterpret_cast<const char *>(a.x) + (b * a.x_sb + l0 * a.x_sl + h * a.R) * es;
+    uint4 *dst = reinterpret_cast<uint4 *>(reinterpret_cast<char *>(a.u) + (bh * a.L + l0) * a.R * es);
+#pragma unroll 4
+    for (int i = lane; i < n; i += 32) {
+      const int t = i / a.u_pieces, p = i - t * a.u_pieces;
+      dst[i] = *reinterpret_cast<const uint4 *>(src + t * a.x_sl * es + 16 * p);
+    }
+  } else {
+    for (int64_t i = lane; i < (l1 - l0) * a.R; i += 32) {
+      const int64_t t = i / a.R, r = i - t * a.R;
+      st_f32(a.u, (bh * a.L + l0) * a.R + i, a.x_dt, ld_f32(a.x, b * a.x_sb + (l0 + t) * a.x_sl + h * a.R + r, a.x_dt));
+    }
+  }
+}
 
 // element j of a token's row of dyn (base: the row's offset)
 __device__ __forceinline__ float dyn_at(const ParamArgs &a, int64_t base, int64_t j) {
@@ -119,9 +155,9 @@ __global__ void __launch_bounds__(128) compute_params_m128_kernel(const ParamArg
   const int64_t H = a.H, R = a.R;
   constexpr int64_t M = 128;
   float lt[4], inv_tau[4];
+  ld_run(a.log_tau, 4 * lane, a.lt_dt, lt);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    lt[i] = ld_f32(a.log_tau, 4 * lane + i, a.lt_dt);
     inv_tau[i] = 1.f / fmaxf(expf(lt[i]), 1e-6f);
   }
   const float dtb = ld_f32(a.dt_bias, h, a.dtb_dt);
@@ -209,7 +245,8 @@ __global__ void __launch_bounds__(128) compute_params_m128_kernel(const ParamArg
 // 128 modes: 0.598 ms for the kernel above, 0.571 with this layout at 8 tokens per warp, 0.508 at 32 tokens per warp
 // (the per-warp setup paid less often), 0.470 with the next tokens' rows requested one step ahead.  With few tokens
 // in all a warp takes 8 (397 tokens x 24 heads: 17.5 -> 12.8 us); 8 modes, 4 x 1000 tokens x 12 heads: 47.8 us with
-// a warp per token, 8.8 here.
+// a warp per token, 8.8 here.  The copy of u, where one is asked for, is the whole warp's: by the lanes of a token it
+// took 27 of 38 us at 397 tokens x 12 heads x 8 modes.
 template <int Q>
 __device__ __forceinline__ float lanes_max(float v) {
 #pragma unroll
@@ -239,13 +276,18 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 // time constants, the gates) is paid once for all of them
 constexpr int kPairTokens = 32;
 
-template <int Q>
+// PLAIN: the small parameters are float32 and dyn has no bias to add (one token: 4.0 us instead of 4.4 with the looks at
+// the types).
+template <int Q, bool PLAIN>
 __global__ void __launch_bounds__(128) compute_params_lanes_kernel(const ParamArgs a, int per_warp) {
+  const int read_dt = PLAIN ? FRACSSM_F32 : a.read_dt, write_dt = PLAIN ? FRACSSM_F32 : a.write_dt;
+  const int lt_dt = PLAIN ? FRACSSM_F32 : a.lt_dt, dtb_dt = PLAIN ? FRACSSM_F32 : a.dtb_dt;
+  auto dyn = [&](int64_t base, int64_t j) { return PLAIN ? ld_f32(a.dyn, base + j, a.dyn_dt) : dyn_at(a, base, j); };
   constexpr int kStep = 32 / Q;              // tokens a warp works on at a time
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
   const int sub = lane / Q, q = lane % Q;    // token of the step; modes 8 q .. 8 q + 7
-  const float read_gate = sigmoidf_(ld_f32(a.read_logit, 0, a.read_dt));
-  const float write_gate = sigmoidf_(ld_f32(a.write_logit, 0, a.write_dt));
+  const float read_gate = sigmoidf_(ld_f32(a.read_logit, 0, read_dt));
+  const float write_gate = sigmoidf_(ld_f32(a.write_logit, 0, write_dt));
   const int64_t l0 = ((int64_t)blockIdx.x * 4 + warp) * per_warp;
   const int64_t bh = blockIdx.y;
   if (l0 >= a.L) return;
@@ -253,22 +295,22 @@ __global__ void __launch_bounds__(128) compute_params_lanes_kernel(const ParamAr
   const int64_t H = a.H, R = a.R;
   constexpr int64_t M = 8 * Q;
   float lt[8], inv_tau[8];
+  ld_run(a.log_tau, 8 * q, lt_dt, lt);
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    lt[i] = ld_f32(a.log_tau, 8 * q + i, a.lt_dt);
     inv_tau[i] = 1.f / fmaxf(expf(lt[i]), 1e-6f);
   }
-  const float dtb = ld_f32(a.dt_bias, h, a.dtb_dt);
+  const float dtb = ld_f32(a.dt_bias, h, dtb_dt);
   const __nv_bfloat16 *rw = reinterpret_cast<const __nv_bfloat16 *>(a.rw);
   const int64_t l1 = min(l0 + per_warp, a.L);
   // per-token scalars: computed once, by lane t for token l0 + t, handed over by shuffles
   float dt_l = 0.f, alpha_l = 0.f, rate_l = 0.f, keep_l = 1.f;
   if (lane < per_warp && l0 + lane < l1) {
     const int64_t l = l0 + lane, dbase = b * a.dyn_sb + l * a.dyn_sl;
-    dt_l = softplusf_(dyn_at(a, dbase, h) + dtb);
+    dt_l = softplusf_(dyn(dbase, h) + dtb);
     dt_l = fminf(fmaxf(dt_l, a.dt_min), a.dt_max);
-    alpha_l = a.a_min + sigmoidf_(dyn_at(a, dbase, H + h)) * (a.a_max - a.a_min);
-    const float lam = a.l_min + sigmoidf_(dyn_at(a, dbase, 2 * H + h)) * (a.l_max - a.l_min);
+    alpha_l = a.a_min + sigmoidf_(dyn(dbase, H + h)) * (a.a_max - a.a_min);
+    const float lam = a.l_min + sigmoidf_(dyn(dbase, 2 * H + h)) * (a.l_max - a.l_min);
     rate_l = powf(fmaxf(lam, 1e-4f), 1.f / fmaxf(alpha_l, 1e-4f));
     if (a.mask) keep_l = a.mask[b * a.m_sb + l * a.m_sl];
   }
@@ -279,6 +321,7 @@ __global__ void __launch_bounds__(128) compute_params_lanes_kernel(const ParamAr
     rnext = __ldcs(reinterpret_cast<const uint4 *>(rp0 + (l0 + sub) * a.rw_sl));
     wnext = __ldcs(reinterpret_cast<const uint4 *>(rp0 + (l0 + sub) * a.rw_sl + H * M));
   }
+  if (a.u) copy_u(a, b, h, bh, l0, l1, lane);
 #pragma unroll 1
   for (int it = 0; it * kStep < per_warp; ++it) {
     if (l0 + kStep * it >= l1) break;
@@ -347,11 +390,6 @@ __global__ void __launch_bounds__(128) compute_params_lanes_kernel(const ParamAr
         __stcs(reinterpret_cast<uint4 *>(reinterpret_cast<__nv_bfloat16 *>(a.kappa) + obase),
                make_uint4(pack_bf16x2(wl[0], wl[1]), pack_bf16x2(wl[2], wl[3]), pack_bf16x2(wl[4], wl[5]),
                           pack_bf16x2(wl[6], wl[7])));
-      }
-      if (a.u) {
-        const int64_t xbase = b * a.x_sb + l * a.x_sl + h * R;
-        for (int64_t r = q; r < R; r += Q)
-          st_f32(a.u, (bh * a.L + l) * R + r, a.x_dt, ld_f32(a.x, xbase + r, a.x_dt));
       }
     }
   }
@@ -749,21 +787,30 @@ int compute_params_typed(const void *dyn, int dyn_dtype, int64_t dyn_sb, int64_t
   a.l_min = lambda_min; a.l_max = lambda_max;
   a.u = u; a.c = c; a.kappa = kappa; a.ck_dt = ck_dtype; a.rho = rho;
   a.L = L; a.H = H; a.R = R; a.M = M;
+  const int64_t es = (int64_t)dtype_size(x_dtype);
+  const uint64_t x_bits = (uint64_t)(uintptr_t)x_conv | (uint64_t)(uintptr_t)u | (uint64_t)(x_sb * es) |
+                          (uint64_t)(x_sl * es) | (uint64_t)(R * es);
+  a.u_pieces = (x_bits & 15) == 0 && R * es < (int64_t(1) << 28) ? (int)(R * es / 16) : 0;
   auto al = [](const void *p, uintptr_t n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; };
   const bool vec = rw_dtype == FRACSSM_BF16 && (ck_dtype == FRACSSM_F32 || ck_dtype == FRACSSM_BF16) && al(c, 16) &&
                    al(kappa, 16) && al(rho, 16);
-  // 16-byte loads of the residual rows
-  if (vec && al(rw, 16) && rw_sb % 8 == 0 && rw_sl % 8 == 0 && (M == 8 || M == 16 || M == 32 || M == 64 || M == 128)) {
+  // 16-byte loads of the residual rows.  Up to 64 modes a warp per token is the faster way for the fewest tokens: 32 x 1
+  // tokens x 64 heads 8.9 against 11.1 us at 32 modes, 1 x 100 x 12 heads 5.8 against 7.5 at 8.
+  const bool fewest = M < 128 && (L < 4 || (M <= 16 && Bt * H * L < 2048));
+  if (vec && al(rw, 16) && rw_sb % 8 == 0 && rw_sl % 8 == 0 && !fewest &&
+      (M == 8 || M == 16 || M == 32 || M == 64 || M == 128)) {
     // 32 tokens per warp, or as few as 8 while that leaves the GPU less than four blocks per SM
     int per_warp = kPairTokens;
     while (per_warp > 8 && per_warp > 256 / M && Bt * H * ceil_div(L, 4 * per_warp) < 148 * 4) per_warp /= 2;
     const dim3 grid((unsigned)ceil_div(L, 4 * per_warp), (unsigned)(Bt * H));
-    const cudaStream_t st = (cudaStream_t)stream;
-    if (M == 8) compute_params_lanes_kernel<1><<<grid, 128, 0, st>>>(a, per_warp);
-    else if (M == 16) compute_params_lanes_kernel<2><<<grid, 128, 0, st>>>(a, per_warp);
-    else if (M == 32) compute_params_lanes_kernel<4><<<grid, 128, 0, st>>>(a, per_warp);
-    else if (M == 64) compute_params_lanes_kernel<8><<<grid, 128, 0, st>>>(a, per_warp);
-    else compute_params_lanes_kernel<16><<<grid, 128, 0, st>>>(a, per_warp);
+    const bool plain = !dyn_bias && dtb_dt == FRACSSM_F32 && lt_dt == FRACSSM_F32 && read_dt == FRACSSM_F32 &&
+                       write_dt == FRACSSM_F32;
+    auto kernel = plain ? compute_params_lanes_kernel<16, true> : compute_params_lanes_kernel<16, false>;
+    if (M == 8) kernel = plain ? compute_params_lanes_kernel<1, true> : compute_params_lanes_kernel<1, false>;
+    if (M == 16) kernel = plain ? compute_params_lanes_kernel<2, true> : compute_params_lanes_kernel<2, false>;
+    if (M == 32) kernel = plain ? compute_params_lanes_kernel<4, true> : compute_params_lanes_kernel<4, false>;
+    if (M == 64) kernel = plain ? compute_params_lanes_kernel<8, true> : compute_params_lanes_kernel<8, false>;
+    kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(a, per_warp);
     return check_launch("compute_params");
   }
   if (vec && M == 128 && al(rw, 8) && rw_sb % 4 == 0 && rw_sl % 4 == 0) {

@@ -387,3 +387,20 @@ def test_params_with_whole_groups_of_modes_match_the_general_kernel(M, B, L):
         for a, b in zip(got[1:], ref[1:]):
             tol = 2 ** -7 if a.dtype == torch.bfloat16 else 2e-6      # bfloat16: neighbours, if the halfway point lies between
             torch.testing.assert_close(a.float(), b.float(), rtol=tol, atol=2.4e-7)
+
+
+@pytest.mark.parametrize("M", [8, 16, 32, 64, 128, 20])                       # the lanes of a token, and a warp per token
+@pytest.mark.parametrize("R,shift", [(64, 0), (64, 4), (20, 0), (5, 0), (128, 0)])      # rows of 16-byte pieces and others
+@pytest.mark.parametrize("B,L", [(1, 1), (3, 37), (2, 1300)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_compute_params_copies_u_head_major(M, R, shift, B, L, dtype):
+    from frac_ssm_b200.layers.compute_params import compute_params_from_projections
+    H = 3
+    g = torch.Generator(device="cuda").manual_seed(M + R)
+    x = torch.randn(B, L, H * R + shift, device="cuda", generator=g).to(dtype)[..., shift:]
+    dyn, rw = (torch.randn(B, L, n, device="cuda", generator=g).bfloat16() for n in (3 * H, 2 * H * M))
+    args = (torch.zeros(H, device="cuda"), 0.0, 0.0, torch.linspace(0, 3, M, device="cuda"), H, R, M, 1.0, 1e-3, 1.0, 0.1, 0.9, 0.1, 2.0)
+    u, c, kappa, rho = compute_params_from_projections(dyn, rw, x, None, *args)
+    assert torch.equal(u, x.reshape(B, L, H, R).transpose(1, 2).reshape(B * H, L, R))
+    given = compute_params_from_projections(dyn, rw, x, None, *args, u=u)
+    assert all(torch.equal(a, b) for a, b in zip(given[1:], (c, kappa, rho)))
