@@ -244,9 +244,9 @@ __global__ void __launch_bounds__(128) compute_params_m128_kernel(const ParamArg
 // of which about 50 are the per-mode arithmetic; this one about 95.  Measured at batch 16 x 4096 tokens x 24 heads x
 // 128 modes: 0.598 ms for the kernel above, 0.571 with this layout at 8 tokens per warp, 0.508 at 32 tokens per warp
 // (the per-warp setup paid less often), 0.470 with the next tokens' rows requested one step ahead.  With few tokens
-// in all a warp takes 8 (397 tokens x 24 heads: 17.5 -> 12.8 us); 8 modes, 4 x 1000 tokens x 12 heads: 47.8 us with
-// a warp per token, 8.8 here.  The copy of u, where one is asked for, is the whole warp's: by the lanes of a token it
-// took 27 of 38 us at 397 tokens x 12 heads x 8 modes.
+// in all a warp takes 8 (397 tokens x 24 heads: 14.7 -> 7.7 us in a stream); 8 modes, 4 x 1000 tokens x 12 heads: 44
+// us with a warp per token, 4.9 here.  The copy of u, where one is asked for, is the whole warp's: copied by the lanes
+// of a token 397 tokens x 12 heads x 8 modes took 38 us, 7.2 so.
 template <int Q>
 __device__ __forceinline__ float lanes_max(float v) {
 #pragma unroll
