@@ -590,6 +590,8 @@ state_transpose_kernel(const float *__restrict__ fin, float *__restrict__ state,
 constexpr int kEpilogueFull = 0, kEpiloguePartial = 1, kEpilogueApply = 2;
 
 // One block per (b, l) row of width H*R: un-flatten h, add the D skip, gate, normalise.
+// DF32: D is float32 (looked up by type in the loops, the kernel took 4 % longer on float32 models)
+template <bool DF32>
 __global__ void __launch_bounds__(256)
 scan_epilogue_kernel(const void *__restrict__ h, int h_dt, int64_t h_sb, int64_t h_sl,
                      const void *__restrict__ x, int64_t x_sb, int64_t x_sl,
@@ -597,6 +599,7 @@ scan_epilogue_kernel(const void *__restrict__ h, int h_dt, int64_t h_sb, int64_t
                      const void *__restrict__ Dp, int D_dt, const void *__restrict__ w, int w_dt,
                      float gate_bias, float eps, void *__restrict__ y, int64_t L, int64_t H,
                      int64_t R, int mode, float *__restrict__ sumsq, int64_t norm_width) {
+  const int d_dt = DF32 ? FRACSSM_F32 : D_dt;
   __shared__ float red[32];
   const int64_t HR = H * R;
   const int64_t row = blockIdx.x, b = row / L, l = row % L;
@@ -604,7 +607,7 @@ scan_epilogue_kernel(const void *__restrict__ h, int h_dt, int64_t h_sb, int64_t
   for (int64_t j = threadIdx.x; mode != kEpilogueApply && j < HR; j += blockDim.x) {
     const int64_t hh = j / R, r = j % R;
     float v = ld_f32(h, (b * H + hh) * h_sb + l * h_sl + r, h_dt) +
-              ld_f32(x, b * x_sb + l * x_sl + j, dt) * ld_f32(Dp, j, D_dt);
+              ld_f32(x, b * x_sb + l * x_sl + j, dt) * ld_f32(Dp, j, d_dt);
     const float z = ld_f32(gate, b * g_sb + l * g_sl + j, dt) + gate_bias;
     v *= z * sigmoidf_(z);
     ss = fmaf(v, v, ss);
@@ -622,7 +625,7 @@ scan_epilogue_kernel(const void *__restrict__ h, int h_dt, int64_t h_sb, int64_t
   for (int64_t j = threadIdx.x; j < HR; j += blockDim.x) {
     const int64_t hh = j / R, r = j % R;
     float v = ld_f32(h, (b * H + hh) * h_sb + l * h_sl + r, h_dt) +
-              ld_f32(x, b * x_sb + l * x_sl + j, dt) * ld_f32(Dp, j, D_dt);
+              ld_f32(x, b * x_sb + l * x_sl + j, dt) * ld_f32(Dp, j, d_dt);
     const float z = ld_f32(gate, b * g_sb + l * g_sl + j, dt) + gate_bias;
     v *= z * sigmoidf_(z);
     st_f32(y, row * HR + j, dt, v * rs * ld_f32(w, j, w_dt));
@@ -924,7 +927,8 @@ int scan_epilogue_launch(const char *who, const void *h, int h_dtype, int64_t h_
 #undef FRACSSM_EPILOGUE
     return check_launch(who);
   }
-  scan_epilogue_kernel<<<(unsigned)(Bt * L), 256, 0, (cudaStream_t)stream>>>(
+  auto kernel = D_dt == FRACSSM_F32 ? scan_epilogue_kernel<true> : scan_epilogue_kernel<false>;
+  kernel<<<(unsigned)(Bt * L), 256, 0, (cudaStream_t)stream>>>(
       h, h_dtype, h_sb, h_sl, x_conv, x_sb, x_sl, gate, g_sb, g_sl, xg_dtype, D, D_dt, weight, w_dtype,
       gate_bias, eps, y, L, H, R, mode, sumsq, norm_width);
   return check_launch(who);
