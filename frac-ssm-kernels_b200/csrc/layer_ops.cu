@@ -75,10 +75,15 @@ __device__ __forceinline__ float dyn_at(const ParamArgs &a, int64_t base, int64_
 }
 
 // One warp per (bh, token): lanes stride over the M modes; two softmaxes by warp shuffles.
+// PLAIN: the small parameters are float32 and dyn has no bias to add.
+template <bool PLAIN>
 __global__ void __launch_bounds__(128) compute_params_kernel(const ParamArgs a) {
+  const int read_dt = PLAIN ? FRACSSM_F32 : a.read_dt, write_dt = PLAIN ? FRACSSM_F32 : a.write_dt;
+  const int lt_dt = PLAIN ? FRACSSM_F32 : a.lt_dt, dtb_dt = PLAIN ? FRACSSM_F32 : a.dtb_dt;
+  auto dyn = [&](int64_t base, int64_t j) { return PLAIN ? ld_f32(a.dyn, base + j, a.dyn_dt) : dyn_at(a, base, j); };
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  const float read_gate = sigmoidf_(ld_f32(a.read_logit, 0, a.read_dt));
-  const float write_gate = sigmoidf_(ld_f32(a.write_logit, 0, a.write_dt));
+  const float read_gate = sigmoidf_(ld_f32(a.read_logit, 0, read_dt));
+  const float write_gate = sigmoidf_(ld_f32(a.write_logit, 0, write_dt));
   const int64_t l = (int64_t)blockIdx.x * 4 + warp;
   const int64_t bh = blockIdx.y;
   if (l >= a.L) return;
@@ -86,10 +91,10 @@ __global__ void __launch_bounds__(128) compute_params_kernel(const ParamArgs a) 
   const int64_t H = a.H, M = a.M, R = a.R;
 
   const int64_t dbase = b * a.dyn_sb + l * a.dyn_sl;
-  float dt = softplusf_(dyn_at(a, dbase, h) + ld_f32(a.dt_bias, h, a.dtb_dt));
+  float dt = softplusf_(dyn(dbase, h) + ld_f32(a.dt_bias, h, dtb_dt));
   dt = fminf(fmaxf(dt, a.dt_min), a.dt_max);
-  const float alpha = a.a_min + sigmoidf_(dyn_at(a, dbase, H + h)) * (a.a_max - a.a_min);
-  const float lam = a.l_min + sigmoidf_(dyn_at(a, dbase, 2 * H + h)) * (a.l_max - a.l_min);
+  const float alpha = a.a_min + sigmoidf_(dyn(dbase, H + h)) * (a.a_max - a.a_min);
+  const float lam = a.l_min + sigmoidf_(dyn(dbase, 2 * H + h)) * (a.l_max - a.l_min);
   const float rate = powf(fmaxf(lam, 1e-4f), 1.f / fmaxf(alpha, 1e-4f));
   const float keep = a.mask ? a.mask[b * a.m_sb + l * a.m_sl] : 1.f;
 
@@ -97,7 +102,7 @@ __global__ void __launch_bounds__(128) compute_params_kernel(const ParamArgs a) 
   const int64_t wbase = rbase + H * M;                            // write residuals
   float rmax = -INFINITY, wmax = -INFINITY;
   for (int64_t m = lane; m < M; m += 32) {
-    const float prior = -alpha * ld_f32(a.log_tau, m, a.lt_dt);
+    const float prior = -alpha * ld_f32(a.log_tau, m, lt_dt);
     rmax = fmaxf(rmax, (prior + read_gate * ld_f32(a.rw, rbase + m, a.rw_dt)) * a.inv_read_temp);
     wmax = fmaxf(wmax, prior + write_gate * ld_f32(a.rw, wbase + m, a.rw_dt));
   }
@@ -105,14 +110,14 @@ __global__ void __launch_bounds__(128) compute_params_kernel(const ParamArgs a) 
   wmax = warp_max(wmax);
   float rsum = 0.f, wsum = 0.f;
   for (int64_t m = lane; m < M; m += 32) {
-    const float prior = -alpha * ld_f32(a.log_tau, m, a.lt_dt);
+    const float prior = -alpha * ld_f32(a.log_tau, m, lt_dt);
     rsum += __expf((prior + read_gate * ld_f32(a.rw, rbase + m, a.rw_dt)) * a.inv_read_temp - rmax);
     wsum += __expf(prior + write_gate * ld_f32(a.rw, wbase + m, a.rw_dt) - wmax);
   }
   const float rinv = 1.f / warp_sum(rsum), winv = 1.f / warp_sum(wsum);
   const int64_t obase = (bh * a.L + l) * M;
   for (int64_t m = lane; m < M; m += 32) {
-    const float lt = ld_f32(a.log_tau, m, a.lt_dt);
+    const float lt = ld_f32(a.log_tau, m, lt_dt);
     const float prior = -alpha * lt;
     const float cw = __expf((prior + read_gate * ld_f32(a.rw, rbase + m, a.rw_dt)) * a.inv_read_temp - rmax) * rinv;
     const float ww = __expf(prior + write_gate * ld_f32(a.rw, wbase + m, a.rw_dt) - wmax) * winv;
@@ -276,8 +281,7 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 // time constants, the gates) is paid once for all of them
 constexpr int kPairTokens = 32;
 
-// PLAIN: the small parameters are float32 and dyn has no bias to add (one token: 4.0 us instead of 4.4 with the looks at
-// the types).
+// PLAIN: as above (one token: 4.0 us instead of 4.4 with the looks at the types).
 template <int Q, bool PLAIN>
 __global__ void __launch_bounds__(128) compute_params_lanes_kernel(const ParamArgs a, int per_warp) {
   const int read_dt = PLAIN ? FRACSSM_F32 : a.read_dt, write_dt = PLAIN ? FRACSSM_F32 : a.write_dt;
@@ -795,6 +799,8 @@ int compute_params_typed(const void *dyn, int dyn_dtype, int64_t dyn_sb, int64_t
                           (uint64_t)(x_sl * es) | (uint64_t)(R * es);
   a.u_pieces = (x_bits & 15) == 0 && R * es < (int64_t(1) << 28) ? (int)(R * es / 16) : 0;
   auto al = [](const void *p, uintptr_t n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; };
+  const bool plain = !dyn_bias && dtb_dt == FRACSSM_F32 && lt_dt == FRACSSM_F32 && read_dt == FRACSSM_F32 &&
+                     write_dt == FRACSSM_F32;
   const bool vec = rw_dtype == FRACSSM_BF16 && (ck_dtype == FRACSSM_F32 || ck_dtype == FRACSSM_BF16) && al(c, 16) &&
                    al(kappa, 16) && al(rho, 16);
   // 16-byte loads of the residual rows.  Up to 64 modes a warp per token is the faster way for the fewest tokens: 32 x 1
@@ -806,8 +812,6 @@ int compute_params_typed(const void *dyn, int dyn_dtype, int64_t dyn_sb, int64_t
     int per_warp = kPairTokens;
     while (per_warp > 8 && per_warp > 256 / M && Bt * H * ceil_div(L, 4 * per_warp) < 148 * 4) per_warp /= 2;
     const dim3 grid((unsigned)ceil_div(L, 4 * per_warp), (unsigned)(Bt * H));
-    const bool plain = !dyn_bias && dtb_dt == FRACSSM_F32 && lt_dt == FRACSSM_F32 && read_dt == FRACSSM_F32 &&
-                       write_dt == FRACSSM_F32;
     auto kernel = plain ? compute_params_lanes_kernel<16, true> : compute_params_lanes_kernel<16, false>;
     if (M == 8) kernel = plain ? compute_params_lanes_kernel<1, true> : compute_params_lanes_kernel<1, false>;
     if (M == 16) kernel = plain ? compute_params_lanes_kernel<2, true> : compute_params_lanes_kernel<2, false>;
@@ -822,7 +826,8 @@ int compute_params_typed(const void *dyn, int dyn_dtype, int64_t dyn_sb, int64_t
     return check_launch("compute_params");
   }
   dim3 grid((unsigned)ceil_div(L, 4), (unsigned)(Bt * H));
-  compute_params_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(a);
+  auto kernel = plain ? compute_params_kernel<true> : compute_params_kernel<false>;
+  kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(a);
   return check_launch("compute_params");
 }
 }  // namespace
