@@ -3,10 +3,10 @@
 //   S = rho (.) S + u kappa^T,   h = S c,
 // with every row cut into segments so that few long rows fill the GPU too.
 //
-//   1. few_scan_kernel<.., false>: per segment but the last, the state it reaches from zero and the
+//   1. few_scan_kernel<.., false, ..>: per segment but the last, the state it reaches from zero and the
 //      product of its decays;
 //   2. few_carry_kernel: the state that enters every segment (in place of the states of step 1);
-//   3. few_scan_kernel<.., true>: every segment again from its true incoming state, writing h.
+//   3. few_scan_kernel<.., true, ..>:  every segment again from its true incoming state, writing h.
 // Rows that are enough by themselves (see few_plan) take step 3 alone.
 //
 // What bounds it: instruction issue, two fifths of it the FMA pipe.  A state element costs a multiply and two
@@ -93,7 +93,8 @@ __device__ __forceinline__ void ld_pairs(const float *p, f2 (&v)[4]) {   // eigh
 // `lanes` threads work on one segment of one row and block_cols columns of u: thread = (column lane, mode group),
 // columns 4 cl .. 4 cl + 3, modes 8 g .. 8 g + 7 (Mp = 8 G modes, zeros beyond M).  Segments that need less than a
 // warp share one.
-template <int G, int UD, int CK, bool READOUT>
+// PADDED: M < Mp (as a branch of one kernel the care for the padding modes cost the others 2 %).
+template <int G, int UD, int CK, bool READOUT, bool PADDED>
 __global__ void __launch_bounds__(32 * G, G == 1 ? 16 : G == 2 ? 8 : G == 4 ? 4 : G == 8 ? 2 : 1)
 few_scan_kernel(const FewArgs a) {
   constexpr int Mp = kModes * G;
@@ -198,9 +199,9 @@ few_scan_kernel(const FewArgs a) {
       const int t = i / a.block_cols, r = i - t * a.block_cols;
       const float v = r < cols ? ld_f32(u_p + ((int64_t)ib * kGroup + t) * a.u.sl, r, UD) : 0.f;
       wide[t * tok_floats + kOffU + r] = v;
-      meets |= !isfinite(v);
+      if (PADDED) meets |= !isfinite(v);
     }
-    return meets && a.M < Mp;
+    return meets;
   };
   if (a.wide_loads) request(0);
   grid_dep_wait();
@@ -243,7 +244,9 @@ few_scan_kernel(const FewArgs a) {
       request(ib + 1);
       __syncthreads();
     } else {
-      keep_zero = __syncthreads_or(copy_group(ib));
+      const bool meets = copy_group(ib);
+      if constexpr (PADDED) keep_zero = __syncthreads_or(meets);
+      else __syncthreads();
     }
     const int n = max(0, min(kGroup, ntok - ib * kGroup)), n_all = min(kGroup, all_tok - ib * kGroup);
     const float *tok = wide;
@@ -262,7 +265,7 @@ few_scan_kernel(const FewArgs a) {
 #pragma unroll
           for (int p = 0; p < 4; ++p) st[r][p] = fma2(rr[p], st[r][p], mul2(ka[p], uu[r]));
         }
-        if (keep_zero) {
+        if (PADDED && keep_zero) {
 #pragma unroll
           for (int p = 0; p < 4; ++p) {
             const int m = kModes * g + 2 * p;
@@ -528,15 +531,17 @@ int few_launch(FewArgs &a, const FewPlan &p, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
   auto blocks = [&](int64_t segs) { return dim3((unsigned)ceil_div((int64_t)a.B * segs, p.per_block), p.col_blocks); };
   if (p.nseg > 1) {
-    e = few_launch_dep(few_scan_kernel<G, UD, CK, false>, blocks(p.nseg - 1), threads, sum_smem, st, false, a);
+    auto summary = a.M < Mp ? few_scan_kernel<G, UD, CK, false, true> : few_scan_kernel<G, UD, CK, false, false>;
+    e = few_launch_dep(summary, blocks(p.nseg - 1), threads, sum_smem, st, false, a);
     int warps = (int)ceil_div(p.nseg, 8);
     if (warps > kCarryWarps) warps = kCarryWarps;
     if (e == cudaSuccess)
       e = few_launch_dep(few_carry_kernel, dim3((unsigned)ceil_div((int64_t)a.R * Mp, 32), (unsigned)a.B), 32 * warps,
                          0, st, true, a.states, a.decay, a.init, p.nseg, a.R, a.M, Mp);
   }
+  auto readout = a.M < Mp ? few_scan_kernel<G, UD, CK, true, true> : few_scan_kernel<G, UD, CK, true, false>;
   if (e == cudaSuccess)
-    e = few_launch_dep(few_scan_kernel<G, UD, CK, true>, blocks(p.nseg), threads, out_smem, st, p.nseg > 1, a);
+    e = few_launch_dep(readout, blocks(p.nseg), threads, out_smem, st, p.nseg > 1, a);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(FRACSSM_ERR_CUDA, "frac_scan (segment kernels): %s", cudaGetErrorString(e));
