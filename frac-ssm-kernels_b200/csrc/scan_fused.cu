@@ -24,10 +24,10 @@
 // A tile is processed in two passes over the modes (64 + 64): a worker thread owns 8 token rows x 2
 // modes per pass, so its per-token factors (32 registers) and the raw inputs of the other pass
 // (32 registers, requested one pass ahead in two batches of four token rows; full tiles use one
-// address per thread and immediate row offsets) fit in its 96 registers with float32 coefficients; with
-// bfloat16 ones the counted instances spill one register (4 bytes stored, 40 loaded a thread), in layer mode
-// one or two, and the tagged instances, which hold two halves of tagged values as well, 24 to 98 bytes
-// stored and 24 to 104 loaded; each operand tile's two
+// address per thread and immediate row offsets) fit in its 112 registers; with
+// bfloat16 coefficients the counted instances spill one register of the MMA warp (4 bytes stored, 40 loaded a thread), in
+// layer mode one or two, and the tagged instances with float32 ones, which hold two halves of tagged values as well,
+// 24 to 98 bytes stored and 24 to 104 loaded; each operand tile's two
 // 64-column halves are filled by the two passes and the level / base products are issued per pass
 // (4 of their 8 contraction steps), accumulating in tensor memory.
 //
@@ -69,12 +69,21 @@ namespace {
 
 using namespace tile;
 constexpr int kWorkers = 512, kThreads = 640;
-// Registers are re-divided after launch (setmaxnreg): the 16 worker warps grow to kWorkerRegs,
-// the group of the MMA and chain warps shrinks to kControlRegs.  Each SM sub-partition holds four
-// worker warps and one warp of that group: 4 * 112 + 32 = 5 * 96, the launch allocation
+// Registers are re-divided after launch (setmaxnreg): the 16 worker warps grow to kWorker registers,
+// the group of the MMA and chain warps shrinks to kControl.  Each SM sub-partition holds four
+// worker warps and one warp of that group: 4 * 112 + 32 = 4 * 104 + 64 = 5 * 96, the launch allocation
 // (checked on the host: it must cover both, or the growing warps would wait forever).
-constexpr int kWorkerRegs = 112, kControlRegs = 32;
-constexpr int kLaunchRegsNeeded = (kWorkers * kWorkerRegs + (kThreads - kWorkers) * kControlRegs + kThreads - 1) / kThreads;
+// The tagged instances with bfloat16 coefficients take the second division: what they spilled at 112 / 32 (58 bytes
+// stored and 68 loaded a thread) were the MMA warp's 32 registers, their workers fit in 104.  24 rows x 65536 tokens 884
+// and 808 us, 12 x 4096 57.5 and 46.0.  With float32 coefficients the workers need the 112, and so do the counted
+// bfloat16 instances to be the faster ones, although the MMA warp then spills a register (192 x 8192: 655 and 690 us).
+template <bool CKF32, bool LL>
+struct Regs {
+  static constexpr int kWorker = LL && !CKF32 ? 104 : 112, kControl = LL && !CKF32 ? 64 : 32;
+};
+constexpr int kLaunchRegsNeeded = 96;
+static_assert(kWorkers * 112 + (kThreads - kWorkers) * 32 <= kThreads * kLaunchRegsNeeded &&
+              kWorkers * 104 + (kThreads - kWorkers) * 64 <= kThreads * kLaunchRegsNeeded);
 // shared memory map (bytes from the 1024-aligned base)
 constexpr uint32_t kSlot = 32768;
 static_assert(kSlot == 32768, "emit_pair_next_slot stores 32768 bytes further on");
@@ -250,6 +259,7 @@ __device__ __forceinline__ void st_tagged(uint4 *p, float a, float b, uint32_t t
 template <bool CKF32, bool LAYER, bool RAGGED, bool LL>
 __global__ void __launch_bounds__(kThreads, 1)
 scan_fused_kernel(const FusedArgs a, const __grid_constant__ CUtensorMap u_map) {
+  constexpr int kWorkerRegs = Regs<CKF32, LL>::kWorker, kControlRegs = Regs<CKF32, LL>::kControl;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   // mbarriers.  Completed once per tile: cb2 / cbK / barH (tcgen05.commit), barU (TMA), fS / fW / fL / fLb / out_bar
