@@ -1,4 +1,4 @@
-"""One token through all layers in native code (`csrc/decode_layers.cu`): four kernels per layer.
+"""One token through all layers in native code (`csrc/decode_layers.cu`): one kernel, or four per layer.
 
 Covers bfloat16 models on one GPU, one token per sequence, up to 64 sequences, no attention mask.  The
 parameters are looked up in the modules on every call (nothing is remembered between calls), and whatever
