@@ -9,8 +9,10 @@
 //   3. few_scan_kernel<.., true, ..>:  every segment again from its true incoming state, writing h.
 // Rows that are enough by themselves (see few_plan) take step 3 alone.
 //
-// What bounds it: instruction issue, two fifths of it the FMA pipe.  A state element costs a multiply and two
-// fused multiply-adds per token (two instructions without the readout), worked on as packed pairs; a thread
+// What bounds it: instruction issue, half of it the FMA pipe.  A state element costs a multiply and two
+// fused multiply-adds per token in step 3, one fused multiply-add and an eighth of a multiply in step 1: there kappa is
+// multiplied with the decay behind its token within a group of 8 first, once for all columns (22 us as the recurrence, 16
+// so).  Elements are worked on as packed pairs; a thread
 // owns 4 columns of u and 8 modes (32 elements), so that registers leave room for 16 warps per SM.  (8 columns
 // need fewer instructions in all, but 160 registers: 2.5 warps per scheduler, and the whole was slower.)
 // What is not arithmetic is kept small: a group of 8 tokens is requested a group ahead into registers, widened
@@ -18,7 +20,9 @@
 // thread a token took 188 instructions a warp.  (Calls whose rows do not load in 16-byte pieces request a group when it
 // is due; large ones among them are left to the chunked stages, see few_narrow_limit.)
 // Whole call, 2 rows x 32768 tokens, 128 columns, 16 modes, bfloat16: 328 us with the chunked stages, 80 us
-// with the first form of these kernels, 62 us here.
+// with the first form of these kernels, 62 us with a recurrence in step 1 too, 54 us here.
+#include <type_traits>
+
 #include "common.cuh"
 #include "scan_tile.cuh"
 
@@ -40,6 +44,10 @@ constexpr int kGroup = 8;      // tokens per group
 constexpr int kCols = 4;       // columns of u per thread
 constexpr int kModes = 8;      // modes per thread
 constexpr int kMaxBlockCols = 128;
+constexpr int kTokPad = 4;     // floats between a token's values and the next token's in the summary
+// Least decay behind a token that the summary multiplies kappa with: a product of 7 decays may underflow, and zero times an
+// infinity of u would be NaN where the recurrence has the infinity.  (Contributions below 1e-37 |kappa u| are lost in any sum.)
+constexpr float kLeastDecay = 1e-37f;
 
 struct Rows {                  // one input: base and strides in bytes
   const char *p;
@@ -85,10 +93,29 @@ __device__ __forceinline__ void widen(const uint4 &raw, float (&f)[DT == FRACSSM
   }
 }
 
+// four coefficients of a token: 16 bytes of float32, 8 of the 16-bit types
+template <int DT>
+__device__ __forceinline__ void widen4(const uint4 &raw, float (&f)[4]) {
+  widen<FRACSSM_F32>(raw, f);
+}
+template <int DT>
+__device__ __forceinline__ void widen4(const uint2 &raw, float (&f)[4]) {
+  float g[8];
+  widen<DT == FRACSSM_F16 ? FRACSSM_F16 : FRACSSM_BF16>(make_uint4(raw.x, raw.y, 0u, 0u), g);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f[i] = g[i];
+}
+
 __device__ __forceinline__ void ld_pairs(const float *p, f2 (&v)[4]) {   // eight floats
   const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(p), b = *reinterpret_cast<const ulonglong2 *>(p + 4);
   v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
+
+// Room for two groups lets one be stored while the slower warps still read the one before.  A readout of 4 and more warps a
+// segment is faster with one (400 rows x 2000 tokens, 64 columns x 64 modes, float32: 0.85 ms against 0.95; 400 x 2000,
+// 128 x 16, bfloat16: 0.52 against 0.51 with two), and so is one of a warp or less, which needs no barrier to speak of (12 x
+// 400, 128 x 8: 12.5 against 18.3 us for the three launches).
+__host__ __device__ constexpr int few_buffers(int G, bool readout) { return readout && (G == 1 || G >= 8) ? 1 : 2; }
 
 // `lanes` threads work on one segment of one row and block_cols columns of u: thread = (column lane, mode group),
 // columns 4 cl .. 4 cl + 3, modes 8 g .. 8 g + 7 (Mp = 8 G modes, zeros beyond M).  Segments that need less than a
@@ -100,11 +127,12 @@ few_scan_kernel(const FewArgs a) {
   constexpr int Mp = kModes * G;
   constexpr int kUs = UD == FRACSSM_F32 ? 4 : 2, kCk = CK == FRACSSM_F32 ? 4 : 2;
   constexpr int kOffK = Mp, kOffC = 2 * Mp, kOffU = READOUT ? 3 * Mp : 2 * Mp;   // a widened token, in floats
-  constexpr int kRhoPer = Mp / 4, kCkPer = Mp * kCk / 16;    // 16-byte pieces per token
+  constexpr int kBuffers = few_buffers(G, READOUT);
+  constexpr int kPieces = kGroup * Mp / 4;                   // of four modes, of a group of tokens
   constexpr int kUMax = (2 * kUs + G - 1) / G;               // pieces of u per thread and group
   extern __shared__ __align__(16) float few_smem[];
   const int lanes = a.lanes, sub = threadIdx.x / lanes, lane = threadIdx.x - sub * lanes;
-  const int tok_floats = kOffU + a.block_cols;
+  const int tok_floats = kOffU + a.block_cols + (READOUT ? 0 : kTokPad), buf_floats = a.per_block * kGroup * tok_floats;
   // (threads beyond the last segment idle along)
   float *wide = few_smem + min(sub, a.per_block - 1) * kGroup * tok_floats;
   const int segs = READOUT ? a.nseg : a.nseg - 1;
@@ -128,16 +156,21 @@ few_scan_kernel(const FewArgs a) {
   const char *rho_p = a.rho.p + b * a.rho.sb + t0 * a.rho.sl, *kap_p = a.kappa.p + b * a.kappa.sb + t0 * a.kappa.sl;
   const char *c_p = a.c.p + b * a.c.sb + t0 * a.c.sl, *u_p = a.u.p + b * a.u.sb + t0 * a.u.sl + (int64_t)col0 * kUs;
 
-  // ---- a group's raw inputs in registers: one 16-byte piece of rho, kappa and c per thread and some of u
-  uint4 q_rho, q_kap, q_c, q_u[kUMax];
-  const int rt = lane / kRhoPer, rq = lane % kRhoPer, ct = lane / kCkPer, cq = lane % kCkPer;
+  // ---- a group's raw inputs in registers: four modes of rho, kappa and c of a token per thread, and some pieces of u.  In the
+  // summary the 8 tokens of a piece lie in neighbouring lanes (kTokPad keeps their stores apart), in the readout the pieces of a
+  // token.
+  using CkRaw = typename std::conditional<kCk == 4, uint4, uint2>::type;
+  uint4 q_rho, q_u[kUMax];
+  CkRaw q_kap, q_c;
+  const int rt = READOUT ? lane / (Mp / 4) : lane % kGroup, rq = READOUT ? lane % (Mp / 4) : lane / kGroup;
+  const bool owns = lane < kPieces;
   auto request = [&](int ib) {
     const int n = min(kGroup, ntok - ib * kGroup);
     const int64_t t = (int64_t)ib * kGroup;
-    if (rt < n) q_rho = __ldg(reinterpret_cast<const uint4 *>(rho_p + (t + rt) * a.rho.sl) + rq);
-    if (ct < n) {
-      q_kap = __ldg(reinterpret_cast<const uint4 *>(kap_p + (t + ct) * a.kappa.sl) + cq);
-      if (READOUT) q_c = __ldg(reinterpret_cast<const uint4 *>(c_p + (t + ct) * a.c.sl) + cq);
+    if (owns && rt < n) {
+      q_rho = __ldg(reinterpret_cast<const uint4 *>(rho_p + (t + rt) * a.rho.sl) + rq);
+      q_kap = __ldg(reinterpret_cast<const CkRaw *>(kap_p + (t + rt) * a.kappa.sl) + rq);
+      if (READOUT) q_c = __ldg(reinterpret_cast<const CkRaw *>(c_p + (t + rt) * a.c.sl) + rq);
     }
 #pragma unroll
     for (int i = 0; i < kUMax; ++i) {
@@ -145,26 +178,42 @@ few_scan_kernel(const FewArgs a) {
       if (ut < n) q_u[i] = __ldg(reinterpret_cast<const uint4 *>(u_p + (t + ut) * a.u.sl) + uq);
     }
   };
-  auto store_group = [&](int ib) {
+  auto store_group = [&](int ib, float *to) {
     const int n = min(kGroup, ntok - ib * kGroup);
-    if (rt < n) {
-      float f[4];
-      widen<FRACSSM_F32>(q_rho, f);
-      *reinterpret_cast<float4 *>(wide + rt * tok_floats + 4 * rq) =
-          make_float4(fmaxf(f[0], kRhoFloor), fmaxf(f[1], kRhoFloor), fmaxf(f[2], kRhoFloor), fmaxf(f[3], kRhoFloor));
-    }
-    if (ct < n) {
-      constexpr int kN = 16 / kCk;
-      float f[kN];
-      float *d = wide + ct * tok_floats + kOffK + kN * cq;
-      widen<CK>(q_kap, f);
+    const bool mine = owns && rt < n;
+    float *d = to + rt * tok_floats + 4 * rq;
+    if (READOUT) {
+      if (mine) {
+        float r[4], f[4];
+        widen<FRACSSM_F32>(q_rho, r);
+        *reinterpret_cast<float4 *>(d) = make_float4(fmaxf(r[0], kRhoFloor), fmaxf(r[1], kRhoFloor), fmaxf(r[2], kRhoFloor), fmaxf(r[3], kRhoFloor));
+        widen4<CK>(q_kap, f);
+        *reinterpret_cast<float4 *>(d + kOffK) = make_float4(f[0], f[1], f[2], f[3]);
+        widen4<CK>(q_c, f);
+        *reinterpret_cast<float4 *>(d + kOffC) = make_float4(f[0], f[1], f[2], f[3]);
+      }
+    } else {
+      // the decay behind each of the 8 tokens, by three exchanges within 8 lanes (see suffix_kappa)
+      float r[4] = {1.f, 1.f, 1.f, 1.f}, k[4] = {0.f, 0.f, 0.f, 0.f};
+      if (mine) {
+        widen<FRACSSM_F32>(q_rho, r);
+        widen4<CK>(q_kap, k);
+      }
 #pragma unroll
-      for (int i = 0; i < kN; i += 4) *reinterpret_cast<float4 *>(d + i) = make_float4(f[i], f[i + 1], f[i + 2], f[i + 3]);
-      if (READOUT) {
-        widen<CK>(q_c, f);
+      for (int x = 0; x < 4; ++x) {
+        float v = mine ? fmaxf(r[x], kRhoFloor) : 1.f;
 #pragma unroll
-        for (int i = 0; i < kN; i += 4)
-          *reinterpret_cast<float4 *>(d + Mp + i) = make_float4(f[i], f[i + 1], f[i + 2], f[i + 3]);
+        for (int o = 1; o < kGroup; o *= 2) {
+          const float y = __shfl_down_sync(0xffffffffu, v, o, kGroup);
+          if (rt + o < kGroup) v *= y;
+        }
+        const float behind = __shfl_down_sync(0xffffffffu, v, 1, kGroup);
+        k[x] *= rt + 1 < kGroup ? fmaxf(behind, kLeastDecay) : 1.f;
+        r[x] = v;
+      }
+      if (owns) {
+        *reinterpret_cast<float4 *>(d + kOffK) = make_float4(k[0], k[1], k[2], k[3]);
+        if (rt == 0) *reinterpret_cast<float4 *>(d) = make_float4(r[0], r[1], r[2], r[3]);
       }
     }
 #pragma unroll
@@ -174,10 +223,10 @@ few_scan_kernel(const FewArgs a) {
         constexpr int kN = 16 / kUs;
         float f[kN];
         widen<UD>(q_u[i], f);
-        float *d = wide + ut * tok_floats + kOffU + kN * uq;
+        float *du = to + ut * tok_floats + kOffU + kN * uq;
 #pragma unroll
         for (int e = 0; e < kN; e += 4)
-          *reinterpret_cast<float4 *>(d + e) = make_float4(f[e], f[e + 1], f[e + 2], f[e + 3]);
+          *reinterpret_cast<float4 *>(du + e) = make_float4(f[e], f[e + 1], f[e + 2], f[e + 3]);
       }
     }
   };
@@ -202,6 +251,24 @@ few_scan_kernel(const FewArgs a) {
       if (PADDED) meets |= !isfinite(v);
     }
     return meets;
+  };
+  // kappa times the decay behind its token within the group, in place, and the group's decay in place of token 0's rho: the
+  // same products in the same order as in store_group
+  auto suffix_kappa = [&](int n) {
+    for (int m = lane; n > 0 && m < Mp; m += lanes) {   // (n is 0 for threads beyond the last segment)
+      float r[kGroup];
+#pragma unroll
+      for (int t = 0; t < kGroup; ++t) r[t] = t < n ? wide[t * tok_floats + m] : 1.f;
+#pragma unroll
+      for (int o = 1; o < kGroup; o *= 2) {
+#pragma unroll
+        for (int t = 0; t + o < kGroup; ++t) r[t] *= r[t + o];
+      }
+#pragma unroll
+      for (int t = 0; t + 1 < kGroup; ++t)
+        if (t < n) wide[t * tok_floats + kOffK + m] *= fmaxf(r[t + 1], kLeastDecay);
+      wide[m] = r[0];
+    }
   };
   if (a.wide_loads) request(0);
   grid_dep_wait();
@@ -236,106 +303,160 @@ few_scan_kernel(const FewArgs a) {
   }
 
   int64_t row = ((int64_t)b * a.L + t0) * a.R + col0 + my;
-  for (int ib = 0; ib * kGroup < all_tok; ++ib) {
-    if (ib > 0) __syncthreads();   // the previous group has been read
-    bool keep_zero = false;        // the padding modes' state
-    if (a.wide_loads) {
-      store_group(ib);
+  // the sums over the modes of this thread's columns, and the nw first of them to row `row` of h
+  auto read_state = [&](const f2 (&cc)[4], int64_t row, int nw) {
+    float o[kCols];
+#pragma unroll
+    for (int r = 0; r < kCols; ++r) {
+      f2 acc = mul2(cc[0], st[r][0]);
+#pragma unroll
+      for (int p = 1; p < 4; ++p) acc = fma2(cc[p], st[r][p], acc);
+      float lo, hi;
+      un2(acc, lo, hi);
+      o[r] = lo + hi;
+    }
+    if constexpr (G == 1) {
+      if (a.h_vec && nw == kCols) {
+        if constexpr (UD == FRACSSM_F32) {
+          *reinterpret_cast<float4 *>(reinterpret_cast<float *>(a.h) + row) = make_float4(o[0], o[1], o[2], o[3]);
+        } else if constexpr (UD == FRACSSM_BF16) {
+          *reinterpret_cast<uint2 *>(reinterpret_cast<__nv_bfloat16 *>(a.h) + row) =
+              make_uint2(tile::pack2(o[0], o[1]), tile::pack2(o[2], o[3]));
+        } else {
+          const __half2 v0 = __floats2half2_rn(o[0], o[1]), v1 = __floats2half2_rn(o[2], o[3]);
+          *reinterpret_cast<uint2 *>(reinterpret_cast<__half *>(a.h) + row) =
+              make_uint2(*reinterpret_cast<const uint32_t *>(&v0), *reinterpret_cast<const uint32_t *>(&v1));
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < kCols; ++r)
+          if (r < nw) st_f32(a.h, row + r, UD, o[r]);
+      }
+    } else {
+      // sum over the mode groups; the first two steps halve the columns a lane answers for
+      const bool b0 = g & 1;
+      float x0 = __shfl_xor_sync(0xffffffffu, b0 ? o[0] : o[2], 1);
+      float x1 = __shfl_xor_sync(0xffffffffu, b0 ? o[1] : o[3], 1);
+      x0 += b0 ? o[2] : o[0];
+      x1 += b0 ? o[3] : o[1];
+      const int r0 = b0 ? 2 : 0;
+      if constexpr (G == 2) {
+        if (a.h_vec && nw == kCols && UD != FRACSSM_F16) {
+          if (UD == FRACSSM_F32)
+            *reinterpret_cast<float2 *>(reinterpret_cast<float *>(a.h) + row + r0) = make_float2(x0, x1);
+          else *reinterpret_cast<uint32_t *>(reinterpret_cast<__nv_bfloat16 *>(a.h) + row + r0) = tile::pack2(x0, x1);
+        } else {
+          if (r0 < nw) st_f32(a.h, row + r0, UD, x0);
+          if (r0 + 1 < nw) st_f32(a.h, row + r0 + 1, UD, x1);
+        }
+      } else {
+        const bool b1 = g & 2;
+        float y = (b1 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, b1 ? x0 : x1, 2);
+#pragma unroll
+        for (int o2 = 4; o2 < G; o2 *= 2) y += __shfl_xor_sync(0xffffffffu, y, o2);
+        const int r1 = r0 + (b1 ? 1 : 0);
+        if (g < 4 && r1 < nw) st_f32(a.h, row + r1, UD, y);
+      }
+    }
+  };
+  auto columns = [&](const float *tok, f2 (&uu)[kCols]) {
+    const float4 u4 = *reinterpret_cast<const float4 *>(tok + kOffU + my);
+    uu[0] = mk2(u4.x, u4.x); uu[1] = mk2(u4.y, u4.y); uu[2] = mk2(u4.z, u4.z); uu[3] = mk2(u4.w, u4.w);
+  };
+  // a group of n tokens in `tok`
+  auto summarise = [&](const float *tok, int n) {   // state := group's decay (.) state + sum of u kappa^T decayed to its end
+    f2 g8[4];
+    ld_pairs(tok + kModes * g, g8);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      prod[p] = mul2(prod[p], g8[p]);
+#pragma unroll
+      for (int r = 0; r < kCols; ++r) st[r][p] = mul2(st[r][p], g8[p]);
+    }
+#pragma unroll 4
+    for (int t = 0; t < n; ++t, tok += tok_floats) {
+      f2 ka[4], uu[kCols];
+      ld_pairs(tok + kOffK + kModes * g, ka);
+      columns(tok, uu);
+#pragma unroll
+      for (int r = 0; r < kCols; ++r) {
+#pragma unroll
+        for (int p = 0; p < 4; ++p) st[r][p] = fma2(ka[p], uu[r], st[r][p]);
+      }
+    }
+  };
+  auto advance = [&](const float *tok) {
+    f2 rr[4], ka[4], uu[kCols];
+    ld_pairs(tok + kModes * g, rr);
+    ld_pairs(tok + kOffK + kModes * g, ka);
+    columns(tok, uu);
+#pragma unroll
+    for (int r = 0; r < kCols; ++r) {
+#pragma unroll
+      for (int p = 0; p < 4; ++p) st[r][p] = fma2(rr[p], st[r][p], mul2(ka[p], uu[r]));
+    }
+  };
+  // the padding modes' state stays zero (an infinity of u times their zero coefficients would make NaN of it)
+  auto clear_padding = [&]() {
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const int m = kModes * g + 2 * p;
+#pragma unroll
+      for (int r = 0; r < kCols; ++r) {
+        float lo, hi;
+        un2(st[r][p], lo, hi);
+        st[r][p] = mk2(m < a.M ? lo : 0.f, m + 1 < a.M ? hi : 0.f);
+      }
+    }
+  };
+
+  if (!PADDED && a.wide_loads) {
+    // All columns are live, and where the readout exchanges between lanes a block has one segment (see few_wide_shape): no
+    // thread idles along.
+    for (int ib = 0; ib * kGroup < all_tok; ++ib) {
+      if (kBuffers == 1 && ib > 0) __syncthreads();   // the previous group has been read
+      float *const tok = wide + (kBuffers == 2 ? (ib & 1) * buf_floats : 0);
+      store_group(ib, tok);
       request(ib + 1);
       __syncthreads();
-    } else {
+      const int n = max(0, min(kGroup, ntok - ib * kGroup));
+      if constexpr (!READOUT) {
+        if (n > 0) summarise(tok, n);
+      } else {
+#pragma unroll 2
+        for (int t = 0; t < n; ++t, row += a.R) {
+          const float *const at = tok + t * tok_floats;
+          advance(at);
+          f2 cc[4];
+          ld_pairs(at + kOffC + kModes * g, cc);
+          read_state(cc, row, kCols);
+        }
+      }
+    }
+  } else {
+    for (int ib = 0; ib * kGroup < all_tok; ++ib) {
+      if (ib > 0) __syncthreads();   // the previous group has been read
+      bool keep_zero = false;        // the padding modes' state
       const bool meets = copy_group(ib);
       if constexpr (PADDED) keep_zero = __syncthreads_or(meets);
       else __syncthreads();
-    }
-    const int n = max(0, min(kGroup, ntok - ib * kGroup)), n_all = min(kGroup, all_tok - ib * kGroup);
-    const float *tok = wide;
+      const int n = max(0, min(kGroup, ntok - ib * kGroup)), n_all = min(kGroup, all_tok - ib * kGroup);
+      if constexpr (!READOUT) {
+        suffix_kappa(n);
+        __syncthreads();
+        if (n > 0) summarise(wide, n);
+        if (PADDED && keep_zero) clear_padding();
+      } else {
+        const float *tok = wide;
 #pragma unroll 1
-    for (int t = 0; t < n_all; ++t, row += a.R, tok += tok_floats) {
-      const bool on = t < n;
-      f2 rr[4], ka[4], cc[4];
-      ld_pairs(tok + kModes * g, rr);
-      ld_pairs(tok + kOffK + kModes * g, ka);
-      if (READOUT) ld_pairs(tok + kOffC + kModes * g, cc);
-      const float4 u4 = *reinterpret_cast<const float4 *>(tok + kOffU + my);
-      const f2 uu[kCols] = {mk2(u4.x, u4.x), mk2(u4.y, u4.y), mk2(u4.z, u4.z), mk2(u4.w, u4.w)};
-      if (on) {
-#pragma unroll
-        for (int r = 0; r < kCols; ++r) {
-#pragma unroll
-          for (int p = 0; p < 4; ++p) st[r][p] = fma2(rr[p], st[r][p], mul2(ka[p], uu[r]));
-        }
-        if (PADDED && keep_zero) {
-#pragma unroll
-          for (int p = 0; p < 4; ++p) {
-            const int m = kModes * g + 2 * p;
-#pragma unroll
-            for (int r = 0; r < kCols; ++r) {
-              float lo, hi;
-              un2(st[r][p], lo, hi);
-              st[r][p] = mk2(m < a.M ? lo : 0.f, m + 1 < a.M ? hi : 0.f);
-            }
+        for (int t = 0; t < n_all; ++t, row += a.R, tok += tok_floats) {
+          f2 cc[4];
+          ld_pairs(tok + kOffC + kModes * g, cc);
+          if (t < n) {
+            advance(tok);
+            if (PADDED && keep_zero) clear_padding();
           }
-        }
-        if (!READOUT) {
-#pragma unroll
-          for (int p = 0; p < 4; ++p) prod[p] = mul2(prod[p], rr[p]);
-        }
-      }
-      if (READOUT) {
-        float o[kCols];
-#pragma unroll
-        for (int r = 0; r < kCols; ++r) {
-          f2 acc = mul2(cc[0], st[r][0]);
-#pragma unroll
-          for (int p = 1; p < 4; ++p) acc = fma2(cc[p], st[r][p], acc);
-          float lo, hi;
-          un2(acc, lo, hi);
-          o[r] = lo + hi;
-        }
-        const int nw = on ? nr : 0;
-        if constexpr (G == 1) {
-          if (a.h_vec && nw == kCols) {
-            if constexpr (UD == FRACSSM_F32) {
-              *reinterpret_cast<float4 *>(reinterpret_cast<float *>(a.h) + row) = make_float4(o[0], o[1], o[2], o[3]);
-            } else if constexpr (UD == FRACSSM_BF16) {
-              *reinterpret_cast<uint2 *>(reinterpret_cast<__nv_bfloat16 *>(a.h) + row) =
-                  make_uint2(tile::pack2(o[0], o[1]), tile::pack2(o[2], o[3]));
-            } else {
-              const __half2 v0 = __floats2half2_rn(o[0], o[1]), v1 = __floats2half2_rn(o[2], o[3]);
-              *reinterpret_cast<uint2 *>(reinterpret_cast<__half *>(a.h) + row) =
-                  make_uint2(*reinterpret_cast<const uint32_t *>(&v0), *reinterpret_cast<const uint32_t *>(&v1));
-            }
-          } else {
-#pragma unroll
-            for (int r = 0; r < kCols; ++r)
-              if (r < nw) st_f32(a.h, row + r, UD, o[r]);
-          }
-        } else {
-          // sum over the mode groups; the first two steps halve the columns a lane answers for
-          const bool b0 = g & 1;
-          float x0 = __shfl_xor_sync(0xffffffffu, b0 ? o[0] : o[2], 1);
-          float x1 = __shfl_xor_sync(0xffffffffu, b0 ? o[1] : o[3], 1);
-          x0 += b0 ? o[2] : o[0];
-          x1 += b0 ? o[3] : o[1];
-          const int r0 = b0 ? 2 : 0;
-          if constexpr (G == 2) {
-            if (a.h_vec && nw == kCols && UD != FRACSSM_F16) {
-              if (UD == FRACSSM_F32)
-                *reinterpret_cast<float2 *>(reinterpret_cast<float *>(a.h) + row + r0) = make_float2(x0, x1);
-              else *reinterpret_cast<uint32_t *>(reinterpret_cast<__nv_bfloat16 *>(a.h) + row + r0) = tile::pack2(x0, x1);
-            } else {
-              if (r0 < nw) st_f32(a.h, row + r0, UD, x0);
-              if (r0 + 1 < nw) st_f32(a.h, row + r0 + 1, UD, x1);
-            }
-          } else {
-            const bool b1 = g & 2;
-            float y = (b1 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, b1 ? x0 : x1, 2);
-#pragma unroll
-            for (int o2 = 4; o2 < G; o2 *= 2) y += __shfl_xor_sync(0xffffffffu, y, o2);
-            const int r1 = r0 + (b1 ? 1 : 0);
-            if (g < 4 && r1 < nw) st_f32(a.h, row + r1, UD, y);
-          }
+          read_state(cc, row, t < n ? nr : 0);
         }
       }
     }
@@ -373,56 +494,76 @@ few_scan_kernel(const FewArgs a) {
   }
 }
 
-// states[b][s] := the state entering segment s.  A warp owns 32 elements of a row's state and a share of its
-// segments, which it first composes and then walks; up to kCarryBatch segments a share stays in registers in
-// between (read once, written once).  Bound by the latency of that one read.
-constexpr int kCarryWarps = 32, kCarryBatch = 12;
+// states[b][s] := the state entering segment s.  A thread composes the segments of its share, walks them again from
+// the state that enters the share, and keeps up to BATCH of them in registers in between (read once, written once).
+// A warp owns 32 / SUB neighbouring elements of a row's state, and its lanes SUB neighbouring shares of each.  Bound by the
+// latency of the one read: with SUB = 1 throughout, 1185 segments (1 row x 32768 tokens, 64 columns x 8 modes) were read twice
+// in four rounds, 24 us, 13 here.
+constexpr int kCarryWarps = 32;
+template <int BATCH, int SUB>
 __global__ void __launch_bounds__(32 * kCarryWarps)
 few_carry_kernel(float *__restrict__ states, const float *__restrict__ decay, const float *__restrict__ init,
                  int nseg, int R, int M, int Mp) {
-  __shared__ float ps[kCarryWarps][32], ss[kCarryWarps][32];
-  const int lane = threadIdx.x % 32, w = threadIdx.x / 32, warps = blockDim.x / 32;
+  constexpr int kElems = 32 / SUB;
+  __shared__ float ps[kCarryWarps][kElems], ss[kCarryWarps][kElems];
+  const int lane = threadIdx.x % 32, w = threadIdx.x / 32, warps = blockDim.x / 32, el = lane % kElems, sub = lane / kElems;
   const int64_t b = blockIdx.y;
-  const int RM = R * Mp, e = blockIdx.x * 32 + lane;
+  const int RM = R * Mp, e = blockIdx.x * kElems + el;
   const bool live = e < RM;
   const int m = e % Mp, r = e / Mp;
-  const int share = (nseg + warps - 1) / warps;
-  const int lo = min(w * share, nseg), hi = min(lo + share, nseg), last = nseg - 1;   // segment `last` has no summary
+  const int share = (nseg + warps * SUB - 1) / (warps * SUB);
+  const int lo = min((w * SUB + sub) * share, nseg), hi = min(lo + share, nseg), last = nseg - 1;   // `last` has no summary
   float *sp = states + (b * nseg + lo) * RM + (live ? e : 0);
   const float *dp = decay + (b * nseg + lo) * Mp + m;
   grid_dep_launch();
   grid_dep_wait();
   float p = 1.f, v = 0.f;
-  float x[kCarryBatch], d[kCarryBatch];
+  float x[BATCH], d[BATCH];
   auto load = [&](int s0) {
     const float *xs = sp + (int64_t)(s0 - lo) * RM, *ds = dp + (int64_t)(s0 - lo) * Mp;
     const int n = min(hi, last) - s0;
 #pragma unroll
-    for (int i = 0; i < kCarryBatch; ++i, xs += RM, ds += Mp) {
+    for (int i = 0; i < BATCH; ++i, xs += RM, ds += Mp) {
       x[i] = i < n ? __ldcg(xs) : 0.f;
       d[i] = i < n ? __ldcg(ds) : 1.f;
     }
   };
-  for (int s0 = lo; s0 < hi; s0 += kCarryBatch) {
+  for (int s0 = lo; s0 < hi; s0 += BATCH) {
     load(s0);
 #pragma unroll
-    for (int i = 0; i < kCarryBatch; ++i) {
+    for (int i = 0; i < BATCH; ++i) {
       v = fmaf(d[i], v, x[i]);
       p *= d[i];
     }
   }
-  ps[w][lane] = p;
-  ss[w][lane] = v;
+  // the warp's shares one after the other: (p, v) up to and with each, then without it
+#pragma unroll
+  for (int o = 1; o < SUB; o *= 2) {
+    const float p0 = __shfl_up_sync(0xffffffffu, p, o * kElems), v0 = __shfl_up_sync(0xffffffffu, v, o * kElems);
+    if (sub >= o) {
+      v = fmaf(p, v0, v);
+      p *= p0;
+    }
+  }
+  if (sub == SUB - 1) {
+    ps[w][el] = p;
+    ss[w][el] = v;
+  }
+  if constexpr (SUB > 1) {
+    p = __shfl_up_sync(0xffffffffu, p, kElems);
+    v = __shfl_up_sync(0xffffffffu, v, kElems);
+  }
   __syncthreads();
   if (!live) return;
   float run = init && m < M ? init[(b * R + r) * M + m] : 0.f;
-  for (int i = 0; i < w; ++i) run = fmaf(ps[i][lane], run, ss[i][lane]);
-  for (int s0 = lo; s0 < hi; s0 += kCarryBatch) {
-    if (share > kCarryBatch) load(s0);
+  for (int i = 0; i < w; ++i) run = fmaf(ps[i][el], run, ss[i][el]);
+  if (SUB > 1 && sub > 0) run = fmaf(p, run, v);
+  for (int s0 = lo; s0 < hi; s0 += BATCH) {
+    if (share > BATCH) load(s0);
     float *xs = sp + (int64_t)(s0 - lo) * RM;
     const int n = hi - s0;
 #pragma unroll
-    for (int i = 0; i < kCarryBatch; ++i, xs += RM) {
+    for (int i = 0; i < BATCH; ++i, xs += RM) {
       if (i < n) __stcg(xs, run);
       run = fmaf(d[i], run, x[i]);
     }
@@ -525,18 +666,26 @@ int few_launch(FewArgs &a, const FewPlan &p, cudaStream_t st) {
   a.wide_loads = few_wide_shape(p, a.R, a.M, kUs) && few_wide_rows(a.u, a.c, a.kappa, a.rho);
   a.u_shift = 0;
   while ((1 << a.u_shift) < pieces) ++a.u_shift;
-  const size_t sum_smem = (size_t)p.per_block * kGroup * (2 * Mp + p.block_cols) * 4;
-  const size_t out_smem = (size_t)p.per_block * kGroup * (3 * Mp + p.block_cols) * 4;
+  const size_t tokens = (size_t)p.per_block * kGroup;
+  const size_t sum_smem = tokens * (2 * Mp + p.block_cols + kTokPad) * 4 * (a.wide_loads ? few_buffers(G, false) : 1);
+  const size_t out_smem = tokens * (3 * Mp + p.block_cols) * 4 * (a.wide_loads ? few_buffers(G, true) : 1);
   if (out_smem > 48 * 1024) return fail(FRACSSM_ERR_UNSUPPORTED, "frac_scan: shared memory of the segment kernel");
   cudaError_t e = cudaSuccess;
   auto blocks = [&](int64_t segs) { return dim3((unsigned)ceil_div((int64_t)a.B * segs, p.per_block), p.col_blocks); };
   if (p.nseg > 1) {
     auto summary = a.M < Mp ? few_scan_kernel<G, UD, CK, false, true> : few_scan_kernel<G, UD, CK, false, false>;
     e = few_launch_dep(summary, blocks(p.nseg - 1), threads, sum_smem, st, false, a);
+    // (no more registers than a share needs: a place that stays empty costs its instructions all the same)
+    auto carry = p.nseg <= 8 * kCarryWarps ? few_carry_kernel<8, 1>
+                 : p.nseg <= 12 * kCarryWarps ? few_carry_kernel<12, 1>
+                 : p.nseg <= 24 * kCarryWarps ? few_carry_kernel<12, 2>
+                 : p.nseg <= 48 * kCarryWarps ? few_carry_kernel<12, 4>
+                                              : few_carry_kernel<12, 8>;
+    const int elems = p.nseg <= 12 * kCarryWarps ? 32 : p.nseg <= 24 * kCarryWarps ? 16 : p.nseg <= 48 * kCarryWarps ? 8 : 4;
     int warps = (int)ceil_div(p.nseg, 8);
     if (warps > kCarryWarps) warps = kCarryWarps;
     if (e == cudaSuccess)
-      e = few_launch_dep(few_carry_kernel, dim3((unsigned)ceil_div((int64_t)a.R * Mp, 32), (unsigned)a.B), 32 * warps,
+      e = few_launch_dep(carry, dim3((unsigned)ceil_div((int64_t)a.R * Mp, elems), (unsigned)a.B), 32 * warps,
                          0, st, true, a.states, a.decay, a.init, p.nseg, a.R, a.M, Mp);
   }
   auto readout = a.M < Mp ? few_scan_kernel<G, UD, CK, true, true> : few_scan_kernel<G, UD, CK, true, false>;
