@@ -123,8 +123,21 @@ def ptr(t):
     return None if t is None else ctypes.c_void_p(t.data_ptr())
 
 
+def raw_stream(t: torch.Tensor) -> int:
+    """The handle of the current stream of t's device (a stream object for it costs 2 us)."""
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
+
+
 def stream_of(t: torch.Tensor):
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    return ctypes.c_void_p(raw_stream(t))
+
+
+_HERE = contextlib.nullcontext()
+
+
+def device_of(t: torch.Tensor):
+    """A context in which t's device is the current one; nothing to enter (and 3 us to save) where it is already."""
+    return _HERE if torch.cuda.current_device() == t.get_device() else torch.cuda.device(t.device)
 
 
 def rows(t: torch.Tensor) -> torch.Tensor:
@@ -145,5 +158,5 @@ def trace(name: str):
     """NVTX range around a host-side stage when FRACSSM_NVTX=1 (for nsys / ncu timelines; the
     reference marks its stages the same way, `frac_ssm/ops/utils.py:6-23`); a no-op otherwise."""
     if not _NVTX:
-        return contextlib.nullcontext()
+        return _HERE
     return torch.cuda.nvtx.range(name)

@@ -139,18 +139,20 @@ def _launch(u, c, kappa, rho, chunk_size, initial_state, want_final, final_fp32,
         return h, fin
     if B > 0:
         lib = C.lib()
-        with C.trace("frac_scan"), torch.cuda.device(u.device):
+        with C.trace("frac_scan"), C.device_of(u):
+            su, sc, sk, sr = u.stride(), c.stride(), kappa.stride(), rho.stride()
             # (strided inputs may take the chunked stages where dense ones take the segment kernels)
-            if path_code == C.PATH_AUTO and all(t.is_contiguous() for t in (u, c, kappa, rho)):
+            if path_code == C.PATH_AUTO and all([t.is_contiguous() for t in (u, c, kappa, rho)]):
                 nbytes = lib.fracssm_frac_scan_auto_workspace_bytes(B, L, R, M, chunk_size)
             else:
                 nbytes = lib.fracssm_frac_scan_workspace_bytes(B, L, R, M, chunk_size, path_code)
-            ws = torch.empty(max(nbytes, 256), device=u.device, dtype=torch.uint8)
+            nbytes = max(nbytes, 256)
+            ws = torch.empty(nbytes, device=u.device, dtype=torch.uint8)
             C.check(lib.fracssm_frac_scan_fwd(
-                C.ptr(u), C.dt(u), u.stride(0), u.stride(1), C.ptr(c), C.ptr(kappa), C.dt(c),
-                c.stride(0), c.stride(1), kappa.stride(0), kappa.stride(1), C.ptr(rho), rho.stride(0),
-                rho.stride(1), C.ptr(init), C.ptr(h), C.ptr(fin), C.dt_of(final_state_dtype),
-                C.ptr(ws), ws.numel(), B, L, R, M, chunk_size, path_code, C.stream_of(u)), "frac_scan")
+                u.data_ptr(), C.dt(u), su[0], su[1], c.data_ptr(), kappa.data_ptr(), C.dt(c), sc[0], sc[1], sk[0], sk[1],
+                rho.data_ptr(), sr[0], sr[1], None if init is None else init.data_ptr(), h.data_ptr(),
+                None if fin is None else fin.data_ptr(), C.dt_of(final_state_dtype), ws.data_ptr(), nbytes, B, L, R, M,
+                chunk_size, path_code, C.raw_stream(u)), "frac_scan")
             if check and L > 0 and path_code != C.PATH_STAGED and u.is_contiguous() and \
                     lib.fracssm_scan_fused_supported(B, L, R, M, chunk_size, C.dt(u), C.dt(c)):
                 C.check(lib.fracssm_scan_fused_status(C.ptr(ws), C.stream_of(u)), "frac_scan")

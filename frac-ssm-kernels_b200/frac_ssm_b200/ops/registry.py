@@ -9,6 +9,8 @@ from __future__ import annotations
 import importlib
 from types import ModuleType
 
+import torch
+
 BACKENDS = ("b200",)
 
 IMPLS: dict[str, str] = {"b200": "frac_ssm_b200.ops.b200.frac_scan"}
@@ -18,8 +20,6 @@ def available(backend: str) -> tuple[bool, str | None]:
     """Whether this backend can run in the current environment."""
     _check_backend(backend)
     import os
-
-    import torch
 
     from .. import _cabi
 
@@ -33,14 +33,20 @@ def available(backend: str) -> tuple[bool, str | None]:
     return True, None
 
 
+_usable: set[tuple[str, int]] = set()      # backends and devices that were found to go together
+
+
 def load(backend: str | None = None) -> ModuleType:
     """Load a backend module; ``None`` picks "b200"."""
     if backend is None:
         backend = "b200"
     _check_backend(backend)
-    ok, reason = available(backend)
-    if not ok:
-        raise RuntimeError(f"Backend {backend!r} is unavailable: {reason}")
+    # (a device keeps its architecture and the library, once found, stays: the question is 10 us of a call)
+    if not (torch.cuda.is_initialized() and (backend, torch.cuda.current_device()) in _usable):
+        ok, reason = available(backend)
+        if not ok:
+            raise RuntimeError(f"Backend {backend!r} is unavailable: {reason}")
+        _usable.add((backend, torch.cuda.current_device()))
     return importlib.import_module(IMPLS[backend])
 
 
