@@ -5,6 +5,7 @@
 //     (frac_ssm/models/modeling_frac.py:159-179, `_update_state`, and the D skip of :236).
 // Both are bandwidth kernels: every input element is read once, every output written once.
 #include "common.cuh"
+#include "prefill_dyn.cuh"
 
 namespace fracssm {
 namespace {
@@ -220,6 +221,8 @@ causal_conv4_silu_bf16_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_sb,
       }
     }
   }
+  // a grid that this one was started beside ends before this one does (else nothing to wait for)
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // One token of the recurrence for every (batch, head): state [M, R] float32 updated in place,
@@ -271,7 +274,8 @@ static int conv_silu_heads(const void *x, int x_dtype, int64_t x_sb, int64_t x_s
                                               const float *mask, int64_t m_sb, int64_t m_sl,
                                               const void *weight, const void *bias, int w_dtype, void *y,
                                               int y_dtype, void *u_heads, int64_t R, int64_t Bt, int64_t L,
-                                              int64_t C, int64_t K, void *stream, const fracssm::ConvTail &tail) {
+                                              int64_t C, int64_t K, void *stream, const fracssm::ConvTail &tail,
+                                              bool beside) {
   using namespace fracssm;
   if (u_heads && (R <= 0 || C % R != 0))
     return fail(FRACSSM_ERR_ARG, "causal_conv_silu: the head width must divide the channel count");
@@ -295,9 +299,22 @@ static int conv_silu_heads(const void *x, int x_dtype, int64_t x_sb, int64_t x_s
     auto kernel = causal_conv4_silu_bf16_kernel<kConvTokens, false>;
     if (tokens == 16) kernel = same_launch ? causal_conv4_silu_bf16_kernel<16, true> : causal_conv4_silu_bf16_kernel<16, false>;
     if (tokens == 8) kernel = same_launch ? causal_conv4_silu_bf16_kernel<8, true> : causal_conv4_silu_bf16_kernel<8, false>;
-    kernel<<<grid, block, 0, (cudaStream_t)stream>>>(
-        reinterpret_cast<const __nv_bfloat16 *>(x), x_sb, x_sl, mask, m_sb, m_sl, weight, w_dtype, bias,
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = beside ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(
+        &cfg, kernel, reinterpret_cast<const __nv_bfloat16 *>(x), x_sb, x_sl, mask, m_sb, m_sl, weight, w_dtype, bias,
         reinterpret_cast<__nv_bfloat16 *>(y), reinterpret_cast<__nv_bfloat16 *>(u_heads), R, L, C, tail);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return fail(FRACSSM_ERR_CUDA, "causal_conv_silu: %s", cudaGetErrorString(e));
+    }
     if (tail.out && !same_launch)
       conv_tail_kernel<<<dim3((unsigned)ceil_div(C, 128), (unsigned)Bt), 128, 0, (cudaStream_t)stream>>>(
           reinterpret_cast<const __nv_bfloat16 *>(x), x_sb, x_sl, mask, m_sb, m_sl, tail, L, C);
@@ -318,7 +335,7 @@ extern "C" int fracssm_causal_conv_silu_heads(const void *x, int x_dtype, int64_
                                               int y_dtype, void *u_heads, int64_t R, int64_t Bt, int64_t L,
                                               int64_t C, int64_t K, void *stream) {
   return conv_silu_heads(x, x_dtype, x_sb, x_sl, mask, m_sb, m_sl, weight, bias, w_dtype, y, y_dtype, u_heads, R, Bt, L, C, K,
-                         stream, fracssm::ConvTail{nullptr, 0});
+                         stream, fracssm::ConvTail{nullptr, 0}, false);
 }
 
 extern "C" int fracssm_decode_step(const void *u, int u_dtype, const float *c, const float *kappa,
@@ -347,5 +364,16 @@ extern "C" int fracssm_prefill_conv(const void *x, int64_t x_sl, const float *ma
   // bf16 in and out
   const fracssm::ConvTail next{K >= 2 ? reinterpret_cast<__nv_bfloat16 *>(tail) : nullptr, (int)K};
   return conv_silu_heads(x, FRACSSM_BF16, L * x_sl, x_sl, mask, L, 1, weight, bias, FRACSSM_BF16, y, FRACSSM_BF16, u_heads, R,
-                         Bt, L, C, K, stream, next);
+                         Bt, L, C, K, stream, next, false);
+}
+
+extern "C" int fracssm_prefill_conv_dyn(const void *x, int64_t x_sl, const float *mask, const void *weight, const void *bias,
+                                        void *y, void *u_heads, void *tail, const void *dyn_weight, void *dyn,
+                                        int64_t dyn_cols, int64_t R, int64_t Bt, int64_t L, int64_t C, int64_t K,
+                                        void *stream) {
+  const int rc = fracssm::prefill_dyn_launch(x, x_sl, dyn_weight, dyn, Bt * L, C, dyn_cols, (cudaStream_t)stream);
+  if (rc) return rc;
+  const fracssm::ConvTail next{K >= 2 ? reinterpret_cast<__nv_bfloat16 *>(tail) : nullptr, (int)K};
+  return conv_silu_heads(x, FRACSSM_BF16, L * x_sl, x_sl, mask, L, 1, weight, bias, FRACSSM_BF16, y, FRACSSM_BF16, u_heads, R,
+                         Bt, L, C, K, stream, next, true);
 }

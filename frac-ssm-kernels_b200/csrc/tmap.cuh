@@ -12,4 +12,8 @@ namespace fracssm {
 int make_tmap_bf16_3d(CUtensorMap *map, const void *base, uint64_t d0, uint64_t d1, uint64_t d2,
                       uint32_t b0, uint32_t b1);
 
+// The same for d1 rows of d0 elements that lie `pitch` elements apart (loads at z = 0).
+int make_tmap_bf16_rows(CUtensorMap *map, const void *base, uint64_t d0, uint64_t d1, uint64_t pitch, uint32_t b0,
+                        uint32_t b1);
+
 }  // namespace fracssm

@@ -70,6 +70,7 @@ _SIGNATURES = {
     "fracssm_decode_layers": (ci, [vp, vp, i64, vp, vp, vp, sz, i64, i64, i64, i64, i64, i64, vp]),
     "fracssm_add_rmsnorm": (ci, [vp, vp, vp, ci, cf, vp, vp, i64, i64, vp]),
     "fracssm_prefill_conv": (ci, [vp, i64, vp, vp, vp, vp, vp, vp, i64, i64, i64, i64, i64, vp]),
+    "fracssm_prefill_conv_dyn": (ci, [vp, i64, vp, vp, vp, vp, vp, vp, vp, vp, i64, i64, i64, i64, i64, i64, vp]),
     "fracssm_prefill_mix": (ci, [vp, vp, vp, vp, vp, i64, vp, vp, ci, vp, vp, vp, vp, ci, vp, vp, vp, vp, vp, vp, sz,
                                  i64, i64, i64, i64, i64, i64, vp]),
     "fracssm_scan_epilogue_sumsq": (ci, [vp, ci, i64, i64, vp, i64, i64, vp, i64, i64, ci, vp, cf, vp,

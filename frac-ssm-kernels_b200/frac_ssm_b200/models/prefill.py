@@ -1,7 +1,7 @@
 """A prompt through all layers with few calls per layer: bfloat16 models on one GPU.
 
-Between the four library GEMMs of a layer stand three native calls (residual addition + norm; convolution + the
-next token's history; parameter prep, scan, state and epilogue), the small parameters are read in their own types
+Between the three library GEMMs of a layer stand three native calls (residual addition + norm; convolution, the next
+token's history and the narrow dynamic projection; parameter prep, scan, state and epilogue), the small parameters are read in their own types
 and the intermediates live in buffers that all layers share.  As with `decode.py`, nothing is remembered between
 calls and whatever has to see the individual modules or operations keeps the modules' own forward.
 """
@@ -70,6 +70,7 @@ def prefill_layers(layers, h, attention_mask, use_cache, classes):
         return torch.empty(*shape, device=h.device, dtype=dtype)
 
     rows = B * L
+    own_dyn = 3 * H <= 192 and di % 8 == 0 and rows <= 1 << 30      # (what fracssm_prefill_conv_dyn covers)
     with C.trace("prefill_layers"), torch.cuda.device(dev):
         stream = C.stream_of(h)
         nbytes = lib.fracssm_frac_scan_auto_workspace_bytes(B * H, L, R, M, T)
@@ -104,10 +105,16 @@ def prefill_layers(layers, h, attention_mask, use_cache, classes):
             xg = F.linear(n, in_w)
             n = None      # (like xg below: what is no longer read makes room)
             p_x = xg.data_ptr()
-            C.check(lib.fracssm_prefill_conv(p_x, 2 * di, p_mask, conv_w.data_ptr(), 0 if conv_b is None else conv_b.data_ptr(),
-                                             p_conv, p_u, tails[i].data_ptr() if use_cache else 0, R, B, L, di, K, stream),
-                    "prefill_conv")
-            dyn = F.linear(xg[:, :di], dyn_w)      # (its bias is added where it is read)
+            conv = (p_x, 2 * di, p_mask, conv_w.data_ptr(), 0 if conv_b is None else conv_b.data_ptr(), p_conv, p_u,
+                    tails[i].data_ptr() if use_cache else 0)
+            # (the bias of dyn is added where it is read)
+            if own_dyn and not dyn_w.data_ptr() & 15:
+                dyn = empty(rows, 3 * H)
+                C.check(lib.fracssm_prefill_conv_dyn(*conv, dyn_w.data_ptr(), dyn.data_ptr(), 3 * H, R, B, L, di, K, stream),
+                        "prefill_conv_dyn")
+            else:
+                C.check(lib.fracssm_prefill_conv(*conv, R, B, L, di, K, stream), "prefill_conv")
+                dyn = F.linear(xg[:, :di], dyn_w)
             rw = F.linear(x_conv, rw_w)
             params = (ctypes.c_void_p * 6)(dt_bias.data_ptr(), read_logit.data_ptr(), write_logit.data_ptr(),
                                            log_tau.data_ptr(), D.data_ptr(), out_norm_w.data_ptr())

@@ -370,6 +370,10 @@ int fracssm_decode_layers(const uint64_t *layer_ptrs, const float *layer_nums, i
  * mask [Bt, L] or NULL, and, if tail is not NULL, tail [Bt, C, K-1] = the last K-1 masked inputs (zeros before the
  * first token).
  *
+ * prefill_conv_dyn: the same, and beside it the dynamic projection of the unconvolved, unmasked input:
+ * dyn [Bt * L, dyn_cols] = x dyn_weight^T for dyn_weight [dyn_cols, C] (bf16, sums in float32), at most 192 columns,
+ * C and x_sl multiples of 8, x and dyn_weight 16-byte aligned.
+ *
  * prefill_mix: compute_params, frac_scan and scan_epilogue of one layer.  dyn [Bt, L, 3H] (dyn_bias [3H] or NULL is
  * added), rw [Bt, L, 2HM], x_conv [Bt, L, HR], gate rows gate_sl apart, u [Bt*H, L, R], all bf16; params (host array of device pointers): dt_bias,
  * read_residual_logit, write_residual_scale, base_log_tau, D, output norm weight, bit i of params_f32 set where
@@ -382,6 +386,9 @@ int fracssm_add_rmsnorm(const void *x, const void *y, const void *weight, int w_
                         int64_t rows, int64_t D, void *stream);
 int fracssm_prefill_conv(const void *x, int64_t x_sl, const float *mask, const void *weight, const void *bias, void *y,
                          void *u_heads, void *tail, int64_t R, int64_t Bt, int64_t L, int64_t C, int64_t K, void *stream);
+int fracssm_prefill_conv_dyn(const void *x, int64_t x_sl, const float *mask, const void *weight, const void *bias, void *y,
+                             void *u_heads, void *tail, const void *dyn_weight, void *dyn, int64_t dyn_cols, int64_t R,
+                             int64_t Bt, int64_t L, int64_t C, int64_t K, void *stream);
 int fracssm_prefill_mix(const void *dyn, const void *dyn_bias, const void *rw, const void *x_conv, const void *gate,
                         int64_t gate_sl,
                         const float *mask, const void *const *params, int params_f32, const float *nums, const void *u,
