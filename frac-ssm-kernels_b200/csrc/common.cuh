@@ -59,14 +59,20 @@ int scan_fused_launch_ex(const void *u, const void *c, const void *kappa, int ck
                          const float *initial_state, void *h, void *final_state, int final_dtype,
                          void *workspace, size_t workspace_bytes, int64_t B, int64_t L, int64_t R,
                          int64_t M, int64_t T, void *stream, int first_tile, unsigned long long wait_ns,
-                         const ScanLayerOut *layer);
+                         const ScanLayerOut *layer, size_t cleared = 0);
+size_t scan_fused_clear_bytes(int64_t B, int64_t L, int64_t R, int64_t M, size_t workspace_bytes, int first_tile, bool layer);
+int scan_fused_launch(const void *u, const void *c, const void *kappa, int ck_dtype, const float *rho,
+                      const float *initial_state, void *h, void *final_state, int final_dtype,
+                      void *workspace, size_t workspace_bytes, int64_t B, int64_t L, int64_t R,
+                      int64_t M, int64_t T, void *stream, size_t cleared = 0);
 
 // defined in frac_scan.cu: fracssm_frac_scan_fwd; where the route taken can, the final state goes to `state_modes_first`
-// ([B, M, R] float32, may be null) instead of final_state, which *modes_first reports
+// ([B, M, R] float32, may be null) instead of final_state, which *modes_first reports; `cleared`: that many bytes at the
+// start of the workspace are zero already (scan_fused_clear_bytes)
 int frac_scan_route(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, const void *c, const void *kappa, int ck_dtype,
                     int64_t c_sb, int64_t c_sl, int64_t k_sb, int64_t k_sl, const float *rho, int64_t r_sb, int64_t r_sl,
                     const float *initial_state, void *h, void *final_state, int final_dtype, void *workspace,
                     size_t workspace_bytes, int64_t B, int64_t L, int64_t R, int64_t M, int64_t T, int path, void *stream,
-                    float *state_modes_first, bool *modes_first);
+                    float *state_modes_first, bool *modes_first, size_t cleared = 0);
 
 }  // namespace fracssm

@@ -28,12 +28,6 @@ static ScanScratch staged_layout(void *base, int64_t B, int64_t L, int64_t R, in
   return s;
 }
 
-// defined in scan_fused.cu
-size_t scan_fused_workspace_bytes(int64_t B, int64_t L, int64_t R, int64_t M, int64_t T);
-int scan_fused_launch(const void *u, const void *c, const void *kappa, int ck_dtype, const float *rho,
-                      const float *initial_state, void *h, void *final_state, int final_dtype,
-                      void *workspace, size_t workspace_bytes, int64_t B, int64_t L, int64_t R,
-                      int64_t M, int64_t T, void *stream);
 // defined in scan_modes.cu
 bool scan_few_supported(int64_t B, int64_t L, int64_t R, int64_t M, int64_t T);
 size_t scan_few_workspace_bytes(int64_t B, int64_t L, int64_t R, int64_t M);
@@ -81,7 +75,7 @@ int frac_scan_route(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, cons
                     int64_t c_sb, int64_t c_sl, int64_t k_sb, int64_t k_sl, const float *rho, int64_t r_sb, int64_t r_sl,
                     const float *initial_state, void *h, void *final_state, int final_dtype, void *workspace,
                     size_t workspace_bytes, int64_t B, int64_t L, int64_t R, int64_t M, int64_t T, int path, void *stream,
-                    float *state_modes_first, bool *modes_first) {
+                    float *state_modes_first, bool *modes_first, size_t cleared) {
   if (modes_first) *modes_first = false;
   if (B < 0 || L < 0 || R <= 0 || M <= 0 || T <= 0) return fail(FRACSSM_ERR_ARG, "frac_scan: bad sizes");
   if (!known_dtype(u_dtype) || !known_dtype(ck_dtype)) return fail(FRACSSM_ERR_ARG, "frac_scan: unsupported dtype");
@@ -123,7 +117,7 @@ int frac_scan_route(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, cons
     return fail(FRACSSM_ERR_UNSUPPORTED, "frac_scan: shape, dtype, strides or alignment not covered by the single-pass kernel");
   if (fused_ok && path != 1) {
     return scan_fused_launch(u, c, kappa, ck_dtype, rho, initial_state, h, final_state, final_dtype,
-                             workspace, workspace_bytes, B, L, R, M, T, stream);
+                             workspace, workspace_bytes, B, L, R, M, T, stream, cleared);
   }
 
   ScanScratch s = staged_layout(workspace, B, L, R, M, T);

@@ -29,6 +29,7 @@ struct ParamArgs {
   int dtb_dt, lt_dt, read_dt, write_dt;
   float inv_read_temp, dt_min, dt_max, a_min, a_max, l_min, l_max;
   void *u, *c, *kappa; int ck_dt; float *rho;
+  uint4 *clear; int clear_pieces;          // 16-byte pieces to set to zero on the way (with CLEAR)
   int u_pieces;                            // 16-byte pieces of a row of u and x, 0 where rows are no such pieces
   int64_t L, H, R, M;
 };
@@ -282,11 +283,17 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 constexpr int kPairTokens = 32;
 
 // PLAIN: as above (one token: 4.0 us instead of 4.4 with the looks at the types).
-template <int Q, bool PLAIN>
+// CLEAR: the blocks zero a.clear between them.
+template <int Q, bool PLAIN, bool CLEAR = false>
 __global__ void __launch_bounds__(128) compute_params_lanes_kernel(const ParamArgs a, int per_warp) {
   const int read_dt = PLAIN ? FRACSSM_F32 : a.read_dt, write_dt = PLAIN ? FRACSSM_F32 : a.write_dt;
   const int lt_dt = PLAIN ? FRACSSM_F32 : a.lt_dt, dtb_dt = PLAIN ? FRACSSM_F32 : a.dtb_dt;
   auto dyn = [&](int64_t base, int64_t j) { return PLAIN ? ld_f32(a.dyn, base + j, a.dyn_dt) : dyn_at(a, base, j); };
+  if (CLEAR) {
+    const int64_t threads = (int64_t)gridDim.x * gridDim.y * blockDim.x;
+    for (int64_t i = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < a.clear_pieces; i += threads)
+      a.clear[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
   constexpr int kStep = 32 / Q;              // tokens a warp works on at a time
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
   const int sub = lane / Q, q = lane % Q;    // token of the step; modes 8 q .. 8 q + 7
@@ -576,17 +583,25 @@ add_rmsnorm_kernel(const __nv_bfloat16 *x, const __nv_bfloat16 *y, const void *_
 }
 
 // state [rows][M][R] = final [rows][R][M]: a cached state lies modes first, the scan leaves it columns first
-__global__ void __launch_bounds__(256)
-state_transpose_kernel(const float *__restrict__ fin, float *__restrict__ state, int R, int M) {
+struct StateTurn {
+  const float *fin;   // [rows, R, M], or null: nothing to do
+  float *state;       // [rows, M, R]
+  int R, M, m_tiles, r_tiles;
+  int64_t rows;
+};
+// one tile of 32 x 32, by a block of whole warps
+__device__ __forceinline__ void turn_tile(const StateTurn &t, int64_t index) {
   __shared__ float tile[32][33];
-  const int64_t base = (int64_t)blockIdx.z * R * M;
-  const int m0 = blockIdx.x * 32, r0 = blockIdx.y * 32, tx = threadIdx.x % 32, ty = threadIdx.x / 32;
-  for (int i = ty; i < 32; i += 8)
-    if (r0 + i < R && m0 + tx < M) tile[i][tx] = fin[base + (int64_t)(r0 + i) * M + m0 + tx];
+  const int64_t rest = index / t.m_tiles, base = rest / t.r_tiles * t.R * t.M;
+  const int m0 = (int)(index % t.m_tiles) * 32, r0 = (int)(rest % t.r_tiles) * 32;
+  const int tx = threadIdx.x % 32, ty = threadIdx.x / 32, step = blockDim.x / 32;
+  for (int i = ty; i < 32; i += step)
+    if (r0 + i < t.R && m0 + tx < t.M) tile[i][tx] = t.fin[base + (int64_t)(r0 + i) * t.M + m0 + tx];
   __syncthreads();
-  for (int i = ty; i < 32; i += 8)
-    if (m0 + i < M && r0 + tx < R) state[base + (int64_t)(m0 + i) * R + r0 + tx] = tile[tx][i];
+  for (int i = ty; i < 32; i += step)
+    if (m0 + i < t.M && r0 + tx < t.R) t.state[base + (int64_t)(m0 + i) * t.R + r0 + tx] = tile[tx][i];
 }
+__global__ void __launch_bounds__(256) state_transpose_kernel(const StateTurn t) { turn_tile(t, blockIdx.x); }
 
 // Modes of the epilogue kernels.  With the heads of a layer spread over several GPUs the norm spans
 // columns on other GPUs: each GPU first computes its own sum of squares per (b, l) row (partial), the
@@ -641,18 +656,25 @@ scan_epilogue_kernel(const void *__restrict__ h, int h_dt, int64_t h_sb, int64_t
 // instruction count as much as by memory, hence the fast-math gate (silu(z) = z / (1 + e^-z) with
 // the approximate exponential and division: about 2 ulp, the output is bf16) and the norm weight
 // read as one or two 16-byte pieces (WVEC 1: bf16, 2: f32; 0: element by element, any type).
-template <int WVEC, bool DF32>
+// TURN: the first blocks turn the scan's final state around (prefill; 397 tokens x 24 heads: a launch of 2.7 us less)
+template <int WVEC, bool DF32, bool TURN>
 __global__ void __launch_bounds__(1024)
 scan_epilogue_bf16_kernel(const __nv_bfloat16 *__restrict__ h, int64_t h_sb, int64_t h_sl,
                           const __nv_bfloat16 *__restrict__ x, int64_t x_sb, int64_t x_sl,
                           const __nv_bfloat16 *__restrict__ gate, int64_t g_sb, int64_t g_sl,
                           const void *__restrict__ Dp, const void *__restrict__ w, int w_dt,
                           float gate_bias, float eps, __nv_bfloat16 *__restrict__ y, int64_t L, int64_t H,
-                          int64_t R, int mode, float *__restrict__ sumsq, int64_t norm_width) {
+                          int64_t R, int mode, float *__restrict__ sumsq, int64_t norm_width, const StateTurn turn,
+                          int turn_tiles) {
   __shared__ float red[32];
+  if (TURN && (int)blockIdx.x < turn_tiles) {
+    turn_tile(turn, blockIdx.x);
+    return;
+  }
   const int HR = (int)(H * R);
-  const int64_t row = blockIdx.x;   // fewer than 2^31 rows (the grid's x extent), so the row splits in 32 bits
-  const int64_t b = (int)blockIdx.x / (int)L, l = row - b * L;
+  // fewer than 2^31 rows (the grid's x extent), so the row splits in 32 bits
+  const int64_t row = TURN ? (int)blockIdx.x - turn_tiles : (int)blockIdx.x;
+  const int64_t b = (int)row / (int)L, l = row - b * L;
   const int j = (int)threadIdx.x * 8;   // < 8192
   float v[8];
   float ss = 0.f;
@@ -770,7 +792,12 @@ int compute_params_typed(const void *dyn, int dyn_dtype, int64_t dyn_sb, int64_t
                          float dt_min, float dt_max, float alpha_min, float alpha_max,
                          float lambda_min, float lambda_max, void *u, void *c,
                          void *kappa, int ck_dtype, float *rho, int64_t Bt, int64_t L,
-                         int64_t H, int64_t R, int64_t M, void *stream) {
+                         int64_t H, int64_t R, int64_t M, void *stream, void *clear = nullptr,
+                         size_t *clear_bytes = nullptr) {
+  // clear: 16-byte aligned memory of which *clear_bytes (a multiple of 16) are set to zero beside the work where the
+  // kernel taken does that; else *clear_bytes becomes 0
+  const size_t clear_want = clear && clear_bytes ? *clear_bytes : 0;
+  if (clear_bytes) *clear_bytes = 0;
   if (Bt < 0 || L < 0 || H <= 0 || R <= 0 || M <= 0) return fail(FRACSSM_ERR_ARG, "compute_params: bad sizes");
   if (!known_dtype(dyn_dtype) || !known_dtype(rw_dtype) || !known_dtype(x_dtype) || !known_dtype(ck_dtype))
     return fail(FRACSSM_ERR_ARG, "compute_params: unsupported dtype");
@@ -817,6 +844,14 @@ int compute_params_typed(const void *dyn, int dyn_dtype, int64_t dyn_sb, int64_t
     if (M == 16) kernel = plain ? compute_params_lanes_kernel<2, true> : compute_params_lanes_kernel<2, false>;
     if (M == 32) kernel = plain ? compute_params_lanes_kernel<4, true> : compute_params_lanes_kernel<4, false>;
     if (M == 64) kernel = plain ? compute_params_lanes_kernel<8, true> : compute_params_lanes_kernel<8, false>;
+    // A launch for the zeros costs 2 us on the device and 3 on the host (397 tokens, 24 layers: 60 us a prompt); the loop in
+    // here up to 2 % of the kernel, 15 us of 600 at 16 x 4096 tokens x 24 heads.  So it is for up to a twelfth of that.
+    if (M == 128 && clear_want && clear_want < (size_t(1) << 34) && Bt * H * L <= (1 << 17)) {
+      kernel = compute_params_lanes_kernel<16, false, true>;
+      a.clear = reinterpret_cast<uint4 *>(clear);
+      a.clear_pieces = (int)(clear_want / 16);
+      *clear_bytes = clear_want;
+    }
     kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(a, per_warp);
     return check_launch("compute_params");
   }
@@ -898,7 +933,7 @@ int scan_epilogue_launch(const char *who, const void *h, int h_dtype, int64_t h_
                          const void *x_conv, int64_t x_sb, int64_t x_sl, const void *gate, int64_t g_sb,
                          int64_t g_sl, int xg_dtype, const void *D, int D_dt, const void *weight, int w_dtype,
                          float gate_bias, float eps, void *y, int64_t Bt, int64_t L, int64_t H, int64_t R,
-                         int mode, float *sumsq, int64_t norm_width, void *stream) {
+                         int mode, float *sumsq, int64_t norm_width, void *stream, const StateTurn &turn = StateTurn{}) {
   if (Bt < 0 || L < 0 || H <= 0 || R <= 0) return fail(FRACSSM_ERR_ARG, "%s: bad sizes", who);
   if (!known_dtype(h_dtype) || !known_dtype(xg_dtype) || (mode != kEpiloguePartial && !known_dtype(w_dtype)))
     return fail(FRACSSM_ERR_ARG, "%s: unsupported dtype", who);
@@ -909,29 +944,38 @@ int scan_epilogue_launch(const char *who, const void *h, int h_dtype, int64_t h_
   if (mode != kEpilogueFull && !sumsq) return fail(FRACSSM_ERR_ARG, "%s: null pointer", who);
   auto al16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   const int64_t HR = H * R;
+  const int64_t tiles = turn.fin ? turn.rows * turn.m_tiles * turn.r_tiles : 0;
+  if (tiles >= (int64_t(1) << 31)) return fail(FRACSSM_ERR_UNSUPPORTED, "%s: too many rows", who);
+  auto turn_alone = [&] {
+    if (tiles) state_transpose_kernel<<<(unsigned)tiles, 256, 0, (cudaStream_t)stream>>>(turn);
+  };
   if (h_dtype == FRACSSM_BF16 && xg_dtype == FRACSSM_BF16 && R % 8 == 0 && HR <= 8192 && al16(h) && al16(x_conv) &&
       al16(gate) && al16(y) && al16(D) && (D_dt == FRACSSM_F32 || D_dt == FRACSSM_BF16) && h_sb % 8 == 0 &&
       h_sl % 8 == 0 && x_sb % 8 == 0 && x_sl % 8 == 0 &&
       g_sb % 8 == 0 && g_sl % 8 == 0) {
     const unsigned threads = (unsigned)(((HR / 8) + 31) / 32 * 32);
     const int wvec = (mode == kEpiloguePartial || !al16(weight)) ? 0 : w_dtype == FRACSSM_BF16 ? 1 : w_dtype == FRACSSM_F32 ? 2 : 0;
+    const bool beside = tiles && Bt * L + tiles < (int64_t(1) << 31);
+    if (!beside) turn_alone();
 #define FRACSSM_EPILOGUE(WV, DF32)                                                                                 \
-  scan_epilogue_bf16_kernel<WV, DF32><<<(unsigned)(Bt * L), threads, 0, (cudaStream_t)stream>>>(                   \
+  auto kernel = beside ? scan_epilogue_bf16_kernel<WV, DF32, true> : scan_epilogue_bf16_kernel<WV, DF32, false>;   \
+  kernel<<<(unsigned)(Bt * L + (beside ? tiles : 0)), threads, 0, (cudaStream_t)stream>>>(                         \
       reinterpret_cast<const __nv_bfloat16 *>(h), h_sb, h_sl, reinterpret_cast<const __nv_bfloat16 *>(x_conv),     \
       x_sb, x_sl, reinterpret_cast<const __nv_bfloat16 *>(gate), g_sb, g_sl, D, weight, w_dtype, gate_bias, eps,   \
-      reinterpret_cast<__nv_bfloat16 *>(y), L, H, R, mode, sumsq, norm_width)
+      reinterpret_cast<__nv_bfloat16 *>(y), L, H, R, mode, sumsq, norm_width, turn, (int)tiles)
     if (D_dt == FRACSSM_F32) {
-      if (wvec == 1) FRACSSM_EPILOGUE(1, true);
-      else if (wvec == 2) FRACSSM_EPILOGUE(2, true);
-      else FRACSSM_EPILOGUE(0, true);
+      if (wvec == 1) { FRACSSM_EPILOGUE(1, true); }
+      else if (wvec == 2) { FRACSSM_EPILOGUE(2, true); }
+      else { FRACSSM_EPILOGUE(0, true); }
     } else {
-      if (wvec == 1) FRACSSM_EPILOGUE(1, false);
-      else if (wvec == 2) FRACSSM_EPILOGUE(2, false);
-      else FRACSSM_EPILOGUE(0, false);
+      if (wvec == 1) { FRACSSM_EPILOGUE(1, false); }
+      else if (wvec == 2) { FRACSSM_EPILOGUE(2, false); }
+      else { FRACSSM_EPILOGUE(0, false); }
     }
 #undef FRACSSM_EPILOGUE
     return check_launch(who);
   }
+  turn_alone();
   auto kernel = D_dt == FRACSSM_F32 ? scan_epilogue_kernel<true> : scan_epilogue_kernel<false>;
   kernel<<<(unsigned)(Bt * L), 256, 0, (cudaStream_t)stream>>>(
       h, h_dtype, h_sb, h_sl, x_conv, x_sb, x_sl, gate, g_sb, g_sl, xg_dtype, D, D_dt, weight, w_dtype,
@@ -1080,23 +1124,25 @@ extern "C" int fracssm_prefill_mix(const void *dyn, const void *dyn_bias, const 
     return fail(FRACSSM_ERR_UNSUPPORTED, "prefill_mix: too many rows");
   auto dt = [&](int i) { return (params_f32 >> i) & 1 ? FRACSSM_F32 : FRACSSM_BF16; };
   const int64_t di = H * R;
+  // the parameter prep of a short call also zeroes what the single-pass scan needs zero
+  size_t clear = 0;
+  if (workspace && fracssm_scan_fused_supported(Bt * H, L, R, M, T, FRACSSM_BF16, ck_dtype))
+    clear = scan_fused_clear_bytes(Bt * H, L, R, M, workspace_bytes, 0, false);
+  if (clear > workspace_bytes || (reinterpret_cast<uintptr_t>(workspace) & 15) != 0) clear = 0;
   int rc = compute_params_typed(dyn, FRACSSM_BF16, L * 3 * H, 3 * H, dyn_bias, rw, FRACSSM_BF16, L * 2 * H * M,
                                 2 * H * M, x_conv, FRACSSM_BF16, L * di, di, mask, L, 1, params[0], dt(0), params[3], dt(3), params[1], dt(1),
                                 params[2], dt(2), nums[0], nums[1], nums[2], nums[3], nums[4], nums[5], nums[6], nullptr, c,
-                                kappa, ck_dtype, rho, Bt, L, H, R, M, stream);
+                                kappa, ck_dtype, rho, Bt, L, H, R, M, stream, workspace, &clear);
   if (rc) return rc;
   bool modes_first = false;
   rc = frac_scan_route(u, FRACSSM_BF16, L * R, R, c, kappa, ck_dtype, L * M, M, L * M, M, rho, L * M, M, nullptr, h,
                        final_state, FRACSSM_F32, workspace, workspace_bytes, Bt * H, L, R, M, T, 0, stream, state,
-                       &modes_first);
+                       &modes_first, clear);
   if (rc) return rc;
-  if (state && !modes_first) {   // (the single-pass kernel writes [R, M]: a second form of that store made it 5 % slower)
-    state_transpose_kernel<<<dim3((unsigned)ceil_div(M, 32), (unsigned)ceil_div(R, 32), (unsigned)(Bt * H)), 256, 0,
-                             (cudaStream_t)stream>>>(final_state, state, (int)R, (int)M);
-    rc = check_launch("prefill_mix");
-    if (rc) return rc;
-  }
+  // (the single-pass kernel writes [R, M]: a second form of that store made it 5 % slower)
+  StateTurn turn{};
+  if (state && !modes_first) turn = StateTurn{final_state, state, (int)R, (int)M, (int)ceil_div(M, 32), (int)ceil_div(R, 32), Bt * H};
   return scan_epilogue_launch("prefill_mix", h, FRACSSM_BF16, L * R, R, x_conv, L * di, di, gate, L * gate_sl, gate_sl,
                               FRACSSM_BF16, params[4], dt(4), params[5], dt(5), nums[7], nums[8], y, Bt, L, H, R,
-                              kEpilogueFull, nullptr, di, stream);
+                              kEpilogueFull, nullptr, di, stream, turn);
 }

@@ -1140,13 +1140,20 @@ size_t scan_fused_workspace_bytes(int64_t B, int64_t, int64_t R, int64_t M, int6
   return B <= kTaggedRows ? tagged_workspace_bytes(B, R, M) : plain_workspace_bytes(B, R, M);
 }
 
+// The bytes at the start of the workspace that a launch needs zero.
+size_t scan_fused_clear_bytes(int64_t B, int64_t L, int64_t R, int64_t M, size_t workspace_bytes, int first_tile, bool layer) {
+  // (a workspace of the plain size keeps the plain hand-over; the tags start from zeros, which no tile hands over)
+  const bool tagged = tags_pay(B, ceil_div(L, kTile) - first_tile) && !layer && workspace_bytes >= tagged_workspace_bytes(B, R, M);
+  return tagged ? tagged_workspace_bytes(B, R, M) : kCtrlBytes + align256((size_t)B * 4);
+}
+
 // first_tile / wait_ns: 0 and the default limit, except in the wait-limit self-test, which starts
 // at a tile whose predecessor is not part of the launch.
 int scan_fused_launch_ex(const void *u, const void *c, const void *kappa, int ck_dtype, const float *rho,
                          const float *initial_state, void *h, void *final_state, int final_dtype,
                          void *workspace, size_t workspace_bytes, int64_t B, int64_t L, int64_t R,
                          int64_t M, int64_t T, void *stream, int first_tile, unsigned long long wait_ns,
-                         const ScanLayerOut *layer) {
+                         const ScanLayerOut *layer, size_t cleared) {
   (void)T;
   const bool ckf32 = ck_dtype == FRACSSM_F32;
   if (workspace_bytes < plain_workspace_bytes(B, R, M))
@@ -1232,13 +1239,12 @@ int scan_fused_launch_ex(const void *u, const void *c, const void *kappa, int ck
   CUtensorMap map;
   int rc = make_tmap_bf16_3d(&map, u, kR, (uint64_t)L, (uint64_t)B, kR, kTile);
   if (rc) return rc;
-  // (a workspace of the plain size keeps the plain hand-over)
-  const bool tagged = tags_pay(B, a.ntiles - first_tile) && !layer &&
-                      workspace_bytes >= tagged_workspace_bytes(B, R, M);
-  // the tags start from zeros, which no tile hands over
-  cudaError_t e = cudaMemsetAsync(ws, 0, tagged ? tagged_workspace_bytes(B, R, M) : kCtrlBytes + align256((size_t)B * 4),
-                                  (cudaStream_t)stream);
-  if (e != cudaSuccess) return fail(FRACSSM_ERR_CUDA, "frac_scan: %s", cudaGetErrorString(e));
+  const size_t zeros = scan_fused_clear_bytes(B, L, R, M, workspace_bytes, first_tile, layer != nullptr);
+  const bool tagged = zeros > kCtrlBytes + align256((size_t)B * 4);
+  if (cleared < zeros) {
+    cudaError_t e = cudaMemsetAsync(ws, 0, zeros, (cudaStream_t)stream);
+    if (e != cudaSuccess) return fail(FRACSSM_ERR_CUDA, "frac_scan: %s", cudaGetErrorString(e));
+  }
   const int grid = a.total < sms ? a.total : sms;
   const cudaStream_t st = (cudaStream_t)stream;
   const bool ragged = a.L % kTile != 0;
@@ -1261,9 +1267,9 @@ int scan_fused_launch_ex(const void *u, const void *c, const void *kappa, int ck
 int scan_fused_launch(const void *u, const void *c, const void *kappa, int ck_dtype, const float *rho,
                       const float *initial_state, void *h, void *final_state, int final_dtype,
                       void *workspace, size_t workspace_bytes, int64_t B, int64_t L, int64_t R,
-                      int64_t M, int64_t T, void *stream) {
+                      int64_t M, int64_t T, void *stream, size_t cleared) {
   return scan_fused_launch_ex(u, c, kappa, ck_dtype, rho, initial_state, h, final_state, final_dtype, workspace,
-                              workspace_bytes, B, L, R, M, T, stream, 0, kWaitNs, nullptr);
+                              workspace_bytes, B, L, R, M, T, stream, 0, kWaitNs, nullptr, cleared);
 }
 
 }  // namespace fracssm
