@@ -60,7 +60,8 @@ int scan_fused_launch_ex(const void *u, const void *c, const void *kappa, int ck
                          void *workspace, size_t workspace_bytes, int64_t B, int64_t L, int64_t R,
                          int64_t M, int64_t T, void *stream, int first_tile, unsigned long long wait_ns,
                          const ScanLayerOut *layer, size_t cleared = 0);
-size_t scan_fused_clear_bytes(int64_t B, int64_t L, int64_t R, int64_t M, size_t workspace_bytes, int first_tile, bool layer);
+size_t scan_fused_clear_bytes(int64_t B, int64_t L, int64_t R, int64_t M, int ck_dtype, size_t workspace_bytes, int first_tile,
+                              bool layer);
 int scan_fused_launch(const void *u, const void *c, const void *kappa, int ck_dtype, const float *rho,
                       const float *initial_state, void *h, void *final_state, int final_dtype,
                       void *workspace, size_t workspace_bytes, int64_t B, int64_t L, int64_t R,

@@ -1127,7 +1127,7 @@ extern "C" int fracssm_prefill_mix(const void *dyn, const void *dyn_bias, const 
   // the parameter prep of a short call also zeroes what the single-pass scan needs zero
   size_t clear = 0;
   if (workspace && fracssm_scan_fused_supported(Bt * H, L, R, M, T, FRACSSM_BF16, ck_dtype))
-    clear = scan_fused_clear_bytes(Bt * H, L, R, M, workspace_bytes, 0, false);
+    clear = scan_fused_clear_bytes(Bt * H, L, R, M, ck_dtype, workspace_bytes, 0, false);
   if (clear > workspace_bytes || (reinterpret_cast<uintptr_t>(workspace) & 15) != 0) clear = 0;
   int rc = compute_params_typed(dyn, FRACSSM_BF16, L * 3 * H, 3 * H, dyn_bias, rw, FRACSSM_BF16, L * 2 * H * M,
                                 2 * H * M, x_conv, FRACSSM_BF16, L * di, di, mask, L, 1, params[0], dt(0), params[3], dt(3), params[1], dt(1),

@@ -1113,22 +1113,24 @@ size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 }  // namespace
 
-// Where the state is handed over with tags (LL).  A step of a row's chain takes 1.0 us with tags and 2.4 us through the
-// counter (4 rows), a tile of a CTA 10.5 us against 8 (the tags' traffic and instructions), and the tags start from zeros.
-// So with more rows the chain has to be longer before it counts.  Counter / tags in us (bfloat16 coefficients; float32
-// lies the same way):
-//   tiles a row        2             4             6            12            24            32
-//      8 rows    18.5 / 19.7   22.6 / 21.7                                               92 /  55
-//     24 rows    18.6 / 20.2   23.4 / 21.9   29.2 / 23.8   48.7 / 37.7   87.6 / 66.7   109 /  84
-//     32 rows    18.5 / 20.4   23.7 / 22.7   32.6 / 30.9   54.2 / 47.8   96.3 / 79.7   121 /  97
-//     40 rows    18.6 / 20.6   25.4 / 29.8   34.0 / 33.8   56.6 / 54.9   97.4 / 89.4   125 / 110
-//     48 rows    18.6 / 20.6   28.2 / 29.9   35.0 / 34.4   57.8 / 57.2    107 /  99    135 / 122
-//     64 rows    18.8 / 20.6   30.1 / 31.9   41.4 / 42.8   67.8 / 68.8    131 / 123    157 / 149
-//     80 rows, 64 tiles 317 / 343; 96 rows, 64 tiles 351 / 406
-// (24 x 131072 tokens 2.92 / 1.76 ms, 48 x 65536 1.89 / 1.56 ms.)
-constexpr int64_t kTaggedRows = 64;
-static bool tags_pay(int64_t rows, int64_t tiles) {
-  return rows <= kTaggedRows && tiles >= (rows <= 32 ? 4 : rows <= 48 ? 12 : 24);
+// Where the state is handed over with tags (LL).  A step of a row's chain takes 0.6 us with tags and 2.4 us through the
+// counter (4 rows); but the tags are twice the state traffic, instructions and zeros to start from, which counts once the
+// SMs have more than one tile each, and more with float32 coefficients, where the kernel is
+// short of registers.  Counter / tags in us, bfloat16 coefficients | float32:
+//   tiles a row          2                4                 8                 24                 64
+//      8 rows      17 / 15 | 18 / 17  23 / 17 | 22 / 19   32 / 20 | 31 / 23   70 / 34 | 68 / 41   169 / 72  | 168 / 88
+//     32 rows      18 / 16 | 19 / 18  23 / 18 | 23 / 20   36 / 28 | 36 / 32   88 / 62 | 91 / 77   214 / 141 | 221 / 170
+//     40 rows      19 / 16 | 18 / 18  24 / 23 | 24 / 27   37 / 33 | 37 / 39   91 / 73 | 98 / 92   221 / 169 | 230 / 206
+//     48 rows      18 / 16 | 18 / 18  26 / 25 | 27 / 28   40 / 36 | 41 / 43   98 / 84 | 106 / 105 236 / 198 | 254 / 242
+//     64 rows      19 / 17 | 18 / 19  27 / 26 | 28 / 30   46 / 45 | 50 / 54  117 / 108 | 127 / 133  283 / 259 | 310 / 315
+//     72 rows      19 / 17 | 19 / 19  28 / 27 | 30 / 31   47 / 46 | 50 / 57  109 / 118 | 119 / 146  274 / 289 | 299 / 353
+// With a last tile that is not full the tags gain more: float32, 64 rows, 24 tiles 130 / 125, 48 tiles 238 / 226.  Three
+// tiles a row in little more than a wave are a draw: bfloat16, 52 rows 23.1 / 24.1, 64 rows 25.6 / 24.9.
+constexpr int64_t kTaggedRows = 64, kTaggedWave = 148;
+static bool tags_pay(int64_t rows, int64_t tiles, bool ckf32) {
+  if (rows > kTaggedRows || tiles < 2) return false;
+  if (rows * tiles <= kTaggedWave) return true;
+  return tiles >= (!ckf32 || rows <= 32 ? 4 : rows <= 48 ? 12 : 24);
 }
 static size_t plain_workspace_bytes(int64_t B, int64_t R, int64_t M) {
   return kCtrlBytes + align256((size_t)B * 4) + (size_t)B * R * M * 4;
@@ -1141,9 +1143,11 @@ size_t scan_fused_workspace_bytes(int64_t B, int64_t, int64_t R, int64_t M, int6
 }
 
 // The bytes at the start of the workspace that a launch needs zero.
-size_t scan_fused_clear_bytes(int64_t B, int64_t L, int64_t R, int64_t M, size_t workspace_bytes, int first_tile, bool layer) {
+size_t scan_fused_clear_bytes(int64_t B, int64_t L, int64_t R, int64_t M, int ck_dtype, size_t workspace_bytes, int first_tile,
+                              bool layer) {
   // (a workspace of the plain size keeps the plain hand-over; the tags start from zeros, which no tile hands over)
-  const bool tagged = tags_pay(B, ceil_div(L, kTile) - first_tile) && !layer && workspace_bytes >= tagged_workspace_bytes(B, R, M);
+  const bool tagged = tags_pay(B, ceil_div(L, kTile) - first_tile, ck_dtype == FRACSSM_F32) && !layer &&
+                      workspace_bytes >= tagged_workspace_bytes(B, R, M);
   return tagged ? tagged_workspace_bytes(B, R, M) : kCtrlBytes + align256((size_t)B * 4);
 }
 
@@ -1239,7 +1243,7 @@ int scan_fused_launch_ex(const void *u, const void *c, const void *kappa, int ck
   CUtensorMap map;
   int rc = make_tmap_bf16_3d(&map, u, kR, (uint64_t)L, (uint64_t)B, kR, kTile);
   if (rc) return rc;
-  const size_t zeros = scan_fused_clear_bytes(B, L, R, M, workspace_bytes, first_tile, layer != nullptr);
+  const size_t zeros = scan_fused_clear_bytes(B, L, R, M, ck_dtype, workspace_bytes, first_tile, layer != nullptr);
   const bool tagged = zeros > kCtrlBytes + align256((size_t)B * 4);
   if (cleared < zeros) {
     cudaError_t e = cudaMemsetAsync(ws, 0, zeros, (cudaStream_t)stream);

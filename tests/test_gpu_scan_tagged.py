@@ -1,5 +1,5 @@
-"""The single-pass scan's two ways of handing the state from tile to tile: with tags beside the values for few and long
-rows (from 4 tiles on, with more than 32 rows from 12 and with more than 48 from 24, up to 64 rows), else through a counter.  The arithmetic is the same, so the results are the same bits."""
+"""The single-pass scan's two ways of handing the state from tile to tile: with tags beside the values for few
+rows (up to 64; where one wave holds all tiles, or from 4, 12 or 24 tiles on), else through a counter.  The arithmetic is the same, so the results are the same bits."""
 
 import pytest
 import torch
