@@ -13,8 +13,8 @@
 // that what follows the convolution follows both.  us for K = 1536, the convolution alone / with the library's product
 // behind it / with this kernel beside it:
 //   rows            5                 397                4000                16000               65536
-//   36 columns   3.0 / 12.7 / 4.8   4.2 / 16.5 / 6.8   11.3 / 28.9 / 12.6   36.3 / 56.6 / 38.1   127 / 204 / 164
-//   72 columns   3.1 /  7.1 / 5.3   4.2 /  8.3 / 7.7   11.2 / 16.2 / 12.6   36.3 / 44.3 / 38.7   126 / 178 / 163
+//   36 columns   3.0 / 12.7 / 4.9   4.2 / 16.5 / 6.5   11.3 / 28.9 / 12.5   36.3 / 56.6 / 38.1   127 / 204 / 164
+//   72 columns   3.1 /  7.1 / 5.4   4.2 /  8.3 / 7.3   11.2 / 16.2 / 12.6   36.3 / 44.3 / 38.8   126 / 178 / 165
 // (The library takes an old kernel where N is no multiple of 8: 17 us for 4000 rows and 36 columns, 4.6 for 72.)
 #include <mutex>
 
@@ -31,7 +31,8 @@ constexpr int kDynK = 64;            // columns of K a step: one 128-byte row of
 constexpr int kDynThreads = 128;
 constexpr int kDynMaxSplit = 8;
 constexpr int kDynMaxStages = 8;
-constexpr size_t kDynMaxSmem = 112 * 1024;
+constexpr size_t kDynMaxSmem = 224 * 1024;
+constexpr int64_t kDynFewBlocks = 64;
 
 struct DynArgs {
   __nv_bfloat16 *out;
@@ -79,6 +80,10 @@ prefill_dyn_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
     }
     umma::fence_mbar_init();
   }
+  // Nobody who holds tensor memory waits for a block that may yet want some (another stream's kernel may hold it there,
+  // and wait in turn): a block says that it has started before it asks for its own, and gives it back before it waits for
+  // the others' sums.
+  if (SPLIT > 1) cluster_arrive();
   if (warp == 1) umma::tmem_alloc(&tmem, (uint32_t)a.cols);
   umma::tc_fence_before();
   __syncthreads();
@@ -130,15 +135,12 @@ prefill_dyn_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
   __syncthreads();
   umma::tc_fence_after();
 
-  // Each row's sums go to the block that owns the row, into a slot for each block they come from.  The slots lie in the
-  // ring: the owner's products are done when it arrives.
-  if (SPLIT > 1) {
-    cluster_arrive();
-    cluster_wait();
-  }
+  // Each row's sums go to the block that owns the row, into a slot behind its ring for each block they come from.  (A
+  // block alone has its slots in the ring.)
+  if (SPLIT > 1) cluster_wait();      // all blocks have started
   constexpr int kPer = kDynRows / SPLIT;
   const int pitch = a.n16 + 4;      // (16-byte stores of eight rows fall into different banks)
-  const float *part = reinterpret_cast<const float *>(ring);
+  const float *part = reinterpret_cast<const float *>(ring + (SPLIT > 1 ? (uint32_t)a.stages * stage_bytes : 0u));
   const uint32_t slot = umma::smem_u32(part) + (uint32_t)((rank * kPer + (int)threadIdx.x % kPer) * pitch) * 4u;
   const uint32_t to = peer_addr(slot, (int)threadIdx.x / kPer);
   const bool bad = failed != 0, wanted = row0 + (int)threadIdx.x < a.rows;
@@ -155,13 +157,12 @@ prefill_dyn_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
       if (wanted) st_peer(to + (uint32_t)(c + i) * 4u, v[i], v[i + 1], v[i + 2], v[i + 3]);
   }
   umma::tc_fence_before();
+  __syncthreads();
+  if (warp == 1) umma::tmem_dealloc(tmem, (uint32_t)a.cols);
   if (SPLIT > 1) {
     cluster_arrive();
     cluster_wait();
-  } else {
-    __syncthreads();
   }
-  if (warp == 1) umma::tmem_dealloc(tmem, (uint32_t)a.cols);
 
   // this block's rows: a warp four rows at a time, a lane a pair of columns
   const int64_t first = row0 + rank * kPer, left = a.rows - first;
@@ -243,20 +244,27 @@ int prefill_dyn_launch(const void *x, int64_t x_sl, const void *w, void *out, in
   a.wait_ns = tile_default_wait_ns();
   // K is cut as long as the grid has one block per SM and a block two steps.  The kernel alone, us, 72 columns:
   //   blocks a tile        1      2      4      8
-  //     397 rows         10.6    8.2    7.2    6.7
-  //    4000 rows         10.7    8.5    7.6   10.2   (8: 256 blocks)
-  //    9000 rows         10.7    8.7   11.0          (4: 284 blocks)
-  //   16000 rows         11.1   11.2   19.0          (2: 250 blocks)
+  //     397 rows         10.4    8.1    7.0    6.5
+  //    4000 rows         10.5    8.2    8.1   10.2   (8: 256 blocks)
+  //    9000 rows         10.7   10.0   11.1          (4: 284 blocks)
+  //   16000 rows         10.9   12.6   19.7          (2: 250 blocks)
   const int64_t tiles = ceil_div(rows, kDynRows);
   a.split = 1;
   while (a.split < kDynMaxSplit && tiles * a.split * 2 <= sms && a.steps >= a.split * 4) a.split *= 2;
   const size_t stage = kDynRows * 128 + (size_t)a.n16 * 128, sums = (size_t)kDynRows * (a.n16 + 4) * 4;
-  // as many stages as two blocks per SM have room for; 1 KB aligns the ring
-  a.stages = (int)((kDynMaxSmem - 1024) / stage);
-  if (a.stages > kDynMaxStages) a.stages = kDynMaxStages;
+  // As many stages as half an SM has room for, or the whole where blocks are few or that is less than two.  (128 blocks in
+  // clusters of 8 find no place with an SM each: 2000 rows with the convolution 16.4 us instead of 9.9.  128 blocks in
+  // clusters of 4 do, and are 0.5 us faster alone, but the convolution beside them is slower: 4 x 1000 tokens through 24
+  // layers 3152 us instead of 3090.)  1 KB aligns the ring.
   const int most = (int)ceil_div(a.steps, a.split);
+  const size_t behind = a.split > 1 ? sums : 0;
+  auto fit = [&](size_t room) { return room < 1024 + behind ? 0 : (int)((room - 1024 - behind) / stage); };
+  a.stages = tiles * a.split <= kDynFewBlocks ? 0 : fit(kDynMaxSmem / 2);
+  if (a.stages < 2) a.stages = fit(kDynMaxSmem);
+  if (a.stages > kDynMaxStages) a.stages = kDynMaxStages;
   if (a.stages > most) a.stages = most;
-  const size_t smem = 1024 + (a.stages * stage > sums ? a.stages * stage : sums);
+  size_t smem = a.stages * stage + behind;
+  smem = 1024 + (smem > sums ? smem : sums);
 
   CUtensorMap x_map, w_map;
   int rc = make_tmap_bf16_rows(&x_map, x, (uint64_t)K, (uint64_t)rows, (uint64_t)x_sl, kDynK, kDynRows);
