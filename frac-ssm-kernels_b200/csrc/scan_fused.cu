@@ -1113,7 +1113,7 @@ size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 }  // namespace
 
-// Where the state is handed over with tags (LL).  A step of a row's chain takes 0.6 us with tags and 2.4 us through the
+// Where the state is handed over with tags (LL).  A step of a row's chain takes 0.6 to 0.8 us with tags and 2.4 us through the
 // counter (4 rows); but the tags are twice the state traffic, instructions and zeros to start from, which counts once the
 // SMs have more than one tile each, and more with float32 coefficients, where the kernel is
 // short of registers.  Counter / tags in us, bfloat16 coefficients | float32:
