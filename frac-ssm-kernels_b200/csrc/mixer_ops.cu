@@ -6,6 +6,7 @@
 // Both are bandwidth kernels: every input element is read once, every output written once.
 #include "common.cuh"
 #include "prefill_dyn.cuh"
+#include "scan_tile.cuh"
 
 namespace fracssm {
 namespace {
@@ -59,6 +60,13 @@ causal_conv_silu_kernel(const void *__restrict__ x, int x_dt, int64_t x_sb, int6
   }
 }
 
+using tile::f2;
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
 // bf16 path for the usual width 4.
 __device__ __forceinline__ void unpack8(const uint4 &p, float (&f)[8]) {
   const uint32_t wds[4] = {p.x, p.y, p.z, p.w};
@@ -67,13 +75,6 @@ __device__ __forceinline__ void unpack8(const uint4 &p, float (&f)[8]) {
     f[2 * i] = __uint_as_float(wds[i] << 16);
     f[2 * i + 1] = __uint_as_float(wds[i] & 0xFFFF0000u);
   }
-}
-
-__device__ __forceinline__ void unpack4(const uint2 &p, float (&f)[4]) {
-  f[0] = __uint_as_float(p.x << 16);
-  f[1] = __uint_as_float(p.x & 0xFFFF0000u);
-  f[2] = __uint_as_float(p.y << 16);
-  f[3] = __uint_as_float(p.y & 0xFFFF0000u);
 }
 
 // What the convolution of the next token needs: tail[b, ch, k] = the last K - 1 inputs times their mask (rounded to
@@ -103,14 +104,16 @@ conv_tail_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_sb, int64_t x_sl
 }
 
 // Four channels (8 bytes) per thread, TOKENS (32 at full size) tokens walked with the window in registers, the next
-// four tokens requested before the current four are worked on; at most 80 registers, so 6 blocks of
-// 128 threads per SM.  At batch 16 x 4096 tokens x 1536 channels: 0.154 ms with 16 tokens per thread and
-// the loads of a group issued right before their use, 0.143 ms with 32 tokens (the three window tokens and
-// the weights are read once per 32), 0.125 ms with the loads one group ahead.  A short sequence is cut into runs of 16
-// or 8 tokens so that the grid covers the GPU (397 tokens: 12.2 -> 7.5 us).  With TAIL, the last row of blocks writes it;
-// at full size a launch of its own does, since that branch costs the kernel registers and 6 % of its time.
+// four tokens requested before the current four are worked on.  Bound by the instructions a thread issues until its next
+// request as much as by memory: with the channels as packed pairs and running addresses 16 x 4096 tokens x 1536
+// channels take 109 us (125 with an fma per channel and 64-bit index products a token; 8 blocks of 128 threads per SM,
+// 114 with 6), 4 x 1000 10.0 (11.6), 397 3.9 (4.4; 6 blocks, 8 are 12 % slower there).  Before: 0.154 ms with 16 tokens per
+// thread and the loads of a group issued right before their use, 0.143 with 32 tokens (the three window tokens and the
+// weights are read once per 32).  A short sequence is cut into runs of 16 or 8 tokens so that the grid covers the GPU.
+// With TAIL, the last row of blocks writes it; at full size a launch of its own does, since that branch costs the kernel
+// registers and 6 % of its time.
 template <int TOKENS, bool TAIL>
-__global__ void __launch_bounds__(128, 6)
+__global__ void __launch_bounds__(128, TOKENS == kConvTokens ? 8 : 6)
 causal_conv4_silu_bf16_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_sb, int64_t x_sl,
                               const float *__restrict__ mask, int64_t m_sb, int64_t m_sl,
                               const void *__restrict__ w, int w_dt, const void *__restrict__ bias,
@@ -126,7 +129,7 @@ causal_conv4_silu_bf16_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_sb,
   __nv_bfloat16 *u_row = nullptr;
   if (u_heads) u_row = u_heads + ((int64_t)blockIdx.z * (C / R) + ch / R) * L * R + ch % R;
   const int64_t b = blockIdx.z, l0 = (int64_t)blockIdx.y * TOKENS;
-  float wk[4][4], bv[4], w0[4], w1[4], w2[4];
+  f2 wk[4][2], bv[2], w0[2], w1[2], w2[2];      // pairs of channels: half the multiply-adds
   if (w_dt == FRACSSM_BF16) {   // 4 channels x 4 taps = 32 contiguous bytes (ch is a multiple of 4)
     const uint4 *wp = reinterpret_cast<const uint4 *>(reinterpret_cast<const __nv_bfloat16 *>(w) + ch * 4);
 #pragma unroll
@@ -134,90 +137,95 @@ causal_conv4_silu_bf16_kernel(const __nv_bfloat16 *__restrict__ x, int64_t x_sb,
       float f[8];
       unpack8(__ldg(wp + q), f);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) { wk[k][2 * q] = f[k]; wk[k][2 * q + 1] = f[4 + k]; }
+      for (int k = 0; k < 4; ++k) wk[k][q] = tile::mk2(f[k], f[4 + k]);
     }
   } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int q = 0; q < 2; ++q) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) wk[k][i] = ld_f32(w, (ch + i) * 4 + k, w_dt);
+      for (int k = 0; k < 4; ++k)
+        wk[k][q] = tile::mk2(ld_f32(w, (ch + 2 * q) * 4 + k, w_dt), ld_f32(w, (ch + 2 * q + 1) * 4 + k, w_dt));
     }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) bv[i] = bias ? ld_f32(bias, ch + i, w_dt) : 0.f;
-  auto in = [&](int64_t l, float (&f)[4]) {
+  for (int q = 0; q < 2; ++q)
+    bv[q] = bias ? tile::mk2(ld_f32(bias, ch + 2 * q, w_dt), ld_f32(bias, ch + 2 * q + 1, w_dt)) : tile::mk2(0.f, 0.f);
+  const __nv_bfloat16 *xp = x + b * x_sb + ch;
+  const float *mp = mask ? mask + b * m_sb : nullptr;
+  auto widen = [&](const uint2 &p, float m, f2 (&f)[2]) {
+    f[0] = tile::mk2(__uint_as_float(p.x << 16), __uint_as_float(p.x & 0xFFFF0000u));
+    f[1] = tile::mk2(__uint_as_float(p.y << 16), __uint_as_float(p.y & 0xFFFF0000u));
+    if (mask) {
+      f[0] = tile::mul2(f[0], tile::mk2(m, m));
+      f[1] = tile::mul2(f[1], tile::mk2(m, m));
+    }
+  };
+  auto in = [&](int64_t l, f2 (&f)[2]) {
     if (l < 0) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) f[i] = 0.f;
+      f[0] = f[1] = tile::mk2(0.f, 0.f);
       return;
     }
-    unpack4(__ldcs(reinterpret_cast<const uint2 *>(x + b * x_sb + l * x_sl + ch)), f);
-    if (mask) {
-      const float m = mask[b * m_sb + l * m_sl];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) f[i] *= m;
-    }
+    widen(__ldcs(reinterpret_cast<const uint2 *>(xp + l * x_sl)), mask ? mp[l * m_sl] : 1.f, f);
   };
   in(l0 - 3, w0);
   in(l0 - 2, w1);
   in(l0 - 1, w2);
-  const int64_t l1 = min(l0 + TOKENS, L);
+  const int n = (int)(min(l0 + TOKENS, L) - l0);
+  xp += l0 * x_sl;
+  if (mask) mp += l0 * m_sl;
+  __nv_bfloat16 *yp = y + (b * L + l0) * C + ch;
+  if (u_row) u_row += l0 * R;
   // the next four tokens are requested before the current four are worked on
   uint2 nraw[4];
   float nmk[4];
-  auto request = [&](int64_t lg) {
+  auto request = [&](int g) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       nraw[j] = make_uint2(0u, 0u);
       nmk[j] = 1.f;
-      if (lg + j < l1) {
-        nraw[j] = __ldcs(reinterpret_cast<const uint2 *>(x + b * x_sb + (lg + j) * x_sl + ch));
-        if (mask) nmk[j] = mask[b * m_sb + (lg + j) * m_sl];
+      if (g + j < n) {
+        nraw[j] = __ldcs(reinterpret_cast<const uint2 *>(xp + j * x_sl));
+        if (mask) nmk[j] = mp[j * m_sl];
       }
     }
+    xp += 4 * x_sl;
+    if (mask) mp += 4 * m_sl;
   };
-  request(l0);
-  for (int64_t lg = l0; lg < l1; lg += 4) {
+  request(0);
+  for (int g = 0; g < n; g += 4) {
     uint2 raw[4];
     float mk[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) { raw[j] = nraw[j]; mk[j] = nmk[j]; }
-    if (lg + 4 < l1) request(lg + 4);
+    if (g + 4 < n) request(g + 4);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      if (lg + j < l1) {
-        const int64_t l = lg + j;
-        float cur[4];
-        unpack4(raw[j], cur);
-        if (mask) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) cur[i] *= mk[j];
-        }
+      if (g + j < n) {
+        f2 cur[2];
+        widen(raw[j], mk[j], cur);
         uint32_t o[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          float r[2];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int c = 2 * i + e;
-            float acc = bv[c];
-            acc = fmaf(wk[0][c], w0[c], acc);
-            acc = fmaf(wk[1][c], w1[c], acc);
-            acc = fmaf(wk[2][c], w2[c], acc);
-            acc = fmaf(wk[3][c], cur[c], acc);
-            r[e] = __fdividef(acc, 1.f + __expf(-acc));   // silu, about 2 ulp: the output is bf16
-          }
-          const __nv_bfloat162 t = __floats2bfloat162_rn(r[0], r[1]);
+          f2 acc = fma2(wk[0][i], w0[i], bv[i]);
+          acc = fma2(wk[1][i], w1[i], acc);
+          acc = fma2(wk[2][i], w2[i], acc);
+          acc = fma2(wk[3][i], cur[i], acc);
+          float r0, r1;
+          tile::un2(acc, r0, r1);
+          r0 = __fdividef(r0, 1.f + __expf(-r0));   // silu, about 2 ulp: the output is bf16
+          r1 = __fdividef(r1, 1.f + __expf(-r1));
+          const __nv_bfloat162 t = __floats2bfloat162_rn(r0, r1);
           o[i] = *reinterpret_cast<const uint32_t *>(&t);
-        }
-        __stcs(reinterpret_cast<uint2 *>(y + (b * L + l) * C + ch), make_uint2(o[0], o[1]));
-        if (u_row) __stcs(reinterpret_cast<uint2 *>(u_row + l * R), make_uint2(o[0], o[1]));
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
           w0[i] = w1[i];
           w1[i] = w2[i];
           w2[i] = cur[i];
         }
+        __stcs(reinterpret_cast<uint2 *>(yp), make_uint2(o[0], o[1]));
+        if (u_row) {
+          __stcs(reinterpret_cast<uint2 *>(u_row), make_uint2(o[0], o[1]));
+          u_row += R;
+        }
+        yp += C;
       }
     }
   }
