@@ -76,4 +76,14 @@ int frac_scan_route(const void *u, int u_dtype, int64_t u_sb, int64_t u_sl, cons
                     size_t workspace_bytes, int64_t B, int64_t L, int64_t R, int64_t M, int64_t T, int path, void *stream,
                     float *state_modes_first, bool *modes_first, size_t cleared = 0);
 
+// defined in decode_layers.cu: fracssm_decode_layers, with the form of the step and what the self-tests set
+struct DecodeForm {
+  enum { kByRule = 0, kOneKernel = 1, kStages = 2 };
+  int form = kByRule;      // (kOneKernel covers up to 32 sequences)
+  int blocks = 0;          // of the one-kernel form; 0: one per SM
+};
+int decode_layers_launch(const uint64_t *layer_ptrs, const float *layer_nums, int64_t layers, const void *hidden_in,
+                         void *hidden_out, void *workspace, size_t workspace_bytes, int64_t B, int64_t hidden, int64_t H,
+                         int64_t R, int64_t M, int64_t K, void *stream, const DecodeForm &how);
+
 }  // namespace fracssm

@@ -22,12 +22,15 @@
 //
 // Two forms of the same code (struct Step), with the same results:
 //   * a kernel a stage, launched with programmatic stream serialisation: 97 launches at 24 layers;
-//   * one kernel (a launch per 32 layers) whose blocks, one per SM, meet at a barrier between the stages.  The host makes the
-//     97 launches in more time than the device takes for them at few sequences.  A stage takes 2 to 5 us here, of which
+//   * one kernel (a launch per 32 layers) whose blocks, at most one per SM, meet at a barrier between the stages.  The host makes
+//     the 97 launches in more time than the device takes for them at few sequences.  A stage takes 2 to 5 us here, of which
 //     the barrier is 1.3; what bounds it is the number of instructions a warp gets through with cold instruction
 //     caches, since every stage passes through its code once per layer.  So it is ONE loop over the stages with one copy of each
 //     piece of code, little of it unrolled (with the products and their requests inlined for each stage 117 KB of code and
 //     0.86 ms at one sequence; 68 KB and 0.51 ms as here).
+//     Nothing makes all blocks run at the same time: kernels of other streams may hold SMs, for long, and may wait for this very
+//     step.  So the blocks that have started make up a list and share the work among themselves (see join); a block that comes
+//     later finds the list closed and leaves.  Nobody waits for a block that has not started.
 // Where either is used: see one_kernel_pays.
 #include <mutex>
 
@@ -112,9 +115,11 @@ enum LayerPtr { kNormW, kInW, kConvW, kConvB, kDynW, kDynB, kRwW, kDtBias, kRead
                 kOutNormW, kOutW, kOldState, kOldConv, kNewState, kNewConv, kF32Mask, kLayerPtrs };
 enum LayerNum { kEpsIn, kEpsOut, kReadTemp, kDtMin, kDtMax, kAMin, kAMax, kLMin, kLMax, kGateBias, kLayerNums };
 
-// Where a thread stands: a block is `teams` teams of 8 warps, each of which works on tiles or heads of its own.
+// Where a thread stands: a block is `teams` teams of 8 warps, each of which works on tiles or heads of its own; the blocks that
+// share the work are numbered 0 .. blocks - 1.
 struct Place {
   int team, teams, tid, lane, w;   // tid, w: inside the team
+  int block, blocks;
   __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kTeam) : "memory"); }
 };
 
@@ -125,15 +130,24 @@ struct MixShape {                      // what does not change from layer to lay
   int items, batch, parts;             // parts: sums of squares an item leaves
 };
 
-// The embedding times the first norm's weight, and its sums of squares (one part per row); clears the counter of the one-kernel
-// form's barriers.
+// What the blocks of the one-kernel form count together.
+struct Meeting {
+  unsigned arrived;    // at the barriers, over the whole launch
+  unsigned started;    // blocks that asked to be on the list; kClosed once it is closed
+  unsigned members;    // blocks on the closed list, 0 before
+  unsigned spare;
+};
+constexpr unsigned kClosed = 0x80000000u;
+
+// The embedding times the first norm's weight, and its sums of squares (one part per row); clears what the one-kernel form's
+// blocks count.
 __global__ void __launch_bounds__(kTeam)
 decode_first_kernel(const __nv_bfloat16 *h, const void *w, int w_dt, float *h_f32, __nv_bfloat16 *h_w, float *ss, int d,
-                    unsigned *counter) {
+                    Meeting *meeting) {
   __shared__ float red[kWarps];
   const int64_t b = blockIdx.x;
   grid_dep_launch();
-  if (b == 0 && threadIdx.x == 0) *counter = 0;
+  if (b == 0 && threadIdx.x == 0) *meeting = Meeting{};
   float sq = 0.f;
   for (int i = threadIdx.x; i < d; i += kTeam) {
     const float v = __bfloat162float(h[b * d + i]);
@@ -165,11 +179,11 @@ struct StepArgs {
   const void *after_w;               // the norm weight behind the last of them, or null: the model's last layer
   int after_dt;
   int layers, first;                 // first: index of tab[0] in the model
-  int B, d, H, R, M, splits, l2_state, blocks2;   // blocks2: blocks that take dyn_proj's tiles
+  int B, d, H, R, M, splits, l2_state, blocks2;   // blocks2: blocks that take dyn_proj's tiles (the kernel of a stage)
   MixShape mix;
   __nv_bfloat16 *x, *x_conv, *vals, *hid_w, *out;
   float *gate, *rw, *dyn, *ss, *hid[2], *hid_ss;
-  unsigned *counter, met;            // the barriers' counter, and what it holds when the launch begins
+  Meeting *meeting;
   uint32_t act_bytes, red_bytes, mix_bytes;
 };
 
@@ -196,6 +210,7 @@ struct Step {
   const __nv_bfloat16 *W, *act;
   int N, K, tile0, tile_step, tiles, k_lo, k_hi;
   bool second, any;   // second: dyn_proj's tiles; any: a team of this block has a tile
+  int blocks2;        // blocks that take dyn_proj's tiles
 
   __device__ __forceinline__ const __nv_bfloat16 *bfp(int l, int i) const {
     return reinterpret_cast<const __nv_bfloat16 *>(a.tab[l].p[i]);
@@ -206,10 +221,11 @@ struct Step {
   }
 
   // ---------------------------------------------------------------------------------------------- the products
-  __device__ __forceinline__ void product(int l, int kind, int team) {
+  // (`rest`, a block alone: rw_proj's tiles, after dyn_proj's)
+  __device__ __forceinline__ void product(int l, int kind, int team, bool rest = false) {
     const int di = a.H * a.R;
-    int blk = blockIdx.x, blocks = gridDim.x;
-    second = kind == kProj && blk < a.blocks2;
+    int blk = at.block, blocks = at.blocks;
+    second = kind == kProj && blk < blocks2 && !rest;
     if (kind == kIn) {
       W = bfp(l, kInW); act = a.hid_w; N = 2 * di; K = a.d;
     } else if (kind == kOut) {
@@ -218,10 +234,10 @@ struct Step {
       K = di;
       if (second) {
         W = bfp(l, kDynW); act = a.x; N = 3 * a.H;
-        blocks = a.blocks2;
+        blocks = blocks2;
       } else {
         W = bfp(l, kRwW); act = a.x_conv; N = 2 * a.H * a.M;
-        blk -= a.blocks2; blocks -= a.blocks2;
+        if (!rest) { blk -= blocks2; blocks -= blocks2; }
       }
     }
     tiles = tiles_of(N);
@@ -475,11 +491,11 @@ struct Step {
     const float *old = reinterpret_cast<const float *>(a.tab[l].p[kOldState]);
     if (!old || !a.l2_state) return;
 #pragma unroll 1
-    for (int item = blockIdx.x + team * gridDim.x; item < a.mix.items; item += gridDim.x * at.teams)
+    for (int item = at.block + team * at.blocks; item < a.mix.items; item += at.blocks * at.teams)
       if (item % a.splits == 0) umma::prefetch_l2(old + (int64_t)(item / a.splits) * a.M * a.R, a.M * a.R * 4);
   }
   __device__ __forceinline__ void request_state(int l, int q, int mg) {
-    const int first = blockIdx.x + at.team * gridDim.x;
+    const int first = at.block + at.team * at.blocks;
     const float *old = reinterpret_cast<const float *>(a.tab[l].p[kOldState]);
     if (first >= a.mix.items) return;
     const bool have = old && mg < a.mix.groups;
@@ -500,7 +516,7 @@ struct Step {
     return reinterpret_cast<float4 *>(smem + at.team * a.mix_bytes) + slot * a.M;
   }
   __device__ __forceinline__ void mix_inputs(int l) {
-    const int first = blockIdx.x + at.team * gridDim.x;
+    const int first = at.block + at.team * at.blocks;
     if (first >= a.mix.items) return;
     const Item i0 = item_at(first);
     extra[4] = ld_bits(raw(l, kReadLogit), 0, dt(l, kReadLogit));
@@ -576,7 +592,7 @@ struct Step {
   }
 
   __device__ __forceinline__ void run_mix(int l, int q, int mg) {
-    const int first = blockIdx.x + at.team * gridDim.x, step = gridDim.x * at.teams;
+    const int first = at.block + at.team * at.blocks, step = at.blocks * at.teams;
     if (first >= a.mix.items) return;
     const int M = a.M, R = a.R, cols = a.mix.cols, groups = a.mix.groups;
     const bool on = mg < groups;
@@ -706,7 +722,43 @@ struct Step {
   }
 };
 
-// All blocks wait for one another, in two parts: a block arrives when its writes are done, and does what needs no other
+// How long the first block keeps the list open while n of `blocks` have started: until the wait has cost as much as going without
+// the others will (a layer takes some 20 us with all of them), and 10 us at least, which their start takes.
+__device__ __forceinline__ uint64_t patience_ns(int n, int blocks, int layers) {
+  return 10000 + (uint64_t)20000 * layers * (blocks - n) / n;
+}
+// Puts this block on the list of those that share the work.  False where the list was closed before (or, for want of an answer
+// within the limit, *gave_up); by one thread.
+__device__ bool join(Meeting *m, int layers, Place *at, int *gave_up) {
+  const unsigned mine = atomicAdd(&m->started, 1u);
+  if (mine & kClosed) return false;
+  const int grid = (int)gridDim.x;
+  unsigned n = 0;
+  const uint64_t t0 = umma::global_ns();
+  if (mine == 0) {
+#pragma unroll 1
+    do {
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(&m->started) : "memory");
+    } while ((int)n < grid && !umma::past_limit(t0, umma::global_ns(), patience_ns((int)n, grid, layers)));
+    n = atomicOr(&m->started, kClosed);
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&m->members), "r"(n) : "memory");
+  } else {
+#pragma unroll 1
+    for (;;) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(&m->members) : "memory");
+      if (n) break;
+      if (umma::past_limit(t0, umma::global_ns(), kWaitNs)) {
+        *gave_up = 1;
+        return false;
+      }
+    }
+  }
+  at->block = (int)mine;
+  at->blocks = (int)n;
+  return true;
+}
+
+// All blocks of the list wait for one another, in two parts: a block arrives when its writes are done, and does what needs no other
 // block in between.
 __device__ __forceinline__ void arrive(unsigned *counter) {
   __syncthreads();
@@ -738,13 +790,29 @@ __device__ __forceinline__ bool wait_for_all(const unsigned *counter, unsigned t
 template <int NT>
 __global__ void __launch_bounds__(kTeam * max_teams<NT>(), 1) decode_step_kernel(const __grid_constant__ StepArgs<kTabLayers> a) {
   extern __shared__ __align__(16) uint8_t smem[];
-  const Place at{(int)(threadIdx.x / kTeam), (int)(blockDim.x / kTeam), (int)(threadIdx.x % kTeam), (int)(threadIdx.x % 32),
-                 (int)(threadIdx.x % kTeam / 32)};
+  Place at{(int)(threadIdx.x / kTeam), (int)(blockDim.x / kTeam), (int)(threadIdx.x % kTeam), (int)(threadIdx.x % 32),
+           (int)(threadIdx.x % kTeam / 32), 0, 0};
+  int *const listed = reinterpret_cast<int *>(smem);
+  if (threadIdx.x == 0) {
+    int gave_up = 0;
+    Place mine{};
+    join(a.meeting, a.layers, &mine, &gave_up);
+    listed[0] = mine.block;
+    listed[1] = gave_up ? -1 : mine.blocks;
+  }
+  __syncthreads();
+  at.block = listed[0];
+  at.blocks = listed[1];
+  __syncthreads();
+  if (at.blocks == 0) return;
   const int q = at.tid % a.mix.quads, mg = at.tid / a.mix.quads;
   Step<NT, kTabLayers> x{a, at, smem};
-  bool ok = true;
-  unsigned target = a.met;
-  const int stages = 4 * a.layers;
+  bool ok = at.blocks > 0;
+  unsigned target = 0;
+  // dyn_proj's tiles take blocks in proportion (a block alone takes them all, and the others after them)
+  const int t2 = tiles_of(3 * a.H), t12 = t2 + tiles_of(2 * a.H * a.M);
+  x.blocks2 = max(1, min((at.blocks * t2 + t12 - 1) / t12, at.blocks - 1));
+  const int stages = ok ? 4 * a.layers : -1;
   // Stage -1 only requests what the first one needs.  Beside a barrier the teams' shares of the weights of a later product
   // and of the layer's old state go to L2 (a lane of the block's last warp for each team), so that no stage waits for HBM.
   const bool carrier = threadIdx.x >= blockDim.x - 32 && at.lane < at.teams;
@@ -753,9 +821,18 @@ __global__ void __launch_bounds__(kTeam * max_teams<NT>(), 1) decode_step_kernel
     const int kind = stage & 3, next = stage + 1, nl = next >> 2, nk = next & 3;
     if (stage >= 0) {
       if (kind == kMix) x.run_mix(stage >> 2, q, mg);
-      else x.run_product(stage >> 2, kind);
+      else {
+#pragma unroll 1
+        for (;;) {
+          x.run_product(stage >> 2, kind);
+          if (at.blocks > 1 || !x.second) break;
+          __syncthreads();   // (the activations in shared memory are written anew)
+          x.product(stage >> 2, kind, at.team, true);
+          if (x.tile0 < x.tiles) x.request(x.tile0, x.k_lo);
+        }
+      }
       if (next == stages) break;
-      arrive(a.counter);
+      arrive(&a.meeting->arrived);
     }
     if (nk == kMix) {
       x.request_state(nl, q, mg);
@@ -766,6 +843,7 @@ __global__ void __launch_bounds__(kTeam * max_teams<NT>(), 1) decode_step_kernel
       // in front of in_proj (not the first) out_proj's weights, in front of rw_proj the old state, then the next layer's
       // in_proj and rw_proj with dyn_proj; at the start rw_proj, dyn_proj and out_proj
       Step<NT, kTabLayers> y{a, at, smem};
+      y.blocks2 = x.blocks2;
       if (nk == kProj) y.state_to_l2(nl, at.lane);
       const int cl = nk == kIn ? nl : nl + 1;
 #pragma unroll 1
@@ -774,8 +852,8 @@ __global__ void __launch_bounds__(kTeam * max_teams<NT>(), 1) decode_step_kernel
         y.product_to_l2(cl, k, at.lane);
     }
     if (stage >= 0) {
-      target += gridDim.x;
-      if (!(ok = wait_for_all(a.counter, target))) break;
+      target += (unsigned)at.blocks;
+      if (!(ok = wait_for_all(&a.meeting->arrived, target))) break;
     }
   }
   if (!ok)   // a block did not come: NaN is what the caller sees
@@ -789,9 +867,10 @@ template <int NT, int KIND>
 __global__ void __launch_bounds__(kTeam, KIND == kMix ? 3 : NT <= 4 ? 2 : 1)
 decode_stage_kernel(const __grid_constant__ StepArgs<1> a) {
   extern __shared__ __align__(16) uint8_t smem[];
-  const Place at{0, 1, (int)threadIdx.x, (int)(threadIdx.x % 32), (int)(threadIdx.x / 32)};
+  const Place at{0, 1, (int)threadIdx.x, (int)(threadIdx.x % 32), (int)(threadIdx.x / 32), (int)blockIdx.x, (int)gridDim.x};
   grid_dep_launch();
   Step<NT, 1> x{a, at, smem};
+  x.blocks2 = a.blocks2;
   if constexpr (KIND == kMix) {
     const int q = at.tid % a.mix.quads, mg = at.tid / a.mix.quads;
     x.request_state(0, q, mg);
@@ -823,7 +902,7 @@ int mix_splits(int64_t B, int64_t H, int64_t R) {
 }
 
 struct Scratch {
-  size_t x, gate, x_conv, rw, dyn, vals, ss, hid, hid_w, hid_ss, counter, bytes;
+  size_t x, gate, x_conv, rw, dyn, vals, ss, hid, hid_w, hid_ss, meeting, bytes;
 };
 Scratch scratch_layout(int64_t B, int64_t d, int64_t di, int64_t H, int64_t M) {
   Scratch s{};
@@ -839,7 +918,7 @@ Scratch scratch_layout(int64_t B, int64_t d, int64_t di, int64_t H, int64_t M) {
   s.hid = take(2 * align256((size_t)B * d * 4));
   s.hid_w = take((size_t)B * d * 2);
   s.hid_ss = take((size_t)B * tiles_of((int)d) * 4);
-  s.counter = take(4);
+  s.meeting = take(sizeof(Meeting));
   s.bytes = off;
   return s;
 }
@@ -886,7 +965,7 @@ void fill_shape(StepArgs<LAYERS> &a, int nt, const Shape &p, char *ws, void *hid
   a.out = reinterpret_cast<__nv_bfloat16 *>(hidden_out);
   a.gate = fl(s.gate); a.rw = fl(s.rw); a.dyn = fl(s.dyn); a.ss = fl(s.ss); a.hid_ss = fl(s.hid_ss);
   a.hid[0] = fl(s.hid); a.hid[1] = fl(s.hid + align256((size_t)p.B * p.d * 4));
-  a.counter = reinterpret_cast<unsigned *>(ws + s.counter);
+  a.meeting = reinterpret_cast<Meeting *>(ws + s.meeting);
 }
 
 // SM count of the current device; calls `prepare` once per device.
@@ -913,7 +992,7 @@ cudaError_t all_smem(K kernel) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostSmem);
 }
 template <typename Arg>
-cudaError_t launch(void (*kernel)(const Arg), unsigned grid, int threads, size_t smem, cudaStream_t st, cudaLaunchAttributeID how,
+cudaError_t launch(void (*kernel)(const Arg), unsigned grid, int threads, size_t smem, cudaStream_t st, bool dependent,
                    const Arg &arg) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
@@ -921,11 +1000,10 @@ cudaError_t launch(void (*kernel)(const Arg), unsigned grid, int threads, size_t
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
-  attr[0].id = how;
-  if (how == cudaLaunchAttributeCooperative) attr[0].val.cooperative = 1;
-  else attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = dependent ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, arg);
 }
 int launched(cudaError_t e) {
@@ -954,7 +1032,7 @@ bool one_kernel_pays(int64_t B, cudaStream_t st) {
 
 template <int NT>
 int run_one_kernel(const uint64_t *ptrs, const float *nums, int64_t layers, void *hidden_out, char *ws, const Shape &p,
-                   cudaStream_t st, bool *too_large) {
+                   cudaStream_t st, const DecodeForm &how) {
   int sms = 0;
   const int rc = device_sms(&sms, [] { return all_smem(decode_step_kernel<NT>); });
   if (rc) return rc;
@@ -967,17 +1045,13 @@ int run_one_kernel(const uint64_t *ptrs, const float *nums, int64_t layers, void
     return lin > mix ? lin : mix;
   };
   while (teams > 1 && smem_of(teams) > kMostSmem) --teams;
-  // dyn_proj's tiles take blocks in proportion
-  const int64_t t1 = tiles_of((int)(2 * p.H * p.M)), t2 = tiles_of((int)(3 * p.H));
-  a.blocks2 = (int)ceil_div((int64_t)sms * t2, t1 + t2);
-  if (a.blocks2 > sms - 1) a.blocks2 = sms - 1;
+  const int grid = how.blocks > 0 ? how.blocks : sms;
   cudaError_t e = cudaSuccess;
   for (int64_t l0 = 0; l0 < layers && e == cudaSuccess; l0 += kTabLayers) {
     fill_table(a, ptrs, nums, layers, l0);
-    // (cooperative: the blocks wait for one another, so all of them have to run at the same time)
-    e = launch(decode_step_kernel<NT>, (unsigned)sms, kTeam * teams, smem_of(teams), st, cudaLaunchAttributeCooperative, a);
-    *too_large = l0 == 0 && e == cudaErrorCooperativeLaunchTooLarge;   // (a context with a share of the device)
-    a.met += (unsigned)(4 * a.layers - 1) * (unsigned)sms;
+    // (the first kernel clears it for the first launch)
+    if (l0) e = cudaMemsetAsync(a.meeting, 0, sizeof(Meeting), st);
+    if (e == cudaSuccess) e = launch(decode_step_kernel<NT>, (unsigned)grid, kTeam * teams, smem_of(teams), st, false, a);
   }
   return launched(e);
 }
@@ -1006,27 +1080,23 @@ int run_stages(const uint64_t *ptrs, const float *nums, int64_t layers, void *hi
     return (unsigned)(NT == 1 ? tiles : ceil_div(tiles, ceil_div(tiles, most)));
   };
   a.blocks2 = tiles_of((int)(3 * p.H));
-  constexpr cudaLaunchAttributeID kDep = cudaLaunchAttributeProgrammaticStreamSerialization;
   cudaError_t e = cudaSuccess;
   for (int64_t l = 0; l < layers && e == cudaSuccess; ++l) {
     fill_table(a, ptrs, nums, layers, l);
-    e = launch(decode_stage_kernel<NT, kIn>, blocks(2 * di), kTeam, smem, st, kDep, a);
-    if (e == cudaSuccess) e = launch(decode_stage_kernel<NT, kProj>, a.blocks2 + blocks(2 * p.H * p.M), kTeam, smem, st, kDep, a);
-    if (e == cudaSuccess) e = launch(decode_stage_kernel<NT, kMix>, (unsigned)a.mix.items, kTeam, a.mix_bytes, st, kDep, a);
-    if (e == cudaSuccess) e = launch(decode_stage_kernel<NT, kOut>, blocks(p.d), kTeam, smem, st, kDep, a);
+    e = launch(decode_stage_kernel<NT, kIn>, blocks(2 * di), kTeam, smem, st, true, a);
+    if (e == cudaSuccess) e = launch(decode_stage_kernel<NT, kProj>, a.blocks2 + blocks(2 * p.H * p.M), kTeam, smem, st, true, a);
+    if (e == cudaSuccess) e = launch(decode_stage_kernel<NT, kMix>, (unsigned)a.mix.items, kTeam, a.mix_bytes, st, true, a);
+    if (e == cudaSuccess) e = launch(decode_stage_kernel<NT, kOut>, blocks(p.d), kTeam, smem, st, true, a);
   }
   return launched(e);
 }
 
 template <int NT>
 int run_layers(const uint64_t *ptrs, const float *nums, int64_t layers, void *hidden_out, char *ws, const Shape &p,
-               cudaStream_t st) {
+               cudaStream_t st, const DecodeForm &how) {
   if constexpr (NT <= 4) {
-    if (one_kernel_pays(p.B, st)) {
-      bool too_large = false;
-      const int rc = run_one_kernel<NT>(ptrs, nums, layers, hidden_out, ws, p, st, &too_large);
-      if (!too_large) return rc;
-    }
+    if (how.form == DecodeForm::kOneKernel || (how.form == DecodeForm::kByRule && one_kernel_pays(p.B, st)))
+      return run_one_kernel<NT>(ptrs, nums, layers, hidden_out, ws, p, st, how);
   }
   return run_stages<NT>(ptrs, nums, layers, hidden_out, ws, p, st);
 }
@@ -1049,10 +1119,9 @@ extern "C" size_t fracssm_decode_layers_workspace_bytes(int64_t B, int64_t hidde
   return fracssm::scratch_layout(B, hidden, H * R, H, M).bytes;
 }
 
-extern "C" int fracssm_decode_layers(const uint64_t *layer_ptrs, const float *layer_nums, int64_t layers,
-                                     const void *hidden_in, void *hidden_out, void *workspace, size_t workspace_bytes,
-                                     int64_t B, int64_t hidden, int64_t H, int64_t R, int64_t M, int64_t K, void *stream) {
-  using namespace fracssm;
+int fracssm::decode_layers_launch(const uint64_t *layer_ptrs, const float *layer_nums, int64_t layers, const void *hidden_in,
+                                  void *hidden_out, void *workspace, size_t workspace_bytes, int64_t B, int64_t hidden,
+                                  int64_t H, int64_t R, int64_t M, int64_t K, void *stream, const DecodeForm &how) {
   if (layers < 1 || !layer_ptrs || !layer_nums || !hidden_in || !hidden_out || !workspace)
     return fail(FRACSSM_ERR_ARG, "decode_layers: null pointer or no layer");
   if (!fracssm_decode_layers_supported(B, hidden, H, R, M, K))
@@ -1077,12 +1146,19 @@ extern "C" int fracssm_decode_layers(const uint64_t *layer_ptrs, const float *la
       reinterpret_cast<const __nv_bfloat16 *>(hidden_in), reinterpret_cast<const void *>(layer_ptrs[kNormW]),
       layer_ptrs[kF32Mask] & 1 ? FRACSSM_F32 : FRACSSM_BF16, reinterpret_cast<float *>(ws + s.hid),
       reinterpret_cast<__nv_bfloat16 *>(ws + s.hid_w), reinterpret_cast<float *>(ws + s.hid_ss), (int)hidden,
-      reinterpret_cast<unsigned *>(ws + s.counter));
+      reinterpret_cast<Meeting *>(ws + s.meeting));
   const int rc = check_launch("decode_layers");
   if (rc) return rc;
   const Shape p{B, hidden, H, R, M};
-  if (B <= 8) return run_layers<1>(layer_ptrs, layer_nums, layers, hidden_out, ws, p, st);
-  if (B <= 16) return run_layers<2>(layer_ptrs, layer_nums, layers, hidden_out, ws, p, st);
-  if (B <= 32) return run_layers<4>(layer_ptrs, layer_nums, layers, hidden_out, ws, p, st);
-  return run_layers<8>(layer_ptrs, layer_nums, layers, hidden_out, ws, p, st);
+  if (B <= 8) return run_layers<1>(layer_ptrs, layer_nums, layers, hidden_out, ws, p, st, how);
+  if (B <= 16) return run_layers<2>(layer_ptrs, layer_nums, layers, hidden_out, ws, p, st, how);
+  if (B <= 32) return run_layers<4>(layer_ptrs, layer_nums, layers, hidden_out, ws, p, st, how);
+  return run_layers<8>(layer_ptrs, layer_nums, layers, hidden_out, ws, p, st, how);
+}
+
+extern "C" int fracssm_decode_layers(const uint64_t *layer_ptrs, const float *layer_nums, int64_t layers,
+                                     const void *hidden_in, void *hidden_out, void *workspace, size_t workspace_bytes,
+                                     int64_t B, int64_t hidden, int64_t H, int64_t R, int64_t M, int64_t K, void *stream) {
+  return fracssm::decode_layers_launch(layer_ptrs, layer_nums, layers, hidden_in, hidden_out, workspace, workspace_bytes, B,
+                                       hidden, H, R, M, K, stream, fracssm::DecodeForm{});
 }

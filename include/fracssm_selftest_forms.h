@@ -1,0 +1,25 @@
+/*
+ * fracssm_selftest_forms.h -- further test-only entry points of libfracssm_selftest.so (see fracssm_selftest.h): a product
+ * call in a form that its own rule would not take here.  None has a counterpart in quorbix/frac-ssm-kernels.
+ */
+#ifndef FRACSSM_SELFTEST_FORMS_H
+#define FRACSSM_SELFTEST_FORMS_H
+
+#include "fracssm.h"
+
+#ifdef __cplusplus
+extern "C" {
+#endif
+
+/*
+ * fracssm_decode_layers as a kernel per stage (one_kernel 0) or as one kernel (up to 32 sequences) of `blocks` blocks, 0: one
+ * per SM.  The results are the same bits in every form and with every number of blocks.
+ */
+int fracssm_selftest_decode_layers(const uint64_t *layer_ptrs, const float *layer_nums, int64_t layers, const void *hidden_in,
+                                   void *hidden_out, void *workspace, size_t workspace_bytes, int64_t B, int64_t hidden,
+                                   int64_t H, int64_t R, int64_t M, int64_t K, void *stream, int one_kernel, int blocks);
+
+#ifdef __cplusplus
+}
+#endif
+#endif /* FRACSSM_SELFTEST_FORMS_H */

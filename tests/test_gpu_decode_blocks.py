@@ -1,0 +1,92 @@
+"""The one-kernel decode step (csrc/decode_layers.cu) works with the blocks that are there: any number of them gives the bits of
+the kernel-per-stage form, and SMs that other streams hold for long stop nothing."""
+
+import ctypes
+
+import pytest
+import torch
+
+from tests.helpers import selftest_lib
+from tests.test_gpu_decode_layers import _flat, _model, _past
+
+pytestmark = pytest.mark.gpu
+
+
+class _Form:
+    """Calls of fracssm_decode_layers go to the self-test entry with these last arguments."""
+
+    def __init__(self, *last):
+        self.last = last
+
+    def __enter__(self):
+        from frac_ssm_b200 import _cabi as C
+        self.lib = C.lib()
+        self.fn, form = self.lib.fracssm_decode_layers, selftest_lib().fracssm_selftest_decode_layers
+        form.argtypes, form.restype = [*self.fn.argtypes, ctypes.c_int, ctypes.c_int], ctypes.c_int
+        self.lib.fracssm_decode_layers = lambda *a: form(*a, *self.last)
+
+    def __exit__(self, *exc):
+        self.lib.fracssm_decode_layers = self.fn
+
+
+# one block; two, of which one takes dyn_proj; fewer and more blocks than tiles or items; more blocks than run at a time, whose
+# last ones find the list closed; groups of 8, 16 and 32 sequences; two launches of the one-kernel form
+@pytest.mark.parametrize("hidden,H,M,B,layers", [(256, 4, 128, 1, 3), (768, 12, 8, 9, 2), (768, 24, 128, 17, 2), (320, 5, 20, 29, 2), (64, 2, 8, 32, 35)])
+def test_any_number_of_blocks_gives_the_same_bits(hidden, H, M, B, layers):
+    model = _model(hidden, H, M, layers).to(torch.bfloat16)
+    ids = torch.randint(1, 50, (B, 1), generator=torch.Generator().manual_seed(B)).cuda()
+    past = _past(model, B, torch.bfloat16)
+
+    def step():
+        return [t.clone() for t in _flat(model(ids, past_key_values=past, use_cache=True))]
+    with torch.no_grad():
+        with _Form(0, 0):
+            want = step()
+        for blocks in (1, 2, 3, 37, 147, 0, 300):
+            with _Form(1, blocks):
+                assert all(torch.equal(a, b) for a, b in zip(step(), want)), blocks
+
+
+@pytest.mark.parametrize("B", [1, 20])
+def test_a_step_beside_kernels_that_hold_sms(B):
+    """Eight kernels of other streams keep eight SMs for half a second: the step neither waits for them nor goes wrong."""
+    model = _model(768, 24, 128, 4).to(torch.bfloat16)
+    ids = torch.randint(1, 50, (B, 1)).cuda()
+    past = _past(model, B, torch.bfloat16)
+    with torch.no_grad():
+        want = [t.clone() for t in _flat(model(ids, past_key_values=past, use_cache=True))]
+        torch.cuda.synchronize()
+        held = []
+        for _ in range(8):
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                torch.cuda._sleep(1_000_000_000)
+                held.append(torch.cuda.Event())
+                held[-1].record()
+        got = _flat(model(ids, past_key_values=past, use_cache=True))
+        torch.cuda.current_stream().synchronize()
+        assert not any(e.query() for e in held)
+        torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("B", [17, 20, 32])
+def test_captured_steps_give_the_same_bits(B):
+    model = _model(768, 24, 128, 3).to(torch.bfloat16)
+    ids = torch.randint(1, 50, (B, 1)).cuda()
+    past = _past(model, B, torch.bfloat16)
+    with torch.no_grad():
+        plain = [t.clone() for t in _flat(model(ids, past_key_values=past, use_cache=True))]
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            captured = _flat(model(ids, past_key_values=past, use_cache=True))
+        for _ in range(2):
+            graph.replay()
+        torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(plain, captured))
+
+
+def test_the_forms_entry_is_part_of_the_test_library_alone():
+    from frac_ssm_b200 import _cabi as C
+    assert not hasattr(ctypes.CDLL(C.lib_path()), "fracssm_selftest_decode_layers")
