@@ -801,8 +801,10 @@ __global__ void __launch_bounds__(kTeam * max_teams<NT>(), 1) decode_step_kernel
     listed[1] = gave_up ? -1 : mine.blocks;
   }
   __syncthreads();
-  at.block = listed[0];
-  at.blocks = listed[1];
+  // (through a reduction, whose result the compiler knows to be the same in the whole warp: 24 layers at one sequence 496 us
+  // against 498, at 32 sequences 879 against 883; as blockIdx and gridDim they were 495 and 869)
+  at.block = __reduce_max_sync(0xffffffffu, listed[0]);
+  at.blocks = __reduce_max_sync(0xffffffffu, listed[1]);
   __syncthreads();
   if (at.blocks == 0) return;
   const int q = at.tid % a.mix.quads, mg = at.tid / a.mix.quads;
