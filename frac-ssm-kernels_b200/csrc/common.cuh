@@ -81,6 +81,8 @@ struct DecodeForm {
   enum { kByRule = 0, kOneKernel = 1, kStages = 2 };
   int form = kByRule;      // (kOneKernel covers up to 32 sequences)
   int blocks = 0;          // of the one-kernel form; 0: one per SM
+  unsigned long long wait_ns = tile_default_wait_ns();
+  int lost = 0;            // n > 0: block 0 waits at the n-th barrier for arrivals that are not to come
 };
 int decode_layers_launch(const uint64_t *layer_ptrs, const float *layer_nums, int64_t layers, const void *hidden_in,
                          void *hidden_out, void *workspace, size_t workspace_bytes, int64_t B, int64_t hidden, int64_t H,

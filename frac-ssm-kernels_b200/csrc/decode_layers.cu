@@ -135,8 +135,11 @@ struct Meeting {
   unsigned arrived;    // at the barriers, over the whole launch
   unsigned started;    // blocks that asked to be on the list; kClosed once it is closed
   unsigned members;    // blocks on the closed list, 0 before
-  unsigned spare;
+  unsigned left;       // blocks at their end
+  unsigned failed;     // set once a wait has run out, for the whole call
+  unsigned spare[3];
 };
+constexpr size_t kPerLaunch = 16;      // bytes of it that every launch starts with as zeros: all but `failed`
 constexpr unsigned kClosed = 0x80000000u;
 
 // The embedding times the first norm's weight, and its sums of squares (one part per row); clears what the one-kernel form's
@@ -167,7 +170,6 @@ decode_first_kernel(const __nv_bfloat16 *h, const void *w, int w_dt, float *h_f3
 }
 
 constexpr int kTabLayers = 32;       // layers of one launch of the one-kernel form
-constexpr unsigned long long kWaitNs = 2000000000ull;   // limit of a wait for the other blocks
 struct LayerTab {
   uint64_t p[kLayerPtrs];
   float f[kLayerNums];
@@ -184,6 +186,8 @@ struct StepArgs {
   __nv_bfloat16 *x, *x_conv, *vals, *hid_w, *out;
   float *gate, *rw, *dyn, *ss, *hid[2], *hid_ss;
   Meeting *meeting;
+  unsigned long long wait_ns;        // limit of a wait for the other blocks
+  int lost;                          // self-test: at this barrier, counted from 1, block 0 waits for the next one's arrivals too
   uint32_t act_bytes, red_bytes, mix_bytes;
 };
 
@@ -727,11 +731,11 @@ struct Step {
 __device__ __forceinline__ uint64_t patience_ns(int n, int blocks, int layers) {
   return 10000 + (uint64_t)20000 * layers * (blocks - n) / n;
 }
-// Puts this block on the list of those that share the work.  False where the list was closed before (or, for want of an answer
-// within the limit, *gave_up); by one thread.
-__device__ bool join(Meeting *m, int layers, Place *at, int *gave_up) {
+// Puts this block on the list of those that share the work, by one thread.  Nothing is set where the list was closed before; for
+// want of an answer within the limit *gave_up is.
+__device__ void join(Meeting *m, int layers, uint64_t wait_ns, Place *at, int *gave_up) {
   const unsigned mine = atomicAdd(&m->started, 1u);
-  if (mine & kClosed) return false;
+  if (mine & kClosed) return;
   const int grid = (int)gridDim.x;
   unsigned n = 0;
   const uint64_t t0 = umma::global_ns();
@@ -747,15 +751,14 @@ __device__ bool join(Meeting *m, int layers, Place *at, int *gave_up) {
     for (;;) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(&m->members) : "memory");
       if (n) break;
-      if (umma::past_limit(t0, umma::global_ns(), kWaitNs)) {
+      if (umma::past_limit(t0, umma::global_ns(), wait_ns)) {
         *gave_up = 1;
-        return false;
+        return;
       }
     }
   }
   at->block = (int)mine;
   at->blocks = (int)n;
-  return true;
 }
 
 // All blocks of the list wait for one another, in two parts: a block arrives when its writes are done, and does what needs no other
@@ -768,7 +771,7 @@ __device__ __forceinline__ void arrive(unsigned *counter) {
   }
 }
 // False when the limit ran out, for every thread of the block.
-__device__ __forceinline__ bool wait_for_all(const unsigned *counter, unsigned target) {
+__device__ __forceinline__ bool wait_for_all(const unsigned *counter, unsigned target, uint64_t wait_ns) {
   int gave_up = 0;
   if (threadIdx.x == 0) {
     uint64_t t0 = 0;
@@ -778,13 +781,30 @@ __device__ __forceinline__ bool wait_for_all(const unsigned *counter, unsigned t
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
       if (static_cast<int>(seen - target) >= 0) break;
       if (spins == 64) t0 = umma::global_ns();
-      if (spins > 64 && umma::past_limit(t0, umma::global_ns(), kWaitNs)) {
+      if (spins > 64 && umma::past_limit(t0, umma::global_ns(), wait_ns)) {
         gave_up = 1;
         break;
       }
     }
   }
   return __syncthreads_or(gave_up) == 0;
+}
+
+// What a step leaves where a wait ran out: NaN throughout, by one block.
+template <typename T>
+__device__ __noinline__ void fill(T *p, int64_t n, T v) {
+  for (int64_t i = threadIdx.x; p && i < n; i += blockDim.x) p[i] = v;
+}
+template <int LAYERS>
+__device__ void mark_failed(const StepArgs<LAYERS> &a) {
+  const unsigned short nan16 = 0x7fc0;
+  const int64_t di = (int64_t)a.H * a.R;
+  if (!a.after_w) fill(reinterpret_cast<unsigned short *>(a.out), (int64_t)a.B * a.d, nan16);
+#pragma unroll 1
+  for (int l = 0; l < a.layers; ++l) {
+    fill(reinterpret_cast<float *>(a.tab[l].p[kNewState]), a.B * di * a.M, __int_as_float(0x7fc00000));
+    fill(reinterpret_cast<unsigned short *>(a.tab[l].p[kNewConv]), a.B * di * 3, nan16);
+  }
 }
 
 template <int NT>
@@ -796,7 +816,7 @@ __global__ void __launch_bounds__(kTeam * max_teams<NT>(), 1) decode_step_kernel
   if (threadIdx.x == 0) {
     int gave_up = 0;
     Place mine{};
-    join(a.meeting, a.layers, &mine, &gave_up);
+    join(a.meeting, a.layers, a.wait_ns, &mine, &gave_up);
     listed[0] = mine.block;
     listed[1] = gave_up ? -1 : mine.blocks;
   }
@@ -806,15 +826,14 @@ __global__ void __launch_bounds__(kTeam * max_teams<NT>(), 1) decode_step_kernel
   at.block = __reduce_max_sync(0xffffffffu, listed[0]);
   at.blocks = __reduce_max_sync(0xffffffffu, listed[1]);
   __syncthreads();
-  if (at.blocks == 0) return;
   const int q = at.tid % a.mix.quads, mg = at.tid / a.mix.quads;
   Step<NT, kTabLayers> x{a, at, smem};
-  bool ok = at.blocks > 0;
+  bool ok = at.blocks >= 0;
   unsigned target = 0;
   // dyn_proj's tiles take blocks in proportion (a block alone takes them all, and the others after them)
   const int t2 = tiles_of(3 * a.H), t12 = t2 + tiles_of(2 * a.H * a.M);
   x.blocks2 = max(1, min((at.blocks * t2 + t12 - 1) / t12, at.blocks - 1));
-  const int stages = ok ? 4 * a.layers : -1;
+  const int stages = at.blocks > 0 ? 4 * a.layers : -1;   // (none for a block that is not on the list)
   // Stage -1 only requests what the first one needs.  Beside a barrier the teams' shares of the weights of a later product
   // and of the layer's old state go to L2 (a lane of the block's last warp for each team), so that no stage waits for HBM.
   const bool carrier = threadIdx.x >= blockDim.x - 32 && at.lane < at.teams;
@@ -855,12 +874,21 @@ __global__ void __launch_bounds__(kTeam * max_teams<NT>(), 1) decode_step_kernel
     }
     if (stage >= 0) {
       target += (unsigned)at.blocks;
-      if (!(ok = wait_for_all(&a.meeting->arrived, target))) break;
+      if (!(ok = wait_for_all(&a.meeting->arrived, target + (at.block == 0 && next == a.lost ? at.blocks : 0), a.wait_ns))) break;
     }
   }
-  if (!ok)   // a block did not come: NaN is what the caller sees
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (int64_t)a.B * a.d; i += (int64_t)gridDim.x * blockDim.x)
-      a.out[i] = __float2bfloat16_rn(__int_as_float(0x7fc00000));
+  // A block that gave up says so, and whoever leaves last, when nobody writes any more, sees it.
+  __syncthreads();
+  int bad = 0;
+  if (threadIdx.x == 0) {
+    if (!ok) atomicExch(&a.meeting->failed, 1u);
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    if (atomicAdd(&a.meeting->left, 1u) + 1 == gridDim.x) {
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      bad = atomicAdd(&a.meeting->failed, 0u) != 0;
+    }
+  }
+  if (__syncthreads_or(bad)) mark_failed(a);
 }
 
 // One stage of one layer as a kernel: a block is a team.  (Two blocks per SM for the products up to 32 sequences: with three, and
@@ -910,6 +938,7 @@ Scratch scratch_layout(int64_t B, int64_t d, int64_t di, int64_t H, int64_t M) {
   Scratch s{};
   size_t off = 0;
   auto take = [&](size_t n) { const size_t at = off; off += align256(n); return at; };
+  s.meeting = take(sizeof(Meeting));   // (at the start: fracssm_decode_layers_status)
   s.x = take((size_t)B * di * 2);
   s.gate = take((size_t)B * di * 4);
   s.x_conv = take((size_t)B * di * 2);
@@ -920,7 +949,6 @@ Scratch scratch_layout(int64_t B, int64_t d, int64_t di, int64_t H, int64_t M) {
   s.hid = take(2 * align256((size_t)B * d * 4));
   s.hid_w = take((size_t)B * d * 2);
   s.hid_ss = take((size_t)B * tiles_of((int)d) * 4);
-  s.meeting = take(sizeof(Meeting));
   s.bytes = off;
   return s;
 }
@@ -1048,11 +1076,13 @@ int run_one_kernel(const uint64_t *ptrs, const float *nums, int64_t layers, void
   };
   while (teams > 1 && smem_of(teams) > kMostSmem) --teams;
   const int grid = how.blocks > 0 ? how.blocks : sms;
+  a.wait_ns = how.wait_ns;
   cudaError_t e = cudaSuccess;
   for (int64_t l0 = 0; l0 < layers && e == cudaSuccess; l0 += kTabLayers) {
     fill_table(a, ptrs, nums, layers, l0);
     // (the first kernel clears it for the first launch)
-    if (l0) e = cudaMemsetAsync(a.meeting, 0, sizeof(Meeting), st);
+    if (l0) e = cudaMemsetAsync(a.meeting, 0, kPerLaunch, st);
+    a.lost = l0 ? 0 : how.lost;
     if (e == cudaSuccess) e = launch(decode_step_kernel<NT>, (unsigned)grid, kTeam * teams, smem_of(teams), st, false, a);
   }
   return launched(e);
@@ -1163,4 +1193,15 @@ extern "C" int fracssm_decode_layers(const uint64_t *layer_ptrs, const float *la
                                      int64_t B, int64_t hidden, int64_t H, int64_t R, int64_t M, int64_t K, void *stream) {
   return fracssm::decode_layers_launch(layer_ptrs, layer_nums, layers, hidden_in, hidden_out, workspace, workspace_bytes, B,
                                        hidden, H, R, M, K, stream, fracssm::DecodeForm{});
+}
+
+extern "C" int fracssm_decode_layers_status(const void *workspace, void *stream) {
+  using namespace fracssm;
+  if (!workspace) return fail(FRACSSM_ERR_ARG, "decode_layers_status: null workspace");
+  Meeting m{};
+  cudaError_t e = cudaMemcpyAsync(&m, workspace, sizeof(m), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
+  if (e != cudaSuccess) return fail(FRACSSM_ERR_CUDA, "decode_layers_status: %s", cudaGetErrorString(e));
+  if (m.failed) return fail(FRACSSM_ERR_WAIT, "decode step: a device-side wait ran out");
+  return FRACSSM_OK;
 }

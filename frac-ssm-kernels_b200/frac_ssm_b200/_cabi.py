@@ -68,6 +68,7 @@ _SIGNATURES = {
     "fracssm_decode_layers_supported": (ci, [i64, i64, i64, i64, i64, i64]),
     "fracssm_decode_layers_workspace_bytes": (sz, [i64, i64, i64, i64, i64]),
     "fracssm_decode_layers": (ci, [vp, vp, i64, vp, vp, vp, sz, i64, i64, i64, i64, i64, i64, vp]),
+    "fracssm_decode_layers_status": (ci, [vp, vp]),
     "fracssm_add_rmsnorm": (ci, [vp, vp, vp, ci, cf, vp, vp, i64, i64, vp]),
     "fracssm_prefill_conv": (ci, [vp, i64, vp, vp, vp, vp, vp, vp, i64, i64, i64, i64, i64, vp]),
     "fracssm_prefill_conv_dyn": (ci, [vp, i64, vp, vp, vp, vp, vp, vp, vp, vp, i64, i64, i64, i64, i64, i64, vp]),

@@ -357,6 +357,12 @@ size_t fracssm_decode_layers_workspace_bytes(int64_t B, int64_t hidden, int64_t 
 int fracssm_decode_layers(const uint64_t *layer_ptrs, const float *layer_nums, int64_t layers,
                           const void *hidden_in, void *hidden_out, void *workspace, size_t workspace_bytes,
                           int64_t B, int64_t hidden, int64_t H, int64_t R, int64_t M, int64_t K, void *stream);
+/*
+ * Reads back the error word of the last fracssm_decode_layers that used `workspace` (this call synchronises the stream).
+ * Returns 0, or FRACSSM_ERR_WAIT when a bounded wait of a block for the others ran out: hidden_out, the new states and the
+ * new conv states are NaN then.  No counterpart in the reference.
+ */
+int fracssm_decode_layers_status(const void *workspace, void *stream);
 
 /*
  * The steps of a bfloat16 mixer's prefill around its library GEMMs, few calls per layer.

@@ -18,6 +18,15 @@ extern "C" {
 int fracssm_selftest_decode_layers(const uint64_t *layer_ptrs, const float *layer_nums, int64_t layers, const void *hidden_in,
                                    void *hidden_out, void *workspace, size_t workspace_bytes, int64_t B, int64_t hidden,
                                    int64_t H, int64_t R, int64_t M, int64_t K, void *stream, int one_kernel, int blocks);
+/*
+ * The one-kernel form whose block 0 waits at the `barrier`-th meeting of the blocks (4 a layer, less one) for the arrivals
+ * of the next one, which needs its own.  After wait_ns nanoseconds it gives up, the kernel returns by itself, fracssm_decode_layers_status reports
+ * FRACSSM_ERR_WAIT and all outputs are NaN, also where the other blocks have finished.
+ */
+int fracssm_selftest_decode_wait_limit(const uint64_t *layer_ptrs, const float *layer_nums, int64_t layers,
+                                       const void *hidden_in, void *hidden_out, void *workspace, size_t workspace_bytes,
+                                       int64_t B, int64_t hidden, int64_t H, int64_t R, int64_t M, int64_t K, void *stream,
+                                       int barrier, unsigned long long wait_ns);
 
 #ifdef __cplusplus
 }

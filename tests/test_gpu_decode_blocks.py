@@ -2,6 +2,7 @@
 the kernel-per-stage form, and SMs that other streams hold for long stop nothing."""
 
 import ctypes
+import time
 
 import pytest
 import torch
@@ -11,19 +12,28 @@ from tests.test_gpu_decode_layers import _flat, _model, _past
 
 pytestmark = pytest.mark.gpu
 
+ERR_WAIT = 4
+
 
 class _Form:
-    """Calls of fracssm_decode_layers go to the self-test entry with these last arguments."""
+    """Calls of fracssm_decode_layers go to a self-test entry with these last arguments; status: what its status call said."""
 
-    def __init__(self, *last):
-        self.last = last
+    def __init__(self, *last, entry="decode_layers", types=(ctypes.c_int, ctypes.c_int)):
+        self.last, self.name, self.types, self.status = last, "fracssm_selftest_" + entry, types, None
 
     def __enter__(self):
         from frac_ssm_b200 import _cabi as C
-        self.lib = C.lib()
-        self.fn, form = self.lib.fracssm_decode_layers, selftest_lib().fracssm_selftest_decode_layers
-        form.argtypes, form.restype = [*self.fn.argtypes, ctypes.c_int, ctypes.c_int], ctypes.c_int
-        self.lib.fracssm_decode_layers = lambda *a: form(*a, *self.last)
+        self.lib, test = C.lib(), selftest_lib()
+        self.fn, form = self.lib.fracssm_decode_layers, getattr(test, self.name)
+        form.argtypes, form.restype = [*self.fn.argtypes, *self.types], ctypes.c_int
+        test.fracssm_decode_layers_status.argtypes = [ctypes.c_void_p, ctypes.c_void_p]
+
+        def call(*a):
+            rc = form(*a, *self.last)
+            self.status = test.fracssm_decode_layers_status(a[5], a[13])      # synchronises
+            return rc
+        self.lib.fracssm_decode_layers = call
+        return self
 
     def __exit__(self, *exc):
         self.lib.fracssm_decode_layers = self.fn
@@ -43,8 +53,9 @@ def test_any_number_of_blocks_gives_the_same_bits(hidden, H, M, B, layers):
         with _Form(0, 0):
             want = step()
         for blocks in (1, 2, 3, 37, 147, 0, 300):
-            with _Form(1, blocks):
+            with _Form(1, blocks) as form:
                 assert all(torch.equal(a, b) for a, b in zip(step(), want)), blocks
+            assert form.status == 0
 
 
 @pytest.mark.parametrize("B", [1, 20])
@@ -87,6 +98,25 @@ def test_captured_steps_give_the_same_bits(B):
     assert all(torch.equal(a, b) for a, b in zip(plain, captured))
 
 
-def test_the_forms_entry_is_part_of_the_test_library_alone():
+# the first barrier, after which the others wait in vain too; the last one, after which they finish; one of a first launch of two
+@pytest.mark.parametrize("B,layers,barrier", [(1, 2, 1), (1, 2, 7), (20, 2, 7), (3, 35, 127), (3, 35, 60)])
+def test_a_wait_that_runs_out_marks_everything(B, layers, barrier):
+    """One block waits for an arrival that is not to come, for two milliseconds at most."""
+    model = _model(64, 2, 8, layers).to(torch.bfloat16)
+    ids = torch.randint(1, 50, (B, 1)).cuda()
+    past = _past(model, B, torch.bfloat16)
+    with torch.no_grad():
+        want = [t.clone() for t in _flat(model(ids, past_key_values=past, use_cache=True))]
+        t0 = time.time()
+        with _Form(barrier, 2_000_000, entry="decode_wait_limit", types=(ctypes.c_int, ctypes.c_uint64)) as form:
+            got = _flat(model(ids, past_key_values=past, use_cache=True))
+        assert time.time() - t0 < 5.0 and form.status == ERR_WAIT
+        assert all(torch.isnan(t).all() for t in got)
+        again = _flat(model(ids, past_key_values=past, use_cache=True))      # the context is usable as before
+    assert all(torch.equal(a, b) for a, b in zip(again, want))
+
+
+def test_the_entries_are_part_of_the_test_library_alone():
     from frac_ssm_b200 import _cabi as C
-    assert not hasattr(ctypes.CDLL(C.lib_path()), "fracssm_selftest_decode_layers")
+    product = ctypes.CDLL(C.lib_path())
+    assert not any(hasattr(product, "fracssm_selftest_" + n) for n in ("decode_layers", "decode_wait_limit"))
