@@ -1042,16 +1042,25 @@ int launched(cudaError_t e) {
   return fail(FRACSSM_ERR_CUDA, "decode_layers: %s", cudaGetErrorString(e));
 }
 
-// Where one kernel is the form to take.  24 layers as the whole model call, ms, a kernel per stage / one kernel:
-//                                sequences   1             8             12            32            64
-//   hidden 768, 128 modes   plain call   0.69 / 0.51   0.69 / 0.55   0.67 / 0.59   1.06 / 0.88   1.57 / 1.75
-//                           captured     0.39 / 0.49   0.44 / 0.53   0.50 / 0.57   1.02 / 0.86   1.52 / 1.74
-//   FracConfig()            plain call   0.68 / 0.47   0.69 / 0.48   0.68 / 0.49   0.69 / 0.58   0.86 / 1.06
-//                           captured     0.30 / 0.38   0.31 / 0.42   0.37 / 0.44   0.52 / 0.56   0.81 / 1.04
-// (a plain call of the kernels waits for the host up to some 20 sequences; a captured one has no launches to save.)
-bool one_kernel_pays(int64_t B, cudaStream_t st) {
-  if (B > 32) return false;
-  if (B > 16) return true;
+// Where one kernel is the form to take.  24 layers as the whole model call, us, a kernel per stage / one kernel:
+//                                sequences   1           8          12          16          17          20          32          64
+//   hidden 768, 128 modes   plain call   696 / 503   692 / 543   720 / 592   692 / 628   889 / 766   969 / 786  1055 / 880   1570 / 1750
+//                           captured     394 / 495   440 / 532   496 / 574   527 / 620   846 / 743   935 / 772  1031 / 866   1520 / 1740
+//   FracConfig()            plain call   693 / 451   703 / 461   712 / 460   696 / 460   704 / 551   711 / 540   707 / 574    860 / 1060
+//                           captured     297 / 394   310 / 421   370 / 451   356 / 429   467 / 531   466 / 519   515 / 561    810 / 1040
+// (a plain call of the kernels waits for the host up to some 20 sequences; a captured one has no launches to save.)  Between 17
+// and 32 sequences it depends on the model which of the captured forms is the faster; MB of weights a layer, us at 20 sequences:
+//   hidden  768, 24 heads, modes 16   9.7  574 / 566     hidden 768, 12 heads, modes  32   9.5  482 / 527
+//                                32  12.0  590 / 568                                  64  11.9  531 / 554
+//                                64  16.7  730 / 625                                 128  16.6  749 / 662
+//   hidden 1536, 24 heads, modes  8  31.1  992 / 896     hidden 512, 16 heads, modes 128  11.6  504 / 585
+//   hidden 1024, 32 heads, modes 32  21.4  832 / 761     (32 sequences)
+//   hidden 1024, 16 heads, modes 64  21.2  614 / 675     the one of these on the slower side of the line
+constexpr int64_t kCapturedWeights = 12000000;      // bytes
+bool one_kernel_pays(const Shape &p, cudaStream_t st) {
+  if (p.B > 32) return false;
+  const int64_t di = p.H * p.R;
+  if (p.B > 16 && 2 * di * (3 * p.d + 2 * p.H * p.M + 3 * p.H) > kCapturedWeights) return true;
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
     cudaGetLastError();   // (the legacy stream while another is captured: the launches themselves say so)
@@ -1127,7 +1136,7 @@ template <int NT>
 int run_layers(const uint64_t *ptrs, const float *nums, int64_t layers, void *hidden_out, char *ws, const Shape &p,
                cudaStream_t st, const DecodeForm &how) {
   if constexpr (NT <= 4) {
-    if (how.form == DecodeForm::kOneKernel || (how.form == DecodeForm::kByRule && one_kernel_pays(p.B, st)))
+    if (how.form == DecodeForm::kOneKernel || (how.form == DecodeForm::kByRule && one_kernel_pays(p, st)))
       return run_one_kernel<NT>(ptrs, nums, layers, hidden_out, ws, p, st, how);
   }
   return run_stages<NT>(ptrs, nums, layers, hidden_out, ws, p, st);

@@ -81,17 +81,23 @@ def test_a_step_beside_kernels_that_hold_sms(B):
     assert all(torch.equal(a, b) for a, b in zip(got, want))
 
 
-@pytest.mark.parametrize("B", [17, 20, 32])
-def test_captured_steps_give_the_same_bits(B):
-    model = _model(768, 24, 128, 3).to(torch.bfloat16)
+# which form a captured call takes: 17 to 32 sequences go by the weights of a layer, 12 MB and more are one kernel
+@pytest.mark.parametrize("H,M,B,one", [(24, 128, 17, True), (24, 128, 20, True), (24, 128, 32, True), (24, 128, 16, False), (12, 8, 17, False),
+                                       (12, 8, 32, False), (12, 64, 20, False), (24, 33, 20, True)])
+def test_captured_steps_give_the_same_bits(H, M, B, one):
+    model = _model(768, H, M, 3).to(torch.bfloat16)
     ids = torch.randint(1, 50, (B, 1)).cuda()
     past = _past(model, B, torch.bfloat16)
     with torch.no_grad():
         plain = [t.clone() for t in _flat(model(ids, past_key_values=past, use_cache=True))]
         torch.cuda.synchronize()
-        graph = torch.cuda.CUDAGraph()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
         with torch.cuda.graph(graph):
             captured = _flat(model(ids, past_key_values=past, use_cache=True))
+        nodes = ctypes.c_size_t()
+        handle = ctypes.c_void_p(graph.raw_cuda_graph())
+        assert ctypes.CDLL("libcudart.so.12").cudaGraphGetNodes(handle, None, ctypes.byref(nodes)) == 0
+        assert (nodes.value < 4 * 3) == one
         for _ in range(2):
             graph.replay()
         torch.cuda.synchronize()
