@@ -45,9 +45,16 @@ constexpr int kCols = 4;       // columns of u per thread
 constexpr int kModes = 8;      // modes per thread
 constexpr int kMaxBlockCols = 128;
 constexpr int kTokPad = 4;     // floats between a token's values and the next token's in the summary
-// Least decay behind a token that the summary multiplies kappa with: a product of 7 decays may underflow, and zero times an
-// infinity of u would be NaN where the recurrence has the infinity.  (Contributions below 1e-37 |kappa u| are lost in any sum.)
+// Least decay over several tokens, of a group, a segment or a share of the carry: a product of 7 decays of 1e-6 underflows, and
+// zero times an infinity (of u, or of the state) would be NaN where the recurrence, whose single decays are no less than 1e-6,
+// keeps the infinity.  What has decayed further stays at 1e-37 of its size, 1e-37 |kappa u| too much in a state.
 constexpr float kLeastDecay = 1e-37f;
+__device__ __forceinline__ float decay_over(float a, float b) { return fmaxf(a * b, kLeastDecay); }
+// kappa and the decay behind its token: for the same reason not zero unless kappa is (or below 2e-15)
+__device__ __forceinline__ float kappa_behind(float kappa, float behind) {
+  const float y = kappa * fmaxf(behind, kLeastDecay);
+  return y != 0.f ? y : kappa * 0x1p-100f;
+}
 
 struct Rows {                  // one input: base and strides in bytes
   const char *p;
@@ -208,8 +215,8 @@ few_scan_kernel(const FewArgs a) {
           if (rt + o < kGroup) v *= y;
         }
         const float behind = __shfl_down_sync(0xffffffffu, v, 1, kGroup);
-        k[x] *= rt + 1 < kGroup ? fmaxf(behind, kLeastDecay) : 1.f;
-        r[x] = v;
+        if (rt + 1 < kGroup) k[x] = kappa_behind(k[x], behind);
+        r[x] = fmaxf(v, kLeastDecay);
       }
       if (owns) {
         *reinterpret_cast<float4 *>(d + kOffK) = make_float4(k[0], k[1], k[2], k[3]);
@@ -266,8 +273,8 @@ few_scan_kernel(const FewArgs a) {
       }
 #pragma unroll
       for (int t = 0; t + 1 < kGroup; ++t)
-        if (t < n) wide[t * tok_floats + kOffK + m] *= fmaxf(r[t + 1], kLeastDecay);
-      wide[m] = r[0];
+        if (t < n) wide[t * tok_floats + kOffK + m] = kappa_behind(wide[t * tok_floats + kOffK + m], r[t + 1]);
+      wide[m] = fmaxf(r[0], kLeastDecay);
     }
   };
   if (a.wide_loads) request(0);
@@ -474,7 +481,11 @@ few_scan_kernel(const FewArgs a) {
     if (owner && cl == 0 && blockIdx.y == 0) {
       f2 *dst = reinterpret_cast<f2 *>(a.decay + ((int64_t)b * a.nseg + s) * Mp + kModes * g);
 #pragma unroll
-      for (int p = 0; p < 4; ++p) dst[p] = prod[p];
+      for (int p = 0; p < 4; ++p) {
+        float lo, hi;
+        un2(prod[p], lo, hi);
+        dst[p] = mk2(fmaxf(lo, kLeastDecay), fmaxf(hi, kLeastDecay));
+      }
     }
   } else if (a.fin && s == a.nseg - 1) {
 #pragma unroll
@@ -533,7 +544,7 @@ few_carry_kernel(float *__restrict__ states, const float *__restrict__ decay, co
 #pragma unroll
     for (int i = 0; i < BATCH; ++i) {
       v = fmaf(d[i], v, x[i]);
-      p *= d[i];
+      p = decay_over(p, d[i]);
     }
   }
   // the warp's shares one after the other: (p, v) up to and with each, then without it
@@ -542,7 +553,7 @@ few_carry_kernel(float *__restrict__ states, const float *__restrict__ decay, co
     const float p0 = __shfl_up_sync(0xffffffffu, p, o * kElems), v0 = __shfl_up_sync(0xffffffffu, v, o * kElems);
     if (sub >= o) {
       v = fmaf(p, v0, v);
-      p *= p0;
+      p = decay_over(p, p0);
     }
   }
   if (sub == SUB - 1) {

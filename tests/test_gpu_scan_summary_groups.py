@@ -54,3 +54,25 @@ def test_an_infinity_stays_one_where_decays_underflow():
     h, _ = frac_scan(*(t.cuda() for t in (u, c, kappa, rho)), 32, init.cuda(), True)
     h_ref, _ = _exact(u, c, kappa, rho, init)
     assert torch.equal(torch.isinf(h.cpu()), torch.isinf(h_ref)) and not torch.isnan(h).any()
+
+
+# (64, 16), (128, 64) load in 16-byte pieces, (60, 16) and (64, 30) element by element, the last with padded modes
+@pytest.mark.parametrize("R,M", [(64, 16), (128, 64), (60, 16), (64, 30)])
+@pytest.mark.parametrize("L,where,floored,small", [
+    (64, 3, (8, 16), 1.0),         # the group behind the infinity's, within a segment
+    (64, 3, (16, 32), 1.0),        # the whole segment behind the infinity's: what the carry multiplies with
+    (64, 8, (9, 16), 1e-12),       # a weight whose product with seven decays underflows although neither is zero
+    (5000, 5, (6, 5000), 1.0)])    # every segment behind it, over the carry's shares
+def test_an_infinity_outlasts_decays_that_underflow(R, M, L, where, floored, small):
+    """In the recurrence each decay is 1e-6 or more, and an infinity times that stays one."""
+    from frac_ssm_b200.ops.b200 import frac_scan
+    u, c, kappa, rho, init = O.scan_inputs(1, L, R, M, dtype=torch.float32, gen="model_like", seed=L + R)
+    c, kappa = c.abs().add(0.01), kappa.abs().add(0.01) * small
+    u[0, where, 5] = float("inf")
+    rho = rho.clamp_min(0.5)
+    rho[:, floored[0]:floored[1]] = 1e-6
+    h, fin = frac_scan(*(t.cuda() for t in (u, c, kappa, rho)), 32, init.cuda(), True)
+    h_ref, f_ref = _exact(u, c, kappa, rho, init)
+    assert torch.isinf(h_ref[0, where:, 5]).all()
+    assert torch.equal(torch.isinf(h.cpu()), torch.isinf(h_ref)) and not torch.isnan(h).any()
+    assert torch.equal(torch.isinf(fin.cpu()), torch.isinf(f_ref)) and not torch.isnan(fin).any()
