@@ -47,14 +47,9 @@ constexpr int kMaxBlockCols = 128;
 constexpr int kTokPad = 4;     // floats between a token's values and the next token's in the summary
 // Least decay over several tokens, of a group, a segment or a share of the carry: a product of 7 decays of 1e-6 underflows, and
 // zero times an infinity (of u, or of the state) would be NaN where the recurrence, whose single decays are no less than 1e-6,
-// keeps the infinity.  What has decayed further stays at 1e-37 of its size, 1e-37 |kappa u| too much in a state.
-constexpr float kLeastDecay = 1e-37f;
-__device__ __forceinline__ float decay_over(float a, float b) { return fmaxf(a * b, kLeastDecay); }
-// kappa and the decay behind its token: for the same reason not zero unless kappa is (or below 2e-15)
-__device__ __forceinline__ float kappa_behind(float kappa, float behind) {
-  const float y = kappa * fmaxf(behind, kLeastDecay);
-  return y != 0.f ? y : kappa * 0x1p-100f;
-}
+// keeps the infinity.  What has decayed further stays at 1e-37 of its size.  Behind a token within its group the least is larger,
+// so that a kappa down to 2e-15 times it is not zero either: 1e-30 |kappa u| too much in a state.
+constexpr float kLeastDecay = 1e-37f, kLeastBehind = 1e-30f;
 
 struct Rows {                  // one input: base and strides in bytes
   const char *p;
@@ -215,7 +210,7 @@ few_scan_kernel(const FewArgs a) {
           if (rt + o < kGroup) v *= y;
         }
         const float behind = __shfl_down_sync(0xffffffffu, v, 1, kGroup);
-        if (rt + 1 < kGroup) k[x] = kappa_behind(k[x], behind);
+        k[x] *= rt + 1 < kGroup ? fmaxf(behind, kLeastBehind) : 1.f;
         r[x] = fmaxf(v, kLeastDecay);
       }
       if (owns) {
@@ -273,7 +268,7 @@ few_scan_kernel(const FewArgs a) {
       }
 #pragma unroll
       for (int t = 0; t + 1 < kGroup; ++t)
-        if (t < n) wide[t * tok_floats + kOffK + m] = kappa_behind(wide[t * tok_floats + kOffK + m], r[t + 1]);
+        if (t < n) wide[t * tok_floats + kOffK + m] *= fmaxf(r[t + 1], kLeastBehind);
       wide[m] = fmaxf(r[0], kLeastDecay);
     }
   };
@@ -544,16 +539,17 @@ few_carry_kernel(float *__restrict__ states, const float *__restrict__ decay, co
 #pragma unroll
     for (int i = 0; i < BATCH; ++i) {
       v = fmaf(d[i], v, x[i]);
-      p = decay_over(p, d[i]);
+      p *= d[i];
     }
   }
+  p = fmaxf(p, kLeastDecay);
   // the warp's shares one after the other: (p, v) up to and with each, then without it
 #pragma unroll
   for (int o = 1; o < SUB; o *= 2) {
     const float p0 = __shfl_up_sync(0xffffffffu, p, o * kElems), v0 = __shfl_up_sync(0xffffffffu, v, o * kElems);
     if (sub >= o) {
       v = fmaf(p, v0, v);
-      p = decay_over(p, p0);
+      p = fmaxf(p * p0, kLeastDecay);
     }
   }
   if (sub == SUB - 1) {
