@@ -40,6 +40,7 @@ struct DynArgs {
   int N, n16, cols;    // columns; rounded up to 16; of tensor memory (a power of two)
   int steps, split, stages;
   uint64_t wait_ns;
+  int withhold;        // self-test: the first block of a cluster leaves out its last tile of x
 };
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
@@ -98,7 +99,7 @@ prefill_dyn_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
       if (k >= a.stages && !umma::mbar_wait_parked(&done[s], phase ^ 1, a.wait_ns)) { late = true; break; }
       uint8_t *stage = ring + s * stage_bytes;
       umma::mbar_expect_tx(&full[s], stage_bytes);
-      umma::tma_load_3d(stage, &x_map, &full[s], (k0 + k) * kDynK, (int)row0, 0);
+      if (!(a.withhold && rank == 0 && k == n_steps - 1)) umma::tma_load_3d(stage, &x_map, &full[s], (k0 + k) * kDynK, (int)row0, 0);
       umma::tma_load_3d(stage + a_bytes, &w_map, &full[s], (k0 + k) * kDynK, 0, 0);
       if (++s == (uint32_t)a.stages) {
         s = 0;
@@ -201,7 +202,7 @@ prefill_dyn_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_const
 }  // namespace
 
 int prefill_dyn_launch(const void *x, int64_t x_sl, const void *w, void *out, int64_t rows, int64_t K, int64_t N,
-                       cudaStream_t st) {
+                       cudaStream_t st, uint64_t wait_ns, bool withhold) {
   if (!x || !w || !out) return fail(FRACSSM_ERR_ARG, "prefill_dyn: null pointer");
   if (rows <= 0 || K <= 0 || N <= 0 || x_sl < K) return fail(FRACSSM_ERR_ARG, "prefill_dyn: bad sizes");
   if (N > 192 || K % 8 != 0 || x_sl % 8 != 0 || rows > (1ll << 30) || K > (1ll << 30) ||
@@ -241,7 +242,8 @@ int prefill_dyn_launch(const void *x, int64_t x_sl, const void *w, void *out, in
   a.cols = 32;
   while (a.cols < a.n16) a.cols *= 2;
   a.steps = (int)ceil_div(K, kDynK);
-  a.wait_ns = tile_default_wait_ns();
+  a.wait_ns = wait_ns;
+  a.withhold = withhold;
   // K is cut as long as the grid has one block per SM and a block two steps.  The kernel alone, us, 72 columns:
   //   blocks a tile        1      2      4      8
   //     397 rows         10.4    8.1    7.0    6.5

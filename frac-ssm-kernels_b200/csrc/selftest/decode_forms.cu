@@ -1,7 +1,8 @@
 // Test-only entry points (built into libfracssm_selftest.so, not into the product library): a decode step in either of its
-// forms, the one-kernel form with any number of blocks or with a wait that runs out.
+// forms, the one-kernel form with any number of blocks or with a wait that runs out; the prefill's projection with one that does.
 #include "common.cuh"
 #include "fracssm_selftest_forms.h"
+#include "prefill_dyn.cuh"
 
 extern "C" int fracssm_selftest_decode_layers(const uint64_t *layer_ptrs, const float *layer_nums, int64_t layers,
                                               const void *hidden_in, void *hidden_out, void *workspace,
@@ -31,4 +32,11 @@ extern "C" int fracssm_selftest_decode_wait_limit(const uint64_t *layer_ptrs, co
   how.lost = barrier;
   return decode_layers_launch(layer_ptrs, layer_nums, layers, hidden_in, hidden_out, workspace, workspace_bytes, B, hidden, H,
                               R, M, K, stream, how);
+}
+
+extern "C" int fracssm_selftest_prefill_dyn_wait_limit(const void *x, int64_t x_sl, const void *w, void *dyn, int64_t rows,
+                                                       int64_t K, int64_t cols, unsigned long long wait_ns, void *stream) {
+  using namespace fracssm;
+  if (wait_ns > tile_default_wait_ns()) return fail(FRACSSM_ERR_ARG, "selftest_prefill_dyn_wait_limit: the limit");
+  return prefill_dyn_launch(x, x_sl, w, dyn, rows, K, cols, (cudaStream_t)stream, wait_ns, true);
 }

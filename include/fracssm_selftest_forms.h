@@ -27,6 +27,12 @@ int fracssm_selftest_decode_wait_limit(const uint64_t *layer_ptrs, const float *
                                        const void *hidden_in, void *hidden_out, void *workspace, size_t workspace_bytes,
                                        int64_t B, int64_t hidden, int64_t H, int64_t R, int64_t M, int64_t K, void *stream,
                                        int barrier, unsigned long long wait_ns);
+/*
+ * The projection of fracssm_prefill_conv_dyn alone, dyn [rows, cols] = x [rows, K] w [cols, K]^T, where one load of every 128
+ * rows is left out (not the wait for it).  After wait_ns nanoseconds the kernel carries on and returns, and dyn is NaN.
+ */
+int fracssm_selftest_prefill_dyn_wait_limit(const void *x, int64_t x_sl, const void *w, void *dyn, int64_t rows, int64_t K,
+                                            int64_t cols, unsigned long long wait_ns, void *stream);
 
 #ifdef __cplusplus
 }

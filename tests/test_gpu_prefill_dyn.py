@@ -1,7 +1,11 @@
 """The dynamic projection that prefill runs beside its convolution, against float64."""
 
+import ctypes
+
 import pytest
 import torch
+
+from tests.helpers import selftest_lib
 
 pytestmark = pytest.mark.gpu
 
@@ -50,3 +54,19 @@ def test_prefill_conv_dyn_refuses_what_it_does_not_cover():
     for cols, K, w in ((193, 64, p(x)), (3, 60, p(x)), (3, 64, x.data_ptr() + 2), (0, 64, p(x))):
         assert lib.fracssm_prefill_conv_dyn(p(x), 64, None, p(x), None, p(x), None, None, w, p(x), cols, 4, 1, 1, K, 4,
                                             C.stream_of(x)) != 0
+
+
+# a block alone and clusters of 2, 4 and 8, one row and tiles with rows beyond the last
+@pytest.mark.parametrize("rows,K,N", [(1, 40, 3), (9000, 1536, 72), (4000, 1536, 36), (397, 1536, 72), (19000, 200, 192)])
+def test_a_wait_that_runs_out_marks_every_row(rows, K, N):
+    """One load of every 128 rows is left out: its wait gives up after two milliseconds, for all blocks of the cluster."""
+    from frac_ssm_b200 import _cabi as C
+    fn = selftest_lib().fracssm_selftest_prefill_dyn_wait_limit
+    vp, i64 = ctypes.c_void_p, ctypes.c_int64
+    fn.argtypes, fn.restype = [vp, i64, vp, vp, i64, i64, i64, ctypes.c_uint64, vp], ctypes.c_int
+    x = torch.ones(rows, K, device="cuda", dtype=torch.bfloat16)
+    w = torch.ones(N, K, device="cuda", dtype=torch.bfloat16)
+    dyn = torch.zeros(rows * N + 8, device="cuda", dtype=torch.bfloat16)
+    assert fn(C.ptr(x), K, C.ptr(w), C.ptr(dyn), rows, K, N, 2_000_000, C.stream_of(x)) == 0
+    torch.cuda.synchronize()
+    assert torch.isnan(dyn[:rows * N]).all() and (dyn[rows * N:] == 0).all()
