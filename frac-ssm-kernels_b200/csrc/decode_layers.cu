@@ -186,6 +186,7 @@ struct StepArgs {
   __nv_bfloat16 *x, *x_conv, *vals, *hid_w, *out;
   float *gate, *rw, *dyn, *ss, *hid[2], *hid_ss;
   Meeting *meeting;
+  unsigned long long work_ns;        // what the launch takes one block per SM, about
   unsigned long long wait_ns;        // limit of a wait for the other blocks
   int lost;                          // self-test: at this barrier, counted from 1, block 0 waits for the next one's arrivals too
   uint32_t act_bytes, red_bytes, mix_bytes;
@@ -726,24 +727,19 @@ struct Step {
   }
 };
 
-// How long the first block keeps the list open while n of `blocks` have started: until the wait has cost as much as going without
-// the others will (a layer takes some 20 us with all of them), and 10 us at least, which their start takes.
-__device__ __forceinline__ uint64_t patience_ns(int n, int blocks, int layers) {
-  return 10000 + (uint64_t)20000 * layers * (blocks - n) / n;
-}
 // Puts this block on the list of those that share the work, by one thread.  Nothing is set where the list was closed before; for
 // want of an answer within the limit *gave_up is.
-__device__ void join(Meeting *m, int layers, uint64_t wait_ns, Place *at, int *gave_up) {
+__device__ void join(Meeting *m, uint64_t work_ns, uint64_t wait_ns, Place *at, int *gave_up) {
   const unsigned mine = atomicAdd(&m->started, 1u);
   if (mine & kClosed) return;
-  const int grid = (int)gridDim.x;
+  const unsigned grid = gridDim.x;
   unsigned n = 0;
   const uint64_t t0 = umma::global_ns();
   if (mine == 0) {
 #pragma unroll 1
     do {
       asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(&m->started) : "memory");
-    } while ((int)n < grid && !umma::past_limit(t0, umma::global_ns(), patience_ns((int)n, grid, layers)));
+    } while (n < grid && !umma::past_limit(t0, umma::global_ns(), list_patience_ns(n, grid, work_ns)));
     n = atomicOr(&m->started, kClosed);
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&m->members), "r"(n) : "memory");
   } else {
@@ -751,7 +747,7 @@ __device__ void join(Meeting *m, int layers, uint64_t wait_ns, Place *at, int *g
     for (;;) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(&m->members) : "memory");
       if (n) break;
-      if (umma::past_limit(t0, umma::global_ns(), wait_ns)) {
+      if (umma::past_limit(t0, umma::global_ns(), wait_ns + list_patience_ns(1, grid, work_ns))) {
         *gave_up = 1;
         return;
       }
@@ -771,7 +767,7 @@ __device__ __forceinline__ void arrive(unsigned *counter) {
   }
 }
 // False when the limit ran out, for every thread of the block.
-__device__ __forceinline__ bool wait_for_all(const unsigned *counter, unsigned target, uint64_t wait_ns) {
+__device__ __forceinline__ bool wait_for_all(const unsigned *counter, unsigned target, int blocks, uint64_t wait_ns) {
   int gave_up = 0;
   if (threadIdx.x == 0) {
     uint64_t t0 = 0;
@@ -781,7 +777,7 @@ __device__ __forceinline__ bool wait_for_all(const unsigned *counter, unsigned t
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
       if (static_cast<int>(seen - target) >= 0) break;
       if (spins == 64) t0 = umma::global_ns();
-      if (spins > 64 && umma::past_limit(t0, umma::global_ns(), wait_ns)) {
+      if (spins > 64 && umma::past_limit(t0, umma::global_ns(), barrier_limit_ns(blocks, gridDim.x, wait_ns))) {
         gave_up = 1;
         break;
       }
@@ -816,7 +812,7 @@ __global__ void __launch_bounds__(kTeam * max_teams<NT>(), 1) decode_step_kernel
   if (threadIdx.x == 0) {
     int gave_up = 0;
     Place mine{};
-    join(a.meeting, a.layers, a.wait_ns, &mine, &gave_up);
+    join(a.meeting, a.work_ns, a.wait_ns, &mine, &gave_up);
     listed[0] = mine.block;
     listed[1] = gave_up ? -1 : mine.blocks;
   }
@@ -874,7 +870,7 @@ __global__ void __launch_bounds__(kTeam * max_teams<NT>(), 1) decode_step_kernel
     }
     if (stage >= 0) {
       target += (unsigned)at.blocks;
-      if (!(ok = wait_for_all(&a.meeting->arrived, target + (at.block == 0 && next == a.lost ? at.blocks : 0), a.wait_ns))) break;
+      if (!(ok = wait_for_all(&a.meeting->arrived, target + (at.block == 0 && next == a.lost ? at.blocks : 0), at.blocks, a.wait_ns))) break;
     }
   }
   // A block that gave up says so, and whoever leaves last, when nobody writes any more, sees it.
@@ -971,6 +967,7 @@ void fill_table(StepArgs<LAYERS> &a, const uint64_t *ptrs, const float *nums, in
 struct Shape {
   int64_t B, d, H, R, M;
 };
+int64_t layer_weights(const Shape &p) { return 2 * p.H * p.R * (3 * p.d + 2 * p.H * p.M + 3 * p.H); }   // bytes
 template <int LAYERS>
 void fill_shape(StepArgs<LAYERS> &a, int nt, const Shape &p, char *ws, void *hidden_out) {
   const int64_t di = p.H * p.R;
@@ -1059,8 +1056,7 @@ int launched(cudaError_t e) {
 constexpr int64_t kCapturedWeights = 12000000;      // bytes
 bool one_kernel_pays(const Shape &p, cudaStream_t st) {
   if (p.B > 32) return false;
-  const int64_t di = p.H * p.R;
-  if (p.B > 16 && 2 * di * (3 * p.d + 2 * p.H * p.M + 3 * p.H) > kCapturedWeights) return true;
+  if (p.B > 16 && layer_weights(p) > kCapturedWeights) return true;
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
     cudaGetLastError();   // (the legacy stream while another is captured: the launches themselves say so)
@@ -1092,6 +1088,7 @@ int run_one_kernel(const uint64_t *ptrs, const float *nums, int64_t layers, void
     // (the first kernel clears it for the first launch)
     if (l0) e = cudaMemsetAsync(a.meeting, 0, kPerLaunch, st);
     a.lost = l0 ? 0 : how.lost;
+    a.work_ns = a.layers * (20000ull + (unsigned long long)layer_weights(p) / 4);   // (latency; 4 TB/s)
     if (e == cudaSuccess) e = launch(decode_step_kernel<NT>, (unsigned)grid, kTeam * teams, smem_of(teams), st, false, a);
   }
   return launched(e);

@@ -20,5 +20,17 @@ FRACSSM_HD bool past_limit(uint64_t start, uint64_t now, uint64_t limit_ns) {
 }
 
 }  // namespace umma
+
+// Blocks that share work with those that have started (csrc/decode_layers.cu).
+
+// How long the first block keeps the list open while n of `blocks` have started: until the wait has cost as much as going without
+// the others will, for work that takes all of them work_ns, and 10 us at least, which their start takes.
+FRACSSM_HD uint64_t list_patience_ns(uint32_t n, uint32_t blocks, uint64_t work_ns) {
+  return 10000 + work_ns * (blocks - n) / n;
+}
+// Limit of a wait at a barrier of n blocks: what takes `blocks` of them milliseconds takes a few of them longer, and the longest
+// share may be all of it.
+FRACSSM_HD uint64_t barrier_limit_ns(uint32_t n, uint32_t blocks, uint64_t limit_ns) { return limit_ns * (blocks - n + 1); }
+
 }  // namespace fracssm
 #undef FRACSSM_HD
