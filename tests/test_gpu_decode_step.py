@@ -36,7 +36,7 @@ def test_both_forms_give_the_same_bits(hidden, H, M, B, layers):
 
 
 def test_two_streams_at_a_time():
-    """Two threads of kernels whose blocks all have to run at the same time: neither waits for the other's."""
+    """Two streams of kernels whose blocks share their work: neither waits for the other's."""
     models = [_model(256, 4, 128, 4).to(torch.bfloat16), _model(768, 12, 8, 3).to(torch.bfloat16)]
     ids = [torch.randint(1, 50, (b, 1)).cuda() for b in (1, 20)]
     pasts = [_past(m, i.shape[0], torch.bfloat16) for m, i in zip(models, ids)]

@@ -20,8 +20,6 @@ def test_groups_match_recurrence(B, L, R, M, dtype, coeff):
     u, c, kappa = u.to(dtype), c.to(coeff), kappa.to(coeff)
     rho[:, L // 3:2 * L // 3, ::2] = 1e-7        # whole groups at the floor of 1e-6: seven such decays are 1e-42
     h, fin = frac_scan(*(t.cuda() for t in (u, c, kappa, rho)), 32, init.cuda(), True, final_state_dtype=torch.float32)
-    if (R, M, dtype) == (64, 128, torch.bfloat16):
-        pytest.skip("the single-pass kernel's shape")
     h_ref, f_ref = _exact(u, c, kappa, rho, init)
     # outputs are rounded once; float32 sums of at most L * M terms whose roundings are of either sign
     assert _rel(h, h_ref) <= {torch.bfloat16: 2 ** -8, torch.float32: 2e-6}[dtype]
