@@ -747,7 +747,7 @@ __device__ void join(Meeting *m, uint64_t work_ns, uint64_t wait_ns, Place *at, 
     for (;;) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(&m->members) : "memory");
       if (n) break;
-      if (umma::past_limit(t0, umma::global_ns(), wait_ns + list_patience_ns(1, grid, work_ns))) {
+      if (umma::past_limit(t0, umma::global_ns(), wait_ns)) {
         *gave_up = 1;
         return;
       }
@@ -767,7 +767,7 @@ __device__ __forceinline__ void arrive(unsigned *counter) {
   }
 }
 // False when the limit ran out, for every thread of the block.
-__device__ __forceinline__ bool wait_for_all(const unsigned *counter, unsigned target, int blocks, uint64_t wait_ns) {
+__device__ __forceinline__ bool wait_for_all(const unsigned *counter, unsigned target, uint64_t wait_ns) {
   int gave_up = 0;
   if (threadIdx.x == 0) {
     uint64_t t0 = 0;
@@ -777,7 +777,7 @@ __device__ __forceinline__ bool wait_for_all(const unsigned *counter, unsigned t
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
       if (static_cast<int>(seen - target) >= 0) break;
       if (spins == 64) t0 = umma::global_ns();
-      if (spins > 64 && umma::past_limit(t0, umma::global_ns(), barrier_limit_ns(blocks, gridDim.x, wait_ns))) {
+      if (spins > 64 && umma::past_limit(t0, umma::global_ns(), wait_ns)) {
         gave_up = 1;
         break;
       }
@@ -870,7 +870,7 @@ __global__ void __launch_bounds__(kTeam * max_teams<NT>(), 1) decode_step_kernel
     }
     if (stage >= 0) {
       target += (unsigned)at.blocks;
-      if (!(ok = wait_for_all(&a.meeting->arrived, target + (at.block == 0 && next == a.lost ? at.blocks : 0), at.blocks, a.wait_ns))) break;
+      if (!(ok = wait_for_all(&a.meeting->arrived, target + (at.block == 0 && next == a.lost ? at.blocks : 0), a.wait_ns))) break;
     }
   }
   // A block that gave up says so, and whoever leaves last, when nobody writes any more, sees it.
@@ -1081,7 +1081,6 @@ int run_one_kernel(const uint64_t *ptrs, const float *nums, int64_t layers, void
   };
   while (teams > 1 && smem_of(teams) > kMostSmem) --teams;
   const int grid = how.blocks > 0 ? how.blocks : sms;
-  a.wait_ns = how.wait_ns;
   cudaError_t e = cudaSuccess;
   for (int64_t l0 = 0; l0 < layers && e == cudaSuccess; l0 += kTabLayers) {
     fill_table(a, ptrs, nums, layers, l0);
@@ -1089,6 +1088,7 @@ int run_one_kernel(const uint64_t *ptrs, const float *nums, int64_t layers, void
     if (l0) e = cudaMemsetAsync(a.meeting, 0, kPerLaunch, st);
     a.lost = l0 ? 0 : how.lost;
     a.work_ns = a.layers * (20000ull + (unsigned long long)layer_weights(p) / 4);   // (latency; 4 TB/s)
+    a.wait_ns = list_limit_ns(grid, a.work_ns, how.wait_ns);
     if (e == cudaSuccess) e = launch(decode_step_kernel<NT>, (unsigned)grid, kTeam * teams, smem_of(teams), st, false, a);
   }
   return launched(e);

@@ -28,9 +28,9 @@ FRACSSM_HD bool past_limit(uint64_t start, uint64_t now, uint64_t limit_ns) {
 FRACSSM_HD uint64_t list_patience_ns(uint32_t n, uint32_t blocks, uint64_t work_ns) {
   return 10000 + work_ns * (blocks - n) / n;
 }
-// Limit of a wait at a barrier of n blocks: what takes `blocks` of them milliseconds takes a few of them longer, and the longest
-// share may be all of it.
-FRACSSM_HD uint64_t barrier_limit_ns(uint32_t n, uint32_t blocks, uint64_t limit_ns) { return limit_ns * (blocks - n + 1); }
+// Limit of the waits among them: on top of `limit_ns` what one of them alone would take for the whole of it, since few may have
+// started and the shares of two may be all and nothing.
+FRACSSM_HD uint64_t list_limit_ns(uint32_t blocks, uint64_t work_ns, uint64_t limit_ns) { return limit_ns + work_ns * blocks; }
 
 }  // namespace fracssm
 #undef FRACSSM_HD

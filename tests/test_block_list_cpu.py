@@ -25,7 +25,9 @@ def test_the_list_stays_open_no_longer_than_the_missing_blocks_are_worth(tmp_pat
     assert 0 < _values(tmp_path, [f"list_patience_ns(1u, 148u, {50_000_000_000}ull)"])[0] < 2 ** 63
 
 
-def test_the_fewer_blocks_the_longer_a_barrier_waits(tmp_path):
-    counts = [148, 147, 74, 2, 1]
-    got = _values(tmp_path, [f"barrier_limit_ns({n}u, 148u, 2000000000ull)" for n in counts])
-    assert got == [2_000_000_000 * (149 - n) for n in counts] and got[-1] < 2 ** 63
+def test_the_limit_covers_the_work_of_all_by_one(tmp_path):
+    work = [640_000, 50_000_000_000]      # 24 layers of hidden 768; layers whose weights fill the device's memory
+    got = _values(tmp_path, [f"list_limit_ns(148u, {w}ull, 2000000000ull)" for w in work])
+    assert got == [2_000_000_000 + 148 * w for w in work] and got[-1] < 2 ** 63
+    # and with it the time that the list may stay open
+    assert all(g > p for g, p in zip(got, _values(tmp_path, [f"list_patience_ns(1u, 148u, {w}ull)" for w in work])))
