@@ -27,7 +27,7 @@
 //     the barrier is 1.3; what bounds it is the number of instructions a warp gets through with cold instruction
 //     caches, since every stage passes through its code once per layer.  So it is ONE loop over the stages with one copy of each
 //     piece of code, little of it unrolled (with the products and their requests inlined for each stage 117 KB of code and
-//     0.86 ms at one sequence; 68 KB and 0.51 ms as here).
+//     0.86 ms at one sequence; 68 KB and 0.50 ms as here).
 //     Nothing makes all blocks run at the same time: kernels of other streams may hold SMs, for long, and may wait for this very
 //     step.  So the blocks that have started make up a list and share the work among themselves (see join); a block that comes
 //     later finds the list closed and leaves.  Nobody waits for a block that has not started.

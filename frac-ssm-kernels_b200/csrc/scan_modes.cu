@@ -20,7 +20,7 @@
 // thread a token took 188 instructions a warp.  (Calls whose rows do not load in 16-byte pieces request a group when it
 // is due; large ones among them are left to the chunked stages, see few_narrow_limit.)
 // Whole call, 2 rows x 32768 tokens, 128 columns, 16 modes, bfloat16: 328 us with the chunked stages, 80 us
-// with the first form of these kernels, 62 us with a recurrence in step 1 too, 54 us here.
+// with the first form of these kernels, 62 us with a recurrence in step 1 too, 52 us here.
 #include <type_traits>
 
 #include "common.cuh"
